@@ -374,15 +374,15 @@ uint32_t emit_wide4(const Tree& t, uint32_t bi, const std::vector<uint32_t>& cod
   Wide4Node& w = hb.wide4_nodes[me];
   for (int k = 0; k < 4; k++) {
     const bool used = k < n;
-    const Box b = used ? t.nodes[slot[k]].box : Box{{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
-    w.lo_x[k] = b.lo.x;
-    w.lo_y[k] = b.lo.y;
-    w.lo_z[k] = b.lo.z;
-    w.hi_x[k] = b.hi.x;
-    w.hi_y[k] = b.hi.y;
-    w.hi_z[k] = b.hi.z;
-    w.code[k] = codes[k];
-    w.pad[k] = 0;
+    const Box b = used ? t.nodes[slot[k]].box : Box{{NAN, NAN, NAN}, {NAN, NAN, NAN}};
+    w.child[k].lo_x = b.lo.x;
+    w.child[k].lo_y = b.lo.y;
+    w.child[k].lo_z = b.lo.z;
+    w.child[k].hi_x = b.hi.x;
+    w.child[k].hi_y = b.hi.y;
+    w.child[k].hi_z = b.hi.z;
+    w.child[k].code = codes[k];
+    w.child[k].pad = 0;
   }
   return me;
 }

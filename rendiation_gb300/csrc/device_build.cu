@@ -878,21 +878,21 @@ __global__ void wide4_emit_kernel(uint32_t T, const BNode* __restrict__ pool, co
   Wide4Node w;
   for (int k = 0; k < 4; k++) {
     const bool used = k < n;
-    const NodeBox b = used ? box_of(pool[slot[k]]) : NodeBox{{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
-    w.lo_x[k] = b.lo.x;
-    w.lo_y[k] = b.lo.y;
-    w.lo_z[k] = b.lo.z;
-    w.hi_x[k] = b.hi.x;
-    w.hi_y[k] = b.hi.y;
-    w.hi_z[k] = b.hi.z;
-    w.pad[k] = 0;
+    const NodeBox b = used ? box_of(pool[slot[k]]) : NodeBox{{NAN, NAN, NAN}, {NAN, NAN, NAN}};
+    w.child[k].lo_x = b.lo.x;
+    w.child[k].lo_y = b.lo.y;
+    w.child[k].lo_z = b.lo.z;
+    w.child[k].hi_x = b.hi.x;
+    w.child[k].hi_y = b.hi.y;
+    w.child[k].hi_z = b.hi.z;
+    w.child[k].pad = 0;
     if (!used) {
-      w.code[k] = EMPTY_SLOT;
+      w.child[k].code = EMPTY_SLOT;
     } else if (pool[slot[k]].left != NONE) {
-      w.code[k] = index4[slot[k]];
+      w.child[k].code = index4[slot[k]];
     } else {
       const uint32_t g = pre[slot[k]];
-      w.code[k] = LEAF_BIT | (g - rank[g]);
+      w.child[k].code = LEAF_BIT | (g - rank[g]);
     }
   }
   out[index4[i]] = w;

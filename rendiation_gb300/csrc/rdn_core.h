@@ -104,16 +104,18 @@ struct WideNode {
 };
 static_assert(sizeof(WideNode) == 64, "64 B node");
 static const uint32_t LEAF_BIT = 0x80000000u;
-// Four-child node, 128 B, children's boxes as SoA rows:
-//   lo_x[4] lo_y[4] lo_z[4] hi_x[4] hi_y[4] hi_z[4] code[4] pad[4]
+// Four-child node, 128 B, one 32 B child after the other: a child is one 32 B
+// load, its planes in the pairs that the packed box test takes.
 // code: bit 31 clear = index of a child Wide4Node, set = index of a leaf range,
-// EMPTY_SLOT = unused slot. Children are binary-tree nodes collapsed from the
+// EMPTY_SLOT = unused slot (its box is NaN, which no slab test passes). Children are binary-tree nodes collapsed from the
 // reference's SAH tree (the inner child with the largest surface area is opened
 // until four slots are used); every child box is an exact reference node box.
+struct Wide4Child {
+  float lo_x, lo_y, hi_x, hi_y, lo_z, hi_z;
+  uint32_t code, pad;
+};
 struct Wide4Node {
-  float lo_x[4], lo_y[4], lo_z[4], hi_x[4], hi_y[4], hi_z[4];
-  uint32_t code[4];
-  uint32_t pad[4];
+  Wide4Child child[4];
 };
 static_assert(sizeof(Wide4Node) == 128, "128 B node");
 static const uint32_t EMPTY_SLOT = 0xFFFFFFFFu;
