@@ -382,7 +382,11 @@ uint32_t emit_wide4(const Tree& t, uint32_t bi, const std::vector<uint32_t>& cod
     w.child[k].hi_y = b.hi.y;
     w.child[k].hi_z = b.hi.z;
     w.child[k].code = codes[k];
-    w.child[k].pad = 0;
+    w.child[k].quad = codes[k];
+    if (used && (codes[k] & LEAF_BIT)) {
+      const uint32_t l = codes[k] & ~LEAF_BIT;
+      w.child[k].quad = quad_leaf_code(l, hb.leaf_ranges[2 * (size_t)l], hb.leaf_ranges[2 * (size_t)l + 1]);
+    }
   }
   return me;
 }

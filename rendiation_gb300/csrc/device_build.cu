@@ -885,14 +885,14 @@ __global__ void wide4_emit_kernel(uint32_t T, const BNode* __restrict__ pool, co
     w.child[k].hi_x = b.hi.x;
     w.child[k].hi_y = b.hi.y;
     w.child[k].hi_z = b.hi.z;
-    w.child[k].pad = 0;
     if (!used) {
-      w.child[k].code = EMPTY_SLOT;
+      w.child[k].code = w.child[k].quad = EMPTY_SLOT;
     } else if (pool[slot[k]].left != NONE) {
-      w.child[k].code = index4[slot[k]];
+      w.child[k].code = w.child[k].quad = index4[slot[k]];
     } else {
       const uint32_t g = pre[slot[k]];
       w.child[k].code = LEAF_BIT | (g - rank[g]);
+      w.child[k].quad = quad_leaf_code(g - rank[g], pool[slot[k]].start, pool[slot[k]].end);
     }
   }
   out[index4[i]] = w;

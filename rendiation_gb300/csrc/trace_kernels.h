@@ -14,6 +14,7 @@ struct TraceParams {
   rdn_hit_ext* hits_ext;
   const uint32_t* tlas_idx;
   uint32_t count, tlas_uniform, ray_flags, cull_mask, anyhit_mode, stack_depth;
+  uint32_t stack_depth4;  // entries of a four-child walk's stack, whatever the traversal asked for
   uint32_t n_binding, n_tlas_root;
   const uint32_t* tlas_binding;
   const uint32_t* tlas_bvh_root;
@@ -49,6 +50,7 @@ struct TraceParams {
   // template argument, so the reference-formula kernels carry no cost for it
   uint32_t watertight;
   const float4* verts;  // 3 per triangle (VertexRecord), sorted order
+  uint32_t quads;       // 1: the triangles are few enough for quad_leaf_code
 };
 
 // 1 + 2 gamma_3 (gamma_n = n u / (1 - n u), u = 2^-24) rounded up to f32:

@@ -396,7 +396,7 @@ __device__ __forceinline__ void push_entry(const TraceParams& p, uint2* stack, u
 // A child of a four-child node (Wide4Child): one 32 B load.
 struct Wide4Load {
   float2 lo_xy, hi_xy, z;  // z = (lo, hi)
-  uint32_t code;
+  uint32_t code, quad;
 };
 __device__ __forceinline__ Wide4Load load_wide4(const float4* w) {
   float a, b, c, d, e, f;
@@ -404,8 +404,19 @@ __device__ __forceinline__ Wide4Load load_wide4(const float4* w) {
   asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
       : "=f"(a), "=f"(b), "=f"(c), "=f"(d), "=f"(e), "=f"(f), "=r"(g), "=r"(h)
       : "l"(w));
-  return Wide4Load{make_float2(a, b), make_float2(c, d), make_float2(e, f), g};
+  return Wide4Load{make_float2(a, b), make_float2(c, d), make_float2(e, f), g, h};
 }
+// The same where `want`; zeros otherwise (no branch around the load).
+__device__ __forceinline__ Wide4Load load_wide4_if(const float4* w, bool want) {
+  float a = 0.f, b = 0.f, c = 0.f, d = 0.f, e = 0.f, f = 0.f;
+  uint32_t g = 0, h = 0;
+  asm("{\n .reg .pred p;\n setp.ne.u32 p, %9, 0;\n"
+      " @p ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n}"
+      : "+f"(a), "+f"(b), "+f"(c), "+f"(d), "+f"(e), "+f"(f), "+r"(g), "+r"(h)
+      : "l"(w), "r"((uint32_t)want));
+  return Wide4Load{make_float2(a, b), make_float2(c, d), make_float2(e, f), g, h};
+}
+
 // slab() on packed pairs of planes: the same subtractions and products (a - b
 // as a + (-b)), two to an instruction. The per-lane four-child walk is bound by
 // instruction issue (55-66 % of the slots, 6 to 17 of 32 lanes active), and a
