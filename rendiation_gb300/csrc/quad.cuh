@@ -15,12 +15,13 @@
 // one, reads its node as one 128 B line, and a warp's longest ray no longer
 // holds 31 others: 24 of 32 lanes active, 0.70 of the issue slots.
 // Measured (rdn_trace, us, one ray per lane -> quads): 777,777 random rays
-// through a 150k soup 1140 -> 898 (watertight 1387 -> 1026), 1,000,000 through
-// the 1024^2 field 455 -> 380, 1,000 through a 10k soup 130 -> 52, 65,536
-// camera rays onto it 121 -> 53. Only large batches of rays that are alike
-// walk faster one per lane, where a warp's lanes share the nodes they read
-// (2.07 M camera rays: 727 against 1082). 64 registers; with 72 the random
-// rays took 910 us, with 56 938 us.
+// through a 150k soup 1140 -> 822 (watertight 1387 -> 935), 1,000,000 through
+// the 1024^2 field 455 -> 344, the 1080p frame's 2.05 M bounce rays 1315 ->
+// 1174, 1,000 rays through a 10k soup 130 -> 45, 65,536 camera rays onto it
+// 121 -> 48. Only large batches of rays that are alike walk faster one per
+// lane, where a warp's lanes share the nodes they read (2.07 M camera rays:
+// 727 against 985). 64 registers a thread; before the steps were unrolled the
+// random rays took 885 us with 64, 910 with 72 and 938 with 56.
 //
 // Results: every child box and every triangle is tested with the operations of
 // the per-lane walk, and a leaf's candidates are committed in the leaf's order
@@ -37,9 +38,19 @@ namespace dev {
 constexpr uint32_t kFullWarp = 0xffffffffu;
 constexpr uint32_t kQuads = 8;  // per warp
 // Quads (in lanes) that may still look for a leaf when the others' leaves are
-// tested: 777,777 rays through a 150k soup took 1326 us with 0, 986 with 8,
-// 949 with 16 and 957 with 20.
-constexpr uint32_t kQuadWait = 16;
+// tested: 64 soups' paths took 5667 us with 12, 5528 with 16, 5460 with 20,
+// 5488 with 24 and 5635 with 28 (0 cost 777,777 rays a third more than 16).
+constexpr uint32_t kQuadWait = 20;
+
+// Rays a warp claims of a queue of n: as many as leave no resident warp
+// without work (the sizes are rdn_trace's, trace.cu).
+__host__ __device__ constexpr uint32_t quad_batch(uint32_t n) { return n < 40000u ? 8u : (n < 100000u ? 16u : 32u); }
+
+// Rows a quad's stack needs: a step pops one entry and pushes at most the four
+// children of its node, so every level of the four-child tree below the top
+// one holds at most three entries and the top one four: 3 D + 1 for D levels
+// (stack_entries(MODE_WIDE4), from the built depth). The steps therefore carry
+// no bounds check (with one, 777,777 rays took 898 us instead of 831).
 
 // One BLAS entry of a lane's ray, read by the quad that walks it; the quad
 // writes the committed hit over it.
@@ -74,9 +85,10 @@ __device__ __forceinline__ QuadWarp quad_warp(unsigned char* smem, uint32_t stac
   return w;
 }
 
-// True when the warp's rays point the same way (within about 11 degrees of the
-// first one's direction) in the same TLAS. Which walk a ray takes does not
+// True when the warp's rays point the same way (within 30 degrees of the first
+// one's direction) in the same TLAS. Which walk a ray takes does not
 // change its result; both kernels of a split query form the same vote.
+constexpr float kAlikeCos2 = 0.75f;
 __device__ __forceinline__ bool coherent_warp(const RayCtx& R, uint32_t tidx, bool valid) {
   const uint32_t m = __ballot_sync(kFullWarp, valid);
   const uint32_t src = m ? (uint32_t)__ffs(m) - 1u : 0u;
@@ -85,7 +97,7 @@ __device__ __forceinline__ bool coherent_warp(const RayCtx& R, uint32_t tidx, bo
   const uint32_t t0 = __shfl_sync(kFullWarp, tidx, src);
   const float dot = R.d.x * dx + R.d.y * dy + R.d.z * dz;
   const float len2 = (R.d.x * R.d.x + R.d.y * R.d.y + R.d.z * R.d.z) * (dx * dx + dy * dy + dz * dz);
-  return __all_sync(kFullWarp, !valid || (tidx == t0 && dot > 0.0f && dot * dot > 0.96f * len2));
+  return __all_sync(kFullWarp, !valid || (tidx == t0 && dot > 0.0f && dot * dot > kAlikeCos2 * len2));
 }
 
 // Walks the n entered rays order[0..n) of the warp. Every lane calls it; all
@@ -103,7 +115,6 @@ __device__ __forceinline__ void quad_walk(const TraceParams& p, const QuadWarp& 
   float3 d = make_float3(0.f, 0.f, 0.f);
   float near_ = 0.f, far_ = 0.f, scaling = 1.f;
   uint32_t bits = 0, slot = 0;
-  bool over = false;
   uint32_t leaf = EMPTY_SLOT, sp = 0;  // the ray is done when both are empty
 
   for (;;) {
@@ -139,36 +150,36 @@ __device__ __forceinline__ void quad_walk(const TraceParams& p, const QuadWarp& 
       }
       __syncwarp();
     } else if (idle_lanes == kFullWarp) {
-      if (over) atomicOr(p.error_word, 1u);
       break;
     }
 
     // inner nodes, until no more than kQuadWait lanes' quads still look for a leaf
     bool stuck;  // holds a leaf and the next entry is one too
     do {
-      // the topmost entry, dropped when its box no longer lies before the far; a leaf goes to a quad that holds none
-      const uint2 e = stack[sp * kQuads];
-      const bool live = __uint_as_float(e.y) < far_;
-      const bool is_leaf = live && (int)e.x < 0;
-      stuck = is_leaf && leaf != EMPTY_SLOT;
-      if (sp != 0u && !stuck) sp--;
-      if (is_leaf && !stuck) leaf = e.x;
-      const bool act = live && !is_leaf;
-      const Wide4Load c = load_wide4_if(p.wide4 + 8 * (size_t)e.x + 2 * l, act);
-      float tn;
-      const bool hit = slab2<WT>(no_xy, no_z, inv_xy, inv_z, near_, far_, c, tn) && act;
-      // near-first: the distance (negative ones equal), the lane in its lowest bits; -1 no hit
-      const int key = hit ? ((__float_as_int(fmaxf(tn, 0.0f)) & ~3) | (int)l) : -1;
-      const int k1 = __shfl_xor_sync(kFullWarp, key, 1), k2 = __shfl_xor_sync(kFullWarp, key, 2),
-                k3 = __shfl_xor_sync(kFullWarp, key, 3);
-      const uint32_t hits = (__ballot_sync(kFullWarp, hit) >> qb) & 15u;
-      // the farthest lowest; the stack is sized from the tree depth, so no row is past it
-      const uint32_t row = sp + 1u + (uint32_t)(k1 > key) + (uint32_t)(k2 > key) + (uint32_t)(k3 > key);
-      if (hit && row <= depth) stack[row * kQuads] = make_uint2(c.quad, __float_as_uint(tn));
-      sp += __popc(hits);
-      over |= sp > depth;
-      sp = min(sp, depth);
-      __syncwarp();
+#pragma unroll
+      for (int rep = 0; rep < 2; rep++) {  // two steps between the votes: 835 us instead of 898 for 777,777 rays
+        // the topmost entry, dropped when its box no longer lies before the far; a leaf goes to a quad that holds none
+        const uint2 e = stack[sp * kQuads];
+        const bool live = __uint_as_float(e.y) < far_;
+        const bool is_leaf = live && (int)e.x < 0;
+        stuck = is_leaf && leaf != EMPTY_SLOT;
+        if (sp != 0u && !stuck) sp--;
+        if (is_leaf && !stuck) leaf = e.x;
+        const bool act = live && !is_leaf;
+        const Wide4Load c = load_wide4_if(p.wide4 + 8 * (size_t)e.x + 2 * l, act);
+        float tn;
+        const bool hit = slab2<WT>(no_xy, no_z, inv_xy, inv_z, near_, far_, c, tn) && act;
+        // near-first: the distance (negative ones equal), the lane in its lowest bits; -1 no hit
+        const int key = hit ? ((__float_as_int(fmaxf(tn, 0.0f)) & ~3) | (int)l) : -1;
+        const int k1 = __shfl_xor_sync(kFullWarp, key, 1), k2 = __shfl_xor_sync(kFullWarp, key, 2),
+                  k3 = __shfl_xor_sync(kFullWarp, key, 3);
+        const uint32_t hits = (__ballot_sync(kFullWarp, hit) >> qb) & 15u;
+        // the farthest lowest
+        const uint32_t row = sp + 1u + (uint32_t)(k1 > key) + (uint32_t)(k2 > key) + (uint32_t)(k3 > key);
+        if (hit) stack[row * kQuads] = make_uint2(c.quad, __float_as_uint(tn));
+        sp += __popc(hits);
+        __syncwarp();
+      }
     } while ((uint32_t)__popc(__ballot_sync(kFullWarp, sp != 0u && !stuck)) > kQuadWait);
 
     // leaves: four triangles at a time, committed in order
@@ -379,5 +390,96 @@ __device__ __forceinline__ void traverse_warp(const TraceParams& p, RayCtx& R, u
   }
 }
 
+// ---- batches of independent rays whose hits go on to per-ray work ----------
+// Blocks of four warps. The first `differing` blocks take 128 rays, a warp 32
+// of its own. The blocks after them take 32 rays each, a warp eight: a quarter
+// of the walk's length for a batch that does not fill the chip, and quads in
+// step on the same nodes where the 32 rays are alike; their hits are gathered
+// so that one warp goes on with all 32. With `split` the former leave out the
+// groups of 32 that are alike and the latter (or a kernel with a ray per lane)
+// those that are not.
+struct QuadShare {
+  uint32_t differing;
+  bool split;
+};
+struct QuadHits {
+  float4 tuvs[32];
+  uint4 where[32];  // sorted triangle, geometry slot, instance, hit
+};
+constexpr uint32_t kShareBlock = 128;
+// From kShareSplit rays on, groups that differ are walked 32 a warp; from
+// kShareLanes on, groups that are alike one ray per lane (trace.cu's sizes).
+constexpr uint32_t kShareSplit = 48000, kShareLanes = 400000;
+__host__ __device__ constexpr uint32_t quad_share_bytes(uint32_t stack_depth) {
+  return (uint32_t)sizeof(QuadHits) + 4u * quad_warp_bytes(stack_depth);
+}
+
+// Closest hits of the block's rays (ray i: two float4 at rays + 2 i). Returns
+// whether this warp goes on, then with its lane's ray i, `valid`, and R.
+template <bool WT>
+__device__ __forceinline__ bool quad_share_query(const TraceParams& p, const QuadShare& S, const float4* rays,
+                                                 uint32_t count, uint32_t tlas, unsigned char* smem, uint32_t& i,
+                                                 bool& valid, RayCtx& R) {
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const bool gather = blockIdx.x >= S.differing;
+  const uint32_t group = gather ? blockIdx.x - S.differing : blockIdx.x * 4u + warp;
+  i = group * 32u + lane;
+  valid = i < count;
+  auto load = [&](uint32_t k) {
+    const float4 r0 = __ldg(rays + 2 * (size_t)k), r1 = __ldg(rays + 2 * (size_t)k + 1);
+    R.o = make_float3(r0.x, r0.y, r0.z);
+    R.tmin = r0.w;
+    R.d = make_float3(r1.x, r1.y, r1.z);
+    R.tmax = r1.w;
+  };
+  if (valid) load(i);
+  // every warp of a gathering block votes on the same 32 rays
+  if (S.split && coherent_warp(R, tlas, valid) != gather) return false;
+  const uint32_t mine = group * 32u + warp * 8u + lane;
+  const bool walks = gather ? lane < 8u && mine < count : valid;
+  if (gather && walks) load(mine);
+  R.cull_mask = 0xFFu;
+  R.ray_flags = 0u;
+  bool bad;
+  traverse_warp<WT>(p, R, tlas, walks, quad_warp(smem + sizeof(QuadHits), p.stack_depth4), bad);
+  if (gather) {
+    QuadHits& H = *reinterpret_cast<QuadHits*>(smem);
+    if (lane < 8u) {
+      const uint32_t at = warp * 8u + lane;
+      H.tuvs[at] = make_float4(R.best.t, R.best.u, R.best.v, R.best.s);
+      H.where[at] = make_uint4(R.best.k, R.best.geom_slot, R.best.inst, R.best.have ? 1u : 0u);
+    }
+    __syncthreads();
+    if (warp != 0u) return false;
+    const float4 t = H.tuvs[lane];
+    const uint4 w = H.where[lane];
+    R.best.t = t.x;
+    R.best.u = t.y;
+    R.best.v = t.z;
+    R.best.s = t.w;
+    R.best.k = w.x;
+    R.best.geom_slot = w.y;
+    R.best.inst = w.z;
+    R.best.have = valid && w.w != 0u;
+  }
+  if (valid) load(i);
+  return true;
+}
+
 }  // namespace dev
+
+// The share of a batch of `count` rays, and whether the groups that are alike
+// are left to a kernel with a ray per lane.
+struct QuadShareLaunch {
+  dev::QuadShare share;
+  uint32_t grid;
+  bool lanes;
+};
+inline QuadShareLaunch quad_share(uint32_t count, bool lanes_ok) {
+  const uint32_t differing = (uint32_t)(((uint64_t)count + 127) / 128), alike = (uint32_t)(((uint64_t)count + 31) / 32);
+  if (count < dev::kShareSplit) return {{0u, false}, alike, false};
+  if (count < dev::kShareLanes || !lanes_ok) return {{differing, true}, differing + alike, false};
+  return {{differing, true}, differing, true};
+}
+
 }  // namespace rdn

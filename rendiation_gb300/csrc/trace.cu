@@ -133,20 +133,22 @@ uint32_t stack_entries(int mode, uint32_t max_binary_depth, uint32_t max_wide4_d
 }
 
 namespace {
-// How a batch query is shared out, by its ray count (ordered walks, us on the
-// 1024^2 field's camera rays / random rays through a 10k soup):
+// How a batch query is shared out, by its ray count (ordered walks; us on
+// camera rays of the 1024^2 / 128^2 field and on random rays through a 10k soup):
 //   below kQuadSplit    quads, eight rays a warp: too few rays to fill the
-//                       chip, so the longest warp decides. 65,536: one ray per
-//                       lane 192 / 163, 8 rays a warp 91 / 114, 16 105 / 101,
-//                       32 150 / 124; 1,000 random rays: 130 -> 52
+//                       chip, so the longest warp decides. 65,536 camera rays
+//                       onto the soup: one ray per lane 121, 8 rays a warp 49,
+//                       16 79, 32 119; 1,000 random rays: 130 -> 45
 //   below kQuadBatch32  quads; rays that differ 16 a warp (48,000 random rays:
 //                       8 a warp 100, 16 88, 32 120), alike ones still 8
 //   below kLaneSplit    the same with 32 (131,072 random: 193 / 159 / 150;
-//                       262,144 camera rays: 8 a warp 186, 32 269, lanes 242)
-//   from there on       alike rays one per lane (1,048,576 camera rays: lanes
-//                       431, quads 567; 524,288: 382 and 344), the rest quads
-//                       (777,777 through a 150k soup: lanes 1140, quads 898)
-constexpr uint32_t kQuadSplit = 40000, kQuadBatch32 = 100000, kLaneSplit = 600000;
+//                       262,144 camera rays: 8 a warp 167 / 110, 32 242 / 134,
+//                       lanes 249 / 99; 131,072: 124 / 70, lanes 240 / 90)
+//   from there on       alike rays one per lane (393,216: quads 243 / 157,
+//                       lanes 330 / 125; 524,288: 311 / 201, 382 / 142;
+//                       786,432: 413 / 283, 411 / 156), the rest quads
+//                       (777,777 through a 150k soup: lanes 1140, quads 822)
+constexpr uint32_t kQuadSplit = 40000, kQuadBatch32 = 100000, kLaneSplit = 400000;
 
 template <int MODE, bool COUNT, bool LOCAL, bool WT, bool SPLIT>
 cudaError_t launch_lanes_wt(const TraceParams& p, uint32_t block, cudaStream_t stream) {
