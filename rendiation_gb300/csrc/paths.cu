@@ -25,6 +25,7 @@
 
 #include "parallel.h"
 #include "paths.h"
+#include "quad.cuh"
 #include "shade.cuh"
 #include "traverse.cuh"
 
@@ -33,8 +34,74 @@ namespace {
 
 using namespace dev;
 
-// Queue of bounce b: rays (2 float4) and states {id, tlas, throughput, 0}.
-// from_user: bounce 0 reads the caller's primary rays instead of a queue.
+struct PathRay {
+  float4 r0, r1;
+  uint32_t id, tlas;
+  float throughput;
+};
+
+// Entry j of a bounce's queue: rays (2 float4) and states {id, tlas,
+// throughput, 0}. from_user: bounce 0 reads the caller's primary rays instead.
+__device__ __forceinline__ PathRay load_path(const PathParams& q, bool from_user, const float4* __restrict__ in_rays,
+                                             const uint4* __restrict__ in_state, uint32_t j) {
+  PathRay e;
+  if (from_user) {
+    const float4* rp = q.primary_rays + 2 * (size_t)j;
+    e.r0 = __ldg(rp);
+    e.r1 = __ldg(rp + 1);
+    e.id = j;
+    e.tlas = q.tlas_idx ? __ldg(q.tlas_idx + j) : q.tlas_uniform;
+    e.throughput = 1.0f;
+  } else {
+    e.r0 = in_rays[2 * (size_t)j];
+    e.r1 = in_rays[2 * (size_t)j + 1];
+    const uint4 s = in_state[j];
+    e.id = s.x;
+    e.tlas = s.y;
+    e.throughput = __uint_as_float(s.z);
+  }
+  return e;
+}
+
+// Ends or continues a path after its query; true when it goes on, with its
+// next queue entry in (nr0, nr1, ns).
+__device__ __forceinline__ bool shade_path(const TraceParams& p, const PathParams& q, uint32_t bounce, uint32_t id,
+                                           uint32_t tlas, float throughput, float3 o, float3 d, const Best& best,
+                                           float4& nr0, float4& nr1, uint4& ns) {
+  if (!best.have) {
+    q.out[id] = make_float2(throughput, __uint_as_float(bounce | RDN_PATH_ESCAPED));
+    return false;
+  }
+  if (bounce == q.max_bounces) {
+    q.out[id] = make_float2(0.0f, __uint_as_float(bounce));
+    return false;
+  }
+  uint32_t st = xxhash32(id, bounce, q.seed);
+  const float s0 = sample_next(st);
+  const float s1 = sample_next(st);
+  const float s2 = sample_next(st);
+  float t_next = throughput * q.albedo;
+  bool survive = true;
+  if (bounce + 1 >= q.rr_start) {
+    survive = s2 < q.rr_survive;
+    t_next = t_next / q.rr_survive;
+  }
+  if (!survive) {
+    q.out[id] = make_float2(0.0f, __uint_as_float(bounce | RDN_PATH_ROULETTE));
+    return false;
+  }
+  const float3 hp = o + d * best.t;
+  const float3 nf = facing_normal(p, best.k, best.inst, d);
+  const float3 org = offset_ray_hit(hp, nf);
+  const float3 dir = cosine_sample_in_dir(nf, s0, s1);
+  nr0 = make_float4(org.x, org.y, org.z, 1.1920929e-7f);
+  nr1 = make_float4(dir.x, dir.y, dir.z, 3.40282347e+38f);
+  ns = make_uint4(id, tlas, __float_as_uint(t_next), 0u);
+  return true;
+}
+
+// One bounce, a ray per lane: the reference order, and structures too large
+// for quad_leaf_code.
 template <int MODE, bool LOCAL, bool WT>
 __global__ void __launch_bounds__(128) path_kernel(TraceParams p, PathParams q, uint32_t bounce, bool from_user,
                                                    const float4* __restrict__ in_rays,
@@ -54,61 +121,74 @@ __global__ void __launch_bounds__(128) path_kernel(TraceParams p, PathParams q, 
     float4 nr0 = make_float4(0.f, 0.f, 0.f, 0.f), nr1 = nr0;
     uint4 ns = make_uint4(0u, 0u, 0u, 0u);
     if (j < n) {
-      float4 r0, r1;
-      uint32_t id, tlas;
-      float throughput;
-      if (from_user) {
-        const float4* rp = q.primary_rays + 2 * (size_t)j;
-        r0 = __ldg(rp);
-        r1 = __ldg(rp + 1);
-        id = j;
-        tlas = q.tlas_idx ? __ldg(q.tlas_idx + j) : q.tlas_uniform;
-        throughput = 1.0f;
-      } else {
-        r0 = in_rays[2 * (size_t)j];
-        r1 = in_rays[2 * (size_t)j + 1];
-        const uint4 s = in_state[j];
-        id = s.x;
-        tlas = s.y;
-        throughput = __uint_as_float(s.z);
-      }
+      const PathRay e = load_path(q, from_user, in_rays, in_state, j);
       RayCtx R;
-      R.o = make_float3(r0.x, r0.y, r0.z);
-      R.tmin = r0.w;
-      R.d = make_float3(r1.x, r1.y, r1.z);
-      R.tmax = r1.w;
+      R.o = make_float3(e.r0.x, e.r0.y, e.r0.z);
+      R.tmin = e.r0.w;
+      R.d = make_float3(e.r1.x, e.r1.y, e.r1.z);
+      R.tmax = e.r1.w;
       R.cull_mask = 0xFFu;
       R.ray_flags = 0u;
       bool bad;
-      traverse_ray<MODE, false, BuiltinAnyHit, WT>(p, R, tlas, stack_ptr, stack_stride, bad);
-      if (!R.best.have) {
-        q.out[id] = make_float2(throughput, __uint_as_float(bounce | RDN_PATH_ESCAPED));
-      } else if (bounce == q.max_bounces) {
-        q.out[id] = make_float2(0.0f, __uint_as_float(bounce));
-      } else {
-        uint32_t st = xxhash32(id, bounce, q.seed);
-        const float s0 = sample_next(st);
-        const float s1 = sample_next(st);
-        const float s2 = sample_next(st);
-        float t_next = throughput * q.albedo;
-        bool survive = true;
-        if (bounce + 1 >= q.rr_start) {
-          survive = s2 < q.rr_survive;
-          t_next = t_next / q.rr_survive;
-        }
-        if (!survive) {
-          q.out[id] = make_float2(0.0f, __uint_as_float(bounce | RDN_PATH_ROULETTE));
-        } else {
-          const float3 hp = R.o + R.d * R.best.t;
-          const float3 nf = facing_normal(p, R.best.k, R.best.inst, R.d);
-          const float3 org = offset_ray_hit(hp, nf);
-          const float3 dir = cosine_sample_in_dir(nf, s0, s1);
-          nr0 = make_float4(org.x, org.y, org.z, 1.1920929e-7f);
-          nr1 = make_float4(dir.x, dir.y, dir.z, 3.40282347e+38f);
-          ns = make_uint4(id, tlas, __float_as_uint(t_next), 0u);
-          keep = true;
-        }
-      }
+      traverse_ray<MODE, false, BuiltinAnyHit, WT>(p, R, e.tlas, stack_ptr, stack_stride, bad);
+      keep = shade_path(p, q, bounce, e.id, e.tlas, e.throughput, R.o, R.d, R.best, nr0, nr1, ns);
+    }
+    const uint32_t slot = warp_append(q.queue_count + bounce, keep);
+    if (keep) {
+      out_rays[2 * (size_t)slot] = nr0;
+      out_rays[2 * (size_t)slot + 1] = nr1;
+      out_state[slot] = ns;
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0 && q.segment_counts) q.segment_counts[bounce] = n;
+}
+
+// One bounce with four lanes per ray (quad.cuh): the ordered walks. A warp
+// claims 32 queue entries, or fewer of a queue that would not give every
+// resident warp 32. The entry is read again for the shading, so that the walk
+// holds no more than its ray. The rays of a bounce differ in scene and
+// direction, the case the quads are for: 64 soups (2.4 M triangles, 3.7 M
+// primaries, up to 4 bounces) 10151 us one ray per lane on two-child nodes,
+// 5515 with quads; blocks of 32, 64 or 128 threads within 0.4 %.
+template <bool WT>
+__global__ void __launch_bounds__(128, 8) path_quad_kernel(TraceParams p, PathParams q, uint32_t bounce, bool from_user,
+                                                           const float4* __restrict__ in_rays,
+                                                           const uint4* __restrict__ in_state,
+                                                           float4* __restrict__ out_rays,
+                                                           uint4* __restrict__ out_state) {
+  extern __shared__ __align__(16) unsigned char quad_smem[];
+  const uint32_t n = bounce == 0 ? q.count : *(volatile uint32_t*)(q.queue_count + bounce - 1);
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t batch = quad_batch(n);
+  uint32_t* work = q.work_counter + bounce;
+  for (;;) {
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(work, batch);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (base >= n) break;
+    const uint32_t j = base + lane;
+    const bool valid = lane < batch && j < n;
+    RayCtx R;
+    uint32_t tlas = 0;
+    if (valid) {
+      const PathRay e = load_path(q, from_user, in_rays, in_state, j);
+      R.o = make_float3(e.r0.x, e.r0.y, e.r0.z);
+      R.tmin = e.r0.w;
+      R.d = make_float3(e.r1.x, e.r1.y, e.r1.z);
+      R.tmax = e.r1.w;
+      tlas = e.tlas;
+    }
+    R.cull_mask = 0xFFu;
+    R.ray_flags = 0u;
+    bool bad;
+    traverse_warp<WT>(p, R, tlas, valid, quad_warp(quad_smem, p.stack_depth4), bad);
+    bool keep = false;
+    float4 nr0 = make_float4(0.f, 0.f, 0.f, 0.f), nr1 = nr0;
+    uint4 ns = make_uint4(0u, 0u, 0u, 0u);
+    if (valid) {
+      const PathRay e = load_path(q, from_user, in_rays, in_state, j);
+      keep = shade_path(p, q, bounce, e.id, e.tlas, e.throughput, make_float3(e.r0.x, e.r0.y, e.r0.z),
+                        make_float3(e.r1.x, e.r1.y, e.r1.z), R.best, nr0, nr1, ns);
     }
     const uint32_t slot = warp_append(q.queue_count + bounce, keep);
     if (keep) {
@@ -161,23 +241,11 @@ __global__ void __launch_bounds__(128, 8) path_dynamic_kernel(TraceParams p, Pat
       if (L.phase == WALK_IDLE) {
         const uint32_t j = base + __popc(idle & lanes_below);
         if (j < n) {
-          float4 r0, r1;
-          if (from_user) {
-            const float4* rp = q.primary_rays + 2 * (size_t)j;
-            r0 = __ldg(rp);
-            r1 = __ldg(rp + 1);
-            id = j;
-            tlas = q.tlas_idx ? __ldg(q.tlas_idx + j) : q.tlas_uniform;
-            throughput = 1.0f;
-          } else {
-            r0 = in_rays[2 * (size_t)j];
-            r1 = in_rays[2 * (size_t)j + 1];
-            const uint4 st = in_state[j];
-            id = st.x;
-            tlas = st.y;
-            throughput = __uint_as_float(st.z);
-          }
-          L.start(p, r0, r1, tlas, 0u);
+          const PathRay e = load_path(q, from_user, in_rays, in_state, j);
+          id = e.id;
+          tlas = e.tlas;
+          throughput = e.throughput;
+          L.start(p, e.r0, e.r1, tlas, 0u);
         }
       }
     }
@@ -187,35 +255,7 @@ __global__ void __launch_bounds__(128, 8) path_dynamic_kernel(TraceParams p, Pat
     float4 nr0 = make_float4(0.f, 0.f, 0.f, 0.f), nr1 = nr0;
     uint4 ns = make_uint4(0u, 0u, 0u, 0u);
     if (L.phase == WALK_DONE) {
-      const RayCtx& R = L.R;
-      if (!R.best.have) {
-        q.out[id] = make_float2(throughput, __uint_as_float(bounce | RDN_PATH_ESCAPED));
-      } else if (bounce == q.max_bounces) {
-        q.out[id] = make_float2(0.0f, __uint_as_float(bounce));
-      } else {
-        uint32_t st = xxhash32(id, bounce, q.seed);
-        const float s0 = sample_next(st);
-        const float s1 = sample_next(st);
-        const float s2 = sample_next(st);
-        float t_next = throughput * q.albedo;
-        bool survive = true;
-        if (bounce + 1 >= q.rr_start) {
-          survive = s2 < q.rr_survive;
-          t_next = t_next / q.rr_survive;
-        }
-        if (!survive) {
-          q.out[id] = make_float2(0.0f, __uint_as_float(bounce | RDN_PATH_ROULETTE));
-        } else {
-          const float3 hp = R.o + R.d * R.best.t;
-          const float3 nf = facing_normal(p, R.best.k, R.best.inst, R.d);
-          const float3 org = offset_ray_hit(hp, nf);
-          const float3 dir = cosine_sample_in_dir(nf, s0, s1);
-          nr0 = make_float4(org.x, org.y, org.z, 1.1920929e-7f);
-          nr1 = make_float4(dir.x, dir.y, dir.z, 3.40282347e+38f);
-          ns = make_uint4(id, tlas, __float_as_uint(t_next), 0u);
-          keep = true;
-        }
-      }
+      keep = shade_path(p, q, bounce, id, tlas, throughput, L.R.o, L.R.d, L.R.best, nr0, nr1, ns);
       L.phase = WALK_IDLE;
     }
     const uint32_t slot = warp_append(q.queue_count + bounce, keep);
@@ -322,47 +362,29 @@ void paths_bind_scratch(PathParams& q, void* scratch) {
 }
 
 namespace {
-// kernel variant: 0 batch, 1 dynamic fetch, 2 batch with local-memory stacks
+// kernel variant: 0 a ray per lane, 1 dynamic fetch, 2 four lanes per ray
+enum PathVariant { PATH_LANES = 0, PATH_DYNAMIC = 1, PATH_QUADS = 2 };
 int path_variant(int mode, const TraceParams& p, const PathParams& q) {
-  if (mode == MODE_THREADED) return 0;
-  if (q.refill != 0) return 1;
-  return p.local_stack ? 2 : 0;
+  if (mode == MODE_THREADED) return PATH_LANES;
+  if (q.refill != 0) return PATH_DYNAMIC;
+  return p.quads ? PATH_QUADS : PATH_LANES;
 }
+// shared memory of a block: the variant's stacks
+size_t path_smem(int mode, int variant, const TraceParams& p, uint32_t block) {
+  if (variant == PATH_QUADS) return (size_t)quad_warp_bytes(p.stack_depth4) * (block / 32);
+  return mode == MODE_THREADED ? 0 : (size_t)p.stack_depth * block * sizeof(uint2);
+}
+using PathKernel = void (*)(TraceParams, PathParams, uint32_t, bool, const float4*, const uint4*, float4*, uint4*);
 template <bool WT>
-const void* path_fn_wt(int mode, int variant) {
+PathKernel path_fn_wt(int mode, int variant) {
+  if (mode == MODE_THREADED) return path_kernel<MODE_THREADED, false, WT>;
+  if (variant == PATH_QUADS) return path_quad_kernel<WT>;
   if (mode == MODE_WIDE4)
-    return variant == 1 ? (const void*)path_dynamic_kernel<MODE_WIDE4, WT>
-                        : (variant == 2 ? (const void*)path_kernel<MODE_WIDE4, true, WT>
-                                        : (const void*)path_kernel<MODE_WIDE4, false, WT>);
-  if (mode == MODE_BINARY)
-    return variant == 1 ? (const void*)path_dynamic_kernel<MODE_BINARY, WT>
-                        : (variant == 2 ? (const void*)path_kernel<MODE_BINARY, true, WT>
-                                        : (const void*)path_kernel<MODE_BINARY, false, WT>);
-  return (const void*)path_kernel<MODE_THREADED, false, WT>;
+    return variant == PATH_DYNAMIC ? path_dynamic_kernel<MODE_WIDE4, WT> : path_kernel<MODE_WIDE4, false, WT>;
+  return variant == PATH_DYNAMIC ? path_dynamic_kernel<MODE_BINARY, WT> : path_kernel<MODE_BINARY, false, WT>;
 }
-const void* path_fn(int mode, int variant, bool wt) {
+PathKernel path_fn(int mode, int variant, bool wt) {
   return wt ? path_fn_wt<true>(mode, variant) : path_fn_wt<false>(mode, variant);
-}
-
-// One bounce launch of the variant chosen by path_variant.
-template <bool WT>
-void launch_bounce(int mode, int variant, uint32_t grid, uint32_t block, size_t smem, cudaStream_t stream,
-                   const TraceParams& p, const PathParams& q, uint32_t b, bool from_user, const float4* in_r,
-                   const uint4* in_s, float4* out_r, uint4* out_s) {
-  if (mode == MODE_WIDE4 && variant == 1)
-    path_dynamic_kernel<MODE_WIDE4, WT><<<grid, block, smem, stream>>>(p, q, b, from_user, in_r, in_s, out_r, out_s);
-  else if (mode == MODE_WIDE4 && variant == 2)
-    path_kernel<MODE_WIDE4, true, WT><<<grid, block, smem, stream>>>(p, q, b, from_user, in_r, in_s, out_r, out_s);
-  else if (mode == MODE_WIDE4)
-    path_kernel<MODE_WIDE4, false, WT><<<grid, block, smem, stream>>>(p, q, b, from_user, in_r, in_s, out_r, out_s);
-  else if (mode == MODE_BINARY && variant == 1)
-    path_dynamic_kernel<MODE_BINARY, WT><<<grid, block, smem, stream>>>(p, q, b, from_user, in_r, in_s, out_r, out_s);
-  else if (mode == MODE_BINARY && variant == 2)
-    path_kernel<MODE_BINARY, true, WT><<<grid, block, smem, stream>>>(p, q, b, from_user, in_r, in_s, out_r, out_s);
-  else if (mode == MODE_BINARY)
-    path_kernel<MODE_BINARY, false, WT><<<grid, block, smem, stream>>>(p, q, b, from_user, in_r, in_s, out_r, out_s);
-  else
-    path_kernel<MODE_THREADED, false, WT><<<grid, block, smem, stream>>>(p, q, b, from_user, in_r, in_s, out_r, out_s);
 }
 }  // namespace
 
@@ -370,9 +392,9 @@ cudaError_t prepare_paths(const TraceParams& p, const PathParams& q, int mode, u
                           uint32_t* grid) {
   if (block == 0) block = 64;
   const int variant = path_variant(mode, p, q);
-  const size_t smem = mode != MODE_THREADED && variant != 2 ? (size_t)p.stack_depth * block * sizeof(uint2) : 0;
+  const size_t smem = path_smem(mode, variant, p, block);
   static std::atomic<uint64_t> attr_done[2][3][3] = {};
-  const void* fn = path_fn(mode, variant, p.watertight != 0);
+  const void* fn = (const void*)path_fn(mode, variant, p.watertight != 0);
   cudaError_t e = raise_smem_limit(attr_done[p.watertight ? 1 : 0][variant][mode], {fn});
   if (e != cudaSuccess) return e;
   int per_sm = 0;
@@ -381,7 +403,8 @@ cudaError_t prepare_paths(const TraceParams& p, const PathParams& q, int mode, u
   if (per_sm < 1) per_sm = 1;
   // persistent grid, never larger than the primary queue needs
   uint32_t g = (uint32_t)(sm_count * per_sm);
-  const uint32_t need = (q.count + block - 1) / block;
+  const uint32_t per = variant == PATH_QUADS ? quad_batch(q.count) * (block / 32) : block;  // rays a block takes at a time
+  const uint32_t need = (q.count + per - 1) / per;
   *grid = g > need ? need : g;
   return cudaSuccess;
 }
@@ -391,7 +414,8 @@ cudaError_t record_paths(const TraceParams& p, const PathParams& q, int mode, ui
   if (block == 0) block = 64;
   if (q.count == 0 || grid == 0) return cudaSuccess;
   const int variant = path_variant(mode, p, q);
-  const size_t smem = mode != MODE_THREADED && variant != 2 ? (size_t)p.stack_depth * block * sizeof(uint2) : 0;
+  const size_t smem = path_smem(mode, variant, p, block);
+  const PathKernel fn = path_fn(mode, variant, p.watertight != 0);
   cudaError_t e = cudaMemsetAsync(q.queue_count, 0, sizeof(uint32_t) * 2 * (q.max_bounces + 1), stream);
   if (e != cudaSuccess) return e;
   float4* ra = static_cast<float4*>(q.rays_a);
@@ -431,10 +455,7 @@ cudaError_t record_paths(const TraceParams& p, const PathParams& q, int mode, ui
       out_r = (b & 1) ? ra : rb;
       out_s = (b & 1) ? sa : sb;
     }
-    if (p.watertight)
-      launch_bounce<true>(mode, variant, grid, block, smem, stream, p, q, b, from_user, in_r, in_s, out_r, out_s);
-    else
-      launch_bounce<false>(mode, variant, grid, block, smem, stream, p, q, b, from_user, in_r, in_s, out_r, out_s);
+    fn<<<grid, block, smem, stream>>>(p, q, b, from_user, in_r, in_s, out_r, out_s);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
