@@ -1,13 +1,13 @@
 // Differentiable closest hit: attribute-interpolation loss and its adjoint at
 // frozen visibility, sm_103a.
 //
-// Forward (attr_forward_kernel): per ray, closest hit (the traversal of
+// Forward (ray_pass_kernel, ATTR_FORWARD): per ray, closest hit (the traversal of
 // traverse.cuh), value = (1-u-v)*a[i0] + u*a[i1] + v*a[i2] with the hit
 // triangle's vertex attributes, loss = (value - target)^2; a miss contributes
 // nothing. The per-ray value and loss are written; the loss sum is accumulated
-// per block and added once per block.
+// per warp and added once per warp.
 //
-// Adjoint (attr_adjoint_kernel): the hit is recomputed by tracing the ray again
+// Adjoint (ATTR_ADJOINT): the hit is recomputed by tracing the ray again
 // instead of being stored by the forward pass. With r = 2 (value - target) * g
 // (g = upstream gradient of the loss sum):
 //   dL/da_k = r * w_k                       (w = (1-u-v, u, v))
@@ -34,6 +34,7 @@
 #include <cstdint>
 
 #include "adjoint.h"
+#include "quad.cuh"
 #include "shade.cuh"
 #include "traverse.cuh"
 
@@ -41,6 +42,12 @@ namespace rdn {
 namespace {
 
 using namespace dev;
+
+// Least resident blocks of 128 threads of the quad kernels: 72 registers. 64
+// (8 blocks) spill in the float-float part and 80 (6) hold fewer warps: the
+// 16-field paths' forward + adjoint took 5991 / 5873 / 6060 us with 8 / 7 / 6,
+// the 256^2 loss step 339 / 322 / 326 us.
+constexpr int kQuadBlocks = 7;
 
 // float-float value hi + lo
 struct ff {
@@ -175,94 +182,15 @@ __device__ __forceinline__ float residual(const HitGeom& h, float a0, float a1, 
   return d.hi + d.lo;
 }
 
-template <int MODE, bool LOCAL, bool WT>
-__global__ void __launch_bounds__(128) attr_forward_kernel(TraceParams p, AdjointParams a) {
-  RDN_TRAVERSAL_STACK(LOCAL);
-  __shared__ double block_sum[4];
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  float loss = 0.0f;
-  if (i < a.count) {
-    const float4* rp = a.rays + 2 * (size_t)i;
-    const float4 r0 = __ldg(rp), r1 = __ldg(rp + 1);
-    RayCtx R;
-    R.o = make_float3(r0.x, r0.y, r0.z);
-    R.tmin = r0.w;
-    R.d = make_float3(r1.x, r1.y, r1.z);
-    R.tmax = r1.w;
-    R.cull_mask = 0xFFu;
-    R.ray_flags = 0u;
-    bool bad;
-    traverse_ray<MODE, false, BuiltinAnyHit, WT>(p, R, a.tlas_uniform, stack_ptr, stack_stride, bad);
-    float value = 0.0f;
-    if (R.best.have) {
-      const InstanceRay ir = to_instance(p.tlas_data + R.best.inst, R.o, R.d, 0u);
-      const HitGeom h = hit_vertices(p, a.indices, a.vertices, R, ir);
-      const float diff = residual(h, __ldg(a.attributes + h.i0), __ldg(a.attributes + h.i1),
-                                  __ldg(a.attributes + h.i2), a.targets ? __ldg(a.targets + i) : 0.0f, &value);
-      loss = diff * diff;
-    }
-    if (a.hit_tri) a.hit_tri[i] = R.best.have ? __ldg(p.redirect + R.best.k) : INVALID_NEXT;
-    if (a.hit_inst) a.hit_inst[i] = R.best.have ? R.best.inst : INVALID_NEXT;
-    if (a.ray_value) a.ray_value[i] = value;
-    if (a.ray_loss) a.ray_loss[i] = loss;
-  }
-  if (a.loss_sum) {
-    double s = loss;
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-    if ((threadIdx.x & 31) == 0) block_sum[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (uint32_t w = 0; w < (blockDim.x + 31) / 32; w++) t += block_sum[w];
-      atomicAdd(a.loss_sum, t);
-    }
-  }
-}
+// What each of the four per-ray passes does with its ray's hit.
+enum RayPass { ATTR_FORWARD, ATTR_ADJOINT, HIT_FORWARD, HIT_ADJOINT };
 
-template <int MODE, bool LOCAL, bool WT>
-__global__ void __launch_bounds__(128) attr_adjoint_kernel(TraceParams p, AdjointParams a) {
-  RDN_TRAVERSAL_STACK(LOCAL);
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.count) return;
-  const float4* rp = a.rays + 2 * (size_t)i;
-  const float4 r0 = __ldg(rp), r1 = __ldg(rp + 1);
-  RayCtx R;
-  R.o = make_float3(r0.x, r0.y, r0.z);
-  R.tmin = r0.w;
-  R.d = make_float3(r1.x, r1.y, r1.z);
-  R.tmax = r1.w;
-  R.cull_mask = 0xFFu;
-  R.ray_flags = 0u;
-  bool bad;
-  traverse_ray<MODE, false, BuiltinAnyHit, WT>(p, R, a.tlas_uniform, stack_ptr, stack_stride, bad);
-  float3 go = make_float3(0.f, 0.f, 0.f), gd = go;
-  if (R.best.have) {
-    const InstanceRay ir = to_instance(p.tlas_data + R.best.inst, R.o, R.d, 0u);
-    const HitGeom h = hit_vertices(p, a.indices, a.vertices, R, ir);
-    const float a0 = __ldg(a.attributes + h.i0), a1 = __ldg(a.attributes + h.i1), a2 = __ldg(a.attributes + h.i2);
-    float value;
-    const float target = a.targets ? __ldg(a.targets + i) : 0.0f;
-    const float r = 2.0f * residual(h, a0, a1, a2, target, &value) * a.grad_scale;
-    const float gu = r * (a1 - a0), gv = r * (a2 - a0);
-    const float3 lam = adjoint_lambda(h, gu, gv);
-    float4* g = reinterpret_cast<float4*>(a.grad_vertices);
-    atomicAdd(g + h.i0, make_float4(-h.w0 * lam.x, -h.w0 * lam.y, -h.w0 * lam.z, r * h.w0));
-    atomicAdd(g + h.i1, make_float4(-h.u * lam.x, -h.u * lam.y, -h.u * lam.z, r * h.u));
-    atomicAdd(g + h.i2, make_float4(-h.v * lam.x, -h.v * lam.y, -h.v * lam.z, r * h.v));
-    // d(o + s d)/dd = s: s the hit's parameter along the object-space direction
-    go = lam;
-    gd = make_float3(h.t_unnorm * lam.x, h.t_unnorm * lam.y, h.t_unnorm * lam.z);
-  }
-  if (a.grad_ray_origin) {
-    a.grad_ray_origin[3 * (size_t)i] = go.x;
-    a.grad_ray_origin[3 * (size_t)i + 1] = go.y;
-    a.grad_ray_origin[3 * (size_t)i + 2] = go.z;
-  }
-  if (a.grad_ray_direction) {
-    a.grad_ray_direction[3 * (size_t)i] = gd.x;
-    a.grad_ray_direction[3 * (size_t)i + 1] = gd.y;
-    a.grad_ray_direction[3 * (size_t)i + 2] = gd.z;
-  }
+// Three floats per ray to an array of them, where there is one.
+__device__ __forceinline__ void store3(float* out, uint32_t i, float3 v) {
+  if (!out) return;
+  out[3 * (size_t)i] = v.x;
+  out[3 * (size_t)i + 1] = v.y;
+  out[3 * (size_t)i + 2] = v.z;
 }
 
 // lambda = M^{-T} (0, gu, gv) with M = [-d | e1 | e2] (object space),
@@ -277,42 +205,93 @@ __device__ __forceinline__ float3 scatter_vertex_grads(const HitGeom& h, const I
   return lam;
 }
 
-// Persistent warps over paths; ADJOINT selects the gradient pass.
-template <int MODE, bool ADJOINT, bool LOCAL, bool WT>
-__global__ void __launch_bounds__(128) attr_path_kernel(TraceParams p, PathAdjointParams a) {
-  RDN_TRAVERSAL_STACK(LOCAL);
+// Loss forward of one ray: its loss, with the per-ray records written.
+__device__ __forceinline__ float attr_forward_ray(const TraceParams& p, const AdjointParams& a, uint32_t i,
+                                                  const RayCtx& R) {
+  float value = 0.0f, loss = 0.0f;
+  if (R.best.have) {
+    const InstanceRay ir = to_instance(p.tlas_data + R.best.inst, R.o, R.d, 0u);
+    const HitGeom h = hit_vertices(p, a.indices, a.vertices, R, ir);
+    const float diff = residual(h, __ldg(a.attributes + h.i0), __ldg(a.attributes + h.i1),
+                                __ldg(a.attributes + h.i2), a.targets ? __ldg(a.targets + i) : 0.0f, &value);
+    loss = diff * diff;
+  }
+  if (a.hit_tri) a.hit_tri[i] = R.best.have ? __ldg(p.redirect + R.best.k) : INVALID_NEXT;
+  if (a.hit_inst) a.hit_inst[i] = R.best.have ? R.best.inst : INVALID_NEXT;
+  if (a.ray_value) a.ray_value[i] = value;
+  if (a.ray_loss) a.ray_loss[i] = loss;
+  return loss;
+}
+
+// Loss adjoint of one ray's hit (triangle `tri` of instance `inst`).
+__device__ __forceinline__ void attr_scatter(const TraceParams& p, const AdjointParams& a, uint32_t i, uint32_t tri,
+                                             uint32_t inst, float3 o, float3 d, float3& go, float3& gd) {
+  const InstanceRay ir = to_instance(p.tlas_data + inst, o, d, 0u);
+  const HitGeom h = hit_vertices_at(p, a.indices, a.vertices, tri, inst, d, ir);
+  const float a0 = __ldg(a.attributes + h.i0), a1 = __ldg(a.attributes + h.i1), a2 = __ldg(a.attributes + h.i2);
+  float value;
+  const float target = a.targets ? __ldg(a.targets + i) : 0.0f;
+  const float r = 2.0f * residual(h, a0, a1, a2, target, &value) * a.grad_scale;
+  const float3 lam = scatter_vertex_grads(h, ir, r, r * (a1 - a0), r * (a2 - a0), a.grad_vertices);
+  // d(o + s d)/dd = s: s the hit's parameter along the object-space direction
+  go = lam;
+  gd = make_float3(h.t_unnorm * lam.x, h.t_unnorm * lam.y, h.t_unnorm * lam.z);
+}
+
+// Persistent warps over paths; ADJOINT selects the gradient pass. QUADS: the
+// ordered walks with four lanes per ray (quad.cuh), every lane of the warp
+// going through all segments; else a ray per lane in MODE's order. 16 fields,
+// 2.2 M paths of three segments, forward + adjoint: 6166 us one ray per lane
+// on two-child nodes, 5363 with quads (6490 with the first segments, whose
+// rays are alike, one per lane in the same kernel: its registers and shared
+// memory cost both walks more than that saves).
+template <int MODE, bool ADJOINT, bool QUADS, bool WT>
+__global__ void __launch_bounds__(128, QUADS ? kQuadBlocks : 0) attr_path_kernel(TraceParams p, PathAdjointParams a) {
+  extern __shared__ __align__(16) unsigned char dyn_smem[];
   __shared__ double block_sum[4];
   const uint32_t lane = threadIdx.x & 31u;
   double loss_acc = 0.0;
+  const uint32_t batch = QUADS ? quad_batch(a.count) : 32u;
   for (;;) {
     uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(a.work_counter, 32u);
+    if (lane == 0) base = atomicAdd(a.work_counter, batch);
     base = __shfl_sync(0xffffffffu, base, 0);
     if (base >= a.count) break;
     const uint32_t i = base + lane;
-    if (i >= a.count) continue;
-    const float4* rp = a.rays + 2 * (size_t)i;
-    float4 r0 = __ldg(rp), r1 = __ldg(rp + 1);
-    const uint32_t tlas = a.tlas_idx ? __ldg(a.tlas_idx + i) : a.tlas_uniform;
-    bool alive = true;
+    const bool mine = lane < batch && i < a.count;
+    if (!QUADS && !mine) continue;
+    float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0;
+    uint32_t tlas = a.tlas_uniform;
+    if (mine) {
+      r0 = __ldg(a.rays + 2 * (size_t)i);
+      r1 = __ldg(a.rays + 2 * (size_t)i + 1);
+      if (a.tlas_idx) tlas = __ldg(a.tlas_idx + i);
+    }
+    bool alive = mine;
     for (uint32_t k = 0; k < a.segments; k++) {
       const size_t seg = (size_t)i * a.segments + k;
       float value = 0.0f;
       uint32_t tri_out = INVALID_NEXT, inst_out = INVALID_NEXT;
+      if (alive && a.seg_rays) {
+        a.seg_rays[2 * seg] = r0;
+        a.seg_rays[2 * seg + 1] = r1;
+      }
+      RayCtx R;
+      R.o = make_float3(r0.x, r0.y, r0.z);
+      R.tmin = r0.w;
+      R.d = make_float3(r1.x, r1.y, r1.z);
+      R.tmax = r1.w;
+      R.cull_mask = 0xFFu;
+      R.ray_flags = 0u;
+      bool bad;
+      if constexpr (QUADS) {
+        if (!__any_sync(kFullWarp, alive || (mine && !ADJOINT))) break;
+        traverse_warp<WT>(p, R, tlas, alive, quad_warp(dyn_smem, p.stack_depth4), bad);
+      } else if (alive) {
+        traverse_ray<MODE, false, BuiltinAnyHit, WT>(p, R, tlas, reinterpret_cast<uint2*>(dyn_smem) + threadIdx.x,
+                                                     blockDim.x, bad);
+      }
       if (alive) {
-        if (a.seg_rays) {
-          a.seg_rays[2 * seg] = r0;
-          a.seg_rays[2 * seg + 1] = r1;
-        }
-        RayCtx R;
-        R.o = make_float3(r0.x, r0.y, r0.z);
-        R.tmin = r0.w;
-        R.d = make_float3(r1.x, r1.y, r1.z);
-        R.tmax = r1.w;
-        R.cull_mask = 0xFFu;
-        R.ray_flags = 0u;
-        bool bad;
-        traverse_ray<MODE, false, BuiltinAnyHit, WT>(p, R, tlas, stack_ptr, stack_stride, bad);
         if (!R.best.have) {
           alive = false;
           if (!ADJOINT && a.targets) {
@@ -346,14 +325,14 @@ __global__ void __launch_bounds__(128) attr_path_kernel(TraceParams p, PathAdjoi
             r1 = make_float4(dir.x, dir.y, dir.z, 3.40282347e+38f);
           }
         }
-      } else if (!ADJOINT && a.targets) {
+      } else if (mine && !ADJOINT && a.targets) {
         // a missed segment has value 0 against its target
         const float t = __ldg(a.targets + seg);
         loss_acc += (double)(t * t);
       }
-      if (!ADJOINT && a.values) a.values[seg] = value;
-      if (!ADJOINT && a.seg_tri) a.seg_tri[seg] = tri_out;
-      if (!ADJOINT && a.seg_inst) a.seg_inst[seg] = inst_out;
+      if (mine && !ADJOINT && a.values) a.values[seg] = value;
+      if (mine && !ADJOINT && a.seg_tri) a.seg_tri[seg] = tri_out;
+      if (mine && !ADJOINT && a.seg_inst) a.seg_inst[seg] = inst_out;
     }
   }
   if (!ADJOINT && a.loss_sum) {
@@ -432,30 +411,12 @@ __global__ void __launch_bounds__(256) attr_recorded_adjoint_kernel(TraceParams 
     const uint32_t tri = __ldg(a.hit_tri + i);
     float3 go = make_float3(0.f, 0.f, 0.f), gd = go;
     if (tri != INVALID_NEXT) {
-      const uint32_t inst = __ldg(a.hit_inst + i);
       const float4 r0 = __ldg(a.rays + 2 * (size_t)i), r1 = __ldg(a.rays + 2 * (size_t)i + 1);
-      const float3 o = make_float3(r0.x, r0.y, r0.z), d = make_float3(r1.x, r1.y, r1.z);
-      const InstanceRay ir = to_instance(p.tlas_data + inst, o, d, 0u);
-      const HitGeom h = hit_vertices_at(p, a.indices, a.vertices, tri, inst, d, ir);
-      const float a0 = __ldg(a.attributes + h.i0), a1 = __ldg(a.attributes + h.i1), a2 = __ldg(a.attributes + h.i2);
-      float value;
-      const float target = a.targets ? __ldg(a.targets + i) : 0.0f;
-      const float r = 2.0f * residual(h, a0, a1, a2, target, &value) * a.grad_scale;
-      const float3 lam = scatter_vertex_grads(h, ir, r, r * (a1 - a0), r * (a2 - a0), a.grad_vertices);
-      // d(o + s d)/dd = s: s the hit's parameter along the object-space direction
-      go = lam;
-      gd = make_float3(h.t_unnorm * lam.x, h.t_unnorm * lam.y, h.t_unnorm * lam.z);
+      attr_scatter(p, a, i, tri, __ldg(a.hit_inst + i), make_float3(r0.x, r0.y, r0.z), make_float3(r1.x, r1.y, r1.z),
+                   go, gd);
     }
-    if (a.grad_ray_origin) {
-      a.grad_ray_origin[3 * (size_t)i] = go.x;
-      a.grad_ray_origin[3 * (size_t)i + 1] = go.y;
-      a.grad_ray_origin[3 * (size_t)i + 2] = go.z;
-    }
-    if (a.grad_ray_direction) {
-      a.grad_ray_direction[3 * (size_t)i] = gd.x;
-      a.grad_ray_direction[3 * (size_t)i + 1] = gd.y;
-      a.grad_ray_direction[3 * (size_t)i + 2] = gd.z;
-    }
+    store3(a.grad_ray_origin, i, go);
+    store3(a.grad_ray_direction, i, gd);
   }
 }
 
@@ -484,21 +445,9 @@ __device__ __forceinline__ void hit_diff_store(const AdjointParams& a, uint32_t 
   if (a.hit_inst) a.hit_inst[i] = inst;
 }
 
-template <int MODE, bool LOCAL, bool WT>
-__global__ void __launch_bounds__(128) hit_diff_forward_kernel(TraceParams p, AdjointParams a) {
-  RDN_TRAVERSAL_STACK(LOCAL);
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.count) return;
-  const float4 r0 = __ldg(a.rays + 2 * (size_t)i), r1 = __ldg(a.rays + 2 * (size_t)i + 1);
-  RayCtx R;
-  R.o = make_float3(r0.x, r0.y, r0.z);
-  R.tmin = r0.w;
-  R.d = make_float3(r1.x, r1.y, r1.z);
-  R.tmax = r1.w;
-  R.cull_mask = 0xFFu;
-  R.ray_flags = 0u;
-  bool bad;
-  traverse_ray<MODE, false, BuiltinAnyHit, WT>(p, R, a.tlas_uniform, stack_ptr, stack_stride, bad);
+// Hit query forward of one ray.
+__device__ __forceinline__ void hit_diff_forward_ray(const TraceParams& p, const AdjointParams& a, uint32_t i,
+                                                     const RayCtx& R) {
   if (!R.best.have) {
     hit_diff_store(a, i, make_float4(R.tmax, 0.0f, 0.0f, 0.0f), INVALID_NEXT, INVALID_NEXT);
     return;
@@ -538,37 +487,74 @@ __device__ __forceinline__ void hit_diff_scatter(const TraceParams& p, const Adj
   gd = make_float3(h.t_unnorm * go.x, h.t_unnorm * go.y, h.t_unnorm * go.z);
 }
 
-__device__ __forceinline__ void hit_diff_store_ray_grads(const AdjointParams& a, uint32_t i, float3 go, float3 gd) {
-  if (a.grad_ray_origin) {
-    a.grad_ray_origin[3 * (size_t)i] = go.x;
-    a.grad_ray_origin[3 * (size_t)i + 1] = go.y;
-    a.grad_ray_origin[3 * (size_t)i + 2] = go.z;
+// What `PASS` does with a ray whose query is done; the loss forward's loss.
+template <int PASS>
+__device__ __forceinline__ float ray_pass(const TraceParams& p, const AdjointParams& a, uint32_t i, const RayCtx& R) {
+  if (PASS == ATTR_FORWARD) return attr_forward_ray(p, a, i, R);
+  if (PASS == HIT_FORWARD) {
+    hit_diff_forward_ray(p, a, i, R);
+    return 0.0f;
   }
-  if (a.grad_ray_direction) {
-    a.grad_ray_direction[3 * (size_t)i] = gd.x;
-    a.grad_ray_direction[3 * (size_t)i + 1] = gd.y;
-    a.grad_ray_direction[3 * (size_t)i + 2] = gd.z;
+  float3 go = make_float3(0.f, 0.f, 0.f), gd = go;
+  if (R.best.have) {
+    const uint32_t tri = __ldg(p.redirect + R.best.k);
+    if (PASS == ATTR_ADJOINT) attr_scatter(p, a, i, tri, R.best.inst, R.o, R.d, go, gd);
+    else hit_diff_scatter(p, a, i, tri, R.best.inst, R.o, R.d, go, gd);
   }
+  store3(a.grad_ray_origin, i, go);
+  store3(a.grad_ray_direction, i, gd);
+  return 0.0f;
 }
 
-template <int MODE, bool LOCAL, bool WT>
-__global__ void __launch_bounds__(128) hit_diff_adjoint_kernel(TraceParams p, AdjointParams a) {
+// The warp's losses to the sum: in double, one addition per warp.
+__device__ __forceinline__ void add_loss(const AdjointParams& a, float loss) {
+  if (!a.loss_sum) return;
+  double s = loss;
+  for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
+  if ((threadIdx.x & 31) == 0) atomicAdd(a.loss_sum, s);
+}
+
+// A ray per lane, in MODE's order. SPLIT: only the warps whose rays are alike.
+template <int PASS, int MODE, bool LOCAL, bool WT, bool SPLIT>
+__global__ void __launch_bounds__(128) ray_pass_kernel(TraceParams p, AdjointParams a) {
   RDN_TRAVERSAL_STACK(LOCAL);
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.count) return;
-  const float4 r0 = __ldg(a.rays + 2 * (size_t)i), r1 = __ldg(a.rays + 2 * (size_t)i + 1);
+  const bool valid = i < a.count;
   RayCtx R;
-  R.o = make_float3(r0.x, r0.y, r0.z);
-  R.tmin = r0.w;
-  R.d = make_float3(r1.x, r1.y, r1.z);
-  R.tmax = r1.w;
-  R.cull_mask = 0xFFu;
-  R.ray_flags = 0u;
-  bool bad;
-  traverse_ray<MODE, false, BuiltinAnyHit, WT>(p, R, a.tlas_uniform, stack_ptr, stack_stride, bad);
-  float3 go = make_float3(0.f, 0.f, 0.f), gd = go;
-  if (R.best.have) hit_diff_scatter(p, a, i, __ldg(p.redirect + R.best.k), R.best.inst, R.o, R.d, go, gd);
-  hit_diff_store_ray_grads(a, i, go, gd);
+  if (valid) {
+    const float4 r0 = __ldg(a.rays + 2 * (size_t)i), r1 = __ldg(a.rays + 2 * (size_t)i + 1);
+    R.o = make_float3(r0.x, r0.y, r0.z);
+    R.tmin = r0.w;
+    R.d = make_float3(r1.x, r1.y, r1.z);
+    R.tmax = r1.w;
+  }
+  if (SPLIT && !coherent_warp(R, a.tlas_uniform, valid)) return;
+  float loss = 0.0f;
+  if (valid) {
+    R.cull_mask = 0xFFu;
+    R.ray_flags = 0u;
+    bool bad;
+    traverse_ray<MODE, false, BuiltinAnyHit, WT>(p, R, a.tlas_uniform, stack_ptr, stack_stride, bad);
+    loss = ray_pass<PASS>(p, a, i, R);
+  }
+  __syncwarp();
+  if (PASS == ATTR_FORWARD) add_loss(a, loss);
+}
+
+// Four lanes per ray (quad.cuh): the ordered walks. 262,144 rays on the 256^2
+// field, loss forward + traced adjoint: 442 us one ray per lane, 297 here;
+// 198,779 rays, hit query + recorded adjoint: 175 and 123; 4,096 rays: 302 and
+// 79.
+template <int PASS, bool WT>
+__global__ void __launch_bounds__(kShareBlock, kQuadBlocks) ray_pass_quad_kernel(TraceParams p, AdjointParams a, QuadShare S) {
+  extern __shared__ __align__(16) unsigned char dyn_smem[];
+  uint32_t i;
+  bool valid;
+  RayCtx R;
+  if (!quad_share_query<WT>(p, S, a.rays, a.count, a.tlas_uniform, dyn_smem, i, valid, R)) return;
+  const float loss = valid ? ray_pass<PASS>(p, a, i, R) : 0.0f;
+  __syncwarp();
+  if (PASS == ATTR_FORWARD) add_loss(a, loss);
 }
 
 __global__ void __launch_bounds__(256) hit_diff_recorded_adjoint_kernel(TraceParams p, AdjointParams a) {
@@ -580,7 +566,8 @@ __global__ void __launch_bounds__(256) hit_diff_recorded_adjoint_kernel(TracePar
       hit_diff_scatter(p, a, i, tri, __ldg(a.hit_inst + i), make_float3(r0.x, r0.y, r0.z),
                        make_float3(r1.x, r1.y, r1.z), go, gd);
     }
-    hit_diff_store_ray_grads(a, i, go, gd);
+    store3(a.grad_ray_origin, i, go);
+    store3(a.grad_ray_direction, i, gd);
   }
 }
 
@@ -590,97 +577,72 @@ inline uint32_t recorded_grid(size_t items, int sm_count) {
   return (uint32_t)(need < cap ? (need ? need : 1) : cap);
 }
 
-template <int MODE, bool LOCAL, bool WT>
-cudaError_t launch_attr_paths_variant(const TraceParams& p, const PathAdjointParams& a, bool adjoint, uint32_t block,
-                                      int sm_count, cudaStream_t stream) {
+template <int MODE, bool QUADS, bool WT>
+cudaError_t launch_attr_paths_wt(const TraceParams& p, const PathAdjointParams& a, bool adjoint, uint32_t block,
+                                 int sm_count, cudaStream_t stream) {
   static std::atomic<uint64_t> done[2] = {};
-  const void* fn = adjoint ? (const void*)attr_path_kernel<MODE, true, LOCAL, WT>
-                           : (const void*)attr_path_kernel<MODE, false, LOCAL, WT>;
-  cudaError_t e = raise_smem_limit(done[adjoint], {fn});
+  const auto fn = adjoint ? attr_path_kernel<MODE, true, QUADS, WT> : attr_path_kernel<MODE, false, QUADS, WT>;
+  cudaError_t e = raise_smem_limit(done[adjoint], {(const void*)fn});
   if (e != cudaSuccess) return e;
-  const size_t smem = MODE != MODE_THREADED && !LOCAL ? (size_t)p.stack_depth * block * sizeof(uint2) : 0;
+  const size_t smem = QUADS                   ? (size_t)quad_warp_bytes(p.stack_depth4) * (block / 32)
+                      : MODE != MODE_THREADED ? (size_t)p.stack_depth * block * sizeof(uint2)
+                                              : 0;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, (int)block, smem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) per_sm = 1;
   uint32_t grid = (uint32_t)(sm_count * per_sm);
-  const uint32_t need = (a.count + block - 1) / block;
+  const uint32_t per = QUADS ? quad_batch(a.count) * (block / 32) : block;  // paths a block takes at a time
+  const uint32_t need = (uint32_t)(((uint64_t)a.count + per - 1) / per);
   if (grid > need) grid = need;
   e = cudaMemsetAsync(a.work_counter, 0, 4, stream);
   if (e != cudaSuccess) return e;
-  if (adjoint) attr_path_kernel<MODE, true, LOCAL, WT><<<grid, block, smem, stream>>>(p, a);
-  else attr_path_kernel<MODE, false, LOCAL, WT><<<grid, block, smem, stream>>>(p, a);
+  fn<<<grid, block, smem, stream>>>(p, a);
   return cudaGetLastError();
 }
 
-template <int MODE>
+template <int MODE, bool QUADS>
 cudaError_t launch_attr_paths_mode(const TraceParams& p, const PathAdjointParams& a, bool adjoint, uint32_t block,
                                    int sm_count, cudaStream_t stream) {
-  const bool local = MODE != MODE_THREADED && p.local_stack;
-  if (p.watertight)
-    return local ? launch_attr_paths_variant<MODE, MODE != MODE_THREADED, true>(p, a, adjoint, block, sm_count, stream)
-                 : launch_attr_paths_variant<MODE, false, true>(p, a, adjoint, block, sm_count, stream);
-  return local ? launch_attr_paths_variant<MODE, MODE != MODE_THREADED, false>(p, a, adjoint, block, sm_count, stream)
-               : launch_attr_paths_variant<MODE, false, false>(p, a, adjoint, block, sm_count, stream);
+  return p.watertight ? launch_attr_paths_wt<MODE, QUADS, true>(p, a, adjoint, block, sm_count, stream)
+                      : launch_attr_paths_wt<MODE, QUADS, false>(p, a, adjoint, block, sm_count, stream);
 }
 
-template <int MODE, bool LOCAL, bool WT>
-cudaError_t launch_attr_variant(const TraceParams& p, const AdjointParams& a, bool adjoint, uint32_t block,
-                                cudaStream_t stream) {
-  static std::atomic<uint64_t> done[2] = {};
-  const cudaError_t e = raise_smem_limit(done[adjoint], {adjoint ? (const void*)attr_adjoint_kernel<MODE, LOCAL, WT>
-                                                                 : (const void*)attr_forward_kernel<MODE, LOCAL, WT>});
+template <int PASS, int MODE, bool LOCAL, bool WT, bool SPLIT>
+cudaError_t launch_ray_lanes(const TraceParams& p, const AdjointParams& a, uint32_t block, cudaStream_t stream) {
+  static std::atomic<uint64_t> done{0};
+  const auto fn = ray_pass_kernel<PASS, MODE, LOCAL, WT, SPLIT>;
+  const cudaError_t e = raise_smem_limit(done, {(const void*)fn});
   if (e != cudaSuccess) return e;
   const size_t smem = MODE != MODE_THREADED && !LOCAL ? (size_t)p.stack_depth * block * sizeof(uint2) : 0;
-  const uint32_t grid = (a.count + block - 1) / block;
-  if (adjoint) attr_adjoint_kernel<MODE, LOCAL, WT><<<grid, block, smem, stream>>>(p, a);
-  else attr_forward_kernel<MODE, LOCAL, WT><<<grid, block, smem, stream>>>(p, a);
+  fn<<<(uint32_t)(((uint64_t)a.count + block - 1) / block), block, smem, stream>>>(p, a);
   return cudaGetLastError();
 }
 
-template <int MODE>
-cudaError_t launch_attr_mode(const TraceParams& p, const AdjointParams& a, bool adjoint, uint32_t block,
-                             cudaStream_t stream) {
-  const bool local = MODE != MODE_THREADED && p.local_stack;
-  if (p.watertight)
-    return local ? launch_attr_variant<MODE, MODE != MODE_THREADED, true>(p, a, adjoint, block, stream)
-                 : launch_attr_variant<MODE, false, true>(p, a, adjoint, block, stream);
-  return local ? launch_attr_variant<MODE, MODE != MODE_THREADED, false>(p, a, adjoint, block, stream)
-               : launch_attr_variant<MODE, false, false>(p, a, adjoint, block, stream);
-}
-
-template <int MODE, bool LOCAL, bool WT>
-cudaError_t launch_hit_diff_variant(const TraceParams& p, const AdjointParams& a, bool adjoint, uint32_t block,
-                                    cudaStream_t stream) {
-  static std::atomic<uint64_t> done[2] = {};
-  const cudaError_t e = raise_smem_limit(done[adjoint], {adjoint ? (const void*)hit_diff_adjoint_kernel<MODE, LOCAL, WT>
-                                                                 : (const void*)hit_diff_forward_kernel<MODE, LOCAL, WT>});
+template <int PASS, bool WT>
+cudaError_t launch_ray_pass_wt(const TraceParams& p, const AdjointParams& a, int mode, uint32_t block,
+                               cudaStream_t stream) {
+  if (mode == MODE_THREADED) return launch_ray_lanes<PASS, MODE_THREADED, false, WT, false>(p, a, block, stream);
+  TraceParams q = p;
+  q.stack_depth = p.stack_depth4;
+  if (!p.quads) return launch_ray_lanes<PASS, MODE_WIDE4, false, WT, false>(q, a, block, stream);
+  const QuadShareLaunch L = quad_share(a.count, q.stack_depth <= kLocalStackEntries);
+  static std::atomic<uint64_t> done{0};
+  const auto fn = ray_pass_quad_kernel<PASS, WT>;
+  const cudaError_t e = raise_smem_limit(done, {(const void*)fn});
   if (e != cudaSuccess) return e;
-  const size_t smem = MODE != MODE_THREADED && !LOCAL ? (size_t)p.stack_depth * block * sizeof(uint2) : 0;
-  const uint32_t grid = (a.count + block - 1) / block;
-  if (adjoint) hit_diff_adjoint_kernel<MODE, LOCAL, WT><<<grid, block, smem, stream>>>(p, a);
-  else hit_diff_forward_kernel<MODE, LOCAL, WT><<<grid, block, smem, stream>>>(p, a);
+  fn<<<L.grid, kShareBlock, quad_share_bytes(p.stack_depth4), stream>>>(q, a, L.share);
+  if (L.lanes) return launch_ray_lanes<PASS, MODE_WIDE4, true, WT, true>(q, a, block, stream);
   return cudaGetLastError();
 }
 
-template <int MODE>
-cudaError_t launch_hit_diff_mode(const TraceParams& p, const AdjointParams& a, bool adjoint, uint32_t block,
-                                 cudaStream_t stream) {
-  const bool local = MODE != MODE_THREADED && p.local_stack;
-  if (p.watertight)
-    return local ? launch_hit_diff_variant<MODE, MODE != MODE_THREADED, true>(p, a, adjoint, block, stream)
-                 : launch_hit_diff_variant<MODE, false, true>(p, a, adjoint, block, stream);
-  return local ? launch_hit_diff_variant<MODE, MODE != MODE_THREADED, false>(p, a, adjoint, block, stream)
-               : launch_hit_diff_variant<MODE, false, false>(p, a, adjoint, block, stream);
-}
-
-cudaError_t launch_attr(const TraceParams& p, const AdjointParams& a, int mode, bool adjoint, uint32_t block,
-                        cudaStream_t stream) {
+template <int PASS>
+cudaError_t launch_ray_pass(const TraceParams& p, const AdjointParams& a, int mode, uint32_t block,
+                            cudaStream_t stream) {
   if (a.count == 0) return cudaSuccess;
   if (block == 0) block = 64;
-  if (mode == MODE_WIDE4) return launch_attr_mode<MODE_WIDE4>(p, a, adjoint, block, stream);
-  if (mode == MODE_BINARY) return launch_attr_mode<MODE_BINARY>(p, a, adjoint, block, stream);
-  return launch_attr_mode<MODE_THREADED>(p, a, adjoint, block, stream);
+  return p.watertight ? launch_ray_pass_wt<PASS, true>(p, a, mode, block, stream)
+                      : launch_ray_pass_wt<PASS, false>(p, a, mode, block, stream);
 }
 
 }  // namespace
@@ -693,14 +655,16 @@ cudaError_t launch_attr_paths(const TraceParams& p, const PathAdjointParams& a, 
     return cudaGetLastError();
   }
   if (block == 0) block = 64;
-  if (mode == MODE_WIDE4) return launch_attr_paths_mode<MODE_WIDE4>(p, a, adjoint, block, sm_count, stream);
-  if (mode == MODE_BINARY) return launch_attr_paths_mode<MODE_BINARY>(p, a, adjoint, block, sm_count, stream);
-  return launch_attr_paths_mode<MODE_THREADED>(p, a, adjoint, block, sm_count, stream);
+  if (mode == MODE_THREADED) return launch_attr_paths_mode<MODE_THREADED, false>(p, a, adjoint, block, sm_count, stream);
+  if (p.quads) return launch_attr_paths_mode<MODE_WIDE4, true>(p, a, adjoint, block, sm_count, stream);
+  TraceParams w = p;  // too many triangles for quad_leaf_code
+  w.stack_depth = p.stack_depth4;
+  return launch_attr_paths_mode<MODE_WIDE4, false>(w, a, adjoint, block, sm_count, stream);
 }
 
 cudaError_t launch_attr_forward(const TraceParams& p, const AdjointParams& a, int mode, uint32_t block,
                                 cudaStream_t stream) {
-  return launch_attr(p, a, mode, false, block, stream);
+  return launch_ray_pass<ATTR_FORWARD>(p, a, mode, block, stream);
 }
 
 cudaError_t launch_attr_adjoint(const TraceParams& p, const AdjointParams& a, int mode, uint32_t block,
@@ -710,7 +674,7 @@ cudaError_t launch_attr_adjoint(const TraceParams& p, const AdjointParams& a, in
     attr_recorded_adjoint_kernel<<<recorded_grid(a.count, sm_count), 256, 0, stream>>>(p, a);
     return cudaGetLastError();
   }
-  return launch_attr(p, a, mode, true, block, stream);
+  return launch_ray_pass<ATTR_ADJOINT>(p, a, mode, block, stream);
 }
 
 cudaError_t launch_hit_diff(const TraceParams& p, const AdjointParams& a, int mode, bool adjoint, uint32_t block,
@@ -720,10 +684,8 @@ cudaError_t launch_hit_diff(const TraceParams& p, const AdjointParams& a, int mo
     hit_diff_recorded_adjoint_kernel<<<recorded_grid(a.count, sm_count), 256, 0, stream>>>(p, a);
     return cudaGetLastError();
   }
-  if (block == 0) block = 64;
-  if (mode == MODE_WIDE4) return launch_hit_diff_mode<MODE_WIDE4>(p, a, adjoint, block, stream);
-  if (mode == MODE_BINARY) return launch_hit_diff_mode<MODE_BINARY>(p, a, adjoint, block, stream);
-  return launch_hit_diff_mode<MODE_THREADED>(p, a, adjoint, block, stream);
+  return adjoint ? launch_ray_pass<HIT_ADJOINT>(p, a, mode, block, stream)
+                 : launch_ray_pass<HIT_FORWARD>(p, a, mode, block, stream);
 }
 
 }  // namespace rdn

@@ -123,3 +123,96 @@ def test_first_hit_queries_agree_on_hit_and_miss(cuda, n):
             res[traversal, str(kw)] = rt.hits_to_numpy(hits)["prim"] != rt.MISS
     first = next(iter(res.values()))
     assert all(np.array_equal(first, r) for r in res.values())
+
+
+def field_system(n=64):
+    m = scenes.heightfield(n, seed=4)
+    P = rt.AccelerationStructureSystem(device=0)
+    b = P.create_bottom_level_acceleration_structure([rt.BottomLevelAccelerationStructureBuildSource(m.positions, m.indices)])
+    P.bind_tlas([P.create_top_level_acceleration_structure([rt.TopLevelAccelerationStructureSourceInstance(b)])])
+    P.build(blas_bin_size=4)
+    return P, m
+
+
+def field_rays(n, seed):
+    """Stretches of camera rays and of rays in random directions into the field."""
+    w = 640
+    cam = scenes.pinhole_rays(scenes.heightfield_camera(w, -(-n // w)))[:n]
+    rnd = scenes.sphere_rays(n, (0, 0, -0.1), (1, 1, 0.4), seed=seed)
+    return np.where(((np.arange(n) + 16) // 96) % 2 == 0, cam, rnd)
+
+
+@pytest.mark.parametrize("watertight", [0, rt.INTERSECT_WATERTIGHT])
+@pytest.mark.parametrize("n", [1, 33, 47_999, 48_001, 399_999, 400_033])
+def test_differentiable_batches(cuda, n, watertight):
+    """Loss and hit query, forward and traced adjoint, against the reference order: the same hits and values; vertex
+    gradients up to the order of their f32 sums (at most m terms a vertex: m 2^-24 of the norm)."""
+    import ctypes as C
+
+    import torch
+    from rendiation_gb300 import native
+
+    P, mesh = field_system()
+    L = native.lib()
+    rays = torch.from_numpy(field_rays(n, n).view(np.float32).reshape(-1, 8).copy()).cuda()
+    g = torch.Generator(device="cuda").manual_seed(1)
+    attr = torch.rand(mesh.positions.shape[0], generator=g, device="cuda")
+    target = torch.rand(n, generator=g, device="cuda")
+    grad_hit = torch.randn((n, 4), generator=g, device="cuda")
+
+    def run(traversal, query):
+        z = lambda *s, dtype=torch.float32: torch.zeros(s, dtype=dtype, device="cuda")  # noqa: E731
+        r = dict(tri=z(n, dtype=torch.int32), inst=z(n, dtype=torch.int32), grad=z(attr.shape[0], 4), go=z(n, 3),
+                 gd=z(n, 3), loss=z(1, dtype=torch.float64), value=z(n), hit=z(n, 4))
+        base = dict(rays=rays.data_ptr(), count=n, attributes=attr.data_ptr(), traversal=traversal | watertight)
+        grads = dict(grad_vertices=r["grad"].data_ptr(), grad_ray_origin=r["go"].data_ptr(),
+                     grad_ray_direction=r["gd"].data_ptr())
+        rec = dict(hit_tri=r["tri"].data_ptr(), hit_inst=r["inst"].data_ptr())
+        if query:
+            f = native.HitDiffDesc(**base, **rec, hit=r["hit"].data_ptr())
+            a = native.HitDiffDesc(**base, **grads, grad_hit=grad_hit.data_ptr())
+            assert L.rdn_hit_diff_forward(P._h, C.byref(f), None) == 0
+            assert L.rdn_hit_diff_adjoint(P._h, C.byref(a), None) == 0
+        else:
+            f = native.AttrLossDesc(**base, **rec, targets=target.data_ptr(), ray_value=r["value"].data_ptr(),
+                                    loss_sum=r["loss"].data_ptr(), grad_scale=1.0)
+            a = native.AttrLossDesc(**base, **grads, targets=target.data_ptr(), grad_scale=1.0)
+            assert L.rdn_attr_loss_forward(P._h, C.byref(f), None) == 0
+            assert L.rdn_attr_loss_adjoint(P._h, C.byref(a), None) == 0
+        torch.cuda.synchronize()
+        return {k: v.cpu().numpy() for k, v in r.items()}
+
+    for query in (False, True):
+        want, got = run(rt.TRAVERSAL_REFERENCE, query), run(rt.TRAVERSAL_ORDERED, query)
+        same = want["tri"] == got["tri"]
+        assert np.count_nonzero(~same) <= 1 + n // 20_000  # exact-distance ties
+        for k in ("inst", "value", "hit", "go", "gd"):
+            assert np.array_equal(want[k][same], got[k][same]), k
+        if same.all():
+            assert abs(want["loss"] - got["loss"]) <= 1e-12 * np.abs(want["loss"])
+            hit = want["tri"] != -1
+            idx = mesh.indices.reshape(-1, 3)[want["tri"][hit]]
+            m = np.bincount(idx.reshape(-1), minlength=1).max() if hit.any() else 0
+            diff = np.linalg.norm(want["grad"].astype(np.float64) - got["grad"])
+            assert diff <= m * 2.0**-24 * np.linalg.norm(want["grad"].astype(np.float64))
+
+
+@pytest.mark.parametrize("n", [5, 1000, 39_999, 100_001])
+def test_path_batches(cuda, n):
+    """Paths of both executors against the reference order (a tie may send a path elsewhere)."""
+    import torch
+
+    P = soup_system([scenes.triangle_soup(k, seed=k) for k in (400, 3000, 9000)])
+    rays = torch.from_numpy(mixed_rays(n, seed=n).view(np.float32).reshape(-1, 8).copy()).cuda()
+    tidx = torch.from_numpy(np.random.default_rng(n).integers(0, 3, n).astype(np.int32)).cuda()
+    out = {}
+    for traversal in (rt.TRAVERSAL_REFERENCE, rt.TRAVERSAL_ORDERED, rt.TRAVERSAL_ORDERED_WIDE):
+        for watertight in (0, rt.INTERSECT_WATERTIGHT):
+            for sort_key in (0, 2):
+                p = rt.Paths(P, rays, tidx, max_bounces=3, seed=7, traversal=traversal | watertight, sort_key=sort_key)
+                p.run()
+                torch.cuda.synchronize()
+                out[traversal, watertight, sort_key] = p.results()
+                assert P.check_errors() == (0, 0)
+    for (traversal, watertight, sort_key), got in out.items():
+        assert np.count_nonzero(got != out[rt.TRAVERSAL_REFERENCE, watertight, 0]) <= n // 20_000
