@@ -1,13 +1,14 @@
 // Fused ambient-occlusion frame for sm_103a: the reference AO renderer's ray
 // generation, primary closest hit, occlusion ray and miss shaders
-// (feature/ao.rs:193-296) as one kernel, one thread per pixel, warps over 4x8
-// pixel tiles. It computes what the task-graph form of the same pipeline
+// (feature/ao.rs:193-296) as one kernel, one thread per pixel over 4x8 pixel
+// tiles, or four lanes per ray for frames that do not fill the chip. It computes what the task-graph form of the same pipeline
 // computes, without the task pools. Built with -fmad=false: see ao.cuh.
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
 #include "ao.cuh"
+#include "quad.cuh"
 #include "traverse.cuh"
 
 namespace rdn {
@@ -54,6 +55,65 @@ __global__ void __launch_bounds__(128) ao_kernel(TraceParams P, AoEnv A) {
   ao_accumulate(A, y * A.width + x, payload);
 }
 
+// Four lanes per ray (quad.cuh), a warp `batch` pixels, for frames of up to
+// kQuadPixels: below that the slowest warps decide a frame's time, and a warp
+// of eight or sixteen pixels is done in less than half the time of one of 32
+// (us for four samples on the 1024^2 field: 128^2 pixels, one per thread 863,
+// 8 a warp 303; 256^2 1008, 8 477, 16 520; 512^2 1275, 8 1188, 16 1085, 32
+// 1133; 1280x720 2249, 16 3139). Above it pixels that are alike share their
+// nodes better one per lane.
+constexpr uint32_t kQuadPixels = 400000;
+constexpr uint32_t ao_quad_batch(uint32_t pixels) { return pixels < 100000u ? 8u : 16u; }
+
+template <bool WT>
+__global__ void __launch_bounds__(128, 8) ao_quad_kernel(TraceParams P, AoEnv A, uint32_t batch) {
+  extern __shared__ __align__(16) unsigned char quad_smem[];
+  const QuadWarp W = quad_warp(quad_smem, P.stack_depth4);
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t x = 0, y = 0;
+  const uint32_t idx = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * batch + lane;
+  const bool valid = lane < batch && ao_pixel(A, idx, x, y);
+  RayCtx R;
+  if (valid) ao_camera_ray(A, x, y, R.o, R.d);
+  R.tmin = F32_EPSILON;
+  R.tmax = F32_MAX;
+  R.ray_flags = RAY_FLAG_CULL_BACK;
+  R.cull_mask = 0xFFFFFFFFu;
+  bool bad;
+  traverse_warp<WT>(P, R, A.tlas, valid, W, bad);
+  const bool hit = valid && R.best.have;
+  RayCtx S;
+  if (hit) {
+    float3 o, d;
+    ao_camera_ray(A, x, y, o, d);
+    S.o = o + d * R.best.t;
+    const float3 n =
+        ao_shading_normal(A, P.tlas_data + R.best.inst, __ldg(P.redirect + R.best.k), R.best.u, R.best.v, o, S.o);
+    S.d = ao_direction(n, ao_sample(A));
+  }
+  S.tmin = AO_TEST_MIN;
+  S.tmax = AO_TEST_MAX;
+  S.ray_flags = RAY_FLAG_END_SEARCH;
+  S.cull_mask = 0xFFFFFFFFu;
+  bool bad2;
+  traverse_warp<WT>(P, S, A.tlas, hit, W, bad2);
+  if (!valid) return;
+  if (bad || (hit && bad2)) atomicOr(P.error_word, 2u);
+  ao_count(A, 0, true);
+  ao_count(A, 1, hit);
+  ao_accumulate(A, y * A.width + x, hit && S.best.have ? 0.0f : 1.0f);  // 1: the camera ray or the occlusion ray missed
+}
+
+template <bool WT>
+cudaError_t launch_quads(const TraceParams& p, const AoEnv& a, uint32_t pixels, cudaStream_t st) {
+  static std::atomic<uint64_t> attr_done{0};
+  const cudaError_t e = raise_smem_limit(attr_done, {(const void*)ao_quad_kernel<WT>});
+  if (e != cudaSuccess) return e;
+  const uint32_t batch = ao_quad_batch(pixels);
+  ao_quad_kernel<WT><<<(pixels + batch - 1) / batch, 32, quad_warp_bytes(p.stack_depth4), st>>>(p, a, batch);
+  return cudaGetLastError();
+}
+
 template <int MODE, bool LOCAL, bool WT>
 cudaError_t launch_variant_wt(const TraceParams& p, const AoEnv& a, cudaStream_t st) {
   const uint32_t block = a.block ? a.block : 128;
@@ -82,6 +142,9 @@ cudaError_t launch_ao_advance(uint32_t* counter, cudaStream_t st) {
 
 cudaError_t launch_ao(const TraceParams& p, const AoEnv& a, int mode, cudaStream_t st) {
   if (a.width == 0 || a.height == 0) return cudaSuccess;
+  const uint32_t pixels = ao_dispatch_count(a.width, a.height);
+  if (mode != MODE_THREADED && p.quads && pixels <= kQuadPixels)
+    return p.watertight ? launch_quads<true>(p, a, pixels, st) : launch_quads<false>(p, a, pixels, st);
   if (mode == MODE_WIDE4)
     return p.local_stack ? launch_variant<MODE_WIDE4, true>(p, a, st) : launch_variant<MODE_WIDE4, false>(p, a, st);
   if (mode == MODE_BINARY)

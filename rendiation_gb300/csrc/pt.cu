@@ -22,6 +22,7 @@
 #include <cstdint>
 
 #include "pt.cuh"
+#include "quad.cuh"
 #include "traverse.cuh"
 
 namespace rdn {
@@ -264,6 +265,69 @@ __global__ void __launch_bounds__(128, pt_min_blocks(TIER)) pt_refill_kernel(Tra
   pt_count(E, core, shadow);
 }
 
+// The same with four lanes per ray (quad.cuh), a warp `batch` paths at a time,
+// for frames of up to kQuadPixels: fewer do not fill the chip one path per
+// lane, and the warp's rays (camera, bounce and shadow ones of different
+// paths) differ. Us for two samples of depth 3 on the 1024^2 field: 128^2
+// pixels, one path per lane 786, 8 a warp 358, 16 447; 256^2 1029, 16 645, 8
+// 662; 682x384 1281, 32 1153, 16 1317; 1280x720 2545, 32 2906. 72 registers (7
+// blocks): 64 and 80 took 1192 and 1169 us at 682x384.
+constexpr uint32_t kQuadPixels = 400000;
+template <bool WT>
+__global__ void __launch_bounds__(128, 7) pt_refill_quad_kernel(TraceParams P, PtEnv E, uint32_t total, uint32_t batch) {
+  extern __shared__ __align__(16) unsigned char quad_smem[];
+  const QuadWarp W = quad_warp(quad_smem, P.stack_depth4);
+  __shared__ float stash[kPtStash][128];
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t sample = ao_sample(E.view);
+  PtPath q;
+  bool active = false, exhausted = false, bad = false;
+  uint32_t core = 0, shadow = 0;
+  for (;;) {
+    // lanes without a path take the next dispatch indices, one atomic per warp
+    const bool need = lane < batch && !active && !exhausted;
+    const uint32_t m = __ballot_sync(0xffffffffu, need);
+    if (m) {
+      const uint32_t leader = __ffs(m) - 1u;
+      uint32_t base = 0;
+      if (lane == leader) base = atomicAdd(E.fetch, __popc(m));
+      base = __shfl_sync(0xffffffffu, base, leader);
+      if (need) {
+        const uint32_t idx = base + __popc(m & ((1u << lane) - 1u));
+        uint32_t x, y;
+        if (idx >= total) {
+          exhausted = true;
+        } else if (ao_pixel(E.view, idx, x, y)) {
+          pt_begin(E, q, x, y);
+          if (E.max_depth == 0u) pt_finish(E, q);  // a path of no rays resolves at once
+          else active = true;
+        }
+      }
+    }
+    if (!__any_sync(0xffffffffu, active)) {
+      if (__all_sync(0xffffffffu, exhausted || lane >= batch)) break;
+      continue;
+    }
+    RayCtx R;
+    pt_ray(q, R);
+    if (active) pt_park(stash, q);
+    bool b;
+    traverse_warp<WT>(P, R, E.view.tlas, active, W, b);
+    if (active) {
+      bad |= b;
+      pt_unpark(stash, q);
+      if (pt_advance(P, E, sample, q, R)) {
+        pt_finish(E, q);
+        core += q.core;
+        shadow += q.shadow;
+        active = false;
+      }
+    }
+  }
+  if (bad) atomicOr(P.error_word, 2u);
+  pt_count(E, core, shadow);
+}
+
 // ---- wavefront schedule ----
 // Path state word-major (word k of pixel i at state[k * n_pix + i]):
 // o 0-2, d 3-5, throughput 6-8, radiance 9-11, shading normal 12-14,
@@ -431,6 +495,27 @@ cudaError_t launch_refill(const TraceParams& p, const PtEnv& e, int sm_count, ui
   return cudaGetLastError();
 }
 
+template <bool WT>
+cudaError_t launch_refill_quads(const TraceParams& p, const PtEnv& e, int sm_count, cudaStream_t st) {
+  constexpr uint32_t block = 128;
+  static std::atomic<uint64_t> attr_done{0};
+  cudaError_t err = raise_smem_limit(attr_done, {(const void*)pt_refill_quad_kernel<WT>});
+  if (err != cudaSuccess) return err;
+  const size_t smem = (size_t)quad_warp_bytes(p.stack_depth4) * (block / 32);
+  int per_sm = 0;
+  err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pt_refill_quad_kernel<WT>, (int)block, smem);
+  if (err != cudaSuccess) return err;
+  if (per_sm < 1) per_sm = 1;
+  const uint32_t total = ao_dispatch_count(e.view.width, e.view.height), batch = quad_batch(total);
+  uint32_t grid = (uint32_t)((sm_count > 0 ? sm_count : 1) * per_sm);
+  const uint32_t per = batch * (block / 32), need = (total + per - 1) / per;
+  if (grid > need) grid = need;
+  err = cudaMemsetAsync(e.fetch, 0, 4, st);
+  if (err != cudaSuccess) return err;
+  pt_refill_quad_kernel<WT><<<grid, block, smem, st>>>(p, e, total, batch);
+  return cudaGetLastError();
+}
+
 template <int MODE, bool LOCAL, bool WT>
 cudaError_t launch_variant_wt(const TraceParams& p, const PtEnv& e, const PtWave* w, int sm_count, cudaStream_t st) {
   const uint32_t block = e.view.block ? e.view.block : 128;
@@ -450,6 +535,8 @@ cudaError_t launch_variant_wt(const TraceParams& p, const PtEnv& e, const PtWave
     pt_kernel<MODE, LOCAL, WT><<<(total + block - 1) / block, block, smem, st>>>(p, e);
     return cudaGetLastError();
   }
+  if constexpr (MODE != MODE_THREADED)
+    if (p.quads && total <= kQuadPixels) return launch_refill_quads<WT>(p, e, sm_count, st);
   // register tiers apply to the local-stack walks
   if constexpr (LOCAL) {
     if (e.register_tier == 1) return launch_refill<MODE, LOCAL, WT, 1>(p, e, sm_count, block, smem, st);

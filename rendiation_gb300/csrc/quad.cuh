@@ -105,7 +105,6 @@ __device__ __forceinline__ bool coherent_warp(const RayCtx& R, uint32_t tidx, bo
 template <bool WT>
 __device__ __forceinline__ void quad_walk(const TraceParams& p, const QuadWarp& W, uint32_t n) {
   const uint32_t lane = threadIdx.x & 31u, l = lane & 3u, qb = lane & ~3u;
-  const uint32_t depth = p.stack_depth4;
   uint2* const stack = W.stack + (lane >> 2);
   uint32_t next = 0;
   if (l == 0u) stack[0] = make_uint2(EMPTY_SLOT, 0x7f800000u);

@@ -216,3 +216,35 @@ def test_path_batches(cuda, n):
                 assert P.check_errors() == (0, 0)
     for (traversal, watertight, sort_key), got in out.items():
         assert np.count_nonzero(got != out[rt.TRAVERSAL_REFERENCE, watertight, 0]) <= n // 20_000
+
+
+@pytest.mark.parametrize("width,height", [(7, 5), (316, 312), (316, 320), (632, 632), (640, 640)])
+def test_frames_of_both_walks(cuda, width, height):
+    """AO and path-traced frames on either side of the sizes where their walks change, against the reference order:
+    the same texels, except where a ray meets two triangles at exactly the same distance."""
+    import torch
+
+    from rendiation_gb300 import path_tracing as pt
+    from rendiation_gb300 import task_graph as tg
+
+    P, _ = field_system(128)
+    eye = (0.5, -0.4, 0.6)
+    vp = tg.look_at_view_projection_inv(eye, (0.5, 0.5, 0.0), (0, 0, 1), 40.0, width / height)
+    lights = [pt.directional_light((3.0, 2.5, 2.0), (0.3, 0.2, -1.0))]
+    images = {}
+    for traversal in (rt.TRAVERSAL_REFERENCE, rt.TRAVERSAL_ORDERED, rt.TRAVERSAL_ORDERED_WIDE):
+        ao = tg.AmbientOcclusion(P, width, height, vp, eye, traversal=traversal)
+        ao.sample_count = 200
+        ao.render()
+        R = pt.DeviceReferencePathTracingRenderer(P, width, height, vp, eye, lights=lights, traversal=traversal,
+                                                  background_color=(0.3, 0.4, 0.6), count_rays=True)
+        R.render()
+        torch.cuda.synchronize()
+        images[traversal] = ao.result().copy(), R.result().copy(), R.rays_traced()
+    want = images[rt.TRAVERSAL_REFERENCE]
+    n = width * height
+    for traversal in (rt.TRAVERSAL_ORDERED, rt.TRAVERSAL_ORDERED_WIDE):
+        for k in (0, 1):
+            assert np.count_nonzero((images[traversal][k] != want[k]).any(-1)) <= n // 20_000
+        assert all(abs(a - b) <= 3 * (n // 20_000) for a, b in zip(images[traversal][2], want[2]))
+    assert P.check_errors() == (0, 0)
