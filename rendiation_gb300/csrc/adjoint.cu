@@ -623,10 +623,9 @@ template <int PASS, bool WT>
 cudaError_t launch_ray_pass_wt(const TraceParams& p, const AdjointParams& a, int mode, uint32_t block,
                                cudaStream_t stream) {
   if (mode == MODE_THREADED) return launch_ray_lanes<PASS, MODE_THREADED, false, WT, false>(p, a, block, stream);
-  TraceParams q = p;
-  q.stack_depth = p.stack_depth4;
-  if (!p.quads) return launch_ray_lanes<PASS, MODE_WIDE4, false, WT, false>(q, a, block, stream);
-  const QuadShareLaunch L = quad_share(a.count, q.stack_depth <= kLocalStackEntries);
+  const TraceParams q = wide4_params(p);
+  if (!p.packed) return launch_ray_lanes<PASS, MODE_WIDE4, false, WT, false>(q, a, block, stream);
+  const QuadShareLaunch L = quad_share(a.count, q.local_stack != 0);
   static std::atomic<uint64_t> done{0};
   const auto fn = ray_pass_quad_kernel<PASS, WT>;
   const cudaError_t e = raise_smem_limit(done, {(const void*)fn});
@@ -656,10 +655,8 @@ cudaError_t launch_attr_paths(const TraceParams& p, const PathAdjointParams& a, 
   }
   if (block == 0) block = 64;
   if (mode == MODE_THREADED) return launch_attr_paths_mode<MODE_THREADED, false>(p, a, adjoint, block, sm_count, stream);
-  if (p.quads) return launch_attr_paths_mode<MODE_WIDE4, true>(p, a, adjoint, block, sm_count, stream);
-  TraceParams w = p;  // too many triangles for quad_leaf_code
-  w.stack_depth = p.stack_depth4;
-  return launch_attr_paths_mode<MODE_WIDE4, false>(w, a, adjoint, block, sm_count, stream);
+  if (p.packed) return launch_attr_paths_mode<MODE_WIDE4, true>(p, a, adjoint, block, sm_count, stream);
+  return launch_attr_paths_mode<MODE_WIDE4, false>(wide4_params(p), a, adjoint, block, sm_count, stream);
 }
 
 cudaError_t launch_attr_forward(const TraceParams& p, const AdjointParams& a, int mode, uint32_t block,

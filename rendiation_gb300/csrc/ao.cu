@@ -143,13 +143,12 @@ cudaError_t launch_ao_advance(uint32_t* counter, cudaStream_t st) {
 cudaError_t launch_ao(const TraceParams& p, const AoEnv& a, int mode, cudaStream_t st) {
   if (a.width == 0 || a.height == 0) return cudaSuccess;
   const uint32_t pixels = ao_dispatch_count(a.width, a.height);
-  if (mode != MODE_THREADED && p.quads && pixels <= kQuadPixels)
+  if (mode != MODE_THREADED && p.packed && pixels <= kQuadPixels)
     return p.watertight ? launch_quads<true>(p, a, pixels, st) : launch_quads<false>(p, a, pixels, st);
-  if (mode == MODE_WIDE4)
-    return p.local_stack ? launch_variant<MODE_WIDE4, true>(p, a, st) : launch_variant<MODE_WIDE4, false>(p, a, st);
-  if (mode == MODE_BINARY)
-    return p.local_stack ? launch_variant<MODE_BINARY, true>(p, a, st)
-                         : launch_variant<MODE_BINARY, false>(p, a, st);
+  if (mode != MODE_THREADED) {
+    const TraceParams q = wide4_params(p);
+    return q.local_stack ? launch_variant<MODE_WIDE4, true>(q, a, st) : launch_variant<MODE_WIDE4, false>(q, a, st);
+  }
   return launch_variant<MODE_THREADED, false>(p, a, st);
 }
 

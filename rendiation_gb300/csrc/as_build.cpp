@@ -371,6 +371,7 @@ uint32_t emit_wide4(const Tree& t, uint32_t bi, const std::vector<uint32_t>& cod
     const TreeNode& c = t.nodes[slot[k]];
     codes[k] = c.left_count ? emit_wide4(t, slot[k], code2, hb, level + 1, depth) : code2[slot[k]];
   }
+  const bool packed = hb.indices_redirect.size() < kPackedTriangles;
   Wide4Node& w = hb.wide4_nodes[me];
   for (int k = 0; k < 4; k++) {
     const bool used = k < n;
@@ -382,11 +383,11 @@ uint32_t emit_wide4(const Tree& t, uint32_t bi, const std::vector<uint32_t>& cod
     w.child[k].hi_y = b.hi.y;
     w.child[k].hi_z = b.hi.z;
     w.child[k].code = codes[k];
-    w.child[k].quad = codes[k];
-    if (used && (codes[k] & LEAF_BIT)) {
+    if (used && packed && (codes[k] & LEAF_BIT)) {
       const uint32_t l = codes[k] & ~LEAF_BIT;
-      w.child[k].quad = quad_leaf_code(l, hb.leaf_ranges[2 * (size_t)l], hb.leaf_ranges[2 * (size_t)l + 1]);
+      w.child[k].code = packed_leaf(l, hb.leaf_ranges[2 * (size_t)l], hb.leaf_ranges[2 * (size_t)l + 1]);
     }
+    w.child[k].pad = 0;
   }
   return me;
 }

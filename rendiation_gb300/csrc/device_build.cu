@@ -868,7 +868,7 @@ __global__ void wide4_mark_kernel(uint32_t lb, uint32_t W, const BNode* __restri
     }
 }
 
-__global__ void wide4_emit_kernel(uint32_t T, const BNode* __restrict__ pool, const uint32_t* __restrict__ croot,
+__global__ void wide4_emit_kernel(uint32_t T, bool packed, const BNode* __restrict__ pool, const uint32_t* __restrict__ croot,
                                   const uint32_t* __restrict__ index4, const uint32_t* __restrict__ pre,
                                   const uint32_t* __restrict__ rank, Wide4Node* __restrict__ out) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -885,14 +885,15 @@ __global__ void wide4_emit_kernel(uint32_t T, const BNode* __restrict__ pool, co
     w.child[k].hi_x = b.hi.x;
     w.child[k].hi_y = b.hi.y;
     w.child[k].hi_z = b.hi.z;
+    w.child[k].pad = 0;
     if (!used) {
-      w.child[k].code = w.child[k].quad = EMPTY_SLOT;
+      w.child[k].code = EMPTY_SLOT;
     } else if (pool[slot[k]].left != NONE) {
-      w.child[k].code = w.child[k].quad = index4[slot[k]];
+      w.child[k].code = index4[slot[k]];
     } else {
       const uint32_t g = pre[slot[k]];
-      w.child[k].code = LEAF_BIT | (g - rank[g]);
-      w.child[k].quad = quad_leaf_code(g - rank[g], pool[slot[k]].start, pool[slot[k]].end);
+      const uint32_t leaf = g - rank[g];
+      w.child[k].code = packed ? packed_leaf(leaf, pool[slot[k]].start, pool[slot[k]].end) : (LEAF_BIT | leaf);
     }
   }
   out[index4[i]] = w;
@@ -1255,7 +1256,7 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
   uint32_t tail4[3] = {0, 0, 0};  // index4[T-1], croot[T-1], deepest level
   CK(cudaStreamWaitEvent(st, side.join, 0));
   if (T) {
-    wide4_emit_kernel<<<blocks_for(T), kBlock, 0, st>>>(T, pool, croot, index4, pre, rank, d.wide4_nodes.ptr);
+    wide4_emit_kernel<<<blocks_for(T), kBlock, 0, st>>>(T, N < kPackedTriangles, pool, croot, index4, pre, rank, d.wide4_nodes.ptr);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(&tail4[0], index4 + (T - 1), 4, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(&tail4[1], croot + (T - 1), 4, cudaMemcpyDeviceToHost, st));

@@ -101,7 +101,7 @@ __device__ __forceinline__ bool shade_path(const TraceParams& p, const PathParam
 }
 
 // One bounce, a ray per lane: the reference order, and structures too large
-// for quad_leaf_code.
+// for packed_leaf.
 template <int MODE, bool LOCAL, bool WT>
 __global__ void __launch_bounds__(128) path_kernel(TraceParams p, PathParams q, uint32_t bounce, bool from_user,
                                                    const float4* __restrict__ in_rays,
@@ -367,21 +367,19 @@ enum PathVariant { PATH_LANES = 0, PATH_DYNAMIC = 1, PATH_QUADS = 2 };
 int path_variant(int mode, const TraceParams& p, const PathParams& q) {
   if (mode == MODE_THREADED) return PATH_LANES;
   if (q.refill != 0) return PATH_DYNAMIC;
-  return p.quads ? PATH_QUADS : PATH_LANES;
+  return p.packed ? PATH_QUADS : PATH_LANES;
 }
 // shared memory of a block: the variant's stacks
 size_t path_smem(int mode, int variant, const TraceParams& p, uint32_t block) {
   if (variant == PATH_QUADS) return (size_t)quad_warp_bytes(p.stack_depth4) * (block / 32);
-  return mode == MODE_THREADED ? 0 : (size_t)p.stack_depth * block * sizeof(uint2);
+  return mode == MODE_THREADED ? 0 : (size_t)p.stack_depth4 * block * sizeof(uint2);
 }
 using PathKernel = void (*)(TraceParams, PathParams, uint32_t, bool, const float4*, const uint4*, float4*, uint4*);
 template <bool WT>
 PathKernel path_fn_wt(int mode, int variant) {
   if (mode == MODE_THREADED) return path_kernel<MODE_THREADED, false, WT>;
   if (variant == PATH_QUADS) return path_quad_kernel<WT>;
-  if (mode == MODE_WIDE4)
-    return variant == PATH_DYNAMIC ? path_dynamic_kernel<MODE_WIDE4, WT> : path_kernel<MODE_WIDE4, false, WT>;
-  return variant == PATH_DYNAMIC ? path_dynamic_kernel<MODE_BINARY, WT> : path_kernel<MODE_BINARY, false, WT>;
+  return variant == PATH_DYNAMIC ? path_dynamic_kernel<MODE_WIDE4, WT> : path_kernel<MODE_WIDE4, false, WT>;
 }
 PathKernel path_fn(int mode, int variant, bool wt) {
   return wt ? path_fn_wt<true>(mode, variant) : path_fn_wt<false>(mode, variant);
@@ -416,6 +414,7 @@ cudaError_t record_paths(const TraceParams& p, const PathParams& q, int mode, ui
   const int variant = path_variant(mode, p, q);
   const size_t smem = path_smem(mode, variant, p, block);
   const PathKernel fn = path_fn(mode, variant, p.watertight != 0);
+  const TraceParams walk = mode == MODE_THREADED ? p : wide4_params(p);
   cudaError_t e = cudaMemsetAsync(q.queue_count, 0, sizeof(uint32_t) * 2 * (q.max_bounces + 1), stream);
   if (e != cudaSuccess) return e;
   float4* ra = static_cast<float4*>(q.rays_a);
@@ -455,7 +454,7 @@ cudaError_t record_paths(const TraceParams& p, const PathParams& q, int mode, ui
       out_r = (b & 1) ? ra : rb;
       out_s = (b & 1) ? sa : sb;
     }
-    fn<<<grid, block, smem, stream>>>(p, q, b, from_user, in_r, in_s, out_r, out_s);
+    fn<<<grid, block, smem, stream>>>(walk, q, b, from_user, in_r, in_s, out_r, out_s);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }

@@ -536,7 +536,7 @@ cudaError_t launch_variant_wt(const TraceParams& p, const PtEnv& e, const PtWave
     return cudaGetLastError();
   }
   if constexpr (MODE != MODE_THREADED)
-    if (p.quads && total <= kQuadPixels) return launch_refill_quads<WT>(p, e, sm_count, st);
+    if (p.packed && total <= kQuadPixels) return launch_refill_quads<WT>(p, e, sm_count, st);
   // register tiers apply to the local-stack walks
   if constexpr (LOCAL) {
     if (e.register_tier == 1) return launch_refill<MODE, LOCAL, WT, 1>(p, e, sm_count, block, smem, st);
@@ -577,12 +577,11 @@ PtWave pt_wave_layout(void* scratch, uint32_t width, uint32_t height) {
 
 cudaError_t launch_pt(const TraceParams& p, const PtEnv& e, const PtWave* w, int mode, int sm_count, cudaStream_t st) {
   if (e.view.width == 0 || e.view.height == 0) return cudaSuccess;
-  if (mode == MODE_WIDE4)
-    return p.local_stack ? launch_variant<MODE_WIDE4, true>(p, e, w, sm_count, st)
-                         : launch_variant<MODE_WIDE4, false>(p, e, w, sm_count, st);
-  if (mode == MODE_BINARY)
-    return p.local_stack ? launch_variant<MODE_BINARY, true>(p, e, w, sm_count, st)
-                         : launch_variant<MODE_BINARY, false>(p, e, w, sm_count, st);
+  if (mode != MODE_THREADED) {
+    const TraceParams q = wide4_params(p);
+    return q.local_stack ? launch_variant<MODE_WIDE4, true>(q, e, w, sm_count, st)
+                         : launch_variant<MODE_WIDE4, false>(q, e, w, sm_count, st);
+  }
   return launch_variant<MODE_THREADED, false>(p, e, w, sm_count, st);
 }
 

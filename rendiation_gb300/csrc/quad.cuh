@@ -175,7 +175,7 @@ __device__ __forceinline__ void quad_walk(const TraceParams& p, const QuadWarp& 
         const uint32_t hits = (__ballot_sync(kFullWarp, hit) >> qb) & 15u;
         // the farthest lowest
         const uint32_t row = sp + 1u + (uint32_t)(k1 > key) + (uint32_t)(k2 > key) + (uint32_t)(k3 > key);
-        if (hit) stack[row * kQuads] = make_uint2(c.quad, __float_as_uint(tn));
+        if (hit) stack[row * kQuads] = make_uint2(c.code, __float_as_uint(tn));
         sp += __popc(hits);
         __syncwarp();
       }
@@ -185,14 +185,9 @@ __device__ __forceinline__ void quad_walk(const TraceParams& p, const QuadWarp& 
     if (__any_sync(kFullWarp, leaf != EMPTY_SLOT)) {
       uint32_t k = 0, ke = 0;
       if (leaf != EMPTY_SLOT) {
-        const uint32_t count = (leaf >> kLeafCountShift) & kLeafCountMask;
-        k = leaf & kLeafStartMask;
-        ke = k + count;
-        if (count == 0u) {  // a leaf of another size: by its range
-          const uint2 lr = __ldg(p.leaves + k);
-          k = lr.x;
-          ke = lr.y;
-        }
+        const uint2 lr = packed_range(p, leaf);
+        k = lr.x;
+        ke = lr.y;
       }
       leaf = EMPTY_SLOT;
       bool ended = false;
@@ -259,14 +254,6 @@ __device__ __forceinline__ void quad_walk(const TraceParams& p, const QuadWarp& 
   }
 }
 
-// Quad code of a geometry's root.
-__device__ __forceinline__ uint32_t quad_root(const TraceParams& p, uint32_t g) {
-  const uint32_t code = __ldg(p.geom_root_code4 + g);
-  if (!(code & LEAF_BIT)) return code;
-  const uint2 lr = __ldg(p.leaves + (code & ~LEAF_BIT));
-  return quad_leaf_code(code & ~LEAF_BIT, lr.x, lr.y);
-}
-
 // Where a lane's ray stands in its TLAS walk.
 struct TlasCursor {
   uint32_t node, ti, ti_end, inst, g, g_end;
@@ -292,7 +279,7 @@ __device__ __forceinline__ bool quad_enter(const TraceParams& p, const RayCtx& R
         continue;
       s.a = make_float4(ir.o.x, ir.o.y, ir.o.z, R.tmin);
       s.b = make_float4(ir.d.x, ir.d.y, ir.d.z, ir.scaling);
-      s.c = make_uint4(quad_root(p, g), __float_as_uint(R.far_world),
+      s.c = make_uint4(wide4_root(p, g), __float_as_uint(R.far_world),
                        (is_opaque ? QB_OPAQUE : 0u) | (cull_enable ? QB_CULL : 0u) | (cull_back ? QB_CULL_BACK : 0u) |
                            ((ir.flags & TF_END_SEARCH) ? QB_END : 0u) | ((gm.z & 1u) ? QB_ODD_START : 0u),
                        0u);

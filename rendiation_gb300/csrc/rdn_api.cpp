@@ -221,7 +221,7 @@ rdn_status fill_params(rdn_ctx* c, const rdn_trace_desc* desc, rdn::TraceParams&
   p.anyhit_mask = desc->anyhit_mask;
   p.stack_depth = rdn::stack_entries(mode_of(desc->traversal), d.max_blas_depth, d.max_wide4_depth);
   p.stack_depth4 = rdn::stack_entries(rdn::MODE_WIDE4, d.max_blas_depth, d.max_wide4_depth);
-  p.quads = d.indices_redirect.count < rdn::kQuadTriangles;
+  p.packed = d.indices_redirect.count < rdn::kPackedTriangles;
   p.n_binding = (uint32_t)d.tlas_binding.count;
   p.n_tlas_root = (uint32_t)d.tlas_bvh_root.count;
   p.tlas_binding = d.tlas_binding.ptr;

@@ -106,14 +106,14 @@ static_assert(sizeof(WideNode) == 64, "64 B node");
 static const uint32_t LEAF_BIT = 0x80000000u;
 // Four-child node, 128 B, one 32 B child after the other: a child is one 32 B
 // load, its planes in the pairs that the packed box test takes.
-// code: bit 31 clear = index of a child Wide4Node, set = index of a leaf range,
+// code: bit 31 clear = index of a child Wide4Node, set = a leaf (packed_leaf;
+// the index of its range in a structure of kPackedTriangles or more),
 // EMPTY_SLOT = unused slot (its box is NaN, which no slab test passes). Children are binary-tree nodes collapsed from the
 // reference's SAH tree (the inner child with the largest surface area is opened
 // until four slots are used); every child box is an exact reference node box.
 struct Wide4Child {
   float lo_x, lo_y, hi_x, hi_y, lo_z, hi_z;
-  uint32_t code;
-  uint32_t quad;  // what a quad's stack holds of it (quad.cuh): the inner child's index, or quad_leaf_code
+  uint32_t code, pad;
 };
 struct Wide4Node {
   Wide4Child child[4];
@@ -121,15 +121,15 @@ struct Wide4Node {
 static_assert(sizeof(Wide4Node) == 128, "128 B node");
 static const uint32_t EMPTY_SLOT = 0xFFFFFFFFu;
 
-// A leaf as a quad's stack holds it, so that no leaf range is looked up on the
-// way to its triangles: bit 31, three bits of count and the first triangle
-// (sorted order); count 0 is a leaf of none or more than seven triangles, with
-// its leaf index in place of the first triangle. EMPTY_SLOT would be the last
-// seven triangles of 2^28: structures of kQuadTriangles and more are walked
-// one ray per lane.
+// A leaf of the four-child tree, so that no range is looked up on the way to
+// its triangles: bit 31, three bits of count and the first triangle (sorted
+// order); count 0 is a leaf of none or more than seven triangles, with its leaf
+// index in place of the first triangle. Structures of kPackedTriangles and more
+// hold plain leaf indices (EMPTY_SLOT would be the last triangles of 2^28) and
+// are walked one ray per lane.
 static const uint32_t kLeafCountShift = 28, kLeafCountMask = 7, kLeafStartMask = (1u << 28) - 1;
-static const uint64_t kQuadTriangles = (1ull << 28) - 8;
-__host__ __device__ inline uint32_t quad_leaf_code(uint32_t leaf, uint32_t start, uint32_t end) {
+static const uint64_t kPackedTriangles = (1ull << 28) - 8;
+__host__ __device__ inline uint32_t packed_leaf(uint32_t leaf, uint32_t start, uint32_t end) {
   const uint32_t count = end - start;
   return LEAF_BIT | (count >= 1u && count <= kLeafCountMask ? count << kLeafCountShift | (start & kLeafStartMask)
                                                            : (leaf & kLeafStartMask));

@@ -190,10 +190,9 @@ cudaError_t launch_trace(const TraceParams& p, int mode, bool counted, uint32_t 
   if (counted)
     return mode == MODE_WIDE4 ? launch_lanes<MODE_WIDE4, true, false>(p, block, stream)
                               : launch_lanes<MODE_BINARY, true, false>(p, block, stream);
-  TraceParams q = p;
-  q.stack_depth = q.stack_depth4;
-  const bool local = q.stack_depth <= kLocalStackEntries;
-  if (!p.quads) return local ? launch_lanes<MODE_WIDE4, false, true>(q, block, stream)
+  const TraceParams q = wide4_params(p);
+  const bool local = q.local_stack != 0;
+  if (!p.packed) return local ? launch_lanes<MODE_WIDE4, false, true>(q, block, stream)
                              : launch_lanes<MODE_WIDE4, false, false>(q, block, stream);
   if (p.count < kQuadSplit) return launch_quads(q, 8, 0, stream);
   if (p.count < kLaneSplit || !local) return launch_quads(q, p.count < kQuadBatch32 ? 16 : 32, 2, stream);

@@ -396,7 +396,7 @@ __device__ __forceinline__ void push_entry(const TraceParams& p, uint2* stack, u
 // A child of a four-child node (Wide4Child): one 32 B load.
 struct Wide4Load {
   float2 lo_xy, hi_xy, z;  // z = (lo, hi)
-  uint32_t code, quad;
+  uint32_t code;
 };
 __device__ __forceinline__ Wide4Load load_wide4(const float4* w) {
   float a, b, c, d, e, f;
@@ -404,7 +404,7 @@ __device__ __forceinline__ Wide4Load load_wide4(const float4* w) {
   asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
       : "=f"(a), "=f"(b), "=f"(c), "=f"(d), "=f"(e), "=f"(f), "=r"(g), "=r"(h)
       : "l"(w));
-  return Wide4Load{make_float2(a, b), make_float2(c, d), make_float2(e, f), g, h};
+  return Wide4Load{make_float2(a, b), make_float2(c, d), make_float2(e, f), g};
 }
 // The same where `want`; zeros otherwise (no branch around the load).
 __device__ __forceinline__ Wide4Load load_wide4_if(const float4* w, bool want) {
@@ -414,7 +414,7 @@ __device__ __forceinline__ Wide4Load load_wide4_if(const float4* w, bool want) {
       " @p ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n}"
       : "+f"(a), "+f"(b), "+f"(c), "+f"(d), "+f"(e), "+f"(f), "+r"(g), "+r"(h)
       : "l"(w), "r"((uint32_t)want));
-  return Wide4Load{make_float2(a, b), make_float2(c, d), make_float2(e, f), g, h};
+  return Wide4Load{make_float2(a, b), make_float2(c, d), make_float2(e, f), g};
 }
 
 // slab() on packed pairs of planes: the same subtractions and products (a - b
@@ -448,6 +448,26 @@ __device__ __forceinline__ void wide4_child(const float4* __restrict__ w, const 
     t = tn;
     code = c.code;
   }
+}
+
+// Sorted triangles [x, y) of a packed leaf.
+__device__ __forceinline__ uint2 packed_range(const TraceParams& p, uint32_t leaf) {
+  const uint32_t count = (leaf >> kLeafCountShift) & kLeafCountMask, k = leaf & kLeafStartMask;
+  if (count == 0u) return __ldg(p.leaves + k);  // a leaf of another size: by its range
+  return make_uint2(k, k + count);
+}
+// The same of a leaf code met by an ordered walk.
+template <int WIDTH>
+__device__ __forceinline__ uint2 leaf_range(const TraceParams& p, uint32_t leaf) {
+  if (WIDTH == 4 && p.packed) return packed_range(p, leaf);
+  return __ldg(p.leaves + (leaf & ~LEAF_BIT));
+}
+// Four-child code of a geometry's root.
+__device__ __forceinline__ uint32_t wide4_root(const TraceParams& p, uint32_t g) {
+  const uint32_t code = __ldg(p.geom_root_code4 + g);
+  if (!(code & LEAF_BIT) || !p.packed) return code;
+  const uint2 lr = __ldg(p.leaves + (code & ~LEAF_BIT));
+  return packed_leaf(code & ~LEAF_BIT, lr.x, lr.y);
 }
 
 // One interior-node step of the ordered walk: tests the children of node
@@ -521,7 +541,7 @@ __device__ __forceinline__ bool blas_speculative(const TraceParams& p, RayCtx& R
     if (!slab<WT>(ir.o, ir.inv_d, R.tmin * ir.scaling, R.far_world * ir.scaling, a.x, a.y, a.z, b.x, b.y, b.z, tn))
       return false;
   }
-  uint32_t code = __ldg((WIDTH == 2 ? p.geom_root_code : p.geom_root_code4) + gslot);
+  uint32_t code = WIDTH == 2 ? __ldg(p.geom_root_code + gslot) : wide4_root(p, gslot);
   float code_tn = -__int_as_float(0x7f800000);
   uint32_t leaf = EMPTY_SLOT;
   uint32_t sp = 0;
@@ -540,7 +560,7 @@ __device__ __forceinline__ bool blas_speculative(const TraceParams& p, RayCtx& R
       if ((uint32_t)__popc(__ballot_sync(__activemask(), leaf == EMPTY_SLOT)) <= p.spec_threshold) break;
     }
     while (leaf != EMPTY_SLOT) {
-      const uint2 lr = __ldg(p.leaves + (leaf & ~LEAF_BIT));
+      const uint2 lr = leaf_range<WIDTH>(p, leaf);
       if (leaf_triangles<COUNT, AH, WT>(p, R, ir, lr.x, lr.y, gslot, inst_slot, is_opaque, cull_enable, cull_back,
                                         prim_start, anyhit))
         return true;
@@ -736,7 +756,7 @@ struct LaneWalk {
           float tn;
           if (!slab<WT>(ir.o, ir.inv_d, R.tmin * ir.scaling, R.far_world * ir.scaling, a.x, a.y, a.z, b.x, b.y, b.z, tn))
             continue;
-          code = __ldg((WIDTH == 2 ? p.geom_root_code : p.geom_root_code4) + cur);
+          code = WIDTH == 2 ? __ldg(p.geom_root_code + cur) : wide4_root(p, cur);
           code_tn = -inf;
           leaf = EMPTY_SLOT;
           sp = 0;
@@ -777,7 +797,7 @@ struct LaneWalk {
         if ((uint32_t)__popc(__ballot_sync(__activemask(), leaf == EMPTY_SLOT)) <= p.spec_threshold) break;
       }
       while (leaf != EMPTY_SLOT) {
-        const uint2 lr = __ldg(p.leaves + (leaf & ~LEAF_BIT));
+        const uint2 lr = leaf_range<WIDTH>(p, leaf);
         if (leaf_triangles<false, BuiltinAnyHit, WT>(p, R, ir, lr.x, lr.y, gslot, inst_slot, is_opaque, cull_enable, cull_back,
                                   prim_start)) {
           code = leaf = EMPTY_SLOT;
