@@ -31,6 +31,7 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "quad.cuh"
 #include "shade.cuh"
 #include "traverse.cuh"
 #include "wavefront.h"
@@ -60,6 +61,108 @@ __device__ __forceinline__ uint32_t bounce_entry(uint32_t j, uint32_t n_front, u
   return j < n_front ? j : cap - 1u - (j - n_front);
 }
 
+// What a pixel's primary hit sends on: one shadow ray and one bounce ray.
+struct NextRays {
+  bool want;
+  float3 org, ldir, bdir;
+  float dist, bcos;
+};
+
+// Camera ray direction (pixel centre), the same f32 steps as the host generator.
+__device__ __forceinline__ float3 camera_direction(const WavefrontParams& w, uint32_t px, uint32_t py) {
+  const float sx = (((float)px + 0.5f) / (float)w.width * 2.0f - 1.0f) * w.tan_half * w.aspect;
+  const float sy = (1.0f - ((float)(py + w.row0) + 0.5f) / (float)w.frame_height * 2.0f) * w.tan_half;
+  return normalize3(make_float3((w.forward.x + sx * w.right.x) + sy * w.up.x,
+                                (w.forward.y + sx * w.right.y) + sy * w.up.y,
+                                (w.forward.z + sx * w.right.z) + sy * w.up.z));
+}
+
+__device__ __forceinline__ void primary_ray(const WavefrontParams& w, float3 d, RayCtx& R) {
+  R.o = w.origin;
+  R.d = d;
+  R.tmin = 0.0f;
+  R.tmax = __int_as_float(0x7f800000);
+  R.cull_mask = 0xFFu;
+  R.ray_flags = 0u;
+}
+
+// Writes the pixel's record and forms its secondary rays.
+__device__ __forceinline__ NextRays shade_primary(const TraceParams& p, const WavefrontParams& w, uint32_t px,
+                                                  uint32_t py, float3 d, const Best& best) {
+  NextRays n;
+  n.want = false;
+  n.org = n.ldir = n.bdir = make_float3(0.f, 0.f, 0.f);
+  n.dist = n.bcos = 0.0f;
+  PixelResult out;
+  out.primary_prim = INVALID_NEXT;
+  out.primary_t = __int_as_float(0x7f800000);
+  out.bounce_prim = INVALID_NEXT;
+  out.bounce_t = F32_MAX;
+  out.primary_flags = 0u;
+  out.light = 0u;
+  out.direct = 0.0f;
+  out.primary_instance = INVALID_NEXT;
+  if (best.have) {
+    const uint4 gm = __ldg(reinterpret_cast<const uint4*>(p.tri_root + best.geom_slot));
+    out.primary_prim = __ldg(p.redirect + best.k) - gm.z;
+    out.primary_t = best.t;
+    out.primary_flags = 1u;
+    out.primary_instance = best.inst;
+    // hit point and world geometric normal facing the incoming ray
+    const float3 hp = w.origin + d * best.t;
+    const float3 nf = facing_normal(p, best.k, best.inst, d);
+    n.org = offset_ray_hit(hp, nf);
+    const float3 L = w.light - n.org;
+    const float dist2 = dot3(L, L);
+    n.dist = sqrtf(dist2);
+    n.ldir = normalize3(L);
+    out.direct = fmaxf(0.0f, dot3(nf, n.ldir)) / dist2;  // kept only if the light is visible
+    uint32_t state = xxhash32(px, py + w.row0, w.sample_index * 3u);
+    const float s0 = sample_next(state);
+    const float s1 = sample_next(state);
+    n.bdir = cosine_sample_in_dir(nf, s0, s1);
+    n.bcos = dot3(n.bdir, nf);
+    n.want = true;
+  }
+  w.out[(size_t)py * w.width + px] = out;
+  return n;
+}
+
+// Compacted appends: shadow rays to their queue; bounce rays to two bins of
+// theirs, grazing ones (the longer walks) from its front and steep ones
+// from its back, so that a warp of the secondary kernel traces rays of
+// like walk lengths. One 64-bit atomic per warp counts both bins (low and
+// high word); the shadow slot is the sum of the two bases plus the lane's
+// rank, so the shadow queue stays dense. Every lane of the warp is here.
+__device__ __forceinline__ void append_rays(const WavefrontParams& w, uint32_t px, uint32_t py, const NextRays& n) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const bool steep = n.want && n.bcos >= kSteepBounceCos;
+  const uint32_t m_want = __ballot_sync(0xffffffffu, n.want), m_steep = __ballot_sync(0xffffffffu, steep);
+  const uint32_t m_front = m_want & ~m_steep;
+  unsigned long long bases = 0ull;
+  if (lane == 0 && m_want)
+    bases = atomicAdd(w.bins, (unsigned long long)__popc(m_front) | ((unsigned long long)__popc(m_steep) << 32));
+  bases = __shfl_sync(0xffffffffu, bases, 0);
+  const uint32_t below = (1u << lane) - 1u;
+  const uint32_t front = (uint32_t)bases + __popc(m_front & below);
+  const uint32_t back = (uint32_t)(bases >> 32) + __popc(m_steep & below);
+  const uint32_t slot = (uint32_t)bases + (uint32_t)(bases >> 32) + __popc(m_want & below);
+  if (n.want) {
+    const uint32_t pix = py * w.width + px;
+    float4* sq = reinterpret_cast<float4*>(w.shadow_rays) + 2 * (size_t)slot;
+    sq[0] = make_float4(n.org.x, n.org.y, n.org.z, F32_EPSILON);
+    sq[1] = make_float4(n.ldir.x, n.ldir.y, n.ldir.z, n.dist);
+    const uint32_t bslot = steep ? w.width * w.height - 1u - back : front;
+    float4* bq = reinterpret_cast<float4*>(w.bounce_rays) + 2 * (size_t)bslot;
+    bq[0] = make_float4(n.org.x, n.org.y, n.org.z, F32_EPSILON);
+    bq[1] = make_float4(n.bdir.x, n.bdir.y, n.bdir.z, F32_MAX);
+    w.shadow_pixel[slot] = pix;
+    w.bounce_pixel[bslot] = pix;
+  }
+}
+
+// persistent: each warp claims 4x8 pixel tiles from a counter until none is
+// left, so that a warp that finishes early does not wait for its block
 template <int MODE, bool LOCAL, int TIER, bool WT>
 __global__ void __launch_bounds__(128, min_blocks(TIER)) primary_kernel(TraceParams p, WavefrontParams w) {
   extern __shared__ uint2 smem_stack[];
@@ -69,8 +172,6 @@ __global__ void __launch_bounds__(128, min_blocks(TIER)) primary_kernel(TracePar
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t tiles_x = (w.width + 3u) / 4u;
   const uint32_t tiles = tiles_x * ((w.height + 7u) / 8u);
-  // persistent: each warp claims 4x8 pixel tiles from a counter until none is
-  // left, so that a warp that finishes early does not wait for its block
   for (;;) {
     uint32_t tile = 0;
     if (lane == 0) tile = atomicAdd(w.tile_counter, 1u);
@@ -78,89 +179,66 @@ __global__ void __launch_bounds__(128, min_blocks(TIER)) primary_kernel(TracePar
     if (tile >= tiles) break;
     const uint32_t px = (tile % tiles_x) * 4u + (lane & 3u);
     const uint32_t py = (tile / tiles_x) * 8u + (lane >> 2);
-    const bool valid = px < w.width && py < w.height;
-
-    bool want = false;
-    float3 org = make_float3(0.f, 0.f, 0.f), ldir = org, bdir = org;
-    float dist = 0.0f, bcos = 0.0f;
-    if (valid) {
-      // camera ray (pixel centre), the same f32 steps as the host generator
-      const float sx = (((float)px + 0.5f) / (float)w.width * 2.0f - 1.0f) * w.tan_half * w.aspect;
-      const float sy = (1.0f - ((float)(py + w.row0) + 0.5f) / (float)w.frame_height * 2.0f) * w.tan_half;
-      const float3 d = normalize3(make_float3((w.forward.x + sx * w.right.x) + sy * w.up.x,
-                                              (w.forward.y + sx * w.right.y) + sy * w.up.y,
-                                              (w.forward.z + sx * w.right.z) + sy * w.up.z));
+    NextRays n;
+    n.want = false;
+    if (px < w.width && py < w.height) {
+      const float3 d = camera_direction(w, px, py);
       RayCtx R;
-      R.o = w.origin;
-      R.d = d;
-      R.tmin = 0.0f;
-      R.tmax = __int_as_float(0x7f800000);
-      R.cull_mask = 0xFFu;
-      R.ray_flags = 0u;
+      primary_ray(w, d, R);
       bool bad;
       traverse_ray<MODE, false, BuiltinAnyHit, WT>(p, R, w.tlas, stack, stride, bad);
-      PixelResult out;
-      out.primary_prim = INVALID_NEXT;
-      out.primary_t = R.tmax;
-      out.bounce_prim = INVALID_NEXT;
-      out.bounce_t = F32_MAX;
-      out.primary_flags = 0u;
-      out.light = 0u;
-      out.direct = 0.0f;
-      out.primary_instance = INVALID_NEXT;
-      if (R.best.have) {
-        const uint4 gm = __ldg(reinterpret_cast<const uint4*>(p.tri_root + R.best.geom_slot));
-        out.primary_prim = __ldg(p.redirect + R.best.k) - gm.z;
-        out.primary_t = R.best.t;
-        out.primary_flags = 1u;
-        out.primary_instance = R.best.inst;
-        // hit point and world geometric normal facing the incoming ray
-        const float3 hp = R.o + d * R.best.t;
-        const float3 nf = facing_normal(p, R.best.k, R.best.inst, d);
-        org = offset_ray_hit(hp, nf);
-        const float3 L = w.light - org;
-        const float dist2 = dot3(L, L);
-        dist = sqrtf(dist2);
-        ldir = normalize3(L);
-        out.direct = fmaxf(0.0f, dot3(nf, ldir)) / dist2;  // kept only if the light is visible
-        uint32_t state = xxhash32(px, py + w.row0, w.sample_index * 3u);
-        const float s0 = sample_next(state);
-        const float s1 = sample_next(state);
-        bdir = cosine_sample_in_dir(nf, s0, s1);
-        bcos = dot3(bdir, nf);
-        want = true;
-      }
-      w.out[(size_t)py * w.width + px] = out;
+      n = shade_primary(p, w, px, py, d, R.best);
     }
-    // compacted appends: shadow rays to their queue; bounce rays to two bins of
-    // theirs, grazing ones (the longer walks) from its front and steep ones
-    // from its back, so that a warp of the secondary kernel traces rays of
-    // like walk lengths. One 64-bit atomic per warp counts both bins (low and
-    // high word); the shadow slot is the sum of the two bases plus the lane's
-    // rank, so the shadow queue stays dense. Every lane of the warp is here.
-    const bool steep = want && bcos >= kSteepBounceCos;
-    const uint32_t m_want = __ballot_sync(0xffffffffu, want), m_steep = __ballot_sync(0xffffffffu, steep);
-    const uint32_t m_front = m_want & ~m_steep;
-    unsigned long long bases = 0ull;
-    if (lane == 0 && m_want)
-      bases = atomicAdd(w.bins, (unsigned long long)__popc(m_front) | ((unsigned long long)__popc(m_steep) << 32));
-    bases = __shfl_sync(0xffffffffu, bases, 0);
-    const uint32_t below = (1u << lane) - 1u;
-    const uint32_t front = (uint32_t)bases + __popc(m_front & below);
-    const uint32_t back = (uint32_t)(bases >> 32) + __popc(m_steep & below);
-    const uint32_t slot = (uint32_t)bases + (uint32_t)(bases >> 32) + __popc(m_want & below);
-    if (want) {
-      const uint32_t pix = py * w.width + px;
-      float4* sq = reinterpret_cast<float4*>(w.shadow_rays) + 2 * (size_t)slot;
-      sq[0] = make_float4(org.x, org.y, org.z, F32_EPSILON);
-      sq[1] = make_float4(ldir.x, ldir.y, ldir.z, dist);
-      const uint32_t bslot = steep ? w.width * w.height - 1u - back : front;
-      float4* bq = reinterpret_cast<float4*>(w.bounce_rays) + 2 * (size_t)bslot;
-      bq[0] = make_float4(org.x, org.y, org.z, F32_EPSILON);
-      bq[1] = make_float4(bdir.x, bdir.y, bdir.z, F32_MAX);
-      w.shadow_pixel[slot] = pix;
-      w.bounce_pixel[bslot] = pix;
-    }
+    append_rays(w, px, py, n);
+  }
+}
+
+// The same with four lanes per ray (quad.cuh): a warp claims `batch` pixels of
+// a tile. Both kernels of this kind run for frames of up to kQuadPixels, whose
+// slowest warps decide (us, primary + secondary, one ray per lane -> quads):
+// 64^2 pixels 131 + 170 -> 54 + 60, 256^2 208 + 240 -> 93 + 104, 512^2 272 +
+// 305 -> 193 + 230, 800x500 304 + 395 -> 275 + 329, but 1280x720 430 + 674 ->
+// 525 + 709.
+constexpr uint32_t kQuadPixels = 450000;
+template <bool WT>
+__global__ void __launch_bounds__(128, 8) primary_quad_kernel(TraceParams p, WavefrontParams w, uint32_t batch) {
+  extern __shared__ __align__(16) unsigned char quad_smem[];
+  const QuadWarp W = quad_warp(quad_smem, p.stack_depth4);
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t tiles_x = (w.width + 3u) / 4u;
+  const uint32_t parts = tiles_x * ((w.height + 7u) / 8u) * (32u / batch);
+  for (;;) {
+    uint32_t part = 0;
+    if (lane == 0) part = atomicAdd(w.tile_counter, 1u);
+    part = __shfl_sync(0xffffffffu, part, 0);
+    if (part >= parts) break;
+    const uint32_t at = part * batch + lane, tile = at >> 5, in = at & 31u;
+    const uint32_t px = (tile % tiles_x) * 4u + (in & 3u);
+    const uint32_t py = (tile / tiles_x) * 8u + (in >> 2);
+    const bool valid = lane < batch && px < w.width && py < w.height;
+    RayCtx R;
+    primary_ray(w, valid ? camera_direction(w, px, py) : make_float3(0.f, 0.f, 0.f), R);
+    bool bad;
+    traverse_warp<WT>(p, R, w.tlas, valid, W, bad);
+    NextRays n;
+    n.want = false;
+    if (valid) n = shade_primary(p, w, px, py, camera_direction(w, px, py), R.best);
+    append_rays(w, px, py, n);
+  }
+}
+
+// The result of queue entry q to its pixel's record.
+__device__ __forceinline__ void store_secondary(const TraceParams& p, const WavefrontParams& w, bool shadow, uint32_t q,
+                                                const Best& best) {
+  if (shadow) {
+    PixelResult* o = w.out + w.shadow_pixel[q];
+    o->light = best.have ? 2u : 1u;
+    if (best.have) o->direct = 0.0f;
+  } else if (best.have) {
+    PixelResult* o = w.out + w.bounce_pixel[q];
+    const uint4 gm = __ldg(reinterpret_cast<const uint4*>(p.tri_root + best.geom_slot));
+    o->bounce_prim = __ldg(p.redirect + best.k) - gm.z;
+    o->bounce_t = best.t;
   }
 }
 
@@ -203,19 +281,52 @@ __global__ void __launch_bounds__(128, min_blocks(TIER)) secondary_kernel(TraceP
       R.ray_flags = shadow ? TF_END_SEARCH : 0u;
       bool bad;
       traverse_ray<MODE, false, BuiltinAnyHit, WT>(p, R, w.tlas, stack, stride, bad);
-      if (shadow) {
-        PixelResult* o = w.out + w.shadow_pixel[q];
-        o->light = R.best.have ? 2u : 1u;
-        if (R.best.have) o->direct = 0.0f;
-      } else {
-        PixelResult* o = w.out + w.bounce_pixel[q];
-        if (R.best.have) {
-          const uint4 gm = __ldg(reinterpret_cast<const uint4*>(p.tri_root + R.best.geom_slot));
-          o->bounce_prim = __ldg(p.redirect + R.best.k) - gm.z;
-          o->bounce_t = R.best.t;
-        }
-      }
+      store_secondary(p, w, shadow, q, R.best);
     }
+  }
+}
+
+// The same with four lanes per ray (quad.cuh), a warp as many entries at a
+// time as the queues give every resident warp.
+template <bool WT>
+__global__ void __launch_bounds__(128, 8) secondary_quad_kernel(TraceParams p, WavefrontParams w) {
+  extern __shared__ __align__(16) unsigned char quad_smem[];
+  const QuadWarp W = quad_warp(quad_smem, p.stack_depth4);
+  const unsigned long long bins = *(volatile unsigned long long*)w.bins;
+  const uint32_t n_front = (uint32_t)bins, n = n_front + (uint32_t)(bins >> 32);
+  const uint32_t cap = w.width * w.height;
+  const uint32_t total = 2u * n;
+  // 131,072 rays took 104 us with 8 a warp, 127 with 16 and 152 with 32; 524,288 268, 242 and 230
+  const uint32_t batch = total < 200000u ? 8u : (total < 400000u ? 16u : 32u);
+  const uint32_t lane = threadIdx.x & 31u;
+  if (blockIdx.x == 0 && threadIdx.x == 0 && w.ray_counts) {
+    w.ray_counts[0] = w.width * w.height;
+    w.ray_counts[1] = n;
+    w.ray_counts[2] = n;
+  }
+  for (;;) {
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(w.work_counter, batch);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (base >= total) break;
+    const uint32_t j = base + lane;
+    const bool valid = lane < batch && j < total;
+    const bool shadow = j >= n;
+    const uint32_t q = shadow ? j - n : bounce_entry(j, n_front, cap);
+    RayCtx R;
+    if (valid) {
+      const float4* rq = reinterpret_cast<const float4*>(shadow ? w.shadow_rays : w.bounce_rays) + 2 * (size_t)q;
+      const float4 r0 = rq[0], r1 = rq[1];
+      R.o = make_float3(r0.x, r0.y, r0.z);
+      R.tmin = r0.w;
+      R.d = make_float3(r1.x, r1.y, r1.z);
+      R.tmax = r1.w;
+    }
+    R.cull_mask = 0xFFu;
+    R.ray_flags = shadow ? TF_END_SEARCH : 0u;
+    bool bad;
+    traverse_warp<WT>(p, R, w.tlas, valid, W, bad);
+    if (valid) store_secondary(p, w, shadow, q, R.best);
   }
 }
 
@@ -333,7 +444,7 @@ cudaError_t launch_wavefront_mode(const TraceParams& p, const WavefrontParams& w
   static std::atomic<uint64_t> attr_done{0};
   cudaError_t e = raise_smem_limit(
       attr_done, {(const void*)primary_kernel<MODE, LOCAL, TIER, WT>, (const void*)secondary_kernel<MODE, LOCAL, TIER, WT>,
-                  (const void*)secondary_dynamic_kernel<MODE == MODE_THREADED ? MODE_BINARY : MODE, WT>});
+                  (const void*)secondary_dynamic_kernel<MODE_WIDE4, WT>});
   if (e != cudaSuccess) return e;
   if (phases & 1u) {
     e = cudaMemsetAsync(w.queue_count, 0, 64, stream);
@@ -357,7 +468,7 @@ cudaError_t launch_wavefront_mode(const TraceParams& p, const WavefrontParams& w
   // persistent secondary grid: enough resident blocks to fill every SM
   const bool dynamic = MODE != MODE_THREADED && w.refill != 0u && !LOCAL;
   int per_sm = 0;
-  constexpr int DMODE = MODE == MODE_THREADED ? MODE_BINARY : MODE;  // the threaded walk has no dynamic form
+  constexpr int DMODE = MODE_WIDE4;  // the threaded walk has no dynamic form
   if (dynamic)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, secondary_dynamic_kernel<DMODE, WT>, (int)block, smem);
   else
@@ -371,32 +482,68 @@ cudaError_t launch_wavefront_mode(const TraceParams& p, const WavefrontParams& w
 }
 }  // namespace
 
-cudaError_t launch_wavefront(const TraceParams& p, const WavefrontParams& w, int mode, uint32_t block,
+namespace {
+template <bool WT>
+cudaError_t launch_wavefront_quads(const TraceParams& p, const WavefrontParams& w, int sm_count, uint32_t phases,
+                                   cudaStream_t stream) {
+  constexpr uint32_t block = 64;
+  const size_t smem = (size_t)quad_warp_bytes(p.stack_depth4) * (block / 32);
+  static std::atomic<uint64_t> attr_done{0};
+  cudaError_t e =
+      raise_smem_limit(attr_done, {(const void*)primary_quad_kernel<WT>, (const void*)secondary_quad_kernel<WT>});
+  if (e != cudaSuccess) return e;
+  const uint64_t pixels = (uint64_t)((w.width + 3) / 4) * ((w.height + 7) / 8) * 32;
+  // persistent grids: as many resident blocks as fill every SM, or fewer when the rays are
+  auto grid = [&](const void* fn, uint64_t rays, uint32_t batch, uint32_t& blocks) {
+    int per_sm = 0;
+    const cudaError_t r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, (int)block, smem);
+    const uint64_t per = batch * (block / 32);
+    blocks = (uint32_t)std::min<uint64_t>((uint64_t)sm_count * std::max(per_sm, 1), (rays + per - 1) / per);
+    return r;
+  };
+  uint32_t blocks = 0;
+  if (phases & 1u) {
+    const uint32_t batch = pixels < 100000 ? 8u : 16u;
+    e = cudaMemsetAsync(w.queue_count, 0, 64, stream);
+    if (e == cudaSuccess) e = grid((const void*)primary_quad_kernel<WT>, pixels, batch, blocks);
+    if (e != cudaSuccess) return e;
+    primary_quad_kernel<WT><<<blocks, block, smem, stream>>>(p, w, batch);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  if (!(phases & 2u)) return cudaSuccess;
+  e = cudaMemsetAsync(w.work_counter, 0, 64, stream);
+  if (e == cudaSuccess) e = grid((const void*)secondary_quad_kernel<WT>, 2 * pixels, 8u, blocks);
+  if (e != cudaSuccess) return e;
+  secondary_quad_kernel<WT><<<blocks, block, smem, stream>>>(p, w);
+  return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t launch_wavefront(const TraceParams& params, const WavefrontParams& w, int mode, uint32_t block,
                              int sm_count, uint32_t phases, cudaStream_t stream) {
   if (phases == 0) phases = 3;
   if (block == 0) block = 64;
   const size_t n = (size_t)w.width * w.height;
   if (n == 0) return cudaSuccess;
-  // the local-memory stack holds kLocalStackEntries entries; deeper trees keep the shared-memory stack
-  const bool local = w.local_stack && mode != MODE_THREADED && p.stack_depth <= kLocalStackEntries;
-  // register tiers apply to the local-stack kernels
-  const uint32_t tier = local ? w.register_tier : 0u;
 #define RDN_WF(M, L, T)                                                                      \
   return p.watertight ? launch_wavefront_mode<M, L, T, true>(p, w, block, sm_count, phases, stream) \
                       : launch_wavefront_mode<M, L, T, false>(p, w, block, sm_count, phases, stream)
-  if (mode == MODE_WIDE4) {
-    if (!local) RDN_WF(MODE_WIDE4, false, 0);
-    if (tier == 1) RDN_WF(MODE_WIDE4, true, 1);
-    if (tier == 2) RDN_WF(MODE_WIDE4, true, 2);
-    RDN_WF(MODE_WIDE4, true, 0);
+  if (mode == MODE_THREADED) {
+    const TraceParams& p = params;
+    RDN_WF(MODE_THREADED, false, 0);
   }
-  if (mode == MODE_BINARY) {
-    if (!local) RDN_WF(MODE_BINARY, false, 0);
-    if (tier == 1) RDN_WF(MODE_BINARY, true, 1);
-    if (tier == 2) RDN_WF(MODE_BINARY, true, 2);
-    RDN_WF(MODE_BINARY, true, 0);
-  }
-  RDN_WF(MODE_THREADED, false, 0);
+  const TraceParams p = wide4_params(params);
+  // dynamic fetch (w.refill) has its own secondary kernel, with stacks in shared memory
+  const bool dynamic = w.refill != 0u && !(w.local_stack && p.local_stack);
+  if (p.packed && n <= kQuadPixels && !dynamic)
+    return p.watertight ? launch_wavefront_quads<true>(p, w, sm_count, phases, stream)
+                        : launch_wavefront_quads<false>(p, w, sm_count, phases, stream);
+  if (!p.local_stack || dynamic) RDN_WF(MODE_WIDE4, false, 0);
+  // register tiers apply to the local-stack kernels
+  if (w.register_tier == 1) RDN_WF(MODE_WIDE4, true, 1);
+  if (w.register_tier == 2) RDN_WF(MODE_WIDE4, true, 2);
+  RDN_WF(MODE_WIDE4, true, 0);
 #undef RDN_WF
 }
 

@@ -248,3 +248,29 @@ def test_frames_of_both_walks(cuda, width, height):
             assert np.count_nonzero((images[traversal][k] != want[k]).any(-1)) <= n // 20_000
         assert all(abs(a - b) <= 3 * (n // 20_000) for a, b in zip(images[traversal][2], want[2]))
     assert P.check_errors() == (0, 0)
+
+
+@pytest.mark.parametrize("width,height", [(3, 9), (320, 312), (316, 320), (670, 670), (680, 672)])
+def test_wavefront_frames_of_both_walks(cuda, width, height):
+    """Wavefront frames on either side of the sizes where their walks change: every record of the reference order's
+    frame, except after an exact-distance tie."""
+    import torch
+
+    P, _ = field_system(128)
+    cam = scenes.heightfield_camera(width, height)
+    frames = {}
+    for watertight in (0, rt.INTERSECT_WATERTIGHT):
+        for traversal, refill, local in ((rt.TRAVERSAL_REFERENCE, 0, 0), (rt.TRAVERSAL_ORDERED, 0, 1),
+                                         (rt.TRAVERSAL_ORDERED_WIDE, 0, 0), (rt.TRAVERSAL_ORDERED, 8, 0)):
+            wf = rt.Wavefront(P, cam, (0.2, 0.2, 2.0))
+            knobs = (traversal | watertight, 64, local)
+            wf.configure(knobs, knobs, refill=refill)
+            wf.run(3)
+            torch.cuda.synchronize()
+            frames[watertight, traversal, refill] = wf.results().copy(), wf.rays_traced()
+    for (watertight, traversal, refill), (got, rays) in frames.items():
+        want, want_rays = frames[watertight, rt.TRAVERSAL_REFERENCE, 0]
+        assert np.count_nonzero(got.view(np.uint32).reshape(-1, 8) != want.view(np.uint32).reshape(-1, 8)) <= \
+            8 * (width * height // 20_000)
+        assert rays == want_rays
+    assert P.check_errors() == (0, 0)
