@@ -8,7 +8,8 @@
 // of the traversal kernels. The arrays equal the host build's byte for byte.
 //
 // The reference builds one node at a time, depth first, on one thread. Here
-// every geometry's tree is built together, one tree level per round:
+// every geometry's tree is built together. Nodes of more than kSmall primitives
+// go one tree level per round:
 //   prepare   each node of the level decides leaf / split (count > bin_size and
 //             depth < max_depth, utils.rs:35-37) and claims warp tasks of 256
 //             primitives ("chunks") of its range;
@@ -19,10 +20,18 @@
 //   decide    per node: the reference's 3-candidate SAH choice (or the median
 //             fallback when 3 buckets are empty), the two children, and each
 //             chunk's per-bucket offset inside the node (warp scan);
-//   select    median-split nodes run Rust's select_nth_unstable_by
-//             restatement on one thread each;
+//   prefix    the chunk offsets of nodes with many chunks, a block per node;
+//             median-split nodes run Rust's select_nth_unstable_by restatement
+//             on one thread each;
 //   scatter   SAH nodes write their primitives in bucket order, stable inside
-//             a bucket (warp ballots), then copy the range back.
+//             a bucket (warp ballots), into the other of two order arrays;
+//             median-split nodes copy theirs.
+// Nodes of kSmall primitives and fewer are left to small_trees_kernel, which
+// builds the whole subtree below each in shared memory, a block per subtree and
+// a warp or a lane per node: a level of many small nodes is bound by the gaps
+// between its launches and by reductions over empty lanes (2.1 M triangles,
+// bin size 4: all by level rounds 5.2 ms a build, subtrees in blocks 3.35 ms;
+// 8,000 triangles 1.58 and 0.75 ms; 1,000 triangles 1.19 and 0.63 ms).
 // Boxes are merged with integer atomics on an order-preserving key of the
 // float, so a union does not depend on the order primitives arrive in. The
 // reference's pre-order numbering is recovered afterwards from subtree sizes
@@ -48,7 +57,9 @@ constexpr uint32_t NONE = 0xFFFFFFFFu;
 constexpr uint32_t kChunk = 256;
 constexpr uint32_t kBlock = 256;
 constexpr uint32_t kWarps = kBlock / 32;
-constexpr uint32_t F_BOX_PENDING = 1u, F_ACTIVE = 2u, F_FALLBACK = 4u;
+constexpr uint32_t F_BOX_PENDING = 1u, F_ACTIVE = 2u, F_FALLBACK = 4u, F_IN_B = 8u;  // F_IN_B: primitives in the second order array
+// Subtrees of at most this many primitives are built by one block each.
+constexpr uint32_t kSmall = 256;
 
 // Order-preserving int key of a float (no NaN reaches a box: boxes start
 // empty and grow with NaN-ignoring min/max). -0.0 orders below +0.0.
@@ -72,13 +83,14 @@ __host__ __device__ __forceinline__ float val_of(int k) {
 #endif
 }
 
-struct BNode {  // 64 B, one per tree node during the build
+struct alignas(16) BNode {  // 64 B, one per tree node during the build
   int lo[3], hi[3];   // box as keys
   uint32_t start, end;  // range in the global primitive order
   uint32_t depth, left;  // left child id (right = left + 1), NONE for a leaf
   uint32_t tree, flags;
-  uint32_t cbase, nchunks;
-  uint32_t pad[2];
+  uint32_t cbase, nchunks;  // a split's chunks; in the finished tree: subtree size, pre-order place below `sub`
+  uint32_t sub;             // finished tree: root of the subtree that a block built, NONE for a node above those
+  uint32_t pad;
 };
 static_assert(sizeof(BNode) == 64, "64 B build node");
 
@@ -87,7 +99,11 @@ struct LevelCounters {  // one per tree level, zeroed before the first level
 };
 struct BuildCounters {
   unsigned long long sah, fallback;
-  uint32_t bad_index, pad;
+  uint32_t bad_index, max_depth;
+  uint32_t ended;     // nodes that have left the level rounds
+  uint32_t added;     // nodes that the subtrees added to the pool
+  uint32_t unfit;     // a split had an empty child (the subtree blocks count on none)
+  uint32_t overflow;  // a level had more children than the pool holds
 };
 
 struct F3 {
@@ -139,9 +155,13 @@ __device__ __forceinline__ void set_box(BNode& n, const NodeBox& b) {
 // Centre keys of one axis with the reference's comparator
 // (partial_cmp(..).unwrap_or(Less) on the centre coordinate).
 struct CentreLess {
-  const float* key;
-  __host__ __device__ bool operator()(const uint32_t& a, const uint32_t& b) const {
-    const float ka = key[a], kb = key[b];
+  const float* key;  // centres, or lower and upper corners `boxes` floats apart
+  uint32_t boxes;
+  __device__ float of(uint32_t p) const {
+    return boxes ? (key[2 * boxes * (size_t)p] + key[2 * boxes * (size_t)p + boxes]) * 0.5f : key[p];
+  }
+  __device__ bool operator()(const uint32_t& a, const uint32_t& b) const {
+    const float ka = of(a), kb = of(b);
     return ka != ka || kb != kb || ka < kb;  // a NaN on either side compares Less
   }
 };
@@ -150,13 +170,12 @@ struct CentreLess {
 
 // Global vertex indices (BLAS concatenation, naive/mod.rs:155-186), the
 // primitive boxes (BuildPrimitive::new, utils.rs:40-66: grow an empty box by
-// the 3 vertices) and centres (box centre), SoA centres for the bucket pass.
+// the 3 vertices); their centres are computed where they are used.
 __global__ void prepare_primitives_kernel(uint32_t N, uint32_t G, const uint32_t* __restrict__ g_prim_start,
                                           const uint32_t* __restrict__ g_vstart, const uint32_t* __restrict__ g_vcount,
                                           const uint32_t* __restrict__ g_indexed, uint32_t* __restrict__ idx,
                                           const float* __restrict__ vtx, float4* __restrict__ pbox,
-                                          float* __restrict__ cen, uint32_t* __restrict__ order,
-                                          BuildCounters* ctr) {
+                                          uint32_t* __restrict__ order, BuildCounters* ctr) {
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x) {
     uint32_t lo = 0, hi = G;  // last g with g_prim_start[g] <= p
     while (hi - lo > 1) {
@@ -181,11 +200,12 @@ __global__ void prepare_primitives_kernel(uint32_t N, uint32_t G, const uint32_t
     }
     pbox[2 * (size_t)p] = make_float4(b.lo.x, b.lo.y, b.lo.z, 0.0f);
     pbox[2 * (size_t)p + 1] = make_float4(b.hi.x, b.hi.y, b.hi.z, 0.0f);
-    cen[p] = (b.lo.x + b.hi.x) * 0.5f;
-    cen[N + p] = (b.lo.y + b.hi.y) * 0.5f;
-    cen[2 * (size_t)N + p] = (b.lo.z + b.hi.z) * 0.5f;
     order[p] = p;
   }
+}
+
+__global__ void restart_kernel(uint32_t N, uint32_t* __restrict__ order) {
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x) order[p] = p;
 }
 
 // ---- one tree level -----------------------------------------------------
@@ -218,7 +238,8 @@ __device__ __forceinline__ uint32_t warp_claim(uint32_t* ctr, uint32_t amount, u
 __global__ void level_prepare_kernel(const uint32_t* __restrict__ lvl, uint32_t L, uint32_t bin_size,
                                      uint32_t max_depth, BNode* __restrict__ pool, uint32_t* __restrict__ acc_cnt,
                                      int* __restrict__ acc_box, uint32_t* __restrict__ chunk_node,
-                                     LevelCounters* lcs) {
+                                     LevelCounters* lcs, uint32_t small, BuildCounters* bc,
+                                     uint32_t* __restrict__ ended) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t lb = lvl[L], W = lvl[L + 1] - lb;
   LevelCounters* lc = lcs + L;
@@ -230,13 +251,16 @@ __global__ void level_prepare_kernel(const uint32_t* __restrict__ lvl, uint32_t 
     if (i < W) {
       BNode& n = pool[lb + i];
       const uint32_t count = n.end - n.start;
-      active = n.depth < max_depth && count > bin_size;
-      const bool need = active || (n.flags & F_BOX_PENDING);
+      active = n.depth < max_depth && count > bin_size && count > small;
+      const bool need = active || (count > small && (n.flags & F_BOX_PENDING));
       nch = need ? (count + kChunk - 1) / kChunk : 0;
-      n.flags = (n.flags & ~(F_ACTIVE | F_FALLBACK)) | (active ? F_ACTIVE : 0u);
+      n.flags = (n.flags & F_BOX_PENDING) | (active ? F_ACTIVE : 0u) | ((L & 1u) ? F_IN_B : 0u);
       n.left = NONE;
       n.nchunks = nch;
     }
+    const bool ends = i < W && !active;
+    const uint32_t at = warp_claim(&bc->ended, ends ? 1u : 0u, lane);
+    if (ends) ended[at] = lb + i;
     const uint32_t base = warp_claim(&lc->chunks, nch, lane);
     if (i < W) pool[lb + i].cbase = nch ? base : 0u;
     // chunk -> node map: small ranges by their own lane, long ones by the whole warp
@@ -314,13 +338,14 @@ __device__ __forceinline__ SplitPlane plane_of(const BNode& n) {
   return sp;
 }
 
-// Bucket counts and boxes of each chunk, merged into the node.
-__global__ void level_stats_kernel(const uint32_t* __restrict__ lvl, uint32_t L, uint32_t N,
-                                   const LevelCounters* lcs, const BNode* __restrict__ pool,
-                                   const uint32_t* __restrict__ chunk_node, const uint32_t* __restrict__ order,
-                                   const float4* __restrict__ pbox, const float* __restrict__ cen,
-                                   uint32_t* __restrict__ chunk_cnt, uint32_t* __restrict__ acc_cnt,
-                                   int* __restrict__ acc_box) {
+// Bucket counts and boxes of each chunk, merged into the node. Bound by the
+// latency of the gathers: a lane loads four primitives' boxes (one sector each,
+// their centres included) before it uses the first.
+__global__ void level_stats_kernel(const uint32_t* __restrict__ lvl, uint32_t L, const LevelCounters* lcs,
+                                   const BNode* __restrict__ pool, const uint32_t* __restrict__ chunk_node,
+                                   const uint32_t* __restrict__ order, const float4* __restrict__ pbox,
+                                   uint8_t* __restrict__ bucket, uint32_t* __restrict__ chunk_cnt,
+                                   uint32_t* __restrict__ acc_cnt, int* __restrict__ acc_box) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t lb = lvl[L];
   const uint32_t total = lcs[L].chunks;
@@ -329,7 +354,6 @@ __global__ void level_stats_kernel(const uint32_t* __restrict__ lvl, uint32_t L,
     const BNode n = pool[id];
     if (!(n.flags & F_ACTIVE)) continue;
     const SplitPlane sp = plane_of(n);
-    const float* ck = cen + (size_t)sp.axis * N;
     uint32_t s, e;
     chunk_range(n, c, s, e);
     uint32_t cnt[4] = {0, 0, 0, 0};
@@ -339,21 +363,39 @@ __global__ void level_stats_kernel(const uint32_t* __restrict__ lvl, uint32_t L,
       bx[b][0] = bx[b][1] = bx[b][2] = key_of(INFINITY);
       bx[b][3] = bx[b][4] = bx[b][5] = key_of(-INFINITY);
     }
-    for (uint32_t i = s + lane; i < e; i += 32) {
-      const uint32_t p = order[i];
-      const uint32_t bk = bucket_of(ck[p], sp.a0, sp.step);
-      const float4 a = pbox[2 * (size_t)p], b = pbox[2 * (size_t)p + 1];
-      const int k[6] = {key_of(a.x), key_of(a.y), key_of(a.z), key_of(b.x), key_of(b.y), key_of(b.z)};
+    constexpr int kAhead = 4;
+    for (uint32_t i0 = s + lane; i0 < e; i0 += 32 * kAhead) {
+      float4 a[kAhead], b[kAhead];
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        if (bk == (uint32_t)q) {
-          cnt[q]++;
-          bx[q][0] = min(bx[q][0], k[0]);
-          bx[q][1] = min(bx[q][1], k[1]);
-          bx[q][2] = min(bx[q][2], k[2]);
-          bx[q][3] = max(bx[q][3], k[3]);
-          bx[q][4] = max(bx[q][4], k[4]);
-          bx[q][5] = max(bx[q][5], k[5]);
+      for (int m = 0; m < kAhead; m++) {
+        const uint32_t i = i0 + 32 * m;
+        if (i < e) {
+          const size_t p = order[i];
+          a[m] = pbox[2 * p];
+          b[m] = pbox[2 * p + 1];
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < kAhead; m++) {
+        const uint32_t i = i0 + 32 * m;
+        if (i >= e) break;
+        const float centre = sp.axis == 0 ? (a[m].x + b[m].x) * 0.5f
+                             : sp.axis == 1 ? (a[m].y + b[m].y) * 0.5f
+                                            : (a[m].z + b[m].z) * 0.5f;
+        const uint32_t bk = bucket_of(centre, sp.a0, sp.step);
+        bucket[i] = (uint8_t)bk;
+        const int k[6] = {key_of(a[m].x), key_of(a[m].y), key_of(a[m].z), key_of(b[m].x), key_of(b[m].y), key_of(b[m].z)};
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          if (bk == (uint32_t)q) {
+            cnt[q]++;
+            bx[q][0] = min(bx[q][0], k[0]);
+            bx[q][1] = min(bx[q][1], k[1]);
+            bx[q][2] = min(bx[q][2], k[2]);
+            bx[q][3] = max(bx[q][3], k[3]);
+            bx[q][4] = max(bx[q][4], k[4]);
+            bx[q][5] = max(bx[q][5], k[5]);
+          }
         }
       }
     }
@@ -382,70 +424,74 @@ __global__ void level_stats_kernel(const uint32_t* __restrict__ lvl, uint32_t L,
 // their own thread.
 constexpr uint32_t kBigChunks = 8;
 
-// The reference's split decision for one active node (strategy.rs:202-284):
-// the 4 buckets' counts and boxes, then either BalanceTree's median split
-// (3 empty buckets, strategy.rs:67-87) or the first strictly cheaper of the 3
-// SAH candidates. Fills the two children; returns true for the median split.
-__device__ __forceinline__ bool decide_split(const BNode& n, uint32_t i, const uint32_t* __restrict__ acc_cnt,
-                                             const int* __restrict__ acc_box, BNode& l, BNode& r) {
+// The reference's split decision (strategy.rs:202-284) from the 4 buckets'
+// counts and boxes: BalanceTree's median split (3 empty buckets,
+// strategy.rs:67-87; `left` is unset) or the first strictly cheaper of the 3
+// SAH candidates, `left` primitives to the left.
+struct Split {
+  bool fallback;
+  uint32_t left;
+  NodeBox l, r;
+};
+__device__ __forceinline__ Split decide_split(const uint32_t (&cnt)[4], const NodeBox (&bb)[4]) {
+  Split s;
+  const int empties = (cnt[0] == 0) + (cnt[1] == 0) + (cnt[2] == 0) + (cnt[3] == 0);
+  s.fallback = empties == 3;
+  s.left = 0;
+  s.l = s.r = empty_box();
+  if (s.fallback) return s;  // child boxes come from their primitives
+  // candidate j puts buckets 0..=j left; the first strictly cheaper
+  // candidate wins, candidate 0 when no cost is below +inf
+  float best_cost = INFINITY;
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    NodeBox lb_ = empty_box(), rb_ = empty_box();
+    uint32_t lc_ = 0, rc_ = 0;
+#pragma unroll
+    for (int p = 0; p <= j; p++) {
+      grow(lb_, bb[p]);
+      lc_ += cnt[p];
+    }
+#pragma unroll
+    for (int p = j + 1; p < 4; p++) {
+      grow(rb_, bb[p]);
+      rc_ += cnt[p];
+    }
+    const float cost = sah_area(lb_) * (float)lc_ + sah_area(rb_) * (float)rc_;
+    if (j == 0 || cost < best_cost) {
+      s.l = lb_;
+      s.r = rb_;
+      s.left = lc_;
+    }
+    if (cost < best_cost) best_cost = cost;
+  }
+  return s;
+}
+
+// The two children of active node i of the level; true for the median split.
+__device__ __forceinline__ bool split_node(const BNode& n, uint32_t i, const uint32_t* __restrict__ acc_cnt,
+                                           const int* __restrict__ acc_box, BNode& l, BNode& r) {
   uint32_t cnt[4];
   NodeBox bb[4];
+#pragma unroll
   for (int q = 0; q < 4; q++) {
     cnt[q] = acc_cnt[4 * (size_t)i + q];
     const int* k = acc_box + 24 * (size_t)i + 6 * q;
     bb[q] = NodeBox{{val_of(k[0]), val_of(k[1]), val_of(k[2])}, {val_of(k[3]), val_of(k[4]), val_of(k[5])}};
   }
-  const int empties = (cnt[0] == 0) + (cnt[1] == 0) + (cnt[2] == 0) + (cnt[3] == 0);
-  bool fallback = false;
-  if (empties == 3) {
-    // BalanceTree: median by centre on the same axis; child boxes come from
-    // the next level's box pass
-    fallback = true;
-    const uint32_t mid = (n.end + n.start) / 2;
-    l.start = n.start;
-    l.end = mid;
-    r.start = mid;
-    r.end = n.end;
-    l.flags = r.flags = F_BOX_PENDING;
-    set_box(l, empty_box());
-    set_box(r, empty_box());
-  } else {
-    // candidate j puts buckets 0..=j left; the first strictly cheaper
-    // candidate wins, candidate 0 when no cost is below +inf
-    float best_cost = INFINITY;
-    NodeBox best_l = empty_box(), best_r = empty_box();
-    uint32_t best_lc = 0;
-    for (int j = 0; j < 3; j++) {
-      NodeBox lb_ = empty_box(), rb_ = empty_box();
-      uint32_t lc_ = 0, rc_ = 0;
-      for (int p = 0; p <= j; p++) {
-        grow(lb_, bb[p]);
-        lc_ += cnt[p];
-      }
-      for (int p = j + 1; p < 4; p++) {
-        grow(rb_, bb[p]);
-        rc_ += cnt[p];
-      }
-      const float cost = sah_area(lb_) * (float)lc_ + sah_area(rb_) * (float)rc_;
-      if (j == 0 || cost < best_cost) {
-        best_l = lb_;
-        best_r = rb_;
-        best_lc = lc_;
-      }
-      if (cost < best_cost) best_cost = cost;
-    }
-    l.start = n.start;
-    l.end = n.start + best_lc;
-    r.start = n.start + best_lc;
-    r.end = n.end;
-    l.flags = r.flags = 0;
-    set_box(l, best_l);
-    set_box(r, best_r);
-  }
+  const Split s = decide_split(cnt, bb);
+  const uint32_t mid = s.fallback ? (n.end + n.start) / 2 : n.start + s.left;
+  l.start = n.start;
+  l.end = r.start = mid;
+  r.end = n.end;
+  l.flags = r.flags = s.fallback ? F_BOX_PENDING : 0u;
+  set_box(l, s.l);
+  set_box(r, s.r);
   l.depth = r.depth = n.depth + 1;
   l.tree = r.tree = n.tree;
   l.left = r.left = NONE;
-  return fallback;
+  l.sub = r.sub = NONE;
+  return s.fallback;
 }
 
 // One thread per node of the level: the split decision, the two children
@@ -455,7 +501,7 @@ __global__ void level_decide_kernel(const uint32_t* __restrict__ lvl, uint32_t L
                                     const uint32_t* __restrict__ acc_cnt, const int* __restrict__ acc_box,
                                     const uint4* __restrict__ chunk_cnt, uint4* __restrict__ chunk_prefix,
                                     LevelCounters* lcs, BuildCounters* bc, uint32_t* __restrict__ big_list,
-                                    uint32_t big_cap) {
+                                    uint32_t big_cap, uint32_t pool_cap) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t lb = lvl[L], next_base = lvl[L + 1], W = next_base - lb;
   LevelCounters* lc = lcs + L;
@@ -468,7 +514,7 @@ __global__ void level_decide_kernel(const uint32_t* __restrict__ lvl, uint32_t L
     if (i < W) {
       n = pool[lb + i];
       active = (n.flags & F_ACTIVE) != 0;
-      if (active) fallback = decide_split(n, i, acc_cnt, acc_box, l, r);
+      if (active) fallback = split_node(n, i, acc_cnt, acc_box, l, r);
     }
     const uint32_t base = next_base + warp_claim(&lc->children, active ? 2u : 0u, lane);
     const uint32_t n_sah = __popc(__ballot_sync(0xffffffffu, active && !fallback));
@@ -478,6 +524,11 @@ __global__ void level_decide_kernel(const uint32_t* __restrict__ lvl, uint32_t L
     const bool big = active && !fallback && n.nchunks > kBigChunks;
     const uint32_t slot = warp_claim(&lc->big, big ? 1u : 0u, lane);
     if (!active) continue;
+    if (base + 1 >= pool_cap) {
+      bc->overflow = 1u;
+      continue;
+    }
+    if (l.start == l.end || r.start == r.end) bc->unfit = 1u;
     pool[base] = l;
     pool[base + 1] = r;
     pool[lb + i].left = base;
@@ -503,11 +554,22 @@ __global__ void level_decide_kernel(const uint32_t* __restrict__ lvl, uint32_t L
 // per node: each thread takes kPerThread consecutive chunks of a tile, the
 // block scans the thread totals (warp shuffles, then the warp totals).
 constexpr uint32_t kPerThread = 4;
-__global__ void __launch_bounds__(kBlock) level_big_prefix_kernel(const LevelCounters* lcs, uint32_t L,
-                                                                  const BNode* __restrict__ pool,
-                                                                  const uint32_t* __restrict__ big_list,
-                                                                  uint32_t big_cap, const uint4* __restrict__ chunk_cnt,
-                                                                  uint4* __restrict__ chunk_prefix) {
+// The last blocks run the median splits meanwhile: Rust's
+// select_nth_unstable_by on the node's range, one thread per node.
+__global__ void __launch_bounds__(kBlock) level_prefix_select_kernel(
+    const uint32_t* __restrict__ lvl, const LevelCounters* lcs, uint32_t L, const BNode* __restrict__ pool,
+    const uint32_t* __restrict__ big_list, uint32_t big_cap, const uint4* __restrict__ chunk_cnt,
+    uint4* __restrict__ chunk_prefix, const float4* __restrict__ pbox, uint32_t* __restrict__ order) {
+  const uint32_t lb = lvl[L], W = lvl[L + 1] - lb;
+  for (uint32_t i = (gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x; i < W; i += gridDim.x * blockDim.x) {
+    const BNode n = pool[lb + i];
+    if (!(n.flags & F_FALLBACK)) continue;
+    const uint32_t count = n.end - n.start;
+    if (count / 2 == 0) continue;
+    const int axis = split_axis(box_of(n));
+    RustSelectNth<uint32_t, CentreLess> sel(CentreLess{&pbox[0].x + axis, 4u});
+    sel.run(order + n.start, count, count / 2);
+  }
   __shared__ uint4 warp_total[kWarps];
   __shared__ uint4 carry_s;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -566,38 +628,29 @@ __global__ void __launch_bounds__(kBlock) level_big_prefix_kernel(const LevelCou
   }
 }
 
-// Median split: Rust's select_nth_unstable_by on the node's range, one thread per node.
-__global__ void level_select_kernel(const uint32_t* __restrict__ lvl, uint32_t L, uint32_t N,
-                                    const BNode* __restrict__ pool, const float* __restrict__ cen,
-                                    uint32_t* __restrict__ order) {
-  const uint32_t lb = lvl[L], W = lvl[L + 1] - lb;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < W; i += gridDim.x * blockDim.x) {
-    const BNode n = pool[lb + i];
-    if (!(n.flags & F_FALLBACK)) continue;
-    const uint32_t count = n.end - n.start;
-    if (count / 2 == 0) continue;
-    const int axis = split_axis(box_of(n));
-    RustSelectNth<uint32_t, CentreLess> sel(CentreLess{cen + (size_t)axis * N});
-    sel.run(order + n.start, count, count / 2);
-  }
-}
-
-// SAH nodes: each chunk writes its primitives to their bucket-ordered slots.
-__global__ void level_scatter_kernel(const uint32_t* __restrict__ lvl, uint32_t L, uint32_t N,
-                                     const LevelCounters* lcs, const BNode* __restrict__ pool,
+// SAH nodes: each chunk writes its primitives to their bucket-ordered slots of
+// the other order array; a median-split node's are copied as they stand. Also
+// closes the level: the next level's end is its start plus the children that
+// level_decide_kernel created (decide ran before this launch).
+__global__ void level_scatter_kernel(uint32_t* __restrict__ lvl, uint32_t L, const LevelCounters* lcs, const BNode* __restrict__ pool,
                                      const uint32_t* __restrict__ chunk_node, const uint32_t* __restrict__ order,
-                                     const float* __restrict__ cen, const uint32_t* __restrict__ acc_cnt,
+                                     const uint8_t* __restrict__ bucket, const uint32_t* __restrict__ acc_cnt,
                                      const uint32_t* __restrict__ chunk_prefix, uint32_t* __restrict__ scratch) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t lt_mask = (1u << lane) - 1u;
   const uint32_t lb = lvl[L];
   const uint32_t total = lcs[L].chunks;
+  if (blockIdx.x == 0 && threadIdx.x == 0) lvl[L + 2] = lvl[L + 1] + lcs[L].children;
   for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < total; c += (gridDim.x * blockDim.x) >> 5) {
     const uint32_t id = chunk_node[c];
     const BNode n = pool[id];
-    if ((n.flags & (F_ACTIVE | F_FALLBACK)) != F_ACTIVE) continue;
-    const SplitPlane sp = plane_of(n);
-    const float* ck = cen + (size_t)sp.axis * N;
+    if (!(n.flags & F_ACTIVE)) continue;
+    if (n.flags & F_FALLBACK) {
+      uint32_t s, e;
+      chunk_range(n, c, s, e);
+      for (uint32_t i = s + lane; i < e; i += 32) scratch[i] = order[i];
+      continue;
+    }
     const uint32_t li = id - lb;
     uint32_t base[4];
     uint32_t run = n.start;
@@ -612,7 +665,7 @@ __global__ void level_scatter_kernel(const uint32_t* __restrict__ lvl, uint32_t 
       const uint32_t i = i0 + lane;
       const bool valid = i < e;
       const uint32_t p = valid ? order[i] : 0u;
-      const uint32_t bk = valid ? bucket_of(ck[p], sp.a0, sp.step) : 4u;
+      const uint32_t bk = valid ? bucket[i] : 4u;
       uint32_t dest = 0;
 #pragma unroll
       for (int q = 0; q < 4; q++) {
@@ -625,52 +678,404 @@ __global__ void level_scatter_kernel(const uint32_t* __restrict__ lvl, uint32_t 
   }
 }
 
-// Also closes the level: the next level's end is its start plus the children
-// that level_decide_kernel created (decide ran before this launch).
-__global__ void level_copyback_kernel(uint32_t* __restrict__ lvl, uint32_t L, const LevelCounters* lcs,
-                                      const BNode* __restrict__ pool, const uint32_t* __restrict__ chunk_node,
-                                      const uint32_t* __restrict__ scratch, uint32_t* __restrict__ order) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t total = lcs[L].chunks;
-  if (blockIdx.x == 0 && threadIdx.x == 0) lvl[L + 2] = lvl[L + 1] + lcs[L].children;
-  for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < total; c += (gridDim.x * blockDim.x) >> 5) {
-    const BNode n = pool[chunk_node[c]];
-    if ((n.flags & (F_ACTIVE | F_FALLBACK)) != F_ACTIVE) continue;
-    uint32_t s, e;
-    chunk_range(n, c, s, e);
-    for (uint32_t i = s + lane; i < e; i += 32) order[i] = scratch[i];
+// ---- subtrees -------------------------------------------------------------
+
+struct SmallNode {
+  int lo[3], hi[3];
+  uint16_t start, end, left, size, pre;  // left: NO_CHILD for a leaf; pre: place in the subtree's pre-order
+  uint16_t pending;
+};
+constexpr uint16_t NO_CHILD = 0xFFFF;
+struct SmallTree {
+  int lo[3][kSmall], hi[3][kSmall];  // boxes as keys
+  float cen[3][kSmall];
+  uint32_t prim[kSmall], order[kSmall], moved[kSmall];
+  SmallNode node[2 * kSmall];
+  uint16_t level[kSmall + 2];  // first node of each level
+  uint32_t count, sah, fallback, base;
+};
+constexpr uint32_t kSmallThreads = 128, kSmallWarps = kSmallThreads / 32;
+
+// The two children of a node that is split at mid, and the median split's order.
+__device__ __forceinline__ void small_children(SmallTree& S, SmallNode& n, const Split& s, uint32_t mid, const float* cen) {
+  const uint32_t child = atomicAdd(&S.count, 2u), start = n.start, end = n.end;
+  n.left = (uint16_t)child;
+  for (uint32_t c = 0; c < 2; c++) {
+    SmallNode& q = S.node[child + c];
+    const NodeBox& b = c ? s.r : s.l;
+    q.lo[0] = key_of(b.lo.x);
+    q.lo[1] = key_of(b.lo.y);
+    q.lo[2] = key_of(b.lo.z);
+    q.hi[0] = key_of(b.hi.x);
+    q.hi[1] = key_of(b.hi.y);
+    q.hi[2] = key_of(b.hi.z);
+    q.start = (uint16_t)(c ? mid : start);
+    q.end = (uint16_t)(c ? end : mid);
+    q.pending = s.fallback ? 1 : 0;
+  }
+  atomicAdd(s.fallback ? &S.fallback : &S.sah, 1u);
+  if (s.fallback) {
+    RustSelectNth<uint32_t, CentreLess> sel(CentreLess{cen, 0u});
+    sel.run(S.order + start, end - start, (end - start) / 2);
+  }
+}
+
+// Nodes of at most this many primitives (16: their bucket numbers fit a word)
+// are taken by a lane each: they are three of four nodes, and a warp each spends
+// most of its instructions on reductions over empty lanes (2.1 M triangles: the
+// kernel takes 520 us by warps alone, 365 with lanes).
+constexpr uint32_t kLaneNode = 16;
+
+__device__ __forceinline__ bool lane_node(SmallTree& S, uint32_t j, uint32_t bin_size, bool may_split) {
+  SmallNode& n = S.node[j];
+  const uint32_t start = n.start, end = n.end, count = end - start;
+  if (n.pending) {
+    int lo[3] = {key_of(INFINITY), key_of(INFINITY), key_of(INFINITY)};
+    int hi[3] = {key_of(-INFINITY), key_of(-INFINITY), key_of(-INFINITY)};
+    for (uint32_t i = start; i < end; i++) {
+      const uint32_t p = S.order[i];
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        lo[k] = min(lo[k], S.lo[k][p]);
+        hi[k] = max(hi[k], S.hi[k][p]);
+      }
+    }
+    for (int k = 0; k < 3; k++) {
+      n.lo[k] = lo[k];
+      n.hi[k] = hi[k];
+    }
+  }
+  n.left = NO_CHILD;
+  if (!(may_split && count > bin_size)) return true;
+  const NodeBox nb{{val_of(n.lo[0]), val_of(n.lo[1]), val_of(n.lo[2])}, {val_of(n.hi[0]), val_of(n.hi[1]), val_of(n.hi[2])}};
+  const int axis = split_axis(nb);
+  const float a0 = comp(nb.lo, axis), step = (comp(nb.hi, axis) - a0) / 4.0f;
+  const float* cen = S.cen[axis];
+  uint32_t cnt[4] = {0, 0, 0, 0}, buckets = 0;
+  int bx[4][6];
+#pragma unroll
+  for (int b = 0; b < 4; b++) {
+    bx[b][0] = bx[b][1] = bx[b][2] = key_of(INFINITY);
+    bx[b][3] = bx[b][4] = bx[b][5] = key_of(-INFINITY);
+  }
+  for (uint32_t i = 0; i < count; i++) {
+    const uint32_t p = S.order[start + i];
+    const uint32_t bk = bucket_of(cen[p], a0, step);
+    buckets |= bk << (2 * i);
+    const int k[6] = {S.lo[0][p], S.lo[1][p], S.lo[2][p], S.hi[0][p], S.hi[1][p], S.hi[2][p]};
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const bool in = bk == (uint32_t)q;
+      cnt[q] += in;
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        bx[q][c] = in ? min(bx[q][c], k[c]) : bx[q][c];
+        bx[q][3 + c] = in ? max(bx[q][3 + c], k[3 + c]) : bx[q][3 + c];
+      }
+    }
+  }
+  NodeBox bb[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+    bb[q] = NodeBox{{val_of(bx[q][0]), val_of(bx[q][1]), val_of(bx[q][2])}, {val_of(bx[q][3]), val_of(bx[q][4]), val_of(bx[q][5])}};
+  const Split s = decide_split(cnt, bb);
+  const uint32_t mid = s.fallback ? (start + end) / 2 : start + s.left;
+  if (mid == start || mid == end) return false;
+  small_children(S, n, s, mid, cen);
+  if (s.fallback) return true;
+  uint32_t base[4] = {start, start + cnt[0], start + cnt[0] + cnt[1], start + cnt[0] + cnt[1] + cnt[2]};
+  for (uint32_t i = 0; i < count; i++) {
+    const uint32_t bk = (buckets >> (2 * i)) & 3u;
+    uint32_t dest = 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      if (bk == (uint32_t)q) dest = base[q]++;
+    S.moved[dest] = S.order[start + i];
+  }
+  for (uint32_t i = start; i < end; i++) S.order[i] = S.moved[i];
+  return true;
+}
+
+// One node by one warp: its box if it is not known, then leaf or split, as the
+// level kernels do it. False, and a leaf, where a child would be empty.
+__device__ __forceinline__ bool small_node(SmallTree& S, uint32_t j, uint32_t bin_size, bool may_split) {
+  const uint32_t lane = threadIdx.x & 31u, lt_mask = (1u << lane) - 1u;
+  SmallNode& n = S.node[j];
+  const uint32_t start = n.start, end = n.end, count = end - start;
+  if (n.pending) {
+    int lo[3] = {key_of(INFINITY), key_of(INFINITY), key_of(INFINITY)};
+    int hi[3] = {key_of(-INFINITY), key_of(-INFINITY), key_of(-INFINITY)};
+    for (uint32_t i = start + lane; i < end; i += 32) {
+      const uint32_t p = S.order[i];
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        lo[k] = min(lo[k], S.lo[k][p]);
+        hi[k] = max(hi[k], S.hi[k][p]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      lo[k] = __reduce_min_sync(0xffffffffu, lo[k]);
+      hi[k] = __reduce_max_sync(0xffffffffu, hi[k]);
+      if (lane == 0) {
+        n.lo[k] = lo[k];
+        n.hi[k] = hi[k];
+      }
+    }
+    __syncwarp();
+  }
+  if (lane == 0) n.left = NO_CHILD;
+  if (!(may_split && count > bin_size)) return true;
+  const NodeBox nb{{val_of(n.lo[0]), val_of(n.lo[1]), val_of(n.lo[2])}, {val_of(n.hi[0]), val_of(n.hi[1]), val_of(n.hi[2])}};
+  const int axis = split_axis(nb);
+  const float a0 = comp(nb.lo, axis), step = (comp(nb.hi, axis) - a0) / 4.0f;
+  const float* cen = S.cen[axis];
+  uint32_t cnt[4] = {0, 0, 0, 0};
+  int bx[4][6];
+#pragma unroll
+  for (int b = 0; b < 4; b++) {
+    bx[b][0] = bx[b][1] = bx[b][2] = key_of(INFINITY);
+    bx[b][3] = bx[b][4] = bx[b][5] = key_of(-INFINITY);
+  }
+  for (uint32_t i = start + lane; i < end; i += 32) {
+    const uint32_t p = S.order[i];
+    const uint32_t bk = bucket_of(cen[p], a0, step);
+    const int k[6] = {S.lo[0][p], S.lo[1][p], S.lo[2][p], S.hi[0][p], S.hi[1][p], S.hi[2][p]};
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      if (bk == (uint32_t)q) {
+        cnt[q]++;
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          bx[q][c] = min(bx[q][c], k[c]);
+          bx[q][3 + c] = max(bx[q][3 + c], k[3 + c]);
+        }
+      }
+  }
+  NodeBox bb[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    cnt[q] = __reduce_add_sync(0xffffffffu, cnt[q]);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      bx[q][c] = __reduce_min_sync(0xffffffffu, bx[q][c]);
+      bx[q][3 + c] = __reduce_max_sync(0xffffffffu, bx[q][3 + c]);
+    }
+    bb[q] = NodeBox{{val_of(bx[q][0]), val_of(bx[q][1]), val_of(bx[q][2])}, {val_of(bx[q][3]), val_of(bx[q][4]), val_of(bx[q][5])}};
+  }
+  const Split s = decide_split(cnt, bb);
+  const uint32_t mid = s.fallback ? (start + end) / 2 : start + s.left;  // the range starts at a whole number
+  if (mid == start || mid == end) return false;
+  if (lane == 0) small_children(S, n, s, mid, cen);
+  __syncwarp();
+  if (s.fallback) return true;
+  uint32_t base[4] = {start, start + cnt[0], start + cnt[0] + cnt[1], start + cnt[0] + cnt[1] + cnt[2]};
+  for (uint32_t i0 = start; i0 < end; i0 += 32) {
+    const uint32_t i = i0 + lane;
+    const bool valid = i < end;
+    const uint32_t p = valid ? S.order[i] : 0u;
+    const uint32_t bk = valid ? bucket_of(cen[p], a0, step) : 4u;
+    uint32_t dest = 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const uint32_t m = __ballot_sync(0xffffffffu, bk == (uint32_t)q);
+      if (bk == (uint32_t)q) dest = base[q] + __popc(m & lt_mask);
+      base[q] += __popc(m);
+    }
+    if (valid) S.moved[dest] = p;
+  }
+  __syncwarp();
+  for (uint32_t i = start + lane; i < end; i += 32) S.order[i] = S.moved[i];
+  return true;
+}
+
+// Every node that left the level rounds: a subtree of at most `small`
+// primitives is built in shared memory, level by level, and added to the pool
+// in that order (children next to each other, behind their parents); a larger
+// leaf is closed. Afterwards order_a holds the final order, and every node has
+// its subtree's size and its place in that subtree's pre-order.
+__global__ void __launch_bounds__(kSmallThreads) small_trees_kernel(uint32_t small, uint32_t top,
+                                                                    const uint32_t* __restrict__ ended,
+                                                                    uint32_t bin_size, uint32_t max_depth,
+                                                                    BNode* __restrict__ pool, uint32_t* order_a,
+                                                                    const uint32_t* order_b,
+                                                                    const float4* __restrict__ pbox, BuildCounters* bc) {
+  __shared__ SmallTree S;
+  const uint32_t warp = threadIdx.x >> 5, total = bc->ended;
+  for (uint32_t e = blockIdx.x; e < total; e += gridDim.x) {
+    const uint32_t id = ended[e];
+    const BNode root = pool[id];
+    const uint32_t count = root.end - root.start;
+    const uint32_t* src = (root.flags & F_IN_B ? order_b : order_a) + root.start;
+    __syncthreads();  // the previous subtree has been written, and every thread has read this root
+    if (count > small) {
+      if (root.flags & F_IN_B)
+        for (uint32_t i = threadIdx.x; i < count; i += kSmallThreads) order_a[root.start + i] = src[i];
+      if (threadIdx.x == 0) {
+        pool[id].cbase = 1;
+        pool[id].nchunks = 0;
+        pool[id].sub = id;
+        atomicMax(&bc->max_depth, root.depth);
+      }
+      continue;
+    }
+    for (uint32_t i = threadIdx.x; i < count; i += kSmallThreads) {
+      const uint32_t p = src[i];
+      const float4 a = pbox[2 * (size_t)p], b = pbox[2 * (size_t)p + 1];
+      S.prim[i] = p;
+      S.order[i] = i;
+      S.lo[0][i] = key_of(a.x);
+      S.lo[1][i] = key_of(a.y);
+      S.lo[2][i] = key_of(a.z);
+      S.hi[0][i] = key_of(b.x);
+      S.hi[1][i] = key_of(b.y);
+      S.hi[2][i] = key_of(b.z);
+      S.cen[0][i] = (a.x + b.x) * 0.5f;
+      S.cen[1][i] = (a.y + b.y) * 0.5f;
+      S.cen[2][i] = (a.z + b.z) * 0.5f;
+    }
+    if (threadIdx.x == 0) {
+      SmallNode& n = S.node[0];
+      for (int k = 0; k < 3; k++) {
+        n.lo[k] = root.lo[k];
+        n.hi[k] = root.hi[k];
+      }
+      n.start = 0;
+      n.end = (uint16_t)count;
+      n.pending = (root.flags & F_BOX_PENDING) ? 1 : 0;
+      S.count = 1;
+      S.sah = S.fallback = 0;
+    }
+    __syncthreads();
+    uint32_t first = 0, last = 1, levels = 0;
+    while (first < last) {
+      if (threadIdx.x == 0) S.level[levels] = (uint16_t)first;
+      const bool may_split = root.depth + levels < max_depth;
+      for (uint32_t j = first + warp; j < last; j += kSmallWarps)
+        if (S.node[j].end - S.node[j].start > (int)kLaneNode && !small_node(S, j, bin_size, may_split)) bc->unfit = 1u;
+      for (uint32_t j = first + threadIdx.x; j < last; j += kSmallThreads)
+        if (S.node[j].end - S.node[j].start <= (int)kLaneNode && !lane_node(S, j, bin_size, may_split)) bc->unfit = 1u;
+      __syncthreads();
+      levels++;
+      first = last;
+      last = S.count;
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) S.level[levels] = (uint16_t)last;
+    __syncthreads();
+    for (uint32_t l = levels; l-- > 0;) {
+      for (uint32_t j = S.level[l] + threadIdx.x; j < S.level[l + 1]; j += kSmallThreads) {
+        const uint32_t c = S.node[j].left;
+        S.node[j].size = c == NO_CHILD ? 1 : (uint16_t)(1 + S.node[c].size + S.node[c + 1].size);
+      }
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+      S.node[0].pre = 0;
+      S.base = last > 1 ? top + atomicAdd(&bc->added, last - 1) : 0u;
+      if (S.sah) atomicAdd(&bc->sah, (unsigned long long)S.sah);
+      if (S.fallback) atomicAdd(&bc->fallback, (unsigned long long)S.fallback);
+      atomicMax(&bc->max_depth, root.depth + levels - 1);
+    }
+    __syncthreads();
+    for (uint32_t l = 0; l < levels; l++) {
+      for (uint32_t j = S.level[l] + threadIdx.x; j < S.level[l + 1]; j += kSmallThreads) {
+        const uint32_t c = S.node[j].left, pre = S.node[j].pre;
+        if (c != NO_CHILD) {
+          S.node[c].pre = (uint16_t)(pre + 1);
+          S.node[c + 1].pre = (uint16_t)(pre + 1 + S.node[c].size);
+        }
+        const SmallNode& n = S.node[j];
+        BNode o;
+        for (int k = 0; k < 3; k++) {
+          o.lo[k] = n.lo[k];
+          o.hi[k] = n.hi[k];
+        }
+        o.start = root.start + n.start;
+        o.end = root.start + n.end;
+        o.depth = root.depth + l;
+        o.left = c == NO_CHILD ? NONE : S.base + c - 1;
+        o.tree = root.tree;
+        o.flags = 0;
+        o.cbase = n.size;
+        o.nchunks = pre;
+        o.sub = id;
+        o.pad = 0;
+        pool[j == 0 ? id : S.base + j - 1] = o;
+      }
+      __syncthreads();
+    }
+    for (uint32_t i = threadIdx.x; i < count; i += kSmallThreads) order_a[root.start + i] = S.prim[S.order[i]];
   }
 }
 
 // ---- numbering and emission --------------------------------------------
 
-__global__ void subtree_size_kernel(uint32_t lb, uint32_t W, const BNode* __restrict__ pool, uint32_t* __restrict__ size) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= W) return;
-  const uint32_t l = pool[lb + i].left;
-  size[lb + i] = l == NONE ? 1u : 1u + size[l] + size[l + 1];
+// Numbering above the subtrees, by one block: subtree sizes bottom-up (in
+// cbase), the geometries' first nodes by a scan of their trees' sizes, and the
+// reference's pre-order numbers top-down.
+constexpr uint32_t kNumberThreads = 1024;
+__global__ void __launch_bounds__(kNumberThreads) top_numbering_kernel(const uint32_t* __restrict__ lvl, uint32_t levels,
+                                                                       uint32_t G, BNode* __restrict__ pool,
+                                                                       uint32_t* __restrict__ tree_end,
+                                                                       uint32_t* __restrict__ tree_nodes,
+                                                                       uint32_t* __restrict__ pre) {
+  __shared__ uint32_t warp_sums[kNumberThreads / 32], carry;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  for (uint32_t l = levels; l-- > 0;) {
+    for (uint32_t i = lvl[l] + threadIdx.x; i < lvl[l + 1]; i += kNumberThreads) {
+      const uint32_t c = pool[i].left;
+      if (pool[i].sub == NONE) pool[i].cbase = 1u + pool[c].cbase + pool[c + 1].cbase;  // nodes above are inner
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) carry = 0;
+  __syncthreads();
+  for (uint32_t g0 = 0; g0 < G; g0 += kNumberThreads) {
+    const uint32_t g = g0 + threadIdx.x;
+    const uint32_t size = g < G ? pool[g].cbase : 0u;
+    const uint32_t inc = warp_inclusive_u32(size, lane);
+    if (lane == 31) warp_sums[warp] = inc;
+    __syncthreads();
+    uint32_t before = carry + inc - size, total = 0;
+    for (uint32_t w = 0; w < kNumberThreads / 32; w++) {
+      if (w < warp) before += warp_sums[w];
+      total += warp_sums[w];
+    }
+    if (g < G) {
+      pre[g] = before;
+      tree_end[g] = before + size;
+      tree_nodes[g] = size;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) carry += total;
+    __syncthreads();
+  }
+  for (uint32_t l = 0; l < levels; l++) {
+    for (uint32_t i = lvl[l] + threadIdx.x; i < lvl[l + 1]; i += kNumberThreads) {
+      if (pool[i].sub != NONE) continue;
+      const uint32_t c = pool[i].left, me = pre[i];
+      pre[c] = me + 1;
+      pre[c + 1] = me + 1 + pool[c].cbase;
+    }
+    __syncthreads();
+  }
 }
 
-__global__ void preorder_roots_kernel(uint32_t G, const uint32_t* __restrict__ bvh_start, uint32_t* __restrict__ pre) {
-  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g < G) pre[g] = bvh_start[g];
-}
-
-__global__ void preorder_level_kernel(uint32_t lb, uint32_t W, const BNode* __restrict__ pool,
-                                      const uint32_t* __restrict__ size, uint32_t* __restrict__ pre) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= W) return;
-  const uint32_t l = pool[lb + i].left;
-  if (l == NONE) return;
-  const uint32_t me = pre[lb + i];
-  pre[l] = me + 1;
-  pre[l + 1] = me + 1 + size[l];
-}
-
-__global__ void inner_flags_kernel(uint32_t T, const BNode* __restrict__ pool, const uint32_t* __restrict__ pre,
+// Pre-order numbers of the subtrees' nodes, and which numbers are inner nodes.
+__global__ void inner_flags_kernel(uint32_t T, const BNode* __restrict__ pool, uint32_t* __restrict__ pre,
                                    uint32_t* __restrict__ inner_at) {
   const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
-  if (id < T) inner_at[pre[id]] = pool[id].left != NONE ? 1u : 0u;
+  if (id >= T) return;
+  const uint32_t sub = pool[id].sub;
+  uint32_t g;
+  if (sub == NONE || sub == id) {
+    g = pre[id];
+  } else {
+    g = pre[sub] + pool[id].nchunks;
+    pre[id] = g;
+  }
+  inner_at[g] = pool[id].left != NONE ? 1u : 0u;
 }
 
 __device__ __forceinline__ uint32_t code_of(uint32_t id, const BNode* pool, const uint32_t* pre, const uint32_t* rank) {
@@ -678,7 +1083,7 @@ __device__ __forceinline__ uint32_t code_of(uint32_t id, const BNode* pool, cons
   return pool[id].left != NONE ? rank[g] : (LEAF_BIT | (g - rank[g]));
 }
 
-__global__ void emit_nodes_kernel(uint32_t T, uint32_t G, const BNode* __restrict__ pool, const uint32_t* __restrict__ size,
+__global__ void emit_nodes_kernel(uint32_t T, uint32_t G, const BNode* __restrict__ pool,
                                   const uint32_t* __restrict__ pre, const uint32_t* __restrict__ rank,
                                   const uint32_t* __restrict__ tree_end, DeviceBVHNode* __restrict__ forest,
                                   WideNode* __restrict__ wide, uint32_t* __restrict__ leaves,
@@ -689,32 +1094,20 @@ __global__ void emit_nodes_kernel(uint32_t T, uint32_t G, const BNode* __restric
   const NodeBox b = box_of(n);
   const uint32_t g = pre[id];
   const bool inner = n.left != NONE;
-  const uint32_t next = g + size[id];
+  const uint32_t next = g + n.cbase;
   const uint32_t miss = next < tree_end[n.tree] ? next : INVALID_NEXT;
-  DeviceBVHNode o;
-  o.aabb_min[0] = b.lo.x;
-  o.aabb_min[1] = b.lo.y;
-  o.aabb_min[2] = b.lo.z;
-  o.hit_next = inner ? g + 1 : miss;
-  o.aabb_max[0] = b.hi.x;
-  o.aabb_max[1] = b.hi.y;
-  o.aabb_max[2] = b.hi.z;
-  o.miss_next = miss;
-  o.content_range[0] = n.start;
-  o.content_range[1] = n.end;
-  o.tail[0] = 0;
-  o.tail[1] = 0;
-  forest[g] = o;
+  float4* o = reinterpret_cast<float4*>(forest + g);  // DeviceBVHNode
+  o[0] = make_float4(b.lo.x, b.lo.y, b.lo.z, __uint_as_float(inner ? g + 1 : miss));
+  o[1] = make_float4(b.hi.x, b.hi.y, b.hi.z, __uint_as_float(miss));
+  o[2] = make_float4(__uint_as_float(n.start), __uint_as_float(n.end), 0.0f, 0.0f);
   if (inner) {
     const NodeBox a = box_of(pool[n.left]), c = box_of(pool[n.left + 1]);
-    WideNode w;
-    const float vals[12] = {a.lo.x, a.lo.y, a.lo.z, a.hi.x, a.hi.y, a.hi.z, c.lo.x, c.lo.y, c.lo.z, c.hi.x, c.hi.y, c.hi.z};
-    for (int k = 0; k < 12; k++) w.w[k] = vals[k];
-    w.code[0] = code_of(n.left, pool, pre, rank);
-    w.code[1] = code_of(n.left + 1, pool, pre, rank);
-    w.code[2] = 0;
-    w.code[3] = 0;
-    wide[rank[g]] = w;
+    float4* w = reinterpret_cast<float4*>(wide + rank[g]);  // WideNode
+    w[0] = make_float4(a.lo.x, a.lo.y, a.lo.z, a.hi.x);
+    w[1] = make_float4(a.hi.y, a.hi.z, c.lo.x, c.lo.y);
+    w[2] = make_float4(c.lo.z, c.hi.x, c.hi.y, c.hi.z);
+    w[3] = make_float4(__uint_as_float(code_of(n.left, pool, pre, rank)),
+                       __uint_as_float(code_of(n.left + 1, pool, pre, rank)), 0.0f, 0.0f);
   } else {
     const uint32_t l = g - rank[g];
     leaves[2 * (size_t)l] = n.start;
@@ -838,65 +1231,114 @@ __device__ __forceinline__ int collapse_slots(uint32_t b, const BNode* pool, uin
   return n;
 }
 
-// Four-child layout without a host round trip per level: the binary nodes
-// that root a four-child node ("collapse roots") are marked top-down, one
-// binary level per launch (a root's slots lie one to three levels below it,
-// so they are marked before their level runs); one scan numbers the roots in
-// pool order and one launch emits every node.
-__global__ void wide4_roots_kernel(uint32_t G, const BNode* __restrict__ pool, uint32_t* __restrict__ croot,
-                                   uint32_t* __restrict__ level4, uint32_t* __restrict__ max_level4) {
-  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= G || pool[g].left == NONE) return;
-  croot[g] = 1u;
-  level4[g] = 1u;
-  atomicMax(max_level4, 1u);
+__device__ __forceinline__ uint4 collapse(uint32_t b, const BNode* pool) {
+  uint32_t slot[4];
+  const int n = collapse_slots(b, pool, slot);
+  return make_uint4(slot[0], slot[1], n > 2 ? slot[2] : NONE, n > 3 ? slot[3] : NONE);
 }
 
-__global__ void wide4_mark_kernel(uint32_t lb, uint32_t W, const BNode* __restrict__ pool,
-                                  uint32_t* __restrict__ croot, uint32_t* __restrict__ level4,
-                                  uint32_t* __restrict__ max_level4) {
+// Four-child layout: the binary nodes that root a four-child node ("collapse
+// roots") are marked top-down, their slots are kept, one scan numbers the roots
+// in pool order and one launch emits every node. A collapse is a chain of
+// dependent loads, the marks only follow its result: above the subtrees every
+// inner node is collapsed at once, root or not, and one block then walks the
+// levels (2 M triangles: 200 us as a launch per level that collapses its roots).
+__global__ void wide4_slots_kernel(uint32_t top, const BNode* __restrict__ pool, uint4* __restrict__ slots) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= W || !croot[lb + i]) return;
-  uint32_t slot[4];
-  const int n = collapse_slots(lb + i, pool, slot);
-  const uint32_t lv = level4[lb + i] + 1u;
-  for (int k = 0; k < n; k++)
-    if (pool[slot[k]].left != NONE) {
-      croot[slot[k]] = 1u;
-      level4[slot[k]] = lv;
-      atomicMax(max_level4, lv);
+  if (i < top && pool[i].sub == NONE) slots[i] = collapse(i, pool);
+}
+
+// Marks the slots of collapse root b that are roots themselves.
+__device__ __forceinline__ void mark_slots(const uint4& s, uint32_t level, const BNode* pool, volatile uint32_t* croot,
+                                           volatile uint32_t* level4, uint32_t& deepest) {
+  const uint32_t slot[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+    if (slot[q] != NONE && pool[slot[q]].left != NONE) {
+      croot[slot[q]] = 1u;
+      level4[slot[q]] = level + 1u;
+      deepest = max(deepest, level + 1u);
     }
+}
+
+__global__ void __launch_bounds__(kNumberThreads) wide4_top_kernel(const uint32_t* __restrict__ lvl, uint32_t levels,
+                                                                   uint32_t G, const BNode* __restrict__ pool,
+                                                                   const uint4* __restrict__ slots,
+                                                                   volatile uint32_t* croot, volatile uint32_t* level4,
+                                                                   uint32_t* __restrict__ max_level4) {
+  uint32_t deepest = 0;
+  for (uint32_t g = threadIdx.x; g < G; g += kNumberThreads)
+    if (pool[g].left != NONE) {
+      croot[g] = level4[g] = 1u;
+      deepest = 1u;
+    }
+  __syncthreads();
+  for (uint32_t l = 0; l < levels; l++) {
+    for (uint32_t i = lvl[l] + threadIdx.x; i < lvl[l + 1]; i += kNumberThreads)
+      if (croot[i] && pool[i].sub == NONE) mark_slots(slots[i], level4[i], pool, croot, level4, deepest);
+    __syncthreads();
+  }
+  deepest = __reduce_max_sync(0xffffffffu, deepest);
+  if ((threadIdx.x & 31u) == 0 && deepest) atomicMax(max_level4, deepest);
+}
+
+// The same below a subtree's root, a warp per subtree: its nodes lie behind the
+// root's children in level order.
+__global__ void wide4_mark_small_kernel(const uint32_t* __restrict__ ended, const BuildCounters* bc,
+                                        const BNode* __restrict__ pool, uint4* __restrict__ slots,
+                                        volatile uint32_t* croot, volatile uint32_t* level4,
+                                        uint32_t* __restrict__ max_level4) {
+  const uint32_t lane = threadIdx.x & 31u, total = bc->ended;
+  for (uint32_t e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < total; e += (gridDim.x * blockDim.x) >> 5) {
+    const uint32_t id = ended[e];
+    const uint32_t m = pool[id].cbase, first = pool[id].left;  // node j > 0 of the subtree is pool[first + j - 1]
+    if (m <= 1) continue;
+    uint32_t depth = pool[id].depth, deepest = 0;
+    for (uint32_t j = 0; j < m;) {
+      // the nodes of one level, as far as a warp reaches
+      const uint32_t k = j + lane, node = k == 0 ? id : first + k - 1;
+      const bool in = k < m && pool[node].depth == depth;
+      if (in && croot[node]) {
+        const uint4 s = collapse(node, pool);
+        slots[node] = s;
+        mark_slots(s, level4[node], pool, croot, level4, deepest);
+      }
+      __syncwarp();
+      const uint32_t taken = __popc(__ballot_sync(0xffffffffu, in));
+      j += taken;
+      if (taken < 32u) depth++;
+    }
+    deepest = __reduce_max_sync(0xffffffffu, deepest);
+    if (lane == 0 && deepest) atomicMax(max_level4, deepest);
+  }
 }
 
 __global__ void wide4_emit_kernel(uint32_t T, bool packed, const BNode* __restrict__ pool, const uint32_t* __restrict__ croot,
-                                  const uint32_t* __restrict__ index4, const uint32_t* __restrict__ pre,
-                                  const uint32_t* __restrict__ rank, Wide4Node* __restrict__ out) {
+                                  const uint4* __restrict__ slots, const uint32_t* __restrict__ index4,
+                                  const uint32_t* __restrict__ pre, const uint32_t* __restrict__ rank,
+                                  Wide4Node* __restrict__ out) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= T || !croot[i]) return;
-  uint32_t slot[4];
-  const int n = collapse_slots(i, pool, slot);
-  Wide4Node w;
+  const uint4 s = slots[i];
+  const uint32_t slot[4] = {s.x, s.y, s.z, s.w};
+  float4* o = reinterpret_cast<float4*>(out + index4[i]);  // Wide4Child: lo_x lo_y hi_x hi_y lo_z hi_z code pad
+#pragma unroll
   for (int k = 0; k < 4; k++) {
-    const bool used = k < n;
-    const NodeBox b = used ? box_of(pool[slot[k]]) : NodeBox{{NAN, NAN, NAN}, {NAN, NAN, NAN}};
-    w.child[k].lo_x = b.lo.x;
-    w.child[k].lo_y = b.lo.y;
-    w.child[k].lo_z = b.lo.z;
-    w.child[k].hi_x = b.hi.x;
-    w.child[k].hi_y = b.hi.y;
-    w.child[k].hi_z = b.hi.z;
-    w.child[k].pad = 0;
-    if (!used) {
-      w.child[k].code = EMPTY_SLOT;
-    } else if (pool[slot[k]].left != NONE) {
-      w.child[k].code = index4[slot[k]];
-    } else {
-      const uint32_t g = pre[slot[k]];
-      const uint32_t leaf = g - rank[g];
-      w.child[k].code = packed ? packed_leaf(leaf, pool[slot[k]].start, pool[slot[k]].end) : (LEAF_BIT | leaf);
+    NodeBox b{{NAN, NAN, NAN}, {NAN, NAN, NAN}};
+    uint32_t code = EMPTY_SLOT;
+    if (slot[k] != NONE) {
+      const BNode c = pool[slot[k]];
+      b = box_of(c);
+      if (c.left != NONE) {
+        code = index4[slot[k]];
+      } else {
+        const uint32_t g = pre[slot[k]], leaf = g - rank[g];
+        code = packed ? packed_leaf(leaf, c.start, c.end) : (LEAF_BIT | leaf);
+      }
     }
+    o[2 * k] = make_float4(b.lo.x, b.lo.y, b.hi.x, b.hi.y);
+    o[2 * k + 1] = make_float4(b.lo.z, b.hi.z, __uint_as_float(code), 0.0f);
   }
-  out[index4[i]] = w;
 }
 
 // ---- host side -------------------------------------------------------------
@@ -1010,13 +1452,13 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
   }
 
   float4* pbox;
-  float* cen;
-  uint32_t *order, *scratch;
+  uint8_t* bucket;  // per primitive in the level's order
+  uint32_t *order, *order_b;
   BuildCounters* bc;
   CK(S.alloc(&pbox, 2 * (size_t)N));
-  CK(S.alloc(&cen, 3 * (size_t)N));
+  CK(S.alloc(&bucket, N));
   CK(S.alloc(&order, N));
-  CK(S.alloc(&scratch, N));
+  CK(S.alloc(&order_b, N));
   CK(S.alloc(&bc, 1));
   CK(cudaMemsetAsync(bc, 0, sizeof(BuildCounters), st));
   const uint32_t persistent = (uint32_t)(sm_count > 0 ? sm_count : 1) * 8;
@@ -1033,110 +1475,124 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
   CK(cudaEventRecord(ev0, st));
   if (N) {
     prepare_primitives_kernel<<<std::min(blocks_for(N), persistent * 4), kBlock, 0, st>>>(
-        N, G, dg_prim, dg_vs, dg_vc, dg_ix, d.indices.ptr, d.vertices.ptr, pbox, cen, order, bc);
+        N, G, dg_prim, dg_vs, dg_vc, dg_ix, d.indices.ptr, d.vertices.ptr, pbox, order, bc);
     CK(cudaGetLastError());
-    // stop before any kernel reads a vertex through an out-of-range index
-    BuildCounters pre;
-    CK(cudaMemcpyAsync(&pre, bc, sizeof(pre), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    if (pre.bad_index) return "triangle index out of range";
   }
 
   // roots: one per geometry, box pending
   size_t cap = 2 * (size_t)N + 2 * (size_t)G + 64;
   BNode* pool;
   CK(S.alloc(&pool, cap));
-  {
-    std::vector<BNode> roots(G);
-    for (uint32_t g = 0; g < G; g++) {
-      BNode& r = roots[g];
-      std::memset(&r, 0, sizeof(r));
-      for (int k = 0; k < 3; k++) {
-        r.lo[k] = key_of(INFINITY);
-        r.hi[k] = key_of(-INFINITY);
-      }
-      r.start = g_prim[g];
-      r.end = g_prim[g + 1];
-      r.depth = 0;
-      r.left = NONE;
-      r.tree = g;
-      r.flags = F_BOX_PENDING;
+  std::vector<BNode> roots(G);
+  for (uint32_t g = 0; g < G; g++) {
+    BNode& r = roots[g];
+    std::memset(&r, 0, sizeof(r));
+    for (int k = 0; k < 3; k++) {
+      r.lo[k] = key_of(INFINITY);
+      r.hi[k] = key_of(-INFINITY);
     }
-    if (G) CK(cudaMemcpyAsync(pool, roots.data(), sizeof(BNode) * G, cudaMemcpyHostToDevice, st));
+    r.start = g_prim[g];
+    r.end = g_prim[g + 1];
+    r.depth = 0;
+    r.left = r.sub = NONE;
+    r.tree = g;
+    r.flags = F_BOX_PENDING;
   }
+  if (G) CK(cudaMemcpyAsync(pool, roots.data(), sizeof(BNode) * G, cudaMemcpyHostToDevice, st));
 
-  // level rounds. Every buffer is sized for the largest possible level (a
-  // level holds at most N + G nodes: ranges are disjoint and only empty roots
-  // are empty), so that no level waits for the host. The host queues a batch
-  // of levels, then reads the level bounds back once to see whether an empty
-  // level has been reached; levels queued past it do nothing.
+  // level rounds. Every buffer is sized for the largest possible level (nodes
+  // that are split hold more than `small` and more than bin_size primitives,
+  // and their ranges are disjoint), so that no level waits for the host. The
+  // host queues a batch of levels, then reads the level bounds back once to see
+  // whether an empty level has been reached; levels queued past it do nothing.
+  // A split with an empty child (areas beyond the float range) can repeat down
+  // to max_depth, which the subtree blocks have no room for: such a forest is
+  // built over, by level rounds alone.
   const uint32_t level_cap = (uint32_t)std::min<uint64_t>(max_depth, N) + 2;  // possible levels + one empty
-  const size_t node_cap = (size_t)N + G + 1;
-  const size_t chunk_cap = (size_t)N / kChunk + node_cap + 1;
   const uint32_t big_cap = N / (kBigChunks * kChunk) + 2;  // a big node holds > kBigChunks * kChunk primitives
-  uint32_t *lvl, *acc_cnt, *chunk_node, *chunk_cnt, *chunk_prefix, *big_list;
+  uint32_t *lvl, *acc_cnt, *chunk_node, *chunk_cnt, *chunk_prefix, *big_list, *ended;
   LevelCounters* lcs;
   int* acc_box;
   CK(S.alloc(&lvl, (size_t)level_cap + 2));
   CK(S.alloc(&lcs, level_cap));
-  CK(S.alloc(&acc_cnt, 4 * node_cap));
-  CK(S.alloc(&acc_box, 24 * node_cap));
-  CK(S.alloc(&chunk_node, chunk_cap));
-  CK(S.alloc(&chunk_cnt, 4 * chunk_cap));
-  CK(S.alloc(&chunk_prefix, 4 * chunk_cap));
   CK(S.alloc(&big_list, big_cap));
-  CK(cudaMemsetAsync(lcs, 0, sizeof(LevelCounters) * level_cap, st));
+  CK(S.alloc(&ended, cap));
   const uint32_t lvl0[2] = {0, G};
-  CK(cudaMemcpyAsync(lvl, lvl0, sizeof(lvl0), cudaMemcpyHostToDevice, st));
   std::vector<uint32_t> h_lvl((size_t)level_cap + 2);
-  uint32_t queued = 0, levels = 0;
-  bool closed = false;
-  // first batch: about the depth of a balanced tree, then a few levels at a time
-  uint32_t batch = 2;
-  for (uint64_t m = std::max<uint32_t>(bin_size, 1); m < N; m *= 2) batch++;
-  while (!closed) {
-    const uint32_t stop = std::min(queued + batch, level_cap);
-    batch = 4;
-    for (; queued < stop; queued++) {
-      const uint32_t L = queued;
-      level_prepare_kernel<<<persistent, kBlock, 0, st>>>(lvl, L, bin_size, max_depth, pool, acc_cnt, acc_box,
-                                                          chunk_node, lcs);
-      level_box_kernel<<<persistent, kBlock, 0, st>>>(lcs, L, pool, chunk_node, order, pbox);
-      level_stats_kernel<<<persistent, kBlock, 0, st>>>(lvl, L, N, lcs, pool, chunk_node, order, pbox, cen,
-                                                        chunk_cnt, acc_cnt, acc_box);
-      level_decide_kernel<<<persistent, kBlock, 0, st>>>(lvl, L, pool, acc_cnt, acc_box,
-                                                         reinterpret_cast<const uint4*>(chunk_cnt),
-                                                         reinterpret_cast<uint4*>(chunk_prefix), lcs, bc, big_list,
-                                                         big_cap);
-      level_big_prefix_kernel<<<persistent, kBlock, 0, st>>>(lcs, L, pool, big_list, big_cap,
-                                                             reinterpret_cast<const uint4*>(chunk_cnt),
-                                                             reinterpret_cast<uint4*>(chunk_prefix));
-      level_select_kernel<<<persistent, kBlock, 0, st>>>(lvl, L, N, pool, cen, order);
-      level_scatter_kernel<<<persistent, kBlock, 0, st>>>(lvl, L, N, lcs, pool, chunk_node, order, cen, acc_cnt,
-                                                          chunk_prefix, scratch);
-      level_copyback_kernel<<<persistent, kBlock, 0, st>>>(lvl, L, lcs, pool, chunk_node, scratch, order);
-    }
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(h_lvl.data(), lvl, 4 * ((size_t)queued + 2), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    for (uint32_t k = 0; k <= queued && !closed; k++)
-      if (h_lvl[k + 1] == h_lvl[k]) {  // level k is empty: the tree has k levels
-        levels = k;
-        closed = true;
+  uint32_t levels = 0;
+  BuildCounters hbc;
+  for (uint32_t small = kSmall;; small = 0) {
+    const size_t node_cap = 2 * (size_t)N / (std::max(bin_size, small) + 1ull) + G + 1;
+    const size_t chunk_cap = (size_t)N / kChunk + node_cap + 1;
+    CK(S.alloc(&acc_cnt, 4 * node_cap));
+    CK(S.alloc(&acc_box, 24 * node_cap));
+    CK(S.alloc(&chunk_node, chunk_cap));
+    CK(S.alloc(&chunk_cnt, 4 * chunk_cap));
+    CK(S.alloc(&chunk_prefix, 4 * chunk_cap));
+    CK(cudaMemsetAsync(lcs, 0, sizeof(LevelCounters) * level_cap, st));
+    CK(cudaMemcpyAsync(lvl, lvl0, sizeof(lvl0), cudaMemcpyHostToDevice, st));
+    uint32_t queued = 0;
+    bool closed = false;
+    // first batch: about the depth of a balanced tree, then a few levels at a time
+    uint32_t batch = 2;
+    for (uint64_t m = std::max<uint32_t>(std::max(bin_size, small), 1); m < N; m *= 2) batch++;
+    while (!closed) {
+      const uint32_t stop = std::min(queued + batch, level_cap);
+      batch = 4;
+      for (; queued < stop; queued++) {
+        const uint32_t L = queued;
+        uint32_t *from = L & 1 ? order_b : order, *to = L & 1 ? order : order_b;
+        level_prepare_kernel<<<persistent, kBlock, 0, st>>>(lvl, L, bin_size, max_depth, pool, acc_cnt, acc_box,
+                                                            chunk_node, lcs, small, bc, ended);
+        level_box_kernel<<<persistent, kBlock, 0, st>>>(lcs, L, pool, chunk_node, from, pbox);
+        level_stats_kernel<<<persistent, kBlock, 0, st>>>(lvl, L, lcs, pool, chunk_node, from, pbox, bucket,
+                                                          chunk_cnt, acc_cnt, acc_box);
+        level_decide_kernel<<<persistent, kBlock, 0, st>>>(lvl, L, pool, acc_cnt, acc_box,
+                                                           reinterpret_cast<const uint4*>(chunk_cnt),
+                                                           reinterpret_cast<uint4*>(chunk_prefix), lcs, bc, big_list,
+                                                           big_cap, (uint32_t)std::min<uint64_t>(cap, NONE));
+        level_prefix_select_kernel<<<persistent, kBlock, 0, st>>>(lvl, lcs, L, pool, big_list, big_cap,
+                                                                  reinterpret_cast<const uint4*>(chunk_cnt),
+                                                                  reinterpret_cast<uint4*>(chunk_prefix), pbox, from);
+        level_scatter_kernel<<<persistent, kBlock, 0, st>>>(lvl, L, lcs, pool, chunk_node, from, bucket, acc_cnt,
+                                                            chunk_prefix, to);
       }
-    if (!closed && queued >= level_cap) return "device build: tree deeper than its level bound";
+      CK(cudaGetLastError());
+      if (!d.tri_records.ptr) {  // while the levels run
+        CK(alloc_out(d.indices_redirect, N, bytes, st));
+        CK(alloc_out(d.tri_records, N, bytes, st));
+      }
+      CK(cudaMemcpyAsync(h_lvl.data(), lvl, 4 * ((size_t)queued + 2), cudaMemcpyDeviceToHost, st));
+      CK(cudaMemcpyAsync(&hbc, bc, sizeof(hbc), cudaMemcpyDeviceToHost, st));
+      CK(cudaStreamSynchronize(st));
+      if (hbc.bad_index) return "triangle index out of range";  // no kernel has read a vertex through the indices yet
+      if (hbc.overflow) return "device build: more nodes than the build holds";
+      for (uint32_t k = 0; k <= queued && !closed; k++)
+        if (h_lvl[k + 1] == h_lvl[k]) {  // level k is empty: the tree has k levels
+          levels = k;
+          closed = true;
+        }
+      if (!closed && queued >= level_cap) return "device build: tree deeper than its level bound";
+    }
+    if (hbc.ended && !(small && hbc.unfit))
+      small_trees_kernel<<<std::min(hbc.ended, 1u << 20), kSmallThreads, 0, st>>>(small, h_lvl[levels], ended, bin_size, max_depth,
+                                                                  pool, order, order_b, pbox, bc);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(&hbc, bc, sizeof(hbc), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    if (!(small && hbc.unfit)) break;
+    CK(cudaMemsetAsync(bc, 0, sizeof(BuildCounters), st));
+    restart_kernel<<<std::min(blocks_for(N), persistent), kBlock, 0, st>>>(N, order);
+    CK(cudaMemcpyAsync(pool, roots.data(), sizeof(BNode) * G, cudaMemcpyHostToDevice, st));
   }
-  std::vector<uint32_t> level_begin(h_lvl.begin(), h_lvl.begin() + levels + 1);
-  const uint32_t T = h_lvl[levels];
-  level_begin.push_back(T);  // level l = [level_begin[l], level_begin[l+1]); the last entry repeats T
-  const uint32_t L = (uint32_t)level_begin.size() - 2;  // number of levels (0 when G == 0)
-  out.max_depth = L ? L - 1 : 0;
+  // the level rounds' nodes, then those of the subtrees
+  const uint32_t T = h_lvl[levels] + hbc.added;
+  out.max_depth = hbc.max_depth;
   out.nodes = T;
 
   // The four-child collapse reads only the finished binary tree: its marks
-  // and numbering scan run on a side stream, overlapped with the subtree
-  // sizes, the pre-order numbering and their host round trips below; the
-  // emit waits for them.
+  // and numbering scan run on a side stream, overlapped with the
+  // pre-order numbering and the allocations below; the emit waits for them.
   struct SideStream {
     cudaStream_t s = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
@@ -1153,6 +1609,8 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
   CK(S.alloc(&croot, T));
   CK(S.alloc(&level4, T));
   CK(S.alloc(&index4, T));
+  uint4* slots;
+  CK(S.alloc(&slots, T));
   CK(S.alloc(&max_level4, 1));
   void* scan4 = nullptr;
   if (T) CK(S.alloc(reinterpret_cast<char**>(&scan4), scan_scratch_bytes(T) + 256));
@@ -1165,75 +1623,37 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
   CK(cudaEventRecord(side.fork, st));
   CK(cudaStreamWaitEvent(side.s, side.fork, 0));
   if (T) {
-    wide4_roots_kernel<<<blocks_for(G), kBlock, 0, side.s>>>(G, pool, croot, level4, max_level4);
-    for (uint32_t l = 0; l < L; l++) {
-      const uint32_t a = level_begin[l], W = level_begin[l + 1] - a;
-      wide4_mark_kernel<<<blocks_for(W), kBlock, 0, side.s>>>(a, W, pool, croot, level4, max_level4);
-    }
+    wide4_slots_kernel<<<blocks_for(h_lvl[levels]), kBlock, 0, side.s>>>(h_lvl[levels], pool, slots);
+    wide4_top_kernel<<<1, kNumberThreads, 0, side.s>>>(lvl, levels, G, pool, slots, croot, level4, max_level4);
+    wide4_mark_small_kernel<<<std::min(blocks_for(hbc.ended, kWarps), 1u << 20), kBlock, 0, side.s>>>(
+        ended, bc, pool, slots, croot, level4, max_level4);
     CK(scan_u32(croot, index4, T, false, 0, scan4, side.s));
     CK(cudaGetLastError());
   }
   CK(cudaEventRecord(side.join, side.s));
 
-  // subtree sizes, bottom-up
-  uint32_t *size, *pre, *inner_at, *rank, *tree_end, *bvh_start, *root_code;
-  CK(S.alloc(&size, T));
+  uint32_t *pre, *inner_at, *rank, *tree_end, *tree_nodes, *root_code;
   CK(S.alloc(&pre, T));
   CK(S.alloc(&inner_at, T));
   CK(S.alloc(&rank, T));
   CK(S.alloc(&tree_end, G));
-  CK(S.alloc(&bvh_start, G));
+  CK(S.alloc(&tree_nodes, G));
   CK(S.alloc(&root_code, G));
-  for (int l = (int)L - 1; l >= 0; l--) {
-    const uint32_t a = level_begin[l], W = level_begin[l + 1] - a;
-    subtree_size_kernel<<<blocks_for(W), kBlock, 0, st>>>(a, W, pool, size);
-  }
-  CK(cudaGetLastError());
-  out.tree_nodes.resize(G);
-  std::vector<BNode> roots(G);
-  if (G) {
-    CK(cudaMemcpyAsync(out.tree_nodes.data(), size, 4 * (size_t)G, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(roots.data(), pool, sizeof(BNode) * G, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-  }
-  std::vector<uint32_t> h_start(G), h_end(G);
-  {
-    uint32_t acc = 0;
-    for (uint32_t g = 0; g < G; g++) {
-      h_start[g] = acc;
-      acc += out.tree_nodes[g];
-      h_end[g] = acc;
-    }
-  }
-  if (G) {
-    CK(cudaMemcpyAsync(bvh_start, h_start.data(), 4 * (size_t)G, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(tree_end, h_end.data(), 4 * (size_t)G, cudaMemcpyHostToDevice, st));
-    preorder_roots_kernel<<<blocks_for(G), kBlock, 0, st>>>(G, bvh_start, pre);
-  }
-  for (uint32_t l = 0; l < L; l++) {
-    const uint32_t a = level_begin[l], W = level_begin[l + 1] - a;
-    preorder_level_kernel<<<blocks_for(W), kBlock, 0, st>>>(a, W, pool, size, pre);
-  }
-  uint32_t inner_total = 0;
   if (T) {
+    top_numbering_kernel<<<1, kNumberThreads, 0, st>>>(lvl, levels, G, pool, tree_end, tree_nodes, pre);
     inner_flags_kernel<<<blocks_for(T), kBlock, 0, st>>>(T, pool, pre, inner_at);
     void* scan_tmp;
     CK(S.alloc(reinterpret_cast<char**>(&scan_tmp), scan_scratch_bytes(T) + 256));
     CK(scan_u32(inner_at, rank, T, false, 0, scan_tmp, st));
-    uint32_t last[2];
-    CK(cudaMemcpyAsync(&last[0], rank + (T - 1), 4, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(&last[1], inner_at + (T - 1), 4, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    inner_total = last[0] + last[1];
   }
+  const uint32_t inner_total = (T - G) / 2;  // every inner node has two children
   const uint32_t leaf_total = T - inner_total;
   CK(alloc_out(d.tri_bvh_forest, T, bytes, st));
   CK(alloc_out(d.wide_nodes, inner_total, bytes, st));
   CK(alloc_out(d.leaf_ranges, 2 * (size_t)leaf_total, bytes, st));
-  CK(alloc_out(d.indices_redirect, N, bytes, st));
-  CK(alloc_out(d.tri_records, N, bytes, st));
+  CK(alloc_out(d.wide4_nodes, inner_total, bytes, st));
   if (T)
-    emit_nodes_kernel<<<blocks_for(T), kBlock, 0, st>>>(T, G, pool, size, pre, rank, tree_end, d.tri_bvh_forest.ptr,
+    emit_nodes_kernel<<<blocks_for(T), kBlock, 0, st>>>(T, G, pool, pre, rank, tree_end, d.tri_bvh_forest.ptr,
                                                         d.wide_nodes.ptr, d.leaf_ranges.ptr, root_code);
   if (N)
     emit_primitives_kernel<<<std::min(blocks_for(N), persistent * 4), kBlock, 0, st>>>(
@@ -1244,19 +1664,10 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
   // scan in pool order (inner geometry roots first, in geometry order), one emit
   out.root_code.resize(G);
   out.root_code4.resize(G);
-  CK(alloc_out(d.wide4_nodes, inner_total, bytes, st));
-  std::vector<char> leaf_root(G, 0);  // their four-child code is the two-child one, read back at the end
-  {
-    uint32_t inner_roots = 0;
-    for (uint32_t g = 0; g < G; g++) {
-      if (roots[g].left == NONE) leaf_root[g] = 1;
-      else out.root_code4[g] = inner_roots++;
-    }
-  }
   uint32_t tail4[3] = {0, 0, 0};  // index4[T-1], croot[T-1], deepest level
   CK(cudaStreamWaitEvent(st, side.join, 0));
   if (T) {
-    wide4_emit_kernel<<<blocks_for(T), kBlock, 0, st>>>(T, N < kPackedTriangles, pool, croot, index4, pre, rank, d.wide4_nodes.ptr);
+    wide4_emit_kernel<<<blocks_for(T), kBlock, 0, st>>>(T, N < kPackedTriangles, pool, croot, slots, index4, pre, rank, d.wide4_nodes.ptr);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(&tail4[0], index4 + (T - 1), 4, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(&tail4[1], croot + (T - 1), 4, cudaMemcpyDeviceToHost, st));
@@ -1264,14 +1675,17 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
   }
   CK(cudaEventRecord(ev1, st));
 
-  BuildCounters hbc;
+  out.tree_nodes.resize(G);
+  if (G) {
+    CK(cudaMemcpyAsync(out.tree_nodes.data(), tree_nodes, 4 * (size_t)G, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(roots.data(), pool, sizeof(BNode) * G, cudaMemcpyDeviceToHost, st));
+  }
   if (G) CK(cudaMemcpyAsync(out.root_code.data(), root_code, 4 * (size_t)G, cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(&hbc, bc, sizeof(hbc), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   d.wide4_nodes.count = tail4[0] + tail4[1];
   out.max_wide4_depth = tail4[2];
-  for (uint32_t g = 0; g < G; g++)
-    if (leaf_root[g]) out.root_code4[g] = out.root_code[g];
+  uint32_t inner_roots = 0;  // a leaf root's four-child code is the two-child one
+  for (uint32_t g = 0; g < G; g++) out.root_code4[g] = roots[g].left == NONE ? out.root_code[g] : inner_roots++;
   float ms = 0.0f;
   CK(cudaEventElapsedTime(&ms, ev0, ev1));
   out.kernel_seconds = ms / 1000.0;
