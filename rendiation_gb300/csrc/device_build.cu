@@ -175,7 +175,7 @@ __global__ void prepare_primitives_kernel(uint32_t N, uint32_t G, const uint32_t
                                           const uint32_t* __restrict__ g_vstart, const uint32_t* __restrict__ g_vcount,
                                           const uint32_t* __restrict__ g_indexed, uint32_t* __restrict__ idx,
                                           const float* __restrict__ vtx, float4* __restrict__ pbox,
-                                          uint32_t* __restrict__ order, BuildCounters* ctr) {
+                                          BuildCounters* ctr) {
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x) {
     uint32_t lo = 0, hi = G;  // last g with g_prim_start[g] <= p
     while (hi - lo > 1) {
@@ -200,12 +200,51 @@ __global__ void prepare_primitives_kernel(uint32_t N, uint32_t G, const uint32_t
     }
     pbox[2 * (size_t)p] = make_float4(b.lo.x, b.lo.y, b.lo.z, 0.0f);
     pbox[2 * (size_t)p + 1] = make_float4(b.hi.x, b.hi.y, b.hi.z, 0.0f);
-    order[p] = p;
   }
 }
 
-__global__ void restart_kernel(uint32_t N, uint32_t* __restrict__ order) {
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x) order[p] = p;
+// The start of a build: the primitives in their order, one root per geometry
+// (its box pending), level 0, and cleared counters.
+__global__ void start_kernel(uint32_t N, uint32_t G, const uint32_t* __restrict__ g_prim_start,
+                             uint32_t* __restrict__ order, BNode* __restrict__ pool, uint32_t* __restrict__ lvl,
+                             LevelCounters* __restrict__ lcs, uint32_t level_cap, BuildCounters* bc) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  for (uint32_t p = t; p < N; p += stride) order[p] = p;
+  for (uint32_t l = t; l < level_cap; l += stride) lcs[l] = LevelCounters{};
+  if (t == 0) {
+    lvl[0] = 0;
+    lvl[1] = G;
+    *bc = BuildCounters{};
+  }
+  for (uint32_t g = t; g < G; g += stride) {
+    BNode r{};
+    set_box(r, empty_box());
+    r.start = g_prim_start[g];
+    r.end = g_prim_start[g + 1];
+    r.left = r.sub = NONE;
+    r.tree = g;
+    r.flags = F_BOX_PENDING;
+    pool[g] = r;
+  }
+}
+
+// What the host reads of the finished build, in one copy.
+struct BuildRoot {
+  int lo[3], hi[3];
+  uint32_t left, nodes, code;
+};
+struct BuildSummary {
+  uint32_t wide4_nodes, wide4_depth;
+};
+__global__ void summary_kernel(uint32_t G, uint32_t T, const BNode* __restrict__ pool, const uint32_t* __restrict__ tree_nodes,
+                               const uint32_t* __restrict__ root_code, const uint32_t* __restrict__ index4,
+                               const uint32_t* __restrict__ croot, const uint32_t* __restrict__ max_level4,
+                               BuildSummary* __restrict__ summary, BuildRoot* __restrict__ roots) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t == 0) *summary = BuildSummary{index4[T - 1] + croot[T - 1], *max_level4};
+  if (t >= G) return;
+  const BNode n = pool[t];
+  roots[t] = BuildRoot{{n.lo[0], n.lo[1], n.lo[2]}, {n.hi[0], n.hi[1], n.hi[2]}, n.left, tree_nodes[t], root_code[t]};
 }
 
 // ---- one tree level -----------------------------------------------------
@@ -1357,7 +1396,7 @@ struct Scratch {
   cudaError_t alloc(T** out, size_t count) {
     void* p = nullptr;
     const size_t bytes = (count ? count : 1) * sizeof(T);
-    cudaError_t e = pool ? cudaMallocFromPoolAsync(&p, bytes, pool, st) : cudaMallocAsync(&p, bytes, st);
+    cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool, st);
     if (e == cudaSuccess) ptrs.push_back(p);
     *out = static_cast<T*>(p);
     return e;
@@ -1367,9 +1406,9 @@ struct Scratch {
 // Device array owned by DeviceBuilt: at least one element, zeroed when empty
 // (the reference uploads one zeroed element for an empty array).
 template <class T>
-cudaError_t alloc_out(DevBuf<T>& b, size_t count, uint64_t& bytes, cudaStream_t s) {
+cudaError_t alloc_out(DevBuf<T>& b, size_t count, uint64_t& bytes, cudaMemPool_t pool, cudaStream_t s) {
   const size_t n = count ? count : 1;
-  cudaError_t e = cudaMalloc(&b.ptr, n * sizeof(T));
+  const cudaError_t e = alloc_built(b, n, pool, s);
   if (e != cudaSuccess) return e;
   b.count = count;
   bytes += n * sizeof(T);
@@ -1385,7 +1424,7 @@ inline uint32_t blocks_for(uint64_t n, uint32_t per = kBlock) {
 }  // namespace
 
 std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t bin_size, uint32_t max_depth,
-                              int sm_count, cudaMemPool_t mem_pool, DeviceBuilt& d, DeviceBlasOut& out) {
+                              int sm_count, const DeviceBuildQueue& q, DeviceBuilt& d, DeviceBlasOut& out) {
   const uint32_t G = (uint32_t)geoms.size();
   uint64_t N64 = 0, V64 = 0;
   for (const auto& g : geoms) {
@@ -1398,13 +1437,8 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
   out = DeviceBlasOut();
   out.triangles = N;
   out.vertices = V;
-  cudaStream_t st = nullptr;
-  cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-  if (e != cudaSuccess) return std::string("CUDA stream: ") + cudaGetErrorString(e);
-  struct StreamGuard {
-    cudaStream_t s;
-    ~StreamGuard() { cudaStreamDestroy(s); }
-  } guard{st};
+  const cudaStream_t st = q.stream;
+  const cudaMemPool_t mem_pool = q.pool;
   Scratch S{mem_pool, st, {}};
   uint64_t& bytes = out.bytes;
 #define CK(x)                                                                                  \
@@ -1416,9 +1450,11 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
   } while (0)
 
   // geometry arrays
-  CK(alloc_out(d.vertices, 3 * (size_t)V, bytes, st));
-  CK(alloc_out(d.indices, 3 * (size_t)N, bytes, st));
-  std::vector<uint32_t> g_prim(G + 1, 0), g_vs(G), g_vc(G), g_ix(G);
+  CK(alloc_out(d.vertices, 3 * (size_t)V, bytes, mem_pool, st));
+  CK(alloc_out(d.indices, 3 * (size_t)N, bytes, mem_pool, st));
+  // per geometry: first triangle (and their end), first vertex, vertex count, indexed
+  std::vector<uint32_t> g_in(4 * (size_t)G + 1);
+  uint32_t *g_prim = g_in.data(), *g_vs = g_prim + G + 1, *g_vc = g_vs + G, *g_ix = g_vc + G;
   {
     uint32_t ps = 0, vs = 0;
     for (uint32_t g = 0; g < G; g++) {
@@ -1439,66 +1475,23 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
     g_prim[G] = ps;
   }
   d.vertex_count = V;
-  uint32_t *dg_prim, *dg_vs, *dg_vc, *dg_ix;
-  CK(S.alloc(&dg_prim, G + 1));
-  CK(S.alloc(&dg_vs, G));
-  CK(S.alloc(&dg_vc, G));
-  CK(S.alloc(&dg_ix, G));
-  CK(cudaMemcpyAsync(dg_prim, g_prim.data(), 4 * (size_t)(G + 1), cudaMemcpyHostToDevice, st));
-  if (G) {
-    CK(cudaMemcpyAsync(dg_vs, g_vs.data(), 4 * (size_t)G, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(dg_vc, g_vc.data(), 4 * (size_t)G, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(dg_ix, g_ix.data(), 4 * (size_t)G, cudaMemcpyHostToDevice, st));
-  }
+  uint32_t* dg_prim;
+  CK(S.alloc(&dg_prim, g_in.size()));
+  CK(cudaMemcpyAsync(dg_prim, g_in.data(), 4 * g_in.size(), cudaMemcpyHostToDevice, st));
+  const uint32_t *dg_vs = dg_prim + G + 1, *dg_vc = dg_vs + G, *dg_ix = dg_vc + G;
 
   float4* pbox;
   uint8_t* bucket;  // per primitive in the level's order
   uint32_t *order, *order_b;
-  BuildCounters* bc;
   CK(S.alloc(&pbox, 2 * (size_t)N));
   CK(S.alloc(&bucket, N));
   CK(S.alloc(&order, N));
   CK(S.alloc(&order_b, N));
-  CK(S.alloc(&bc, 1));
-  CK(cudaMemsetAsync(bc, 0, sizeof(BuildCounters), st));
   const uint32_t persistent = (uint32_t)(sm_count > 0 ? sm_count : 1) * 8;
-  cudaEvent_t ev0, ev1;
-  CK(cudaEventCreate(&ev0));
-  CK(cudaEventCreate(&ev1));
-  struct EventGuard {
-    cudaEvent_t a, b;
-    ~EventGuard() {
-      cudaEventDestroy(a);
-      cudaEventDestroy(b);
-    }
-  } eg{ev0, ev1};
-  CK(cudaEventRecord(ev0, st));
-  if (N) {
-    prepare_primitives_kernel<<<std::min(blocks_for(N), persistent * 4), kBlock, 0, st>>>(
-        N, G, dg_prim, dg_vs, dg_vc, dg_ix, d.indices.ptr, d.vertices.ptr, pbox, order, bc);
-    CK(cudaGetLastError());
-  }
-
-  // roots: one per geometry, box pending
-  size_t cap = 2 * (size_t)N + 2 * (size_t)G + 64;
+  CK(cudaEventRecord(q.begin, st));
+  const size_t cap = 2 * (size_t)N + 2 * (size_t)G + 64;
   BNode* pool;
   CK(S.alloc(&pool, cap));
-  std::vector<BNode> roots(G);
-  for (uint32_t g = 0; g < G; g++) {
-    BNode& r = roots[g];
-    std::memset(&r, 0, sizeof(r));
-    for (int k = 0; k < 3; k++) {
-      r.lo[k] = key_of(INFINITY);
-      r.hi[k] = key_of(-INFINITY);
-    }
-    r.start = g_prim[g];
-    r.end = g_prim[g + 1];
-    r.depth = 0;
-    r.left = r.sub = NONE;
-    r.tree = g;
-    r.flags = F_BOX_PENDING;
-  }
-  if (G) CK(cudaMemcpyAsync(pool, roots.data(), sizeof(BNode) * G, cudaMemcpyHostToDevice, st));
 
   // level rounds. Every buffer is sized for the largest possible level (nodes
   // that are split hold more than `small` and more than bin_size primitives,
@@ -1513,12 +1506,16 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
   uint32_t *lvl, *acc_cnt, *chunk_node, *chunk_cnt, *chunk_prefix, *big_list, *ended;
   LevelCounters* lcs;
   int* acc_box;
-  CK(S.alloc(&lvl, (size_t)level_cap + 2));
+  // the counters and the level bounds: one copy to the host
+  constexpr size_t kBounds = sizeof(BuildCounters) / 4;
+  CK(S.alloc(&lvl, kBounds + level_cap + 2));
+  BuildCounters* bc = reinterpret_cast<BuildCounters*>(lvl);
+  lvl += kBounds;
   CK(S.alloc(&lcs, level_cap));
   CK(S.alloc(&big_list, big_cap));
   CK(S.alloc(&ended, cap));
-  const uint32_t lvl0[2] = {0, G};
-  std::vector<uint32_t> h_lvl((size_t)level_cap + 2);
+  std::vector<uint32_t> counters(kBounds + level_cap + 2);
+  const uint32_t* h_lvl = counters.data() + kBounds;
   uint32_t levels = 0;
   BuildCounters hbc;
   for (uint32_t small = kSmall;; small = 0) {
@@ -1529,8 +1526,11 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
     CK(S.alloc(&chunk_node, chunk_cap));
     CK(S.alloc(&chunk_cnt, 4 * chunk_cap));
     CK(S.alloc(&chunk_prefix, 4 * chunk_cap));
-    CK(cudaMemsetAsync(lcs, 0, sizeof(LevelCounters) * level_cap, st));
-    CK(cudaMemcpyAsync(lvl, lvl0, sizeof(lvl0), cudaMemcpyHostToDevice, st));
+    start_kernel<<<std::min(blocks_for(std::max(N, G)), persistent * 4), kBlock, 0, st>>>(N, G, dg_prim, order, pool, lvl, lcs,
+                                                                                        level_cap, bc);
+    if (N && small)  // once: it makes the indices global
+      prepare_primitives_kernel<<<std::min(blocks_for(N), persistent * 4), kBlock, 0, st>>>(
+          N, G, dg_prim, dg_vs, dg_vc, dg_ix, d.indices.ptr, d.vertices.ptr, pbox, bc);
     uint32_t queued = 0;
     bool closed = false;
     // first batch: about the depth of a balanced tree, then a few levels at a time
@@ -1559,12 +1559,12 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
       }
       CK(cudaGetLastError());
       if (!d.tri_records.ptr) {  // while the levels run
-        CK(alloc_out(d.indices_redirect, N, bytes, st));
-        CK(alloc_out(d.tri_records, N, bytes, st));
+        CK(alloc_out(d.indices_redirect, N, bytes, mem_pool, st));
+        CK(alloc_out(d.tri_records, N, bytes, mem_pool, st));
       }
-      CK(cudaMemcpyAsync(h_lvl.data(), lvl, 4 * ((size_t)queued + 2), cudaMemcpyDeviceToHost, st));
-      CK(cudaMemcpyAsync(&hbc, bc, sizeof(hbc), cudaMemcpyDeviceToHost, st));
+      CK(cudaMemcpyAsync(counters.data(), bc, 4 * (kBounds + queued + 2), cudaMemcpyDeviceToHost, st));
       CK(cudaStreamSynchronize(st));
+      std::memcpy(&hbc, counters.data(), sizeof(hbc));
       if (hbc.bad_index) return "triangle index out of range";  // no kernel has read a vertex through the indices yet
       if (hbc.overflow) return "device build: more nodes than the build holds";
       for (uint32_t k = 0; k <= queued && !closed; k++)
@@ -1581,9 +1581,6 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
     CK(cudaMemcpyAsync(&hbc, bc, sizeof(hbc), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     if (!(small && hbc.unfit)) break;
-    CK(cudaMemsetAsync(bc, 0, sizeof(BuildCounters), st));
-    restart_kernel<<<std::min(blocks_for(N), persistent), kBlock, 0, st>>>(N, order);
-    CK(cudaMemcpyAsync(pool, roots.data(), sizeof(BNode) * G, cudaMemcpyHostToDevice, st));
   }
   // the level rounds' nodes, then those of the subtrees
   const uint32_t T = h_lvl[levels] + hbc.added;
@@ -1594,17 +1591,13 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
   // and numbering scan run on a side stream, overlapped with the
   // pre-order numbering and the allocations below; the emit waits for them.
   struct SideStream {
-    cudaStream_t s = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
+    cudaStream_t s;
     ~SideStream() {
       // before the scratch it reads is freed (on the main stream, by S's
       // destructor, which runs after this one), also on an early error return
-      if (s) cudaStreamSynchronize(s);
-      if (join) cudaEventDestroy(join);
-      if (fork) cudaEventDestroy(fork);
-      if (s) cudaStreamDestroy(s);
+      cudaStreamSynchronize(s);
     }
-  } side;
+  } side{q.side};
   uint32_t *croot, *level4, *index4, *max_level4;
   CK(S.alloc(&croot, T));
   CK(S.alloc(&level4, T));
@@ -1617,11 +1610,8 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
   CK(cudaMemsetAsync(croot, 0, 4 * (size_t)(T ? T : 1), st));
   CK(cudaMemsetAsync(level4, 0, 4 * (size_t)(T ? T : 1), st));
   CK(cudaMemsetAsync(max_level4, 0, 4, st));
-  CK(cudaStreamCreateWithFlags(&side.s, cudaStreamNonBlocking));
-  CK(cudaEventCreateWithFlags(&side.fork, cudaEventDisableTiming));
-  CK(cudaEventCreateWithFlags(&side.join, cudaEventDisableTiming));
-  CK(cudaEventRecord(side.fork, st));
-  CK(cudaStreamWaitEvent(side.s, side.fork, 0));
+  CK(cudaEventRecord(q.fork, st));
+  CK(cudaStreamWaitEvent(side.s, q.fork, 0));
   if (T) {
     wide4_slots_kernel<<<blocks_for(h_lvl[levels]), kBlock, 0, side.s>>>(h_lvl[levels], pool, slots);
     wide4_top_kernel<<<1, kNumberThreads, 0, side.s>>>(lvl, levels, G, pool, slots, croot, level4, max_level4);
@@ -1630,7 +1620,7 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
     CK(scan_u32(croot, index4, T, false, 0, scan4, side.s));
     CK(cudaGetLastError());
   }
-  CK(cudaEventRecord(side.join, side.s));
+  CK(cudaEventRecord(q.join, side.s));
 
   uint32_t *pre, *inner_at, *rank, *tree_end, *tree_nodes, *root_code;
   CK(S.alloc(&pre, T));
@@ -1648,10 +1638,10 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
   }
   const uint32_t inner_total = (T - G) / 2;  // every inner node has two children
   const uint32_t leaf_total = T - inner_total;
-  CK(alloc_out(d.tri_bvh_forest, T, bytes, st));
-  CK(alloc_out(d.wide_nodes, inner_total, bytes, st));
-  CK(alloc_out(d.leaf_ranges, 2 * (size_t)leaf_total, bytes, st));
-  CK(alloc_out(d.wide4_nodes, inner_total, bytes, st));
+  CK(alloc_out(d.tri_bvh_forest, T, bytes, mem_pool, st));
+  CK(alloc_out(d.wide_nodes, inner_total, bytes, mem_pool, st));
+  CK(alloc_out(d.leaf_ranges, 2 * (size_t)leaf_total, bytes, mem_pool, st));
+  CK(alloc_out(d.wide4_nodes, inner_total, bytes, mem_pool, st));
   if (T)
     emit_nodes_kernel<<<blocks_for(T), kBlock, 0, st>>>(T, G, pool, pre, rank, tree_end, d.tri_bvh_forest.ptr,
                                                         d.wide_nodes.ptr, d.leaf_ranges.ptr, root_code);
@@ -1664,38 +1654,41 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
   // scan in pool order (inner geometry roots first, in geometry order), one emit
   out.root_code.resize(G);
   out.root_code4.resize(G);
-  uint32_t tail4[3] = {0, 0, 0};  // index4[T-1], croot[T-1], deepest level
-  CK(cudaStreamWaitEvent(st, side.join, 0));
+  BuildSummary* summary;
+  std::vector<char> h_summary(sizeof(BuildSummary) + sizeof(BuildRoot) * G);
+  CK(S.alloc(reinterpret_cast<char**>(&summary), h_summary.size()));
+  CK(cudaStreamWaitEvent(st, q.join, 0));
   if (T) {
     wide4_emit_kernel<<<blocks_for(T), kBlock, 0, st>>>(T, N < kPackedTriangles, pool, croot, slots, index4, pre, rank, d.wide4_nodes.ptr);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(&tail4[0], index4 + (T - 1), 4, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(&tail4[1], croot + (T - 1), 4, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(&tail4[2], max_level4, 4, cudaMemcpyDeviceToHost, st));
+    summary_kernel<<<blocks_for(G), kBlock, 0, st>>>(G, T, pool, tree_nodes, root_code, index4, croot, max_level4, summary,
+                                                     reinterpret_cast<BuildRoot*>(summary + 1));
+    CK(cudaGetLastError());
   }
-  CK(cudaEventRecord(ev1, st));
+  CK(cudaEventRecord(q.end, st));
 
   out.tree_nodes.resize(G);
-  if (G) {
-    CK(cudaMemcpyAsync(out.tree_nodes.data(), tree_nodes, 4 * (size_t)G, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(roots.data(), pool, sizeof(BNode) * G, cudaMemcpyDeviceToHost, st));
-  }
-  if (G) CK(cudaMemcpyAsync(out.root_code.data(), root_code, 4 * (size_t)G, cudaMemcpyDeviceToHost, st));
+  out.root_box.resize(G);
+  BuildSummary hs{};
+  if (T) CK(cudaMemcpyAsync(h_summary.data(), summary, h_summary.size(), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  d.wide4_nodes.count = tail4[0] + tail4[1];
-  out.max_wide4_depth = tail4[2];
-  uint32_t inner_roots = 0;  // a leaf root's four-child code is the two-child one
-  for (uint32_t g = 0; g < G; g++) out.root_code4[g] = roots[g].left == NONE ? out.root_code[g] : inner_roots++;
+  if (T) std::memcpy(&hs, h_summary.data(), sizeof(hs));
+  d.wide4_nodes.count = hs.wide4_nodes;
+  out.max_wide4_depth = hs.wide4_depth;
+  uint32_t inner_roots = 0;
+  for (uint32_t g = 0; g < G; g++) {
+    BuildRoot r;
+    std::memcpy(&r, h_summary.data() + sizeof(BuildSummary) + sizeof(BuildRoot) * g, sizeof(r));
+    out.tree_nodes[g] = r.nodes;
+    out.root_code[g] = r.code;
+    out.root_code4[g] = r.left == NONE ? r.code : inner_roots++;  // a leaf root's code is the two-child one
+    out.root_box[g] = Box{{val_of(r.lo[0]), val_of(r.lo[1]), val_of(r.lo[2])}, {val_of(r.hi[0]), val_of(r.hi[1]), val_of(r.hi[2])}};
+  }
   float ms = 0.0f;
-  CK(cudaEventElapsedTime(&ms, ev0, ev1));
+  CK(cudaEventElapsedTime(&ms, q.begin, q.end));
   out.kernel_seconds = ms / 1000.0;
   out.sah_splits = hbc.sah;
   out.median_fallbacks = hbc.fallback;
-  out.root_box.resize(G);
-  for (uint32_t g = 0; g < G; g++) {
-    const BNode& r = roots[g];
-    out.root_box[g] = Box{{val_of(r.lo[0]), val_of(r.lo[1]), val_of(r.lo[2])}, {val_of(r.hi[0]), val_of(r.hi[1]), val_of(r.hi[2])}};
-  }
 #undef CK
   return std::string();
 }

@@ -35,10 +35,10 @@ struct DeviceBlasOut {
 // geometry order exactly as the host build concatenates them. Returns "" or
 // the error ("CUDA ..." for a failed CUDA call, "CUDA OOM ..." when device
 // memory ran out); on error the arrays already written stay in `d` for the
-// caller to free. Scratch memory comes from `pool` (stream-ordered; nullptr =
-// the device's default pool) and goes back to it when the build returns.
+// caller to free (cudaFree). Both they and the scratch come from the queue's
+// pool; the scratch goes back to it when the build returns.
 std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t bin_size, uint32_t max_depth,
-                              int sm_count, cudaMemPool_t pool, DeviceBuilt& d, DeviceBlasOut& out);
+                              int sm_count, const DeviceBuildQueue& q, DeviceBuilt& d, DeviceBlasOut& out);
 
 // Writes d.vertex_records[j] = the three vertices of sorted triangle j
 // (d.indices_redirect, d.indices, d.vertices must be on the device), for j <

@@ -70,17 +70,66 @@ void free_device(rdn::DeviceBuilt& d) {
   d.bytes = 0;
 }
 
+// After a failed build: the arrays of a device build are the pool's, whose
+// memory cudaFree hands on without waiting for the kernels in flight.
+void drop_built(rdn::DeviceBuilt& d) {
+  cudaDeviceSynchronize();
+  free_device(d);
+}
+
 // Uploads one array; an empty array still gets one zeroed element, as the
 // reference's create_gpu_buffer does (naive/mod.rs:401-416).
 template <class T>
-cudaError_t upload(DevBuf<T>& dst, const std::vector<T>& src, uint64_t& bytes) {
+cudaError_t upload(DevBuf<T>& dst, const std::vector<T>& src, uint64_t& bytes, cudaMemPool_t pool, cudaStream_t s) {
   const size_t n = src.empty() ? 1 : src.size();
-  cudaError_t e = cudaMalloc(&dst.ptr, n * sizeof(T));
+  cudaError_t e = rdn::alloc_built(dst, n, pool, s);
   if (e != cudaSuccess) return e;
   dst.count = src.size();
   bytes += n * sizeof(T);
-  if (src.empty()) return cudaMemset(dst.ptr, 0, sizeof(T));
-  return cudaMemcpy(dst.ptr, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice);
+  if (src.empty()) return cudaMemsetAsync(dst.ptr, 0, sizeof(T), s);
+  return cudaMemcpyAsync(dst.ptr, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice, s);
+}
+
+cudaError_t open_build_queue(rdn::DeviceBuildQueue& q, int device) {
+  cudaError_t e = cudaSuccess;
+  if (!q.pool) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    if ((e = cudaMemPoolCreate(&q.pool, &props)) != cudaSuccess) {
+      q.pool = nullptr;
+      return e;
+    }
+    uint64_t keep = ~0ull;
+    if ((e = cudaMemPoolSetAttribute(q.pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) return e;
+  }
+  for (cudaStream_t* s : {&q.stream, &q.side})
+    if (!*s && (e = cudaStreamCreateWithFlags(s, cudaStreamNonBlocking)) != cudaSuccess) return e;
+  for (cudaEvent_t* v : {&q.begin, &q.end})
+    if (!*v && (e = cudaEventCreate(v)) != cudaSuccess) return e;
+  for (cudaEvent_t* v : {&q.fork, &q.join})
+    if (!*v && (e = cudaEventCreateWithFlags(v, cudaEventDisableTiming)) != cudaSuccess) return e;
+  return cudaSuccess;
+}
+
+void close_build_queue(rdn::DeviceBuildQueue& q) {
+  for (cudaEvent_t v : {q.begin, q.end, q.fork, q.join})
+    if (v) cudaEventDestroy(v);
+  for (cudaStream_t s : {q.stream, q.side})
+    if (s) cudaStreamDestroy(s);
+  if (q.pool) cudaMemPoolDestroy(q.pool);
+  q = rdn::DeviceBuildQueue();
+}
+
+// The pool keeps up to twice what the build that has just ended held at its
+// peak (about 200 B per triangle of scratch, and the built arrays) for the next
+// one (64 MB at least), not what an earlier, larger build needed.
+cudaError_t bound_build_pool(cudaMemPool_t pool) {
+  uint64_t peak = 0;
+  cudaError_t e = cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemHigh, &peak);
+  peak = std::max<uint64_t>(2 * peak, 64ull << 20);
+  return e == cudaSuccess ? cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &peak) : e;
 }
 
 rdn_status do_build(rdn_ctx* c) {
@@ -96,36 +145,24 @@ rdn_status do_build(rdn_ctx* c) {
     e = cudaDeviceSynchronize();  // no trace may still read the buffers being replaced
     if (e != cudaSuccess) return cuda_fail(c, e, "synchronize before build");
     free_device(c->dev);
-    if (!c->build_pool) {
-      // the build's scratch (about 200 B per triangle) stays in this pool
-      // between builds, so that a rebuild allocates nothing from the driver
-      cudaMemPoolProps props = {};
-      props.allocType = cudaMemAllocationTypePinned;
-      props.location.type = cudaMemLocationTypeDevice;
-      props.location.id = c->device;
-      e = cudaMemPoolCreate(&c->build_pool, &props);
-      if (e != cudaSuccess) {
-        c->build_pool = nullptr;
-        return cuda_fail(c, e, "cudaMemPoolCreate");
-      }
-      uint64_t keep = ~0ull;
-      e = cudaMemPoolSetAttribute(c->build_pool, cudaMemPoolAttrReleaseThreshold, &keep);
-      if (e != cudaSuccess) return cuda_fail(c, e, "cudaMemPoolSetAttribute");
-    }
+    e = open_build_queue(c->build_queue, c->device);
+    uint64_t none = 0;  // the peak of this build alone
+    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(c->build_queue.pool, cudaMemPoolAttrUsedMemHigh, &none);
+    if (e != cudaSuccess) return cuda_fail(c, e, "build queue");
   }
   try {
-    err = on_device ? rdn::build_with_device_blas(c->blas, c->tlas, c->binding, c->opts, c->sm_count, c->build_pool,
+    err = on_device ? rdn::build_with_device_blas(c->blas, c->tlas, c->binding, c->opts, c->sm_count, c->build_queue,
                                                   *hb, c->dev, &c->device_seconds)
                     : rdn::build_host(c->blas, c->tlas, c->binding, c->opts, *hb);
   } catch (const std::bad_alloc&) {
-    if (on_device) free_device(c->dev);
+    if (on_device) drop_built(c->dev);
     return fail(c, RDN_ERR_OOM, "host allocation failed during build");
   } catch (const std::exception& ex) {
-    if (on_device) free_device(c->dev);
+    if (on_device) drop_built(c->dev);
     return fail(c, RDN_ERR_INVALID_ARG, ex.what());
   }
   if (!err.empty()) {
-    if (on_device) free_device(c->dev);
+    if (on_device) drop_built(c->dev);
     const rdn_status code = err.rfind("CUDA OOM ", 0) == 0 ? RDN_ERR_OOM
                             : err.rfind("CUDA ", 0) == 0   ? RDN_ERR_CUDA
                                                            : RDN_ERR_INVALID_HANDLE;
@@ -141,13 +178,16 @@ rdn_status do_build(rdn_ctx* c) {
       e = cudaDeviceSynchronize();  // no trace may still read the buffers being replaced
       if (e != cudaSuccess) return cuda_fail(c, e, "synchronize before upload");
       free_device(c->dev);
+      if (c->build_queue.pool) cudaMemPoolTrimTo(c->build_queue.pool, 0);
     }
     rdn::DeviceBuilt& d = c->dev;
+    const cudaMemPool_t pool = on_device ? c->build_queue.pool : nullptr;
+    const cudaStream_t st = on_device ? c->build_queue.stream : nullptr;
     uint64_t bytes = hb->device_bytes;
 #define UP(field, src)                                      \
-  e = upload(d.field, hb->src, bytes);                      \
+  e = upload(d.field, hb->src, bytes, pool, st);            \
   if (e != cudaSuccess) {                                   \
-    free_device(d);                                         \
+    drop_built(d);                                          \
     return cuda_fail(c, e, "upload " #src);                 \
   }
     UP(tlas_binding, tlas_binding)
@@ -173,15 +213,16 @@ rdn_status do_build(rdn_ctx* c) {
     {
       // vertices of every sorted triangle, for the watertight test, gathered on the device
       const size_t n = d.indices_redirect.count;
-      e = cudaMalloc(&d.vertex_records.ptr, (n ? n : 1) * sizeof(rdn::VertexRecord));
+      e = rdn::alloc_built(d.vertex_records, n ? n : 1, pool, st);
       if (e == cudaSuccess) {
         d.vertex_records.count = n;
         bytes += (n ? n : 1) * sizeof(rdn::VertexRecord);
-        e = n ? rdn::emit_vertex_records(d, 0) : cudaMemset(d.vertex_records.ptr, 0, sizeof(rdn::VertexRecord));
+        e = n ? rdn::emit_vertex_records(d, st) : cudaMemsetAsync(d.vertex_records.ptr, 0, sizeof(rdn::VertexRecord), st);
       }
-      if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+      if (e == cudaSuccess && pool) e = bound_build_pool(pool);
       if (e != cudaSuccess) {
-        free_device(d);
+        drop_built(d);
         return cuda_fail(c, e, "vertex records");
       }
     }
@@ -358,7 +399,7 @@ rdn_status rdn_destroy(rdn_ctx* c) {
     cudaDeviceSynchronize();
     free_device(c->dev);
     if (c->d_counters) cudaFree(c->d_counters);
-    if (c->build_pool) cudaMemPoolDestroy(c->build_pool);
+    close_build_queue(c->build_queue);
   }
   delete c;
   return RDN_OK;

@@ -204,6 +204,25 @@ struct DeviceBuilt {
   uint64_t bytes = 0;
 };
 
+// What a context keeps between device builds, so that a rebuild takes nothing
+// from the driver: the pool of the built arrays and of the scratch, two
+// streams and the events between them. (With the arrays from cudaMalloc and
+// new streams for each build, 2.1 M triangles took 3.35 ms instead of 2.37 and
+// 1,000 triangles 0.63 instead of 0.35: 18 allocations and frees, each of
+// which maps or unmaps memory.) The device is idle when arrays are replaced.
+struct DeviceBuildQueue {
+  cudaMemPool_t pool = nullptr;
+  cudaStream_t stream = nullptr, side = nullptr;
+  cudaEvent_t begin = nullptr, end = nullptr, fork = nullptr, join = nullptr;
+};
+
+// `n` elements from the pool (in the order of `s`) or, without one, from the driver.
+template <class T>
+cudaError_t alloc_built(DevBuf<T>& b, size_t n, cudaMemPool_t pool, cudaStream_t s) {
+  return pool ? cudaMallocFromPoolAsync(reinterpret_cast<void**>(&b.ptr), n * sizeof(T), pool, s)
+              : cudaMalloc(reinterpret_cast<void**>(&b.ptr), n * sizeof(T));
+}
+
 struct BuildOptions {
   uint32_t blas_bin_size = 2, blas_max_depth = 50, tlas_bin_size = 10, tlas_max_depth = 50, host_threads = 0;
   uint32_t device_build = 0;
@@ -221,7 +240,7 @@ std::string build_host(const std::vector<std::unique_ptr<std::vector<GeometrySou
 std::string build_with_device_blas(const std::vector<std::unique_ptr<std::vector<GeometrySource>>>& blas,
                                    const std::vector<std::unique_ptr<std::vector<InstanceSource>>>& tlas,
                                    const std::vector<uint32_t>& binding, const BuildOptions& opt, int sm_count,
-                                   cudaMemPool_t pool, HostBuilt& out, DeviceBuilt& d, double* device_seconds);
+                                   const DeviceBuildQueue& queue, HostBuilt& out, DeviceBuilt& d, double* device_seconds);
 
 }  // namespace rdn
 
@@ -241,7 +260,7 @@ struct rdn_ctx {
   // context that use the same word must not overlap on the GPU.
   uint32_t* d_counters = nullptr;
   uint32_t iteration_limit = 0;     // cap of the dynamic-fetch loops (0 = built-in)
-  cudaMemPool_t build_pool = nullptr;  // stream-ordered scratch of device builds, kept for the next build
+  rdn::DeviceBuildQueue build_queue;
   double build_seconds = 0.0, upload_seconds = 0.0, device_seconds = 0.0;
   std::string err;
 };
