@@ -58,11 +58,11 @@ __global__ void __launch_bounds__(128) ao_kernel(TraceParams P, AoEnv A) {
 // Four lanes per ray (quad.cuh), a warp `batch` pixels, for frames of up to
 // kQuadPixels: below that the slowest warps decide a frame's time, and a warp
 // of eight or sixteen pixels is done in less than half the time of one of 32
-// (us for four samples on the 1024^2 field: 128^2 pixels, one per thread 863,
-// 8 a warp 303; 256^2 1008, 8 477, 16 520; 512^2 1275, 8 1188, 16 1085, 32
-// 1133; 1280x720 2249, 16 3139). Above it pixels that are alike share their
+// (us for four samples on the 1024^2 field: 128^2 pixels, one per thread 582,
+// 8 a warp 303; 256^2 662, 8 487, 16 520; means of four cameras: 400x300 841,
+// 760; 400^2 930, 890; 512^2 1030, 1180; 800x500 1370, 1710). Above it pixels that are alike share their
 // nodes better one per lane.
-constexpr uint32_t kQuadPixels = 400000;
+constexpr uint32_t kQuadPixels = 200000;
 constexpr uint32_t ao_quad_batch(uint32_t pixels) { return pixels < 100000u ? 8u : 16u; }
 
 template <bool WT>

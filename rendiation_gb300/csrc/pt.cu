@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(128) pt_kernel(TraceParams P, PtEnv E) {
       pt_ray(q, R);
       pt_park(stash, q);
       bool b;
-      traverse_ray<MODE, false, BuiltinAnyHit, WT>(P, R, E.view.tlas, stack_ptr, stack_stride, b);
+      traverse_ray<MODE, false, BuiltinAnyHit, WT, 1>(P, R, E.view.tlas, stack_ptr, stack_stride, b);
       bad |= b;
       pt_unpark(stash, q);
       done = pt_advance(P, E, sample, q, R);
@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(128, pt_min_blocks(TIER)) pt_refill_kernel(Tra
       pt_ray(q, R);
       pt_park(stash, q);
       bool b;
-      traverse_ray<MODE, false, BuiltinAnyHit, WT>(P, R, E.view.tlas, stack_ptr, stack_stride, b);
+      traverse_ray<MODE, false, BuiltinAnyHit, WT, 1>(P, R, E.view.tlas, stack_ptr, stack_stride, b);
       bad |= b;
       pt_unpark(stash, q);
       if (pt_advance(P, E, sample, q, R)) {
@@ -269,10 +269,11 @@ __global__ void __launch_bounds__(128, pt_min_blocks(TIER)) pt_refill_kernel(Tra
 // for frames of up to kQuadPixels: fewer do not fill the chip one path per
 // lane, and the warp's rays (camera, bounce and shadow ones of different
 // paths) differ. Us for two samples of depth 3 on the 1024^2 field: 128^2
-// pixels, one path per lane 786, 8 a warp 358, 16 447; 256^2 1029, 16 645, 8
-// 662; 682x384 1281, 32 1153, 16 1317; 1280x720 2545, 32 2906. 72 registers (7
-// blocks): 64 and 80 took 1192 and 1169 us at 682x384.
-constexpr uint32_t kQuadPixels = 400000;
+// pixels, one path per lane 625, 8 a warp 360, 16 447; 256^2 835, 16 645, 8
+// 662; means of four cameras: 400x300 952, 938; 400^2 1020, 1014; 512^2 1155,
+// 1293; 800x500 1360, 1580. 72 registers (7 blocks): 64 and 80 took 1192 and 1169 us against 1153
+// at 682x384.
+constexpr uint32_t kQuadPixels = 200000;
 template <bool WT>
 __global__ void __launch_bounds__(128, 7) pt_refill_quad_kernel(TraceParams P, PtEnv E, uint32_t total, uint32_t batch) {
   extern __shared__ __align__(16) unsigned char quad_smem[];
@@ -428,7 +429,7 @@ __global__ void __launch_bounds__(128, pt_min_blocks(TIER))
       pt_ray(q, R);
       pt_park(stash, q);
       bool b;
-      traverse_ray<MODE, false, BuiltinAnyHit, WT>(P, R, E.view.tlas, stack_ptr, stack_stride, b);
+      traverse_ray<MODE, false, BuiltinAnyHit, WT, 1>(P, R, E.view.tlas, stack_ptr, stack_stride, b);
       bad |= b;
       pt_unpark(stash, q);
       if (pt_advance(P, E, sample, q, R)) {

@@ -15,12 +15,11 @@
 // one, reads its node as one 128 B line, and a warp's longest ray no longer
 // holds 31 others: 24 of 32 lanes active, 0.70 of the issue slots.
 // Measured (rdn_trace, us, one ray per lane -> quads): 777,777 random rays
-// through a 150k soup 1140 -> 822 (watertight 1387 -> 935), 1,000,000 through
-// the 1024^2 field 455 -> 344, the 1080p frame's 2.05 M bounce rays 1315 ->
-// 1174, 1,000 rays through a 10k soup 130 -> 45, 65,536 camera rays onto it
-// 121 -> 48. Only large batches of rays that are alike walk faster one per
+// through a 150k soup 917 -> 835 (watertight 1200 -> 943), 1,000,000 through
+// the 1024^2 field 407 -> 355, 1,000 rays through a 10k soup 84 -> 47, 65,536
+// camera rays onto it 85 -> 49. Only large batches of rays that are alike walk faster one per
 // lane, where a warp's lanes share the nodes they read (2.07 M camera rays:
-// 727 against 985). 64 registers a thread; before the steps were unrolled the
+// 597 against 985). 64 registers a thread; before the steps were unrolled the
 // random rays took 885 us with 64, 910 with 72 and 938 with 56.
 //
 // Results: every child box and every triangle is tested with the operations of

@@ -137,17 +137,17 @@ namespace {
 // camera rays of the 1024^2 / 128^2 field and on random rays through a 10k soup):
 //   below kQuadSplit    quads, eight rays a warp: too few rays to fill the
 //                       chip, so the longest warp decides. 65,536 camera rays
-//                       onto the soup: one ray per lane 121, 8 rays a warp 49,
-//                       16 79, 32 119; 1,000 random rays: 130 -> 45
+//                       onto the soup: one ray per lane 85, 8 rays a warp 49,
+//                       16 79, 32 119; 1,000 random rays: 84 -> 47
 //   below kQuadBatch32  quads; rays that differ 16 a warp (48,000 random rays:
 //                       8 a warp 100, 16 88, 32 120), alike ones still 8
 //   below kLaneSplit    the same with 32 (131,072 random: 193 / 159 / 150;
-//                       262,144 camera rays: 8 a warp 167 / 110, 32 242 / 134,
-//                       lanes 249 / 99; 131,072: 124 / 70, lanes 240 / 90)
-//   from there on       alike rays one per lane (393,216: quads 243 / 157,
-//                       lanes 330 / 125; 524,288: 311 / 201, 382 / 142;
-//                       786,432: 413 / 283, 411 / 156), the rest quads
-//                       (777,777 through a 150k soup: lanes 1140, quads 822)
+//                       camera rays: 160,000 8 a warp 127 / 70, lanes 173 / 87;
+//                       327,680 215 / 101, lanes 237 / 98)
+//   from there on       alike rays one per lane (400,000: quads 259 / 102,
+//                       lanes 273 / 99; 786,432: 431 / 187, 323 / 112), the
+//                       rest quads (777,777 through a 150k soup: lanes 917,
+//                       quads 835; watertight 1200, 943)
 constexpr uint32_t kQuadSplit = 40000, kQuadBatch32 = 100000, kLaneSplit = 400000;
 
 template <int MODE, bool COUNT, bool LOCAL, bool WT, bool SPLIT>

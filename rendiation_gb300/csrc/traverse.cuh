@@ -421,8 +421,8 @@ __device__ __forceinline__ Wide4Load load_wide4_if(const float4* w, bool want) {
 // as a + (-b)), two to an instruction. The per-lane four-child walk is bound by
 // instruction issue (55-66 % of the slots, 6 to 17 of 32 lanes active), and a
 // box test falls from about 22 to 16 instructions: 2.07 M camera rays on the
-// 1024^2 field 880 -> 727 us (with the child-major node below), 777,777 rays
-// through a 150k soup 1248 -> 1140 us, the 1080p frame 2107 -> 1950 us.
+// 1024^2 field 880 -> 727 us (with the child-major node below; 597 with the
+// steps of descend()), the 1080p frame 2107 -> 1950 us (1659).
 template <bool WT>
 __device__ __forceinline__ bool slab2(float2 neg_o_xy, float2 neg_o_z, float2 inv_xy, float2 inv_z, float tmin,
                                       float tmax, const Wide4Load& c, float& t_near_max) {
@@ -514,11 +514,39 @@ __device__ __forceinline__ uint32_t interior_step(const TraceParams& p, RayCtx& 
     cswap(t1, c1, t3, c3);
     cswap(t1, c1, t2, c2);
     if (c0 == EMPTY_SLOT) return pop_live(stack, stride, sp, far_, code_tn);
-    if (c3 != EMPTY_SLOT) push_entry(p, stack, stride, sp, depth, c3, t3);
-    if (c2 != EMPTY_SLOT) push_entry(p, stack, stride, sp, depth, c2, t2);
-    if (c1 != EMPTY_SLOT) push_entry(p, stack, stride, sp, depth, c1, t1);
+    // no bounds check: a step leaves at most three entries per level of the four-child tree, and the stack has
+    // 3 D + 1 for D levels (stack_entries); with one the 1080p frame took 1912 us instead of 1747
+    if (c3 != EMPTY_SLOT) stack[(sp++) * stride] = make_uint2(c3, __float_as_uint(t3));
+    if (c2 != EMPTY_SLOT) stack[(sp++) * stride] = make_uint2(c2, __float_as_uint(t2));
+    if (c1 != EMPTY_SLOT) stack[(sp++) * stride] = make_uint2(c1, __float_as_uint(t1));
     code_tn = t0;
     return c0;
+  }
+}
+
+// Interior steps of a lane, which keeps the first leaf it meets, until it has
+// none left or no more than spec_threshold lanes still look for a leaf. On the
+// four-child tree the lanes vote after every STEPS steps. Fewer votes against
+// more code, which a kernel that holds two or three walks feels sooner. 1080p
+// frame: 1747 us with one step between the votes, 1682 with two, 1659 with
+// three, 1672 with four (80 registers instead of 64: 1926, 56: 2110). Ambient
+// occlusion, 1280x720: 1742 with one, 1741 with two, 1862 with three. Path
+// tracing, 1280x720: 2210 with one, 2310 with two, 2510 with three.
+template <int STEPS, bool COUNT, int WIDTH, bool WT>
+__device__ __forceinline__ void descend(const TraceParams& p, RayCtx& R, const InstanceRay& ir, uint32_t& code,
+                                        float& code_tn, uint32_t& leaf, uint2* stack, uint32_t stride, uint32_t& sp,
+                                        uint32_t depth) {
+  while (!(code & LEAF_BIT)) {  // EMPTY_SLOT has the bit too
+#pragma unroll
+    for (int step = 0; step < (WIDTH == 4 ? STEPS : 1); step++) {
+      if (code & LEAF_BIT) continue;
+      code = interior_step<COUNT, WIDTH, WT>(p, R, ir, code, code_tn, stack, stride, sp, depth);
+      if (code != EMPTY_SLOT && (code & LEAF_BIT) && leaf == EMPTY_SLOT) {
+        leaf = code;
+        code = pop_live(stack, stride, sp, R.far_world * ir.scaling, code_tn);
+      }
+    }
+    if ((uint32_t)__popc(__ballot_sync(__activemask(), leaf == EMPTY_SLOT)) <= p.spec_threshold) break;
   }
 }
 
@@ -527,7 +555,7 @@ __device__ __forceinline__ uint32_t interior_step(const TraceParams& p, RayCtx& 
 // a leaf (or has finished), then the warp tests triangles together. Nodes are
 // visited in near-first order with the reference's box test; the speculation
 // only adds visits, never removes one, so the closest hit is unchanged.
-template <bool COUNT, int WIDTH, class AH = BuiltinAnyHit, bool WT = false>
+template <int STEPS, bool COUNT, int WIDTH, class AH = BuiltinAnyHit, bool WT = false>
 __device__ __forceinline__ bool blas_speculative(const TraceParams& p, RayCtx& R, const InstanceRay& ir,
                                                  uint32_t root_node, uint32_t gslot, uint32_t inst_slot,
                                                  bool is_opaque, bool cull_enable, bool cull_back, uint32_t prim_start,
@@ -550,15 +578,7 @@ __device__ __forceinline__ bool blas_speculative(const TraceParams& p, RayCtx& R
     code = EMPTY_SLOT;
   }
   while (code != EMPTY_SLOT || leaf != EMPTY_SLOT) {
-    while (code != EMPTY_SLOT && !(code & LEAF_BIT)) {
-      code = interior_step<COUNT, WIDTH, WT>(p, R, ir, code, code_tn, stack, stride, sp, depth);
-      if (code != EMPTY_SLOT && (code & LEAF_BIT) && leaf == EMPTY_SLOT) {
-        leaf = code;
-        code = pop_live(stack, stride, sp, R.far_world * ir.scaling, code_tn);
-      }
-      // keep descending while more than spec_threshold lanes still look for a leaf
-      if ((uint32_t)__popc(__ballot_sync(__activemask(), leaf == EMPTY_SLOT)) <= p.spec_threshold) break;
-    }
+    descend<STEPS, COUNT, WIDTH, WT>(p, R, ir, code, code_tn, leaf, stack, stride, sp, depth);
     while (leaf != EMPTY_SLOT) {
       const uint2 lr = leaf_range<WIDTH>(p, leaf);
       if (leaf_triangles<COUNT, AH, WT>(p, R, ir, lr.x, lr.y, gslot, inst_slot, is_opaque, cull_enable, cull_back,
@@ -579,7 +599,7 @@ __device__ __forceinline__ bool blas_speculative(const TraceParams& p, RayCtx& R
 
 // Full query of one ray (traverse_cpu.rs:52-245). R must hold the ray; on
 // return R.best holds the committed hit. `bad` reports an unbound TLAS index.
-template <int MODE, bool COUNT, class AH = BuiltinAnyHit, bool WT = false>
+template <int MODE, bool COUNT, class AH = BuiltinAnyHit, bool WT = false, int STEPS = 2>
 __device__ __forceinline__ void traverse_ray(const TraceParams& p, RayCtx& R, uint32_t tidx, uint2* stack,
                                              uint32_t stride, bool& bad, const AH& anyhit = AH()) {
   R.inv_d = make_float3(1.0f / R.d.x, 1.0f / R.d.y, 1.0f / R.d.z);
@@ -628,10 +648,10 @@ __device__ __forceinline__ void traverse_ray(const TraceParams& p, RayCtx& R, ui
         if (!pass) continue;
         bool end;
         if (MODE == MODE_WIDE4)
-          end = blas_speculative<COUNT, 4, AH, WT>(p, R, ir, gm.x, g, ti, is_opaque, cull_enable, cull_back, gm.z, stack,
+          end = blas_speculative<STEPS, COUNT, 4, AH, WT>(p, R, ir, gm.x, g, ti, is_opaque, cull_enable, cull_back, gm.z, stack,
                                                stride, p.stack_depth, anyhit);
         else if (MODE == MODE_BINARY)
-          end = blas_speculative<COUNT, 2, AH, WT>(p, R, ir, gm.x, g, ti, is_opaque, cull_enable, cull_back, gm.z, stack,
+          end = blas_speculative<STEPS, COUNT, 2, AH, WT>(p, R, ir, gm.x, g, ti, is_opaque, cull_enable, cull_back, gm.z, stack,
                                                stride, p.stack_depth, anyhit);
         else
           end = blas_threaded<COUNT, AH, WT>(p, R, ir, gm.x, g, ti, is_opaque, cull_enable, cull_back, gm.z, anyhit);
@@ -788,14 +808,7 @@ struct LaneWalk {
         phase = WALK_DONE;
         return;
       }
-      while (code != EMPTY_SLOT && !(code & LEAF_BIT)) {
-        code = interior_step<false, WIDTH, WT>(p, R, ir, code, code_tn, stack, stride, sp, p.stack_depth);
-        if (code != EMPTY_SLOT && (code & LEAF_BIT) && leaf == EMPTY_SLOT) {
-          leaf = code;
-          code = pop_live(stack, stride, sp, R.far_world * ir.scaling, code_tn);
-        }
-        if ((uint32_t)__popc(__ballot_sync(__activemask(), leaf == EMPTY_SLOT)) <= p.spec_threshold) break;
-      }
+      descend<2, false, WIDTH, WT>(p, R, ir, code, code_tn, leaf, stack, stride, sp, p.stack_depth);
       while (leaf != EMPTY_SLOT) {
         const uint2 lr = leaf_range<WIDTH>(p, leaf);
         if (leaf_triangles<false, BuiltinAnyHit, WT>(p, R, ir, lr.x, lr.y, gslot, inst_slot, is_opaque, cull_enable, cull_back,

@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(128, min_blocks(TIER)) primary_kernel(TracePar
       RayCtx R;
       primary_ray(w, d, R);
       bool bad;
-      traverse_ray<MODE, false, BuiltinAnyHit, WT>(p, R, w.tlas, stack, stride, bad);
+      traverse_ray<MODE, false, BuiltinAnyHit, WT, 3>(p, R, w.tlas, stack, stride, bad);
       n = shade_primary(p, w, px, py, d, R.best);
     }
     append_rays(w, px, py, n);
@@ -195,11 +195,10 @@ __global__ void __launch_bounds__(128, min_blocks(TIER)) primary_kernel(TracePar
 
 // The same with four lanes per ray (quad.cuh): a warp claims `batch` pixels of
 // a tile. Both kernels of this kind run for frames of up to kQuadPixels, whose
-// slowest warps decide (us, primary + secondary, one ray per lane -> quads):
-// 64^2 pixels 131 + 170 -> 54 + 60, 256^2 208 + 240 -> 93 + 104, 512^2 272 +
-// 305 -> 193 + 230, 800x500 304 + 395 -> 275 + 329, but 1280x720 430 + 674 ->
-// 525 + 709.
-constexpr uint32_t kQuadPixels = 450000;
+// slowest warps decide (us a frame, one ray per lane -> quads): 64^2 pixels 236
+// -> 110, 256^2 393 -> 216, 400^2 464 -> 340, 512^2 482 -> 442, but 640x512 499
+// -> 525, 1280x720 899 -> 1246.
+constexpr uint32_t kQuadPixels = 300000;
 template <bool WT>
 __global__ void __launch_bounds__(128, 8) primary_quad_kernel(TraceParams p, WavefrontParams w, uint32_t batch) {
   extern __shared__ __align__(16) unsigned char quad_smem[];
@@ -280,7 +279,7 @@ __global__ void __launch_bounds__(128, min_blocks(TIER)) secondary_kernel(TraceP
       R.cull_mask = 0xFFu;
       R.ray_flags = shadow ? TF_END_SEARCH : 0u;
       bool bad;
-      traverse_ray<MODE, false, BuiltinAnyHit, WT>(p, R, w.tlas, stack, stride, bad);
+      traverse_ray<MODE, false, BuiltinAnyHit, WT, 3>(p, R, w.tlas, stack, stride, bad);
       store_secondary(p, w, shadow, q, R.best);
     }
   }
