@@ -238,16 +238,15 @@ __device__ __forceinline__ void attr_scatter(const TraceParams& p, const Adjoint
   gd = make_float3(h.t_unnorm * lam.x, h.t_unnorm * lam.y, h.t_unnorm * lam.z);
 }
 
-// Persistent warps over paths; ADJOINT selects the gradient pass. QUADS: the
-// ordered walks with four lanes per ray (quad.cuh), every lane of the warp
-// going through all segments; else a ray per lane in MODE's order. 16 fields,
-// 2.2 M paths of three segments, forward + adjoint: 6166 us one ray per lane
-// on two-child nodes, 5363 with quads (6490 with the first segments, whose
-// rays are alike, one per lane in the same kernel: its registers and shared
-// memory cost both walks more than that saves).
-template <int MODE, bool ADJOINT, bool QUADS, bool WT>
+// Persistent warps over paths; ADJOINT selects the gradient pass. QUADS: four
+// lanes per ray (quad.cuh), every lane of the warp going through all segments;
+// else a ray per lane in MODE's order. Which of the two an ordered walk takes:
+// launch_attr_paths.
+template <int MODE, bool ADJOINT, bool QUADS, bool LOCAL, bool WT>
 __global__ void __launch_bounds__(128, QUADS ? kQuadBlocks : 0) attr_path_kernel(TraceParams p, PathAdjointParams a) {
   extern __shared__ __align__(16) unsigned char dyn_smem[];
+  uint2 local_stack[LOCAL ? kLocalStackEntries : 1];
+  uint2* const stack = LOCAL ? local_stack : reinterpret_cast<uint2*>(dyn_smem) + threadIdx.x;
   __shared__ double block_sum[4];
   const uint32_t lane = threadIdx.x & 31u;
   double loss_acc = 0.0;
@@ -288,8 +287,7 @@ __global__ void __launch_bounds__(128, QUADS ? kQuadBlocks : 0) attr_path_kernel
         if (!__any_sync(kFullWarp, alive || (mine && !ADJOINT))) break;
         traverse_warp<WT>(p, R, tlas, alive, quad_warp(dyn_smem, p.stack_depth4), bad);
       } else if (alive) {
-        traverse_ray<MODE, false, BuiltinAnyHit, WT>(p, R, tlas, reinterpret_cast<uint2*>(dyn_smem) + threadIdx.x,
-                                                     blockDim.x, bad);
+        traverse_ray<MODE, false, BuiltinAnyHit, WT>(p, R, tlas, stack, LOCAL ? 1u : blockDim.x, bad);
       }
       if (alive) {
         if (!R.best.have) {
@@ -577,16 +575,16 @@ inline uint32_t recorded_grid(size_t items, int sm_count) {
   return (uint32_t)(need < cap ? (need ? need : 1) : cap);
 }
 
-template <int MODE, bool QUADS, bool WT>
+template <int MODE, bool QUADS, bool LOCAL, bool WT>
 cudaError_t launch_attr_paths_wt(const TraceParams& p, const PathAdjointParams& a, bool adjoint, uint32_t block,
                                  int sm_count, cudaStream_t stream) {
   static std::atomic<uint64_t> done[2] = {};
-  const auto fn = adjoint ? attr_path_kernel<MODE, true, QUADS, WT> : attr_path_kernel<MODE, false, QUADS, WT>;
+  const auto fn = adjoint ? attr_path_kernel<MODE, true, QUADS, LOCAL, WT> : attr_path_kernel<MODE, false, QUADS, LOCAL, WT>;
   cudaError_t e = raise_smem_limit(done[adjoint], {(const void*)fn});
   if (e != cudaSuccess) return e;
-  const size_t smem = QUADS                   ? (size_t)quad_warp_bytes(p.stack_depth4) * (block / 32)
-                      : MODE != MODE_THREADED ? (size_t)p.stack_depth * block * sizeof(uint2)
-                                              : 0;
+  const size_t smem = QUADS                             ? (size_t)quad_warp_bytes(p.stack_depth4) * (block / 32)
+                      : MODE != MODE_THREADED && !LOCAL ? (size_t)p.stack_depth * block * sizeof(uint2)
+                                                        : 0;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, (int)block, smem);
   if (e != cudaSuccess) return e;
@@ -601,12 +599,20 @@ cudaError_t launch_attr_paths_wt(const TraceParams& p, const PathAdjointParams& 
   return cudaGetLastError();
 }
 
-template <int MODE, bool QUADS>
+template <int MODE, bool QUADS, bool LOCAL>
 cudaError_t launch_attr_paths_mode(const TraceParams& p, const PathAdjointParams& a, bool adjoint, uint32_t block,
                                    int sm_count, cudaStream_t stream) {
-  return p.watertight ? launch_attr_paths_wt<MODE, QUADS, true>(p, a, adjoint, block, sm_count, stream)
-                      : launch_attr_paths_wt<MODE, QUADS, false>(p, a, adjoint, block, sm_count, stream);
+  return p.watertight ? launch_attr_paths_wt<MODE, QUADS, LOCAL, true>(p, a, adjoint, block, sm_count, stream)
+                      : launch_attr_paths_wt<MODE, QUADS, LOCAL, false>(p, a, adjoint, block, sm_count, stream);
 }
+
+// Ordered path passes of up to this many paths take four lanes per ray, larger
+// ones a lane (fields, forward + adjoint, us, quads / lanes: 104,196 paths of
+// three segments 440 / 445, of one 234 / 262; 135,801 462 / 470, 261 / 264;
+// 175,157 578 / 558, 301 / 297; 1,031,276 of three 2280 / 1945; 2,677,724 5355
+// / 4400). 64 registers without a bound on the blocks; with 5, 6, 7 and 8
+// blocks of 128 the last took 5170, 4790, 5208 and 5105.
+constexpr uint32_t kQuadPaths = 150000;
 
 template <int PASS, int MODE, bool LOCAL, bool WT, bool SPLIT>
 cudaError_t launch_ray_lanes(const TraceParams& p, const AdjointParams& a, uint32_t block, cudaStream_t stream) {
@@ -654,9 +660,13 @@ cudaError_t launch_attr_paths(const TraceParams& p, const PathAdjointParams& a, 
     return cudaGetLastError();
   }
   if (block == 0) block = 64;
-  if (mode == MODE_THREADED) return launch_attr_paths_mode<MODE_THREADED, false>(p, a, adjoint, block, sm_count, stream);
-  if (p.packed) return launch_attr_paths_mode<MODE_WIDE4, true>(p, a, adjoint, block, sm_count, stream);
-  return launch_attr_paths_mode<MODE_WIDE4, false>(wide4_params(p), a, adjoint, block, sm_count, stream);
+  if (mode == MODE_THREADED)
+    return launch_attr_paths_mode<MODE_THREADED, false, false>(p, a, adjoint, block, sm_count, stream);
+  const TraceParams q = wide4_params(p);
+  if (p.packed && (a.count <= kQuadPaths || !q.local_stack))
+    return launch_attr_paths_mode<MODE_WIDE4, true, false>(p, a, adjoint, block, sm_count, stream);
+  return q.local_stack ? launch_attr_paths_mode<MODE_WIDE4, false, true>(q, a, adjoint, block, sm_count, stream)
+                       : launch_attr_paths_mode<MODE_WIDE4, false, false>(q, a, adjoint, block, sm_count, stream);
 }
 
 cudaError_t launch_attr_forward(const TraceParams& p, const AdjointParams& a, int mode, uint32_t block,

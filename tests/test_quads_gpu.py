@@ -274,3 +274,49 @@ def test_wavefront_frames_of_both_walks(cuda, width, height):
             8 * (width * height // 20_000)
         assert rays == want_rays
     assert P.check_errors() == (0, 0)
+
+
+@pytest.mark.parametrize("watertight", [0, rt.INTERSECT_WATERTIGHT])
+@pytest.mark.parametrize("n", [1, 33, 150_000, 150_001])
+def test_attribute_paths_at_the_edges(cuda, n, watertight):
+    """Differentiable paths on both sides of the size from which a lane takes a path."""
+    import ctypes as C
+
+    import torch
+
+    from rendiation_gb300 import native
+
+    P, mesh = field_system()
+    L = native.lib()
+    rays = torch.from_numpy(field_rays(n, n).view(np.float32).reshape(-1, 8).copy()).cuda()
+    g = torch.Generator(device="cuda").manual_seed(2)
+    attr = torch.rand(mesh.positions.shape[0], generator=g, device="cuda")
+    target = torch.rand(2 * n, generator=g, device="cuda")
+
+    def run(traversal):
+        z = lambda *s, dtype=torch.float32: torch.zeros(s, dtype=dtype, device="cuda")  # noqa: E731
+        r = dict(tri=z(n, 2, dtype=torch.int32), inst=z(n, 2, dtype=torch.int32), rays=z(n, 16), values=z(n, 2),
+                 loss=z(1, dtype=torch.float64), grad=z(attr.shape[0], 4))
+        base = dict(rays=rays.data_ptr(), count=n, segments=2, seed=3, attributes=attr.data_ptr(),
+                    targets=target.data_ptr(), grad_scale=1.0, traversal=traversal | watertight)
+        f = native.AttrPathDesc(**base, seg_tri=r["tri"].data_ptr(), seg_inst=r["inst"].data_ptr(),
+                                seg_rays=r["rays"].data_ptr(), values=r["values"].data_ptr(),
+                                loss_sum=r["loss"].data_ptr())
+        a = native.AttrPathDesc(**base, grad_vertices=r["grad"].data_ptr())
+        assert L.rdn_attr_paths_forward(P._h, C.byref(f), None) == 0
+        assert L.rdn_attr_paths_adjoint(P._h, C.byref(a), None) == 0
+        torch.cuda.synchronize()
+        return {k: v.cpu().numpy() for k, v in r.items()}
+
+    want, got = run(rt.TRAVERSAL_REFERENCE), run(rt.TRAVERSAL_ORDERED)
+    same = (want["tri"] == got["tri"]).all(1)
+    assert np.count_nonzero(~same) <= 1 + n // 20_000  # exact-distance ties
+    for k in ("inst", "rays", "values"):
+        assert np.array_equal(want[k][same], got[k][same]), k
+    # a sum of n non-negative doubles in another order, and the ties' own terms (at most 1 each)
+    assert abs(want["loss"][0] - got["loss"][0]) <= 4 * n * 2.0**-53 * abs(want["loss"][0]) + 2 * np.count_nonzero(~same)
+    if same.all():
+        hit = want["tri"] != -1
+        m = np.bincount(mesh.indices.reshape(-1, 3)[want["tri"][hit]].reshape(-1), minlength=1).max() if hit.any() else 0
+        diff = np.linalg.norm(want["grad"].astype(np.float64) - got["grad"])
+        assert diff <= m * 2.0**-24 * np.linalg.norm(want["grad"].astype(np.float64))
