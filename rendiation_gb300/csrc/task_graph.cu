@@ -30,6 +30,7 @@
 #include <cstring>
 
 #include "ao.cuh"
+#include "quad.cuh"
 #include "task_graph.h"
 #include "task_graph_device.cuh"
 #include "traverse.cuh"
@@ -166,23 +167,26 @@ __device__ bool poll_chain(const TaskGraphDev& G, uint32_t g, uint32_t idx, cons
 // spawns the closest-hit or miss task of its trace call (resolving at once
 // when there is none to spawn); the task resolves in the poll that finds that
 // child finished, taking back the child's user payload.
-template <int MODE, bool WT>
-__device__ bool poll_trace(const TaskGraphDev& G, uint32_t g, uint32_t idx, const TraceParams& P, uint2* stack,
-                           uint32_t stride) {
+__device__ __forceinline__ void task_ray(const Rec& self, RayCtx& R) {
+  R.o = make_float3(__uint_as_float(self[0]), __uint_as_float(self[1]), __uint_as_float(self[2]));
+  R.tmin = __uint_as_float(self[3]);
+  R.d = make_float3(__uint_as_float(self[4]), __uint_as_float(self[5]), __uint_as_float(self[6]));
+  R.tmax = __uint_as_float(self[7]);
+  R.ray_flags = self[8];
+  R.cull_mask = self[9];
+}
+__device__ __forceinline__ bool wants_trace(const TaskGroupDev& T, uint32_t idx) {
+  return task_locals(T, idx)[6] == TRACE_SUB_NOT_SPAWNED;
+}
+
+// The poll after the traversal; R and bad are read when the task wanted one.
+__device__ bool poll_traced(const TaskGraphDev& G, uint32_t g, uint32_t idx, const TraceParams& P, const RayCtx& R,
+                            bool bad) {
   const TaskGroupDev& T = G.g[g];
   const Rec L = task_locals(T, idx);
   const Rec self = task_payload(T, idx);
   uint32_t sub_group = L[5], sub_id = L[6], terminated = L[7];
   if (sub_id == TRACE_SUB_NOT_SPAWNED) {
-    RayCtx R;
-    R.o = make_float3(__uint_as_float(self[0]), __uint_as_float(self[1]), __uint_as_float(self[2]));
-    R.tmin = __uint_as_float(self[3]);
-    R.d = make_float3(__uint_as_float(self[4]), __uint_as_float(self[5]), __uint_as_float(self[6]));
-    R.tmax = __uint_as_float(self[7]);
-    R.ray_flags = self[8];
-    R.cull_mask = self[9];
-    bool bad;
-    traverse_ray<MODE, false, BuiltinAnyHit, WT>(P, R, self[10], stack, stride, bad);
     if (bad) atomicOr(P.error_word, 2u);
     uint32_t target = TRACE_SUB_NOT_SPAWNED;
     if (R.best.have) {
@@ -242,6 +246,19 @@ __device__ bool poll_trace(const TaskGraphDev& G, uint32_t g, uint32_t idx, cons
   return resolved;
 }
 
+template <int MODE, bool WT>
+__device__ bool poll_trace(const TaskGraphDev& G, uint32_t g, uint32_t idx, const TraceParams& P, uint2* stack,
+                           uint32_t stride) {
+  RayCtx R;
+  bool bad = false;
+  if (wants_trace(G.g[g], idx)) {
+    const Rec self = task_payload(G.g[g], idx);
+    task_ray(self, R);
+    traverse_ray<MODE, false, BuiltinAnyHit, WT>(P, R, self[10], stack, stride, bad);
+  }
+  return poll_traced(G, g, idx, P, R, bad);
+}
+
 // One thread per active entry of group g: poll(idx) runs the task's program,
 // then the poll is finalised.
 template <class Poll>
@@ -294,6 +311,49 @@ __global__ void __launch_bounds__(kPollThreads, 8) poll_kernel(const TaskGraphDe
   const TaskGraphDev& G = *Gp;
   poll_active_fetch(G, g,
                     [&](uint32_t idx) { return poll_trace<MODE, WT>(G, g, idx, P, stack_ptr, stack_stride); });
+}
+
+// Trace polls of the ordered walks, four lanes per ray (quad.cuh): the warp
+// walks the rays of the entries that it has claimed, then every lane polls its
+// entry. Tasks of one warp differ (rays that start, tasks that wait), and a
+// poll is as long as its slowest warp. Four samples of the AO pipeline on the
+// 1024^2 field, us, a ray per lane (two-child, four-child nodes) -> quads:
+// 128^2 pixels 3950, 3760 -> 2910; 512^2 8600, 8110 -> 7060; 1280x720 25990,
+// 24150 -> 22530.
+template <bool WT>
+__global__ void __launch_bounds__(kPollThreads, 8) poll_quad_kernel(const TaskGraphDev* __restrict__ Gp, uint32_t g,
+                                                                 TraceParams P) {
+  extern __shared__ __align__(16) unsigned char quad_smem[];
+  const TaskGraphDev& G = *Gp;
+  const TaskGroupDev& T = G.g[g];
+  GroupCtl* c = T.ctl;
+  const uint32_t n = c->active.size, batch = quad_batch(n);
+  const uint32_t* list = T.active[c->sel];
+  const uint32_t lane = threadIdx.x & 31u;
+  for (;;) {
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(&c->poll_next, batch);
+    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    if (base >= n) break;
+    const bool mine = lane < batch && base + lane < n;
+    const uint32_t idx = mine ? list[base + lane] : 0u;
+    const bool want = mine && wants_trace(T, idx);
+    RayCtx R;
+    bool bad = false;
+    if (__any_sync(0xFFFFFFFFu, want)) {
+      uint32_t tlas = 0;
+      if (want) {
+        const Rec self = task_payload(T, idx);
+        task_ray(self, R);
+        tlas = self[10];
+      }
+      traverse_warp<WT>(P, R, tlas, want, quad_warp(quad_smem, P.stack_depth4), bad);
+    }
+    if (mine) {
+      const uint32_t pi = T.parent_index[idx], pt = T.parent_type[idx];
+      finalize(G, g, idx, poll_traced(G, g, idx, P, R, bad), pi, pt);
+    }
+  }
 }
 
 // Chain groups alone: without the traversal the kernel fits twice the resident
@@ -581,6 +641,19 @@ cudaError_t launch_poll_wt(const TaskGraphDev* G, uint32_t g, const TraceParams&
   return cudaGetLastError();
 }
 
+template <bool WT>
+cudaError_t launch_poll_quads(const TaskGraphDev* G, uint32_t g, uint32_t cap, const TraceParams& P, int sm_count,
+                              cudaStream_t st) {
+  const size_t smem = (size_t)quad_warp_bytes(P.stack_depth4) * (kPollThreads / 32);
+  static std::atomic<uint64_t> attr_done{0};
+  const cudaError_t e = raise_smem_limit(attr_done, {(const void*)poll_quad_kernel<WT>});
+  if (e != cudaSuccess) return e;
+  const uint32_t per = 8u * (kPollThreads / 32);  // entries a block takes at a time, at least
+  const uint32_t grid = std::min<uint32_t>((cap + per - 1) / per, (uint32_t)sm_count * 8);
+  poll_quad_kernel<WT><<<grid, kPollThreads, smem, st>>>(G, g, P);
+  return cudaGetLastError();
+}
+
 template <int MODE, bool LOCAL>
 cudaError_t launch_poll(const TaskGraphDev* G, uint32_t g, const TraceParams& P, const AoEnv& A, uint32_t grid,
                         cudaStream_t st) {
@@ -765,14 +838,13 @@ cudaError_t TaskGraph::poll(uint32_t g, const TraceParams* p, int mode, const Ao
   }
   // the trace poll's launch bounds guarantee 8 resident blocks per SM
   const uint32_t tgrid = std::min<uint32_t>(cap_blocks, (uint32_t)sm_count_ * 8);
-  if (!p) return launch_poll<MODE_THREADED, false>(G, g, P, A, tgrid, st);
-  if (mode == MODE_WIDE4)
-    return P.local_stack ? launch_poll<MODE_WIDE4, true>(G, g, P, A, tgrid, st)
-                         : launch_poll<MODE_WIDE4, false>(G, g, P, A, tgrid, st);
-  if (mode == MODE_BINARY)
-    return P.local_stack ? launch_poll<MODE_BINARY, true>(G, g, P, A, tgrid, st)
-                         : launch_poll<MODE_BINARY, false>(G, g, P, A, tgrid, st);
-  return launch_poll<MODE_THREADED, false>(G, g, P, A, tgrid, st);
+  if (!p || mode == MODE_THREADED) return launch_poll<MODE_THREADED, false>(G, g, P, A, tgrid, st);
+  if (P.packed)
+    return P.watertight ? launch_poll_quads<true>(G, g, T.cap, P, sm_count_, st)
+                        : launch_poll_quads<false>(G, g, T.cap, P, sm_count_, st);
+  const TraceParams q = wide4_params(P);  // a structure too large for packed leaves
+  return q.local_stack ? launch_poll<MODE_WIDE4, true>(G, g, q, A, tgrid, st)
+                       : launch_poll<MODE_WIDE4, false>(G, g, q, A, tgrid, st);
 }
 
 cudaError_t TaskGraph::dispatch_init(uint32_t group, uint32_t count, uint32_t init_op, cudaStream_t st) {

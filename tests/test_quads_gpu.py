@@ -320,3 +320,26 @@ def test_attribute_paths_at_the_edges(cuda, n, watertight):
         m = np.bincount(mesh.indices.reshape(-1, 3)[want["tri"][hit]].reshape(-1), minlength=1).max() if hit.any() else 0
         diff = np.linalg.norm(want["grad"].astype(np.float64) - got["grad"])
         assert diff <= m * 2.0**-24 * np.linalg.norm(want["grad"].astype(np.float64))
+
+
+@pytest.mark.parametrize("watertight", [0, rt.INTERSECT_WATERTIGHT])
+@pytest.mark.parametrize("width,height", [(1, 1), (7, 5), (33, 31), (250, 200)])
+def test_task_graph_trace_polls(cuda, width, height, watertight):
+    """The AO pipeline on the task graph (its trace tasks start and wait in the same warps) against the reference order."""
+    import torch
+
+    from rendiation_gb300 import task_graph as tg
+
+    P, _ = field_system(128)
+    eye = (0.5, -0.4, 0.6)
+    vp = tg.look_at_view_projection_inv(eye, (0.5, 0.5, 0.0), (0, 0, 1), 40.0, width / height)
+    images = []
+    for traversal in (rt.TRAVERSAL_REFERENCE, rt.TRAVERSAL_ORDERED, rt.TRAVERSAL_ORDERED_WIDE):
+        ao = tg.AmbientOcclusion(P, width, height, vp, eye, traversal=traversal | watertight, mode="graph")
+        ao.sample_count = 200
+        ao.render()
+        torch.cuda.synchronize()
+        images.append(ao.result().copy())
+    for image in images[1:]:
+        assert np.count_nonzero((image != images[0]).any(-1)) <= width * height // 20_000
+    assert P.check_errors() == (0, 0)
