@@ -10,28 +10,26 @@
 // The reference builds one node at a time, depth first, on one thread. Here
 // every geometry's tree is built together. Nodes of more than kSmall primitives
 // go one tree level per round:
-//   prepare   each node of the level decides leaf / split (count > bin_size and
-//             depth < max_depth, utils.rs:35-37) and claims warp tasks of 256
-//             primitives ("chunks") of its range;
-//   box       nodes whose box is not known yet (roots, median-split children)
-//             reduce their primitives' boxes;
 //   stats     per chunk: the 4 centroid buckets on the longest axis of the
 //             node box, their counts and boxes, merged into the node;
 //   decide    per node: the reference's 3-candidate SAH choice (or the median
-//             fallback when 3 buckets are empty), the two children, and each
-//             chunk's per-bucket offset inside the node (warp scan);
+//             fallback when 3 buckets are empty), each chunk's per-bucket
+//             offset inside the node, and the two children, each a leaf or a
+//             split (count > bin_size and depth < max_depth, utils.rs:35-37)
+//             that claims warp tasks of 256 primitives ("chunks");
 //   prefix    the chunk offsets of nodes with many chunks, a block per node;
 //             median-split nodes run Rust's select_nth_unstable_by restatement
 //             on one thread each;
 //   scatter   SAH nodes write their primitives in bucket order, stable inside
 //             a bucket (warp ballots), into the other of two order arrays;
-//             median-split nodes copy theirs.
+//             median-split nodes copy theirs and reduce the children's boxes.
 // Nodes of kSmall primitives and fewer are left to small_trees_kernel, which
 // builds the whole subtree below each in shared memory, a block per subtree and
 // a warp or a lane per node: a level of many small nodes is bound by the gaps
 // between its launches and by reductions over empty lanes (2.1 M triangles,
 // bin size 4: all by level rounds 5.2 ms a build, subtrees in blocks 3.35 ms;
-// 8,000 triangles 1.58 and 0.75 ms; 1,000 triangles 1.19 and 0.63 ms).
+// 8,000 triangles 1.58 and 0.75 ms; 1,000 triangles 1.19 and 0.63 ms; with the arrays
+// kept and four launches a level now 2.04, 0.44 and 0.33 ms).
 // Boxes are merged with integer atomics on an order-preserving key of the
 // float, so a union does not depend on the order primitives arrive in. The
 // reference's pre-order numbering is recovered afterwards from subtree sizes
@@ -274,52 +272,64 @@ __device__ __forceinline__ uint32_t warp_claim(uint32_t* ctr, uint32_t amount, u
 // several levels without reading anything back. Kernels of an empty level
 // (past the last one) find no node and return. Node loops step a whole warp
 // at a time (warp-uniform bounds) so that the lanes can aggregate atomics.
-__global__ void level_prepare_kernel(const uint32_t* __restrict__ lvl, uint32_t L, uint32_t bin_size,
-                                     uint32_t max_depth, BNode* __restrict__ pool, uint32_t* __restrict__ acc_cnt,
-                                     int* __restrict__ acc_box, uint32_t* __restrict__ chunk_node,
-                                     LevelCounters* lcs, uint32_t small, BuildCounters* bc,
-                                     uint32_t* __restrict__ ended) {
+struct LevelBuffers {  // of the nodes of one level, by their place in it
+  uint32_t* acc_cnt;
+  int* acc_box;
+  uint32_t* chunk_node;
+};
+struct SplitRule {
+  uint32_t bin_size, max_depth, small;
+};
+
+// Leaf or split of node n (id, the i-th of level L): a split claims its chunks
+// and clears its sums, any other node goes to the list of ended ones. All 32
+// lanes call, those without a node with `valid` unset.
+__device__ __forceinline__ void prepare_node(bool valid, BNode& n, uint32_t id, uint32_t i, uint32_t L, const SplitRule& rule,
+                                             const LevelBuffers& B, LevelCounters* lcs, BuildCounters* bc,
+                                             uint32_t* __restrict__ ended) {
   const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t lb = lvl[L], W = lvl[L + 1] - lb;
-  LevelCounters* lc = lcs + L;
-  const uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < W; i0 += stride) {
-    const uint32_t i = i0 + lane;
-    uint32_t nch = 0;
-    bool active = false;
-    if (i < W) {
-      BNode& n = pool[lb + i];
-      const uint32_t count = n.end - n.start;
-      active = n.depth < max_depth && count > bin_size && count > small;
-      const bool need = active || (count > small && (n.flags & F_BOX_PENDING));
-      nch = need ? (count + kChunk - 1) / kChunk : 0;
-      n.flags = (n.flags & F_BOX_PENDING) | (active ? F_ACTIVE : 0u) | ((L & 1u) ? F_IN_B : 0u);
-      n.left = NONE;
-      n.nchunks = nch;
-    }
-    const bool ends = i < W && !active;
-    const uint32_t at = warp_claim(&bc->ended, ends ? 1u : 0u, lane);
-    if (ends) ended[at] = lb + i;
-    const uint32_t base = warp_claim(&lc->chunks, nch, lane);
-    if (i < W) pool[lb + i].cbase = nch ? base : 0u;
-    // chunk -> node map: small ranges by their own lane, long ones by the whole warp
-    if (nch && nch <= 32)
-      for (uint32_t j = 0; j < nch; j++) chunk_node[base + j] = lb + i;
-    uint32_t wide = __ballot_sync(0xffffffffu, nch > 32);
-    while (wide) {
-      const uint32_t src = __ffs(wide) - 1;
-      wide &= wide - 1;
-      const uint32_t b = __shfl_sync(0xffffffffu, base, src), c = __shfl_sync(0xffffffffu, nch, src);
-      for (uint32_t j = lane; j < c; j += 32) chunk_node[b + j] = lb + i0 + src;
-    }
-    if (active) {
-      for (int b = 0; b < 4; b++) acc_cnt[4 * (size_t)i + b] = 0;
-      for (int b = 0; b < 4; b++)
-        for (int k = 0; k < 3; k++) {
-          acc_box[24 * (size_t)i + 6 * b + k] = key_of(INFINITY);
-          acc_box[24 * (size_t)i + 6 * b + 3 + k] = key_of(-INFINITY);
-        }
-    }
+  const uint32_t count = n.end - n.start;
+  const bool active = valid && n.depth < rule.max_depth && count > rule.bin_size && count > rule.small;
+  const bool need = active || (valid && count > rule.small && (n.flags & F_BOX_PENDING));
+  const uint32_t nch = need ? (count + kChunk - 1) / kChunk : 0;
+  n.flags = (n.flags & F_BOX_PENDING) | (active ? F_ACTIVE : 0u) | ((L & 1u) ? F_IN_B : 0u);
+  n.left = NONE;
+  n.nchunks = nch;
+  const bool ends = valid && !active;
+  const uint32_t at = warp_claim(&bc->ended, ends ? 1u : 0u, lane);
+  if (ends) ended[at] = id;
+  const uint32_t base = warp_claim(&lcs[L].chunks, nch, lane);
+  n.cbase = nch ? base : 0u;
+  // chunk -> node map: small ranges by their own lane, long ones by the whole warp
+  if (nch && nch <= 32)
+    for (uint32_t j = 0; j < nch; j++) B.chunk_node[base + j] = id;
+  uint32_t wide = __ballot_sync(0xffffffffu, nch > 32);
+  while (wide) {
+    const uint32_t src = __ffs(wide) - 1;
+    wide &= wide - 1;
+    const uint32_t b = __shfl_sync(0xffffffffu, base, src), c = __shfl_sync(0xffffffffu, nch, src),
+                   node = __shfl_sync(0xffffffffu, id, src);
+    for (uint32_t j = lane; j < c; j += 32) B.chunk_node[b + j] = node;
+  }
+  if (active) {
+    for (int b = 0; b < 4; b++) B.acc_cnt[4 * (size_t)i + b] = 0;
+    for (int b = 0; b < 4; b++)
+      for (int k = 0; k < 3; k++) {
+        B.acc_box[24 * (size_t)i + 6 * b + k] = key_of(INFINITY);
+        B.acc_box[24 * (size_t)i + 6 * b + 3 + k] = key_of(-INFINITY);
+      }
+  }
+}
+
+__global__ void prepare_roots_kernel(uint32_t G, SplitRule rule, BNode* __restrict__ pool, LevelBuffers B, LevelCounters* lcs,
+                                     BuildCounters* bc, uint32_t* __restrict__ ended) {
+  const uint32_t lane = threadIdx.x & 31u, stride = gridDim.x * blockDim.x;
+  for (uint32_t g0 = blockIdx.x * blockDim.x + threadIdx.x - lane; g0 < G; g0 += stride) {
+    const uint32_t g = g0 + lane;
+    BNode n{};
+    if (g < G) n = pool[g];
+    prepare_node(g < G, n, g, g, 0, rule, B, lcs, bc, ended);
+    if (g < G) pool[g] = n;
   }
 }
 
@@ -328,12 +338,12 @@ __device__ __forceinline__ void chunk_range(const BNode& n, uint32_t c, uint32_t
   e = min(n.end, s + kChunk);
 }
 
-// Boxes of nodes whose box is still unknown: min/max of the primitive boxes.
-__global__ void level_box_kernel(const LevelCounters* lcs, uint32_t L, BNode* __restrict__ pool,
-                                 const uint32_t* __restrict__ chunk_node, const uint32_t* __restrict__ order,
-                                 const float4* __restrict__ pbox) {
+// Boxes of the roots: min/max of the primitive boxes.
+__global__ void root_box_kernel(const LevelCounters* lcs, BNode* __restrict__ pool,
+                                const uint32_t* __restrict__ chunk_node, const uint32_t* __restrict__ order,
+                                const float4* __restrict__ pbox) {
   const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t total = lcs[L].chunks;
+  const uint32_t total = lcs[0].chunks;
   for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < total; c += (gridDim.x * blockDim.x) >> 5) {
     const uint32_t id = chunk_node[c];
     const BNode n = pool[id];
@@ -523,7 +533,7 @@ __device__ __forceinline__ bool split_node(const BNode& n, uint32_t i, const uin
   l.start = n.start;
   l.end = r.start = mid;
   r.end = n.end;
-  l.flags = r.flags = s.fallback ? F_BOX_PENDING : 0u;
+  l.flags = r.flags = 0u;  // the median split's boxes, empty so far, grow in level_scatter_kernel
   set_box(l, s.l);
   set_box(r, s.r);
   l.depth = r.depth = n.depth + 1;
@@ -534,13 +544,15 @@ __device__ __forceinline__ bool split_node(const BNode& n, uint32_t i, const uin
 }
 
 // One thread per node of the level: the split decision, the two children
-// (slots claimed per warp), and the exclusive per-bucket prefix of the node's
+// (slots claimed per warp, prepared for the next level at once: a launch of
+// their own cost 8 us a level), and the exclusive per-bucket prefix of the node's
 // chunk counts (big nodes: appended to big_list for the block-wide scan).
 __global__ void level_decide_kernel(const uint32_t* __restrict__ lvl, uint32_t L, BNode* __restrict__ pool,
                                     const uint32_t* __restrict__ acc_cnt, const int* __restrict__ acc_box,
                                     const uint4* __restrict__ chunk_cnt, uint4* __restrict__ chunk_prefix,
                                     LevelCounters* lcs, BuildCounters* bc, uint32_t* __restrict__ big_list,
-                                    uint32_t big_cap, uint32_t pool_cap) {
+                                    uint32_t big_cap, uint32_t pool_cap, SplitRule rule, LevelBuffers next,
+                                    uint32_t* __restrict__ ended) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t lb = lvl[L], next_base = lvl[L + 1], W = next_base - lb;
   LevelCounters* lc = lcs + L;
@@ -562,11 +574,14 @@ __global__ void level_decide_kernel(const uint32_t* __restrict__ lvl, uint32_t L
     if (lane == 0 && n_med) atomicAdd(&bc->fallback, (unsigned long long)n_med);
     const bool big = active && !fallback && n.nchunks > kBigChunks;
     const uint32_t slot = warp_claim(&lc->big, big ? 1u : 0u, lane);
-    if (!active) continue;
-    if (base + 1 >= pool_cap) {
+    const bool fits = active && base + 1 < pool_cap;
+    if (active && !fits) {  // the host gives up on the build; no kernel may scatter this node
       bc->overflow = 1u;
-      continue;
+      pool[lb + i].flags = n.flags & ~F_ACTIVE;
     }
+    prepare_node(fits, l, base, base - next_base, L + 1, rule, next, lcs, bc, ended);
+    prepare_node(fits, r, base + 1, base + 1 - next_base, L + 1, rule, next, lcs, bc, ended);
+    if (!fits) continue;
     if (l.start == l.end || r.start == r.end) bc->unfit = 1u;
     pool[base] = l;
     pool[base + 1] = r;
@@ -671,7 +686,8 @@ __global__ void __launch_bounds__(kBlock) level_prefix_select_kernel(
 // the other order array; a median-split node's are copied as they stand. Also
 // closes the level: the next level's end is its start plus the children that
 // level_decide_kernel created (decide ran before this launch).
-__global__ void level_scatter_kernel(uint32_t* __restrict__ lvl, uint32_t L, const LevelCounters* lcs, const BNode* __restrict__ pool,
+__global__ void level_scatter_kernel(uint32_t* __restrict__ lvl, uint32_t L, const LevelCounters* lcs, BNode* __restrict__ pool,
+                                     const float4* __restrict__ pbox,
                                      const uint32_t* __restrict__ chunk_node, const uint32_t* __restrict__ order,
                                      const uint8_t* __restrict__ bucket, const uint32_t* __restrict__ acc_cnt,
                                      const uint32_t* __restrict__ chunk_prefix, uint32_t* __restrict__ scratch) {
@@ -687,7 +703,37 @@ __global__ void level_scatter_kernel(uint32_t* __restrict__ lvl, uint32_t L, con
     if (n.flags & F_FALLBACK) {
       uint32_t s, e;
       chunk_range(n, c, s, e);
-      for (uint32_t i = s + lane; i < e; i += 32) scratch[i] = order[i];
+      const uint32_t mid = pool[n.left].end;
+      int lo[2][3], hi[2][3];
+      for (int c2 = 0; c2 < 2; c2++)
+        for (int k = 0; k < 3; k++) {
+          lo[c2][k] = key_of(INFINITY);
+          hi[c2][k] = key_of(-INFINITY);
+        }
+      for (uint32_t i = s + lane; i < e; i += 32) {
+        const uint32_t p = order[i];
+        scratch[i] = p;
+        const float4 a = pbox[2 * (size_t)p], b = pbox[2 * (size_t)p + 1];
+        const int c2 = i >= mid;
+        const int kl[3] = {key_of(a.x), key_of(a.y), key_of(a.z)}, kh[3] = {key_of(b.x), key_of(b.y), key_of(b.z)};
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+          lo[0][k] = min(lo[0][k], c2 ? lo[0][k] : kl[k]);
+          hi[0][k] = max(hi[0][k], c2 ? hi[0][k] : kh[k]);
+          lo[1][k] = min(lo[1][k], c2 ? kl[k] : lo[1][k]);
+          hi[1][k] = max(hi[1][k], c2 ? kh[k] : hi[1][k]);
+        }
+      }
+#pragma unroll
+      for (int c2 = 0; c2 < 2; c2++)
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+          const int l = __reduce_min_sync(0xffffffffu, lo[c2][k]), h = __reduce_max_sync(0xffffffffu, hi[c2][k]);
+          if (lane == 0) {
+            atomicMin(&pool[n.left + c2].lo[k], l);
+            atomicMax(&pool[n.left + c2].hi[k], h);
+          }
+        }
       continue;
     }
     const uint32_t li = id - lb;
@@ -1503,15 +1549,15 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
   // built over, by level rounds alone.
   const uint32_t level_cap = (uint32_t)std::min<uint64_t>(max_depth, N) + 2;  // possible levels + one empty
   const uint32_t big_cap = N / (kBigChunks * kChunk) + 2;  // a big node holds > kBigChunks * kChunk primitives
-  uint32_t *lvl, *acc_cnt, *chunk_node, *chunk_cnt, *chunk_prefix, *big_list, *ended;
+  uint32_t *lvl, *chunk_cnt, *chunk_prefix, *big_list, *ended;
   LevelCounters* lcs;
-  int* acc_box;
+  LevelBuffers buf[2];  // this level's and the next one's
   // the counters and the level bounds: one copy to the host
   constexpr size_t kBounds = sizeof(BuildCounters) / 4;
   CK(S.alloc(&lvl, kBounds + level_cap + 2));
   BuildCounters* bc = reinterpret_cast<BuildCounters*>(lvl);
   lvl += kBounds;
-  CK(S.alloc(&lcs, level_cap));
+  CK(S.alloc(&lcs, (size_t)level_cap + 1));
   CK(S.alloc(&big_list, big_cap));
   CK(S.alloc(&ended, cap));
   std::vector<uint32_t> counters(kBounds + level_cap + 2);
@@ -1521,16 +1567,23 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
   for (uint32_t small = kSmall;; small = 0) {
     const size_t node_cap = 2 * (size_t)N / (std::max(bin_size, small) + 1ull) + G + 1;
     const size_t chunk_cap = (size_t)N / kChunk + node_cap + 1;
-    CK(S.alloc(&acc_cnt, 4 * node_cap));
-    CK(S.alloc(&acc_box, 24 * node_cap));
-    CK(S.alloc(&chunk_node, chunk_cap));
+    for (LevelBuffers& b : buf) {
+      CK(S.alloc(&b.acc_cnt, 4 * node_cap));
+      CK(S.alloc(&b.acc_box, 24 * node_cap));
+      CK(S.alloc(&b.chunk_node, chunk_cap));
+    }
+    const SplitRule rule{bin_size, max_depth, small};
     CK(S.alloc(&chunk_cnt, 4 * chunk_cap));
     CK(S.alloc(&chunk_prefix, 4 * chunk_cap));
     start_kernel<<<std::min(blocks_for(std::max(N, G)), persistent * 4), kBlock, 0, st>>>(N, G, dg_prim, order, pool, lvl, lcs,
-                                                                                        level_cap, bc);
+                                                                                        level_cap + 1, bc);
     if (N && small)  // once: it makes the indices global
       prepare_primitives_kernel<<<std::min(blocks_for(N), persistent * 4), kBlock, 0, st>>>(
           N, G, dg_prim, dg_vs, dg_vc, dg_ix, d.indices.ptr, d.vertices.ptr, pbox, bc);
+    if (G) {
+      prepare_roots_kernel<<<std::min(blocks_for(G), persistent), kBlock, 0, st>>>(G, rule, pool, buf[0], lcs, bc, ended);
+      root_box_kernel<<<persistent, kBlock, 0, st>>>(lcs, pool, buf[0].chunk_node, order, pbox);
+    }
     uint32_t queued = 0;
     bool closed = false;
     // first batch: about the depth of a balanced tree, then a few levels at a time
@@ -1542,19 +1595,18 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
       for (; queued < stop; queued++) {
         const uint32_t L = queued;
         uint32_t *from = L & 1 ? order_b : order, *to = L & 1 ? order : order_b;
-        level_prepare_kernel<<<persistent, kBlock, 0, st>>>(lvl, L, bin_size, max_depth, pool, acc_cnt, acc_box,
-                                                            chunk_node, lcs, small, bc, ended);
-        level_box_kernel<<<persistent, kBlock, 0, st>>>(lcs, L, pool, chunk_node, from, pbox);
-        level_stats_kernel<<<persistent, kBlock, 0, st>>>(lvl, L, lcs, pool, chunk_node, from, pbox, bucket,
-                                                          chunk_cnt, acc_cnt, acc_box);
-        level_decide_kernel<<<persistent, kBlock, 0, st>>>(lvl, L, pool, acc_cnt, acc_box,
+        const LevelBuffers &B = buf[L & 1], &next = buf[(L + 1) & 1];
+        level_stats_kernel<<<persistent, kBlock, 0, st>>>(lvl, L, lcs, pool, B.chunk_node, from, pbox, bucket, chunk_cnt,
+                                                          B.acc_cnt, B.acc_box);
+        level_decide_kernel<<<persistent, kBlock, 0, st>>>(lvl, L, pool, B.acc_cnt, B.acc_box,
                                                            reinterpret_cast<const uint4*>(chunk_cnt),
                                                            reinterpret_cast<uint4*>(chunk_prefix), lcs, bc, big_list,
-                                                           big_cap, (uint32_t)std::min<uint64_t>(cap, NONE));
+                                                           big_cap, (uint32_t)std::min<uint64_t>(cap, NONE), rule, next,
+                                                           ended);
         level_prefix_select_kernel<<<persistent, kBlock, 0, st>>>(lvl, lcs, L, pool, big_list, big_cap,
                                                                   reinterpret_cast<const uint4*>(chunk_cnt),
                                                                   reinterpret_cast<uint4*>(chunk_prefix), pbox, from);
-        level_scatter_kernel<<<persistent, kBlock, 0, st>>>(lvl, L, lcs, pool, chunk_node, from, bucket, acc_cnt,
+        level_scatter_kernel<<<persistent, kBlock, 0, st>>>(lvl, L, lcs, pool, pbox, B.chunk_node, from, bucket, B.acc_cnt,
                                                             chunk_prefix, to);
       }
       CK(cudaGetLastError());
