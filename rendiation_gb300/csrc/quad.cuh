@@ -84,19 +84,24 @@ __device__ __forceinline__ QuadWarp quad_warp(unsigned char* smem, uint32_t stac
   return w;
 }
 
-// True when the warp's rays point the same way (within 30 degrees of the first
-// one's direction) in the same TLAS. Which walk a ray takes does not
-// change its result; both kernels of a split query form the same vote.
+// True when the warp's rays are alike: but for at most kSeams of them each ray
+// points where the one before it does (within 30 degrees) in the same TLAS. A
+// seam is the end of an image's row, or of a batch of the caller's: with every
+// ray held against the first, the rows' ends of a 1000x524 image, one group in
+// 31, went to the quads and made 305 us of camera rays 430. Which walk a ray
+// takes does not change its result; both kernels of a split query form the
+// same vote.
 constexpr float kAlikeCos2 = 0.75f;
+constexpr int kSeams = 2;
 __device__ __forceinline__ bool coherent_warp(const RayCtx& R, uint32_t tidx, bool valid) {
-  const uint32_t m = __ballot_sync(kFullWarp, valid);
-  const uint32_t src = m ? (uint32_t)__ffs(m) - 1u : 0u;
-  const float dx = __shfl_sync(kFullWarp, R.d.x, src), dy = __shfl_sync(kFullWarp, R.d.y, src),
-              dz = __shfl_sync(kFullWarp, R.d.z, src);
-  const uint32_t t0 = __shfl_sync(kFullWarp, tidx, src);
+  const float dx = __shfl_up_sync(kFullWarp, R.d.x, 1), dy = __shfl_up_sync(kFullWarp, R.d.y, 1),
+              dz = __shfl_up_sync(kFullWarp, R.d.z, 1);
+  const uint32_t t0 = __shfl_up_sync(kFullWarp, tidx, 1);
+  const bool follows = __shfl_up_sync(kFullWarp, valid, 1) && (threadIdx.x & 31u) != 0u;
   const float dot = R.d.x * dx + R.d.y * dy + R.d.z * dz;
   const float len2 = (R.d.x * R.d.x + R.d.y * R.d.y + R.d.z * R.d.z) * (dx * dx + dy * dy + dz * dz);
-  return __all_sync(kFullWarp, !valid || (tidx == t0 && dot > 0.0f && dot * dot > kAlikeCos2 * len2));
+  const bool alike = tidx == t0 && dot > 0.0f && dot * dot > kAlikeCos2 * len2;
+  return __popc(__ballot_sync(kFullWarp, valid && follows && !alike)) <= kSeams;
 }
 
 // Walks the n entered rays order[0..n) of the warp. Every lane calls it; all
