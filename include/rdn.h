@@ -164,13 +164,13 @@ typedef struct rdn_hit_ext {
  * RDN_TRAVERSAL_ORDERED_WIDE: as ORDERED over 128 B four-child nodes collapsed
  *   from the same tree.
  * The two ordered values give the same results, and rdn_trace, the frames, the
- * paths and the differentiable calls walk both on the four-child nodes, one ray
- * per lane or four lanes per ray by their number of rays and by how alike a
- * warp's rays are (rdn_trace_counted and include/rdn_trace.cuh walk the nodes
- * that are asked for). The launch knobs of the descriptors (block_size,
- * local_stack, register_tier, speculation) change no result and act where a
- * ray has a lane of its own; stacks that fit 64 entries are in local memory
- * there unless dynamic fetch is asked for. */
+ * paths, the task graph's trace tasks and the differentiable calls walk both on
+ * the four-child nodes, one ray per lane or four lanes per ray by their number
+ * of rays and by how alike a warp's rays are (rdn_trace_counted and
+ * include/rdn_trace.cuh walk the nodes that are asked for). The launch knobs of
+ * the descriptors (block_size, local_stack, register_tier, speculation) change
+ * no result and act where a ray has a lane of its own; stacks that fit 64
+ * entries are in local memory there unless dynamic fetch is asked for. */
 #define RDN_TRAVERSAL_ORDERED 0u
 #define RDN_TRAVERSAL_REFERENCE 1u
 #define RDN_TRAVERSAL_ORDERED_WIDE 2u

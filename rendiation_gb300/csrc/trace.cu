@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(256) trace_kernel(TraceParams p) {
     R.cull_mask = p.cull_mask;
     R.ray_flags = p.ray_flags;
     bool bad;
-    traverse_ray<MODE, COUNT, BuiltinAnyHit, WT>(p, R, tidx, stack_ptr, stack_stride, bad);
+    traverse_ray<MODE, COUNT, BuiltinAnyHit, WT, 2, WT>(p, R, tidx, stack_ptr, stack_stride, bad);
     store_hit(p, i, R);
     if (bad) atomicOr(p.error_word, 2u);
     if (COUNT) {

@@ -532,21 +532,38 @@ __device__ __forceinline__ uint32_t interior_step(const TraceParams& p, RayCtx& 
 // three, 1672 with four (80 registers instead of 64: 1926, 56: 2110). Ambient
 // occlusion, 1280x720: 1742 with one, 1741 with two, 1862 with three. Path
 // tracing, 1280x720: 2210 with one, 2310 with two, 2510 with three.
-template <int STEPS, bool COUNT, int WIDTH, bool WT>
-__device__ __forceinline__ void descend(const TraceParams& p, RayCtx& R, const InstanceRay& ir, uint32_t& code,
-                                        float& code_tn, uint32_t& leaf, uint2* stack, uint32_t stride, uint32_t& sp,
-                                        uint32_t depth) {
-  while (!(code & LEAF_BIT)) {  // EMPTY_SLOT has the bit too
+//
+// CONVERGE: the lanes of `lanes`, all of which call, leave the loop together
+// (`lanes` is unused otherwise). Without it the compiler decides where they
+// meet again. That suits the frames (1080p 1661 us against 1697 with it,
+// watertight 1890, 1922) and queries (637, 640), but not the batch query with
+// the watertight test (2.07 M camera rays 778 us, 713 with it).
+template <int STEPS, bool COUNT, int WIDTH, bool WT, bool CONVERGE>
+__device__ __forceinline__ void descend(uint32_t lanes, const TraceParams& p, RayCtx& R, const InstanceRay& ir,
+                                        uint32_t& code, float& code_tn, uint32_t& leaf, uint2* stack, uint32_t stride,
+                                        uint32_t& sp, uint32_t depth) {
+  const auto steps = [&] {
 #pragma unroll
     for (int step = 0; step < (WIDTH == 4 ? STEPS : 1); step++) {
-      if (code & LEAF_BIT) continue;
+      if (code & LEAF_BIT) continue;  // EMPTY_SLOT has the bit too
       code = interior_step<COUNT, WIDTH, WT>(p, R, ir, code, code_tn, stack, stride, sp, depth);
       if (code != EMPTY_SLOT && (code & LEAF_BIT) && leaf == EMPTY_SLOT) {
         leaf = code;
         code = pop_live(stack, stride, sp, R.far_world * ir.scaling, code_tn);
       }
     }
-    if ((uint32_t)__popc(__ballot_sync(__activemask(), leaf == EMPTY_SLOT)) <= p.spec_threshold) break;
+  };
+  if constexpr (CONVERGE) {
+    uint32_t looking;
+    do {
+      steps();
+      looking = __ballot_sync(lanes, leaf == EMPTY_SLOT && !(code & LEAF_BIT));
+    } while ((uint32_t)__popc(looking) > p.spec_threshold);
+  } else {
+    while (!(code & LEAF_BIT)) {
+      steps();
+      if ((uint32_t)__popc(__ballot_sync(__activemask(), leaf == EMPTY_SLOT)) <= p.spec_threshold) break;
+    }
   }
 }
 
@@ -555,7 +572,7 @@ __device__ __forceinline__ void descend(const TraceParams& p, RayCtx& R, const I
 // a leaf (or has finished), then the warp tests triangles together. Nodes are
 // visited in near-first order with the reference's box test; the speculation
 // only adds visits, never removes one, so the closest hit is unchanged.
-template <int STEPS, bool COUNT, int WIDTH, class AH = BuiltinAnyHit, bool WT = false>
+template <int STEPS, bool CONVERGE, bool COUNT, int WIDTH, class AH = BuiltinAnyHit, bool WT = false>
 __device__ __forceinline__ bool blas_speculative(const TraceParams& p, RayCtx& R, const InstanceRay& ir,
                                                  uint32_t root_node, uint32_t gslot, uint32_t inst_slot,
                                                  bool is_opaque, bool cull_enable, bool cull_back, uint32_t prim_start,
@@ -577,13 +594,22 @@ __device__ __forceinline__ bool blas_speculative(const TraceParams& p, RayCtx& R
     leaf = code;
     code = EMPTY_SLOT;
   }
-  while (code != EMPTY_SLOT || leaf != EMPTY_SLOT) {
-    descend<STEPS, COUNT, WIDTH, WT>(p, R, ir, code, code_tn, leaf, stack, stride, sp, depth);
+  bool ended = false;
+  uint32_t lanes = __activemask();
+  for (;;) {
+    const bool busy = code != EMPTY_SLOT || leaf != EMPTY_SLOT;
+    if (CONVERGE) lanes = __ballot_sync(lanes, busy);
+    if (!busy) break;
+    descend<STEPS, COUNT, WIDTH, WT, CONVERGE>(lanes, p, R, ir, code, code_tn, leaf, stack, stride, sp, depth);
     while (leaf != EMPTY_SLOT) {
       const uint2 lr = leaf_range<WIDTH>(p, leaf);
       if (leaf_triangles<COUNT, AH, WT>(p, R, ir, lr.x, lr.y, gslot, inst_slot, is_opaque, cull_enable, cull_back,
-                                        prim_start, anyhit))
-        return true;
+                                        prim_start, anyhit)) {
+        if (!CONVERGE) return true;
+        code = leaf = EMPTY_SLOT;
+        ended = true;
+        break;
+      }
       leaf = EMPTY_SLOT;
       // the far may have shrunk: re-check the pending node before descending into it
       if (code != EMPTY_SLOT && !(code_tn < R.far_world * ir.scaling))
@@ -594,12 +620,13 @@ __device__ __forceinline__ bool blas_speculative(const TraceParams& p, RayCtx& R
       }
     }
   }
-  return false;
+  return ended;
 }
 
 // Full query of one ray (traverse_cpu.rs:52-245). R must hold the ray; on
 // return R.best holds the committed hit. `bad` reports an unbound TLAS index.
-template <int MODE, bool COUNT, class AH = BuiltinAnyHit, bool WT = false, int STEPS = 2>
+template <int MODE, bool COUNT, class AH = BuiltinAnyHit, bool WT = false, int STEPS = 2,
+          bool CONVERGE = false>
 __device__ __forceinline__ void traverse_ray(const TraceParams& p, RayCtx& R, uint32_t tidx, uint2* stack,
                                              uint32_t stride, bool& bad, const AH& anyhit = AH()) {
   R.inv_d = make_float3(1.0f / R.d.x, 1.0f / R.d.y, 1.0f / R.d.z);
@@ -648,10 +675,10 @@ __device__ __forceinline__ void traverse_ray(const TraceParams& p, RayCtx& R, ui
         if (!pass) continue;
         bool end;
         if (MODE == MODE_WIDE4)
-          end = blas_speculative<STEPS, COUNT, 4, AH, WT>(p, R, ir, gm.x, g, ti, is_opaque, cull_enable, cull_back, gm.z, stack,
+          end = blas_speculative<STEPS, CONVERGE, COUNT, 4, AH, WT>(p, R, ir, gm.x, g, ti, is_opaque, cull_enable, cull_back, gm.z, stack,
                                                stride, p.stack_depth, anyhit);
         else if (MODE == MODE_BINARY)
-          end = blas_speculative<STEPS, COUNT, 2, AH, WT>(p, R, ir, gm.x, g, ti, is_opaque, cull_enable, cull_back, gm.z, stack,
+          end = blas_speculative<STEPS, CONVERGE, COUNT, 2, AH, WT>(p, R, ir, gm.x, g, ti, is_opaque, cull_enable, cull_back, gm.z, stack,
                                                stride, p.stack_depth, anyhit);
         else
           end = blas_threaded<COUNT, AH, WT>(p, R, ir, gm.x, g, ti, is_opaque, cull_enable, cull_back, gm.z, anyhit);
@@ -808,7 +835,7 @@ struct LaneWalk {
         phase = WALK_DONE;
         return;
       }
-      descend<2, false, WIDTH, WT>(p, R, ir, code, code_tn, leaf, stack, stride, sp, p.stack_depth);
+      descend<2, false, WIDTH, WT, false>(0u, p, R, ir, code, code_tn, leaf, stack, stride, sp, p.stack_depth);
       while (leaf != EMPTY_SLOT) {
         const uint2 lr = leaf_range<WIDTH>(p, leaf);
         if (leaf_triangles<false, BuiltinAnyHit, WT>(p, R, ir, lr.x, lr.y, gslot, inst_slot, is_opaque, cull_enable, cull_back,
