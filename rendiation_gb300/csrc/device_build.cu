@@ -572,9 +572,9 @@ __global__ void level_decide_kernel(const uint32_t* __restrict__ lvl, uint32_t L
     const uint32_t n_med = __popc(__ballot_sync(0xffffffffu, active && fallback));
     if (lane == 0 && n_sah) atomicAdd(&bc->sah, (unsigned long long)n_sah);
     if (lane == 0 && n_med) atomicAdd(&bc->fallback, (unsigned long long)n_med);
-    const bool big = active && !fallback && n.nchunks > kBigChunks;
-    const uint32_t slot = warp_claim(&lc->big, big ? 1u : 0u, lane);
     const bool fits = active && base + 1 < pool_cap;
+    const bool big = fits && !fallback && n.nchunks > kBigChunks;
+    const uint32_t slot = warp_claim(&lc->big, big ? 1u : 0u, lane);
     if (active && !fits) {  // the host gives up on the build; no kernel may scatter this node
       bc->overflow = 1u;
       pool[lb + i].flags = n.flags & ~F_ACTIVE;
@@ -682,20 +682,34 @@ __global__ void __launch_bounds__(kBlock) level_prefix_select_kernel(
   }
 }
 
+// End of the level whose first node is `first`: the children that were claimed,
+// as far as the pool holds them. Children are claimed in pairs from `first` on
+// and a pair is written when both of its slots lie below `cap`, so every node
+// below the end that this returns has been written: the levels that are queued
+// behind an overflow see no other node, and none of theirs fits any more.
+__host__ __device__ constexpr uint32_t level_end(uint32_t first, uint32_t children, uint32_t cap) {
+  const uint32_t room = (cap - first) & ~1u;
+  return first + (children < room ? children : room);
+}
+static_assert(level_end(10, 4, 14) == 14 && level_end(10, 4, 13) == 12 && level_end(10, 4, 11) == 10 &&
+                  level_end(10, 0, 64) == 10 && level_end(10, 6, 10) == 10,
+              "whole pairs below the cap");
+
 // SAH nodes: each chunk writes its primitives to their bucket-ordered slots of
 // the other order array; a median-split node's are copied as they stand. Also
-// closes the level: the next level's end is its start plus the children that
-// level_decide_kernel created (decide ran before this launch).
+// closes the level: the next level's end, from the children that
+// level_decide_kernel claimed (decide ran before this launch).
 __global__ void level_scatter_kernel(uint32_t* __restrict__ lvl, uint32_t L, const LevelCounters* lcs, BNode* __restrict__ pool,
                                      const float4* __restrict__ pbox,
                                      const uint32_t* __restrict__ chunk_node, const uint32_t* __restrict__ order,
                                      const uint8_t* __restrict__ bucket, const uint32_t* __restrict__ acc_cnt,
-                                     const uint32_t* __restrict__ chunk_prefix, uint32_t* __restrict__ scratch) {
+                                     const uint32_t* __restrict__ chunk_prefix, uint32_t* __restrict__ scratch,
+                                     uint32_t pool_cap) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t lt_mask = (1u << lane) - 1u;
   const uint32_t lb = lvl[L];
   const uint32_t total = lcs[L].chunks;
-  if (blockIdx.x == 0 && threadIdx.x == 0) lvl[L + 2] = lvl[L + 1] + lcs[L].children;
+  if (blockIdx.x == 0 && threadIdx.x == 0) lvl[L + 2] = level_end(lvl[L + 1], lcs[L].children, pool_cap);
   for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < total; c += (gridDim.x * blockDim.x) >> 5) {
     const uint32_t id = chunk_node[c];
     const BNode n = pool[id];
@@ -1538,6 +1552,7 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
   const size_t cap = 2 * (size_t)N + 2 * (size_t)G + 64;
   BNode* pool;
   CK(S.alloc(&pool, cap));
+  const uint32_t pool_cap = (uint32_t)std::min<uint64_t>(cap, NONE);
 
   // level rounds. Every buffer is sized for the largest possible level (nodes
   // that are split hold more than `small` and more than bin_size primitives,
@@ -1601,13 +1616,13 @@ std::string build_blas_device(const std::vector<DeviceGeometry>& geoms, uint32_t
         level_decide_kernel<<<persistent, kBlock, 0, st>>>(lvl, L, pool, B.acc_cnt, B.acc_box,
                                                            reinterpret_cast<const uint4*>(chunk_cnt),
                                                            reinterpret_cast<uint4*>(chunk_prefix), lcs, bc, big_list,
-                                                           big_cap, (uint32_t)std::min<uint64_t>(cap, NONE), rule, next,
+                                                           big_cap, pool_cap, rule, next,
                                                            ended);
         level_prefix_select_kernel<<<persistent, kBlock, 0, st>>>(lvl, lcs, L, pool, big_list, big_cap,
                                                                   reinterpret_cast<const uint4*>(chunk_cnt),
                                                                   reinterpret_cast<uint4*>(chunk_prefix), pbox, from);
         level_scatter_kernel<<<persistent, kBlock, 0, st>>>(lvl, L, lcs, pool, pbox, B.chunk_node, from, bucket, B.acc_cnt,
-                                                            chunk_prefix, to);
+                                                            chunk_prefix, to, pool_cap);
       }
       CK(cudaGetLastError());
       if (!d.tri_records.ptr) {  // while the levels run
