@@ -52,7 +52,9 @@ struct Hit {
 // One query: MODE rdn::MODE_THREADED (the reference's order) or
 // rdn::MODE_WIDE4 / rdn::MODE_BINARY (ordered walks; Params from
 // rdn_trace_params with that traversal, whose stack fits this thread's
-// local array). Params asked for with RDN_INTERSECT_WATERTIGHT select the
+// local array; a push past the depth that they state, as when they are of
+// another ordered walk or of an earlier build, sets the context's error word
+// and is left out). Params asked for with RDN_INTERSECT_WATERTIGHT select the
 // watertight triangle test (both forms are compiled into the caller's kernel).
 template <int MODE, class AnyHit>
 __device__ inline Hit trace(const Params& p, const rdn_ray& ray, uint32_t tlas, uint32_t ray_flags,
@@ -67,9 +69,9 @@ __device__ inline Hit trace(const Params& p, const rdn_ray& ray, uint32_t tlas, 
   R.cull_mask = cull_mask;
   bool bad;
   if (p.watertight)
-    rdn::dev::traverse_ray<MODE, false, AnyHit, true>(p, R, tlas, stack, 1u, bad, anyhit);
+    rdn::dev::traverse_ray<MODE, false, AnyHit, true, 2, false, true>(p, R, tlas, stack, 1u, bad, anyhit);
   else
-    rdn::dev::traverse_ray<MODE, false, AnyHit, false>(p, R, tlas, stack, 1u, bad, anyhit);
+    rdn::dev::traverse_ray<MODE, false, AnyHit, false, 2, false, true>(p, R, tlas, stack, 1u, bad, anyhit);
   Hit h;
   h.unbound_tlas = bad;
   if (R.best.have) {

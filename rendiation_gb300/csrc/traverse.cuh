@@ -390,7 +390,7 @@ __device__ __forceinline__ uint32_t pop_live(const uint2* stack, uint32_t stride
 __device__ __forceinline__ void push_entry(const TraceParams& p, uint2* stack, uint32_t stride, uint32_t& sp,
                                            uint32_t depth, uint32_t code, float tn) {
   if (sp < depth) stack[(sp++) * stride] = make_uint2(code, __float_as_uint(tn));
-  else atomicOr(p.error_word, 1u);  // the stack is sized from the tree depth: unreachable
+  else atomicOr(p.error_word, 1u);  // unreachable with a stack that is sized from the tree's depth
 }
 
 // A child of a four-child node (Wide4Child): one 32 B load.
@@ -473,7 +473,7 @@ __device__ __forceinline__ uint32_t wide4_root(const TraceParams& p, uint32_t g)
 // One interior-node step of the ordered walk: tests the children of node
 // `code`, pushes the farther hits and returns the nearest hit child (or the
 // next live stack entry when no child is hit).
-template <bool COUNT, int WIDTH, bool WT = false>
+template <bool COUNT, int WIDTH, bool WT, bool CHECKED>
 __device__ __forceinline__ uint32_t interior_step(const TraceParams& p, RayCtx& R, const InstanceRay& ir, uint32_t code,
                                                   float& code_tn, uint2* stack, uint32_t stride, uint32_t& sp,
                                                   uint32_t depth) {
@@ -514,11 +514,16 @@ __device__ __forceinline__ uint32_t interior_step(const TraceParams& p, RayCtx& 
     cswap(t1, c1, t3, c3);
     cswap(t1, c1, t2, c2);
     if (c0 == EMPTY_SLOT) return pop_live(stack, stride, sp, far_, code_tn);
-    // no bounds check: a step leaves at most three entries per level of the four-child tree, and the stack has
-    // 3 D + 1 for D levels (stack_entries); with one the 1080p frame took 1912 us instead of 1747
-    if (c3 != EMPTY_SLOT) stack[(sp++) * stride] = make_uint2(c3, __float_as_uint(t3));
-    if (c2 != EMPTY_SLOT) stack[(sp++) * stride] = make_uint2(c2, __float_as_uint(t2));
-    if (c1 != EMPTY_SLOT) stack[(sp++) * stride] = make_uint2(c1, __float_as_uint(t1));
+    // the library's own kernels make no bounds check: a step leaves at most three entries per level of the four-child
+    // tree, and their stacks have 3 D + 1 for D levels (stack_entries); with one the 1080p frame took 1912 us instead
+    // of 1747. CHECKED: a caller's kernel, whose stack array and parameters need not be of this tree and walk.
+    const auto push = [&](uint32_t c, float t) {
+      if (CHECKED) push_entry(p, stack, stride, sp, depth, c, t);
+      else stack[(sp++) * stride] = make_uint2(c, __float_as_uint(t));
+    };
+    if (c3 != EMPTY_SLOT) push(c3, t3);
+    if (c2 != EMPTY_SLOT) push(c2, t2);
+    if (c1 != EMPTY_SLOT) push(c1, t1);
     code_tn = t0;
     return c0;
   }
@@ -538,7 +543,7 @@ __device__ __forceinline__ uint32_t interior_step(const TraceParams& p, RayCtx& 
 // meet again. That suits the frames (1080p 1661 us against 1697 with it,
 // watertight 1890, 1922) and queries (637, 640), but not the batch query with
 // the watertight test (2.07 M camera rays 778 us, 713 with it).
-template <int STEPS, bool COUNT, int WIDTH, bool WT, bool CONVERGE>
+template <int STEPS, bool COUNT, int WIDTH, bool WT, bool CONVERGE, bool CHECKED>
 __device__ __forceinline__ void descend(uint32_t lanes, const TraceParams& p, RayCtx& R, const InstanceRay& ir,
                                         uint32_t& code, float& code_tn, uint32_t& leaf, uint2* stack, uint32_t stride,
                                         uint32_t& sp, uint32_t depth) {
@@ -546,7 +551,7 @@ __device__ __forceinline__ void descend(uint32_t lanes, const TraceParams& p, Ra
 #pragma unroll
     for (int step = 0; step < (WIDTH == 4 ? STEPS : 1); step++) {
       if (code & LEAF_BIT) continue;  // EMPTY_SLOT has the bit too
-      code = interior_step<COUNT, WIDTH, WT>(p, R, ir, code, code_tn, stack, stride, sp, depth);
+      code = interior_step<COUNT, WIDTH, WT, CHECKED>(p, R, ir, code, code_tn, stack, stride, sp, depth);
       if (code != EMPTY_SLOT && (code & LEAF_BIT) && leaf == EMPTY_SLOT) {
         leaf = code;
         code = pop_live(stack, stride, sp, R.far_world * ir.scaling, code_tn);
@@ -572,7 +577,7 @@ __device__ __forceinline__ void descend(uint32_t lanes, const TraceParams& p, Ra
 // a leaf (or has finished), then the warp tests triangles together. Nodes are
 // visited in near-first order with the reference's box test; the speculation
 // only adds visits, never removes one, so the closest hit is unchanged.
-template <int STEPS, bool CONVERGE, bool COUNT, int WIDTH, class AH = BuiltinAnyHit, bool WT = false>
+template <int STEPS, bool CONVERGE, bool COUNT, int WIDTH, class AH, bool WT, bool CHECKED>
 __device__ __forceinline__ bool blas_speculative(const TraceParams& p, RayCtx& R, const InstanceRay& ir,
                                                  uint32_t root_node, uint32_t gslot, uint32_t inst_slot,
                                                  bool is_opaque, bool cull_enable, bool cull_back, uint32_t prim_start,
@@ -600,7 +605,7 @@ __device__ __forceinline__ bool blas_speculative(const TraceParams& p, RayCtx& R
     const bool busy = code != EMPTY_SLOT || leaf != EMPTY_SLOT;
     if (CONVERGE) lanes = __ballot_sync(lanes, busy);
     if (!busy) break;
-    descend<STEPS, COUNT, WIDTH, WT, CONVERGE>(lanes, p, R, ir, code, code_tn, leaf, stack, stride, sp, depth);
+    descend<STEPS, COUNT, WIDTH, WT, CONVERGE, CHECKED>(lanes, p, R, ir, code, code_tn, leaf, stack, stride, sp, depth);
     while (leaf != EMPTY_SLOT) {
       const uint2 lr = leaf_range<WIDTH>(p, leaf);
       if (leaf_triangles<COUNT, AH, WT>(p, R, ir, lr.x, lr.y, gslot, inst_slot, is_opaque, cull_enable, cull_back,
@@ -625,8 +630,8 @@ __device__ __forceinline__ bool blas_speculative(const TraceParams& p, RayCtx& R
 
 // Full query of one ray (traverse_cpu.rs:52-245). R must hold the ray; on
 // return R.best holds the committed hit. `bad` reports an unbound TLAS index.
-template <int MODE, bool COUNT, class AH = BuiltinAnyHit, bool WT = false, int STEPS = 2,
-          bool CONVERGE = false>
+template <int MODE, bool COUNT, class AH = BuiltinAnyHit, bool WT = false, int STEPS = 2, bool CONVERGE = false,
+          bool CHECKED = false>
 __device__ __forceinline__ void traverse_ray(const TraceParams& p, RayCtx& R, uint32_t tidx, uint2* stack,
                                              uint32_t stride, bool& bad, const AH& anyhit = AH()) {
   R.inv_d = make_float3(1.0f / R.d.x, 1.0f / R.d.y, 1.0f / R.d.z);
@@ -675,10 +680,10 @@ __device__ __forceinline__ void traverse_ray(const TraceParams& p, RayCtx& R, ui
         if (!pass) continue;
         bool end;
         if (MODE == MODE_WIDE4)
-          end = blas_speculative<STEPS, CONVERGE, COUNT, 4, AH, WT>(p, R, ir, gm.x, g, ti, is_opaque, cull_enable, cull_back, gm.z, stack,
+          end = blas_speculative<STEPS, CONVERGE, COUNT, 4, AH, WT, CHECKED>(p, R, ir, gm.x, g, ti, is_opaque, cull_enable, cull_back, gm.z, stack,
                                                stride, p.stack_depth, anyhit);
         else if (MODE == MODE_BINARY)
-          end = blas_speculative<STEPS, CONVERGE, COUNT, 2, AH, WT>(p, R, ir, gm.x, g, ti, is_opaque, cull_enable, cull_back, gm.z, stack,
+          end = blas_speculative<STEPS, CONVERGE, COUNT, 2, AH, WT, CHECKED>(p, R, ir, gm.x, g, ti, is_opaque, cull_enable, cull_back, gm.z, stack,
                                                stride, p.stack_depth, anyhit);
         else
           end = blas_threaded<COUNT, AH, WT>(p, R, ir, gm.x, g, ti, is_opaque, cull_enable, cull_back, gm.z, anyhit);
@@ -835,7 +840,7 @@ struct LaneWalk {
         phase = WALK_DONE;
         return;
       }
-      descend<2, false, WIDTH, WT, false>(0u, p, R, ir, code, code_tn, leaf, stack, stride, sp, p.stack_depth);
+      descend<2, false, WIDTH, WT, false, false>(0u, p, R, ir, code, code_tn, leaf, stack, stride, sp, p.stack_depth);
       while (leaf != EMPTY_SLOT) {
         const uint2 lr = leaf_range<WIDTH>(p, leaf);
         if (leaf_triangles<false, BuiltinAnyHit, WT>(p, R, ir, lr.x, lr.y, gslot, inst_slot, is_opaque, cull_enable, cull_back,
