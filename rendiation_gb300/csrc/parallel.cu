@@ -26,8 +26,9 @@
 // 10,000 elements: 99 -> 44, 21 -> 11, 15 -> 6.
 //
 // A tile's predecessors have taken their tickets before it, so they run and
-// every wait ends; each wait is bounded all the same, and a block whose wait
-// runs out writes nothing.
+// every wait ends; each wait is bounded all the same. A block whose wait runs
+// out counts the missing tile in the input itself, so that every result is
+// right whatever held the other block up.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -40,7 +41,7 @@ namespace {
 constexpr uint32_t THREADS = 512, WARPS = THREADS / 32, ITEMS = 16, TILE = THREADS * ITEMS;
 constexpr uint32_t SORT_TILE = 4096, HIST_THREADS = 256;
 constexpr uint32_t FULL = 0xffffffffu;
-constexpr uint32_t kMaxWait = 1u << 22;  // polls of one descriptor
+constexpr uint32_t kMaxWait = 1u << 16;  // polls of one descriptor, some 40 ms: waits are of microseconds
 constexpr uint32_t DIGITS = 256;
 constexpr uint32_t kWindow = 4;
 
@@ -67,34 +68,70 @@ __device__ __forceinline__ uint32_t take_tile(uint32_t* ticket, uint32_t* shared
   return *shared;
 }
 
+// The sum over one whole tile of `in`, by a warp, for a look-back whose wait
+// ran out. `in` may be what the scan writes over: see look_back.
+__device__ __forceinline__ uint32_t tile_sum(const uint32_t* in, uint32_t tile, bool as_flags) {
+  const volatile uint32_t* p = in + (size_t)tile * TILE;
+  uint32_t sum = 0;
+#pragma unroll 1
+  for (uint32_t k = threadIdx.x & 31u; k < TILE; k += 32u) sum += as_flags ? (uint32_t)(p[k] != 0u) : p[k];
+  return __reduce_add_sync(FULL, sum);
+}
+
+// Publishes ahead of everything that the block writes after its next barrier:
+// an exchange that acquires. 16,000,000 elements in place take 33.8 us with it,
+// 46.7 with a plain store and a fence after the look-back, and took 43.2 with
+// the store alone, which orders nothing.
+__device__ __forceinline__ void publish_first(volatile TileState* at, TileState s) {
+  TileState old;
+  asm volatile("atom.acquire.gpu.global.exch.b64 %0, [%1], %2;" : "=l"(old) : "l"(const_cast<TileState*>(at)), "l"(s) : "memory");
+}
+
 // One warp: publishes the tile's total and returns the sum of the tiles
-// [first, tile) before it. False when a wait ran out.
-__device__ __forceinline__ bool look_back(volatile TileState* state, uint32_t tile, uint32_t first, uint32_t total,
-                                          uint32_t& before) {
+// [first, tile) before it. A tile that does not publish in time is summed here.
+// That holds in place too: nothing of the block is written before its
+// descriptor is (publish_first), so one that is still empty after the sum was
+// read proves that the tile's input was whole.
+__device__ __forceinline__ uint32_t look_back(volatile TileState* state, uint32_t tile, uint32_t first, uint32_t total,
+                                              const uint32_t* in, bool as_flags, bool in_place) {
   const uint32_t lane = threadIdx.x & 31u;
-  before = 0;
-  if (lane == 0) state[tile] = tile_state(tile == first ? TILE_PREFIX : TILE_SUM, total);
-  if (tile == first) return true;
+  uint32_t before = 0;
+  if (lane == 0) {
+    const TileState own = tile_state(tile == first ? TILE_PREFIX : TILE_SUM, total);
+    if (in_place) publish_first(state + tile, own);
+    else state[tile] = own;
+  }
+  if (tile == first) return 0;
   for (uint32_t behind = 1;; behind += 32) {
     // lane k reads the tile `behind + k` before; the first tile's prefix is its sum
     const uint32_t back = behind + lane;
-    const bool in = back <= tile - first;
+    const bool known = back > tile - first;
     TileState s = 0;
     uint32_t stop = 0;
     for (uint32_t polls = 0;; polls++) {
-      s = in ? state[tile - back] : tile_state(TILE_PREFIX, 0u);
+      s = known ? tile_state(TILE_PREFIX, 0u) : state[tile - back];
       const uint32_t empty = __ballot_sync(FULL, (uint32_t)(s >> 32) == TILE_EMPTY);
       stop = __ballot_sync(FULL, (uint32_t)(s >> 32) == TILE_PREFIX);
       const uint32_t need = stop ? (stop & -stop) - 1u : FULL;  // lanes before the nearest prefix
-      if ((empty & need) == 0u) break;
-      if (polls >= kMaxWait) return false;
+      uint32_t missing = empty & need;
+      if (missing == 0u) break;
+      if (polls < kMaxWait) continue;
+      for (; missing; missing &= missing - 1u) {
+        const uint32_t k = (uint32_t)__ffs(missing) - 1u, at = tile - behind - k;
+        const uint32_t sum = tile_sum(in, at, as_flags);
+        __threadfence();
+        const TileState now = state[at];
+        if (lane == k) s = (uint32_t)(now >> 32) == TILE_EMPTY ? tile_state(at == first ? TILE_PREFIX : TILE_SUM, sum) : now;
+      }
+      stop = __ballot_sync(FULL, (uint32_t)(s >> 32) == TILE_PREFIX);
+      break;
     }
     const uint32_t upto = stop ? (uint32_t)__ffs(stop) - 1u : 31u;
     before += __reduce_add_sync(FULL, lane <= upto ? (uint32_t)s : 0u);
     if (stop) break;
   }
   if (lane == 0) state[tile] = tile_state(TILE_PREFIX, before + total);
-  return true;
+  return before;
 }
 
 // A warp's 512 elements of a tile, four consecutive ones per lane and round.
@@ -155,11 +192,10 @@ __device__ __forceinline__ uint32_t tile_exclusive(const uint4 (&v)[4], uint32_t
 
 // segment_tiles: 0, or the tiles after which the sum restarts.
 template <bool VEC>
-__global__ void __launch_bounds__(THREADS) scan_kernel(const uint32_t* in, uint32_t* out, uint32_t n, bool inclusive,
+__global__ void __launch_bounds__(THREADS, 3) scan_kernel(const uint32_t* in, uint32_t* out, uint32_t n, bool inclusive,
                                                        bool as_flags, uint32_t segment_tiles, TileState* state,
                                                        uint32_t* ticket) {
-  __shared__ uint32_t warp_sums[WARPS], tile_s, before_s, ok_s;
-  uint32_t before;
+  __shared__ uint32_t warp_sums[WARPS], tile_s, before_s;
   const uint32_t tile = take_tile(ticket, &tile_s);
   uint4 v[4];
 #pragma unroll
@@ -170,15 +206,12 @@ __global__ void __launch_bounds__(THREADS) scan_kernel(const uint32_t* in, uint3
   uint32_t base[4];
   const uint32_t total = tile_exclusive(v, base, warp_sums);
   if (threadIdx.x < 32) {
-    const bool ok = look_back(state, tile, segment_tiles ? tile - tile % segment_tiles : 0u, total, before);
-    if (threadIdx.x == 0) {
-      before_s = before;
-      ok_s = ok;
-    }
+    const uint32_t sum =
+        look_back(state, tile, segment_tiles ? tile - tile % segment_tiles : 0u, total, in, as_flags, in == out);
+    if (threadIdx.x == 0) before_s = sum;
   }
   __syncthreads();
-  if (!ok_s) return;
-  before = before_s;
+  const uint32_t before = before_s;
 #pragma unroll
   for (int r = 0; r < 4; r++) {
     const uint4 x = v[r];
@@ -227,7 +260,7 @@ __global__ void __launch_bounds__(THREADS) compact_kernel(const uint32_t* __rest
                                                           uint32_t* __restrict__ out, uint32_t n, uint32_t tiles,
                                                           uint32_t* __restrict__ count, TileState* state,
                                                           uint32_t* ticket) {
-  __shared__ uint32_t warp_sums[WARPS], tile_s, before_s, ok_s, kept[TILE];
+  __shared__ uint32_t warp_sums[WARPS], tile_s, before_s, kept[TILE];
   const uint32_t tile = take_tile(ticket, &tile_s);
   uint4 f[4], v[4];
 #pragma unroll
@@ -246,16 +279,13 @@ __global__ void __launch_bounds__(THREADS) compact_kernel(const uint32_t* __rest
     if (f[r].w) kept[at++] = v[r].w;
   }
   if (threadIdx.x < 32) {
-    uint32_t before;
-    const bool ok = look_back(state, tile, 0u, total, before);
+    const uint32_t before = look_back(state, tile, 0u, total, flags, true, false);
     if (threadIdx.x == 0) {
       before_s = before;
-      ok_s = ok;
-      if (ok && tile == tiles - 1) *count = before + total;
+      if (tile == tiles - 1) *count = before + total;
     }
   }
   __syncthreads();
-  if (!ok_s) return;
   for (uint32_t i = threadIdx.x; i < total; i += THREADS) out[before_s + i] = kept[i];
 }
 
@@ -415,6 +445,17 @@ __device__ __forceinline__ uint32_t rank_tile(SortShared& S, const uint32_t (&ke
   return total;
 }
 
+// The keys of one whole tile with digit `digit`, by a thread whose wait for the
+// tile's count ran out.
+__device__ __forceinline__ uint32_t tile_digits(const uint32_t* __restrict__ keys, uint32_t tile, uint32_t shift,
+                                             uint32_t digit) {
+  const uint32_t* p = keys + (size_t)tile * SORT_TILE;
+  uint32_t count = 0;
+#pragma unroll 1
+  for (uint32_t k = 0; k < SORT_TILE; k++) count += ((__ldg(p + k) >> shift) & 0xFFu) == digit;
+  return count;
+}
+
 // One pass over the tile that this block takes. D: descriptor word, the count
 // in its low bits, the status in its two top ones. first_of: where each
 // digit's run starts in the output.
@@ -455,7 +496,6 @@ __global__ void __launch_bounds__(SORT_THREADS, 3) sort_pass(const uint32_t* __r
       S.key[place[r]] = key[r];
       if (vals_out) S.val[place[r]] = val[r];
     }
-  bool ok = true;
   if (threadIdx.x < DIGITS) {
     D before = 0;
     for (uint32_t back = 1; back <= tile;) {
@@ -463,7 +503,7 @@ __global__ void __launch_bounds__(SORT_THREADS, 3) sort_pass(const uint32_t* __r
 #pragma unroll
       for (uint32_t k = 0; k < kWindow; k++)
         d[k] = back + k <= tile ? own[-(ptrdiff_t)((size_t)(back + k) * DIGITS)] : (D)0;
-      bool done = false;
+      bool done = false, missing = false;
       uint32_t polls = 0;
 #pragma unroll
       for (uint32_t k = 0; k < kWindow; k++) {
@@ -473,8 +513,7 @@ __global__ void __launch_bounds__(SORT_THREADS, 3) sort_pass(const uint32_t* __r
           polls++;
         }
         if ((d[k] >> STATUS) == TILE_EMPTY) {
-          ok = false;
-          done = true;
+          missing = true;
           break;
         }
         before += d[k] & VALUE;
@@ -482,11 +521,12 @@ __global__ void __launch_bounds__(SORT_THREADS, 3) sort_pass(const uint32_t* __r
         back++;
       }
       if (done) break;
+      if (missing) before += tile_digits(keys_in, tile - back++, shift, threadIdx.x);
     }
-    if (ok && tile) *own = ((D)TILE_PREFIX << STATUS) | (before + count);
+    if (tile) *own = ((D)TILE_PREFIX << STATUS) | (before + count);
     S.offset[threadIdx.x] = digit_first + (uint32_t)before - S.first[threadIdx.x];
   }
-  if (__syncthreads_or(!ok)) return;
+  __syncthreads();
   const uint32_t live = (uint32_t)(n - tile0 < SORT_TILE ? n - tile0 : SORT_TILE);
 #pragma unroll
   for (uint32_t r = 0; r < ROUNDS; r++) {
