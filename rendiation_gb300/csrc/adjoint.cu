@@ -663,7 +663,9 @@ cudaError_t launch_attr_paths(const TraceParams& p, const PathAdjointParams& a, 
   if (mode == MODE_THREADED)
     return launch_attr_paths_mode<MODE_THREADED, false, false>(p, a, adjoint, block, sm_count, stream);
   const TraceParams q = wide4_params(p);
-  if (p.packed && (a.count <= kQuadPaths || !q.local_stack))
+  // instanced structures: quads at every size (64 instances of 20,000 triangles, 700,000 paths of two segments: 11300 us
+  // one per lane, whose lanes part at the first of a ray's BLASes, 3430 with quads; 512 of 100: 3290, 1340)
+  if (p.packed && (a.count <= kQuadPaths || !q.local_stack || q.instanced))
     return launch_attr_paths_mode<MODE_WIDE4, true, false>(p, a, adjoint, block, sm_count, stream);
   return q.local_stack ? launch_attr_paths_mode<MODE_WIDE4, false, true>(q, a, adjoint, block, sm_count, stream)
                        : launch_attr_paths_mode<MODE_WIDE4, false, false>(q, a, adjoint, block, sm_count, stream);

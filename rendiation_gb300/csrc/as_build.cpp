@@ -225,6 +225,21 @@ Tree build_tree(const std::vector<Box>& boxes, uint32_t bin_size, uint32_t max_d
   return t;
 }
 
+// Share of `whole`'s area, the chance that a random line through `whole` meets
+// the box `part` of it; 0 where the areas give none.
+double area_share(const Box& part, const Box& whole) {
+  const double a = area(part), b = area(whole);
+  return a > 0.0 && b > 0.0 && a <= b && std::isfinite(b) ? a / b : 0.0;
+}
+
+// HostBuilt::geom_line_nodes of a tree.
+float line_nodes(const Tree& t) {
+  double sum = 0.0;
+  for (const TreeNode& n : t.nodes)
+    if (n.left_count) sum += area_share(n.box, t.nodes[0].box);
+  return (float)sum;
+}
+
 // compute_bvh_next (naive/mod.rs:611-632): threaded hit/miss links, pre-order.
 std::vector<std::pair<uint32_t, uint32_t>> threaded_links(const std::vector<TreeNode>& nodes) {
   std::vector<std::pair<uint32_t, uint32_t>> links(nodes.size());
@@ -476,6 +491,8 @@ Box transform_box(const Box& b, const M4& m) {  // Box3::apply_matrix
 std::string build_tlas_phase(const std::vector<std::unique_ptr<std::vector<InstanceSource>>>& tlas,
                              const std::vector<Box>& blas_box, const std::vector<char>& blas_box_some,
                              const BuildOptions& opt, HostBuilt& hb) {
+  double line_sum = 0.0;
+  uint32_t line_count = 0;
   for (const auto& tp : tlas) {
     if (!tp) {
       hb.tlas_bvh_root.push_back(INVALID_NEXT);
@@ -493,6 +510,20 @@ std::string build_tlas_phase(const std::vector<std::unique_ptr<std::vector<Insta
       aabbs.push_back(transform_box(blas_box[s.blas_handle], m));
     }
     Tree t = build_tree(aabbs, opt.tlas_bin_size, opt.tlas_max_depth, 1);
+    if (!tp->empty()) {
+      double met = line_nodes(t);
+      for (size_t i = 0; i < tp->size(); i++) {
+        const uint32_t blas = (*tp)[i].blas_handle;
+        double below = 0.0;
+        if (blas < hb.blas_meta_info.size())
+          for (uint32_t g = hb.blas_meta_info[blas].tri_root_range[0]; g < hb.blas_meta_info[blas].tri_root_range[1]; g++)
+            below += 1.0 + hb.geom_line_nodes[g];
+        met += (tp->size() == 1 ? 1.0 : area_share(aabbs[i], t.nodes[0].box)) * below;
+      }
+      line_sum += met;
+      line_count++;
+      hb.instanced |= tp->size() > 1;
+    }
     for (uint32_t idx : t.order) {
       const InstanceSource& s = (*tp)[idx];
       M4 m;
@@ -529,6 +560,7 @@ std::string build_tlas_phase(const std::vector<std::unique_ptr<std::vector<Insta
     hb.sah_splits += t.sah_splits;
     hb.median_fallbacks += t.fallbacks;
   }
+  if (line_count) hb.line_nodes = (float)(line_sum / line_count);
   return std::string();
 }
 
@@ -605,6 +637,7 @@ std::string build_host(const std::vector<std::unique_ptr<std::vector<GeometrySou
     const auto links = threaded_links(pd.tree.nodes);
     for (size_t i = 0; i < pd.tree.nodes.size(); i++)
       hb.tri_bvh_forest.push_back(to_device_node(pd.tree.nodes[i], links[i], bvh_start, pd.primitive_start));
+    hb.geom_line_nodes.push_back(line_nodes(pd.tree));
     std::vector<uint32_t> code2;
     hb.geom_root_code.push_back(emit_wide(pd.tree, pd.primitive_start, hb, code2));
     uint32_t d4 = 0;
@@ -696,6 +729,7 @@ std::string build_with_device_blas(const std::vector<std::unique_ptr<std::vector
   }
   hb.geom_root_code = o.root_code;
   hb.geom_root_code4 = o.root_code4;
+  hb.geom_line_nodes = o.line_nodes;
   hb.max_blas_depth = o.max_depth;
   hb.max_wide4_depth = o.max_wide4_depth;
   hb.sah_splits = o.sah_splits;

@@ -22,6 +22,7 @@ struct DeviceBlasOut {
   std::vector<uint32_t> tree_nodes;  // per geometry: nodes of its tree
   std::vector<uint32_t> root_code;   // per geometry: two-child code of the root
   std::vector<uint32_t> root_code4;  // per geometry: four-child code of the root
+  std::vector<float> line_nodes;     // per geometry: HostBuilt::geom_line_nodes
   uint64_t triangles = 0, nodes = 0, vertices = 0, sah_splits = 0, median_fallbacks = 0;
   uint32_t max_depth = 0, max_wide4_depth = 0;
   uint64_t bytes = 0;                // device bytes of the arrays written into DeviceBuilt

@@ -517,13 +517,20 @@ cudaError_t launch_refill_quads(const TraceParams& p, const PtEnv& e, int sm_cou
   return cudaGetLastError();
 }
 
+// Instanced structures whose rays walk more than this many nodes enter their
+// BLASes together (us, two samples of depth 3, 640x512, schedule 1 / 0: 8
+// instances of 1,000 triangles, 34 nodes, 248 / 245 by themselves and 233 / 217
+// together; 64 of 100, 28 nodes, 157 / 160 and 167 / 161; 512 of 12, 24 nodes,
+// 172 / 173 and 202 / 196).
+constexpr float kTogetherNodes = 32.0f;
+
 template <int MODE, bool LOCAL, bool WT>
 cudaError_t launch_variant_wt(const TraceParams& p, const PtEnv& e, const PtWave* w, int sm_count, cudaStream_t st) {
   const uint32_t block = e.view.block ? e.view.block : 128;
   const uint32_t total = ao_dispatch_count(e.view.width, e.view.height);
   const size_t smem = MODE != MODE_THREADED && !LOCAL ? (size_t)p.stack_depth * block * sizeof(uint2) : 0;
   if (e.schedule == 2u) {
-    if constexpr (LOCAL) {
+    if constexpr (LOCAL && MODE == MODE_WIDE4) {
       if (e.register_tier == 1) return launch_passes<MODE, LOCAL, WT, 1>(p, e, *w, sm_count, block, smem, st);
       if (e.register_tier == 2) return launch_passes<MODE, LOCAL, WT, 2>(p, e, *w, sm_count, block, smem, st);
     }
@@ -538,8 +545,8 @@ cudaError_t launch_variant_wt(const TraceParams& p, const PtEnv& e, const PtWave
   }
   if constexpr (MODE != MODE_THREADED)
     if (p.packed && total <= kQuadPixels) return launch_refill_quads<WT>(p, e, sm_count, st);
-  // register tiers apply to the local-stack walks
-  if constexpr (LOCAL) {
+  // register tiers apply to the local-stack walks of MODE_WIDE4
+  if constexpr (LOCAL && MODE == MODE_WIDE4) {
     if (e.register_tier == 1) return launch_refill<MODE, LOCAL, WT, 1>(p, e, sm_count, block, smem, st);
     if (e.register_tier == 2) return launch_refill<MODE, LOCAL, WT, 2>(p, e, sm_count, block, smem, st);
   }
@@ -580,6 +587,8 @@ cudaError_t launch_pt(const TraceParams& p, const PtEnv& e, const PtWave* w, int
   if (e.view.width == 0 || e.view.height == 0) return cudaSuccess;
   if (mode != MODE_THREADED) {
     const TraceParams q = wide4_params(p);
+    if (q.local_stack && q.instanced && q.line_nodes >= kTogetherNodes)
+      return launch_variant<MODE_WIDE4_TOGETHER, true>(q, e, w, sm_count, st);
     return q.local_stack ? launch_variant<MODE_WIDE4, true>(q, e, w, sm_count, st)
                          : launch_variant<MODE_WIDE4, false>(q, e, w, sm_count, st);
   }

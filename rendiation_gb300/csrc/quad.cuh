@@ -258,77 +258,20 @@ __device__ __forceinline__ void quad_walk(const TraceParams& p, const QuadWarp& 
   }
 }
 
-// Where a lane's ray stands in its TLAS walk.
-struct TlasCursor {
-  uint32_t node, ti, ti_end, inst, g, g_end;
-};
-
-// TLAS / instance / geometry steps of traverse_ray up to the next BLAS entry,
-// written to the slot; false when the query has none left.
+// The ray's next BLAS entry, written to the slot; false when the query has none left.
 template <bool WT>
 __device__ __forceinline__ bool quad_enter(const TraceParams& p, const RayCtx& R, TlasCursor& c, QuadSlot& s,
                                            uint32_t& gslot) {
-  for (;;) {
-    while (c.g < c.g_end) {
-      const uint32_t g = c.g++;
-      const InstanceRay ir = to_instance(p.tlas_data + c.inst, R.o, R.d, R.ray_flags);
-      const uint4 gm = __ldg(reinterpret_cast<const uint4*>(p.tri_root + g));
-      bool pass, is_opaque, cull_enable, cull_back;
-      geometry_cull(ir.flags, gm.w, pass, is_opaque, cull_enable, cull_back);
-      if (!pass) continue;
-      const float4* nd = reinterpret_cast<const float4*>(p.tri_forest + gm.x);
-      const float4 a = __ldg(nd), b = __ldg(nd + 1);
-      float tn;
-      if (!slab<WT>(ir.o, ir.inv_d, R.tmin * ir.scaling, R.far_world * ir.scaling, a.x, a.y, a.z, b.x, b.y, b.z, tn))
-        continue;
-      s.a = make_float4(ir.o.x, ir.o.y, ir.o.z, R.tmin);
-      s.b = make_float4(ir.d.x, ir.d.y, ir.d.z, ir.scaling);
-      s.c = make_uint4(wide4_root(p, g), __float_as_uint(R.far_world),
-                       (is_opaque ? QB_OPAQUE : 0u) | (cull_enable ? QB_CULL : 0u) | (cull_back ? QB_CULL_BACK : 0u) |
-                           ((ir.flags & TF_END_SEARCH) ? QB_END : 0u) | ((gm.z & 1u) ? QB_ODD_START : 0u),
-                       0u);
-      gslot = g;
-      return true;
-    }
-    bool entered = false;
-    while (c.ti < c.ti_end) {
-      const uint32_t cur = c.ti++;
-      const float4* tb = reinterpret_cast<const float4*>(p.tlas_bounding + cur);
-      const float4 ba = __ldg(tb), bb = __ldg(tb + 1);
-      float tn;
-      if (!slab<WT>(R.o, R.inv_d, R.tmin, R.tmax, ba.x, ba.y, ba.z, bb.x, bb.y, bb.z, tn)) continue;
-      if ((R.cull_mask & __float_as_uint(ba.w)) == 0) continue;
-      const DeviceInstance* inst = p.tlas_data + cur;
-      if (merge_instance_flags(R.ray_flags, __ldg(&inst->flags)) & TF_SKIP_TRIANGLES) continue;
-      const uint32_t blas = __ldg(&inst->acceleration_structure_handle);
-      const uint2 range = __ldg(reinterpret_cast<const uint2*>(p.blas_meta + blas));
-      c.g = range.x;
-      c.g_end = range.y;
-      c.inst = cur;
-      entered = true;
-      break;
-    }
-    if (entered) continue;
-    bool found = false;
-    while (c.node != INVALID_NEXT) {
-      const float4* nd = reinterpret_cast<const float4*>(p.tlas_forest + c.node);
-      const float4 a = __ldg(nd), b = __ldg(nd + 1);
-      const uint32_t hit_next = __float_as_uint(a.w), miss_next = __float_as_uint(b.w);
-      float tn;
-      if (!slab<WT>(R.o, R.inv_d, R.tmin * 1.0f, R.far_world * 1.0f, a.x, a.y, a.z, b.x, b.y, b.z, tn)) {
-        c.node = miss_next;
-        continue;
-      }
-      c.node = hit_next;
-      if (hit_next != miss_next) continue;
-      const uint2 cr = __ldg(reinterpret_cast<const uint2*>(nd + 2));
-      c.ti = cr.x;
-      c.ti_end = cr.y;
-      found = true;
-      break;
-    }
-    if (!found) return false;
-  }
+  BlasEntry e;
+  if (!next_blas<WT>(p, R, c, e)) return false;
+  s.a = make_float4(e.ir.o.x, e.ir.o.y, e.ir.o.z, R.tmin);
+  s.b = make_float4(e.ir.d.x, e.ir.d.y, e.ir.d.z, e.ir.scaling);
+  s.c = make_uint4(wide4_root(p, e.gslot), __float_as_uint(R.far_world),
+                   (e.is_opaque ? QB_OPAQUE : 0u) | (e.cull_enable ? QB_CULL : 0u) | (e.cull_back ? QB_CULL_BACK : 0u) |
+                       ((e.ir.flags & TF_END_SEARCH) ? QB_END : 0u) | ((e.gm.z & 1u) ? QB_ODD_START : 0u),
+                   0u);
+  gslot = e.gslot;
+  return true;
 }
 
 // Full query of the warp's rays (traverse_cpu.rs:52-245): traverse_ray's
@@ -340,17 +283,7 @@ __device__ __forceinline__ void traverse_warp(const TraceParams& p, RayCtx& R, u
   R.best.have = false;
   bad = false;
   TlasCursor c{INVALID_NEXT, 0u, 0u, 0u, 0u, 0u};
-  if (valid) {
-    R.inv_d = make_float3(1.0f / R.d.x, 1.0f / R.d.y, 1.0f / R.d.z);
-    R.far_world = R.tmax;
-    if (tidx >= p.n_binding) {
-      bad = true;
-    } else {
-      const uint32_t handle = __ldg(p.tlas_binding + tidx);
-      if (handle >= p.n_tlas_root) bad = true;
-      else c.node = __ldg(p.tlas_bvh_root + handle);
-    }
-  }
+  if (valid) c = start_query(p, R, tidx, bad);
   bool more = valid && !bad;
   for (;;) {
     uint32_t gslot = 0;

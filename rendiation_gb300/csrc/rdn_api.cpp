@@ -228,6 +228,8 @@ rdn_status do_build(rdn_ctx* c) {
     }
     d.max_blas_depth = hb->max_blas_depth;
     d.max_wide4_depth = hb->max_wide4_depth;
+    d.line_nodes = hb->line_nodes;
+    d.instanced = hb->instanced;
     d.vertex_count = hb->n_vertices;
     d.bytes = bytes;
     c->upload_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t1).count();
@@ -263,6 +265,8 @@ rdn_status fill_params(rdn_ctx* c, const rdn_trace_desc* desc, rdn::TraceParams&
   p.stack_depth = rdn::stack_entries(mode_of(desc->traversal), d.max_blas_depth, d.max_wide4_depth);
   p.stack_depth4 = rdn::stack_entries(rdn::MODE_WIDE4, d.max_blas_depth, d.max_wide4_depth);
   p.packed = d.indices_redirect.count < rdn::kPackedTriangles;
+  p.instanced = d.instanced ? 1u : 0u;
+  p.line_nodes = d.line_nodes;
   p.n_binding = (uint32_t)d.tlas_binding.count;
   p.n_tlas_root = (uint32_t)d.tlas_bvh_root.count;
   p.tlas_binding = d.tlas_binding.ptr;

@@ -170,6 +170,13 @@ struct HostBuilt {
   std::vector<uint32_t> geom_root_code4;  // per tri_bvh_root entry
   uint32_t max_blas_depth = 0;
   uint32_t max_wide4_depth = 0;
+  // inner nodes of each geometry's binary tree that a random line through its
+  // root box meets: the sum of their areas over the root's
+  std::vector<float> geom_line_nodes;  // per tri_bvh_root entry
+  // the same of a whole TLAS, the trees below it included, as the mean over
+  // the TLASes; and whether any TLAS holds more than one instance
+  float line_nodes = 0.0f;
+  bool instanced = false;
   uint64_t sah_splits = 0, median_fallbacks = 0;
   // sizes of the reference-layout arrays (kept when they live on the device only)
   uint64_t n_triangles = 0, n_nodes = 0, n_indices = 0, n_vertices = 0;
@@ -200,6 +207,8 @@ struct DeviceBuilt {
   DevBuf<uint32_t> geom_root_code4;
   uint32_t max_blas_depth = 0;
   uint32_t max_wide4_depth = 0;
+  float line_nodes = 0.0f;  // as in HostBuilt
+  bool instanced = false;
   uint64_t vertex_count = 0;
   uint64_t bytes = 0;
 };

@@ -51,6 +51,8 @@ struct TraceParams {
   uint32_t watertight;
   const float4* verts;  // 3 per triangle (VertexRecord), sorted order
   uint32_t packed;      // 1: the four-child tree holds packed_leaf codes (needed to walk it with quads)
+  uint32_t instanced;   // 1: a TLAS holds more than one instance
+  float line_nodes;     // HostBuilt::line_nodes: how much a ray walks, by which a launch is given its kind of walk
 };
 
 // 1 + 2 gamma_3 (gamma_n = n u / (1 - n u), u = 2^-24) rounded up to f32:
@@ -61,7 +63,9 @@ constexpr float kWatertightBoxFarScale = 1.000000476837158203125f;
 constexpr uint32_t kLocalStackEntries = 64;
 
 // Traversal modes (template argument of every traversal kernel).
-enum TraversalMode : int { MODE_THREADED = 0, MODE_BINARY = 1, MODE_WIDE4 = 2 };
+// MODE_WIDE4_TOGETHER is the walk of MODE_WIDE4 with the lanes of a warp
+// entering their BLASes together (traverse_together).
+enum TraversalMode : int { MODE_THREADED = 0, MODE_BINARY = 1, MODE_WIDE4 = 2, MODE_WIDE4_TOGETHER = 3 };
 
 // Parameters of an ordered walk on the four-child tree, whichever node width
 // was asked for (the results are the same and the four-child walk is the

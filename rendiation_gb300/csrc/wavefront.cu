@@ -535,14 +535,25 @@ cudaError_t launch_wavefront(const TraceParams& params, const WavefrontParams& w
   const TraceParams p = wide4_params(params);
   // dynamic fetch (w.refill) has its own secondary kernel, with stacks in shared memory
   const bool dynamic = w.refill != 0u && !(w.local_stack && p.local_stack);
-  if (p.packed && n <= kQuadPixels && !dynamic)
-    return p.watertight ? launch_wavefront_quads<true>(p, w, sm_count, phases, stream)
-                        : launch_wavefront_quads<false>(p, w, sm_count, phases, stream);
-  if (!p.local_stack || dynamic) RDN_WF(MODE_WIDE4, false, 0);
-  // register tiers apply to the local-stack kernels
-  if (w.register_tier == 1) RDN_WF(MODE_WIDE4, true, 1);
-  if (w.register_tier == 2) RDN_WF(MODE_WIDE4, true, 2);
-  RDN_WF(MODE_WIDE4, true, 0);
+  // The phases (1 primaries, 2 secondary rays) that go by quads: both of a small frame, the secondary rays of an
+  // instanced structure always. One per lane the lanes part at the first of a ray's BLASes (us, secondary rays of
+  // 640x480 and 1920x1080 pixels, lanes / quads: 512 instances of 300 triangles 900, 1130 / 178, 303; 64 of 5,000
+  // 1040, 1620 / 271, 638; 216 of 6 x 100 2260, 2640 / 416, 925; the primaries are alike: 300, 500 / 525, 1450).
+  uint32_t by_quads = 0u;
+  if (p.packed && !dynamic) by_quads = n <= kQuadPixels ? 3u : (p.instanced ? 2u : 0u);
+  const auto run = [&](uint32_t phases) -> cudaError_t {
+    if (phases & by_quads)
+      return p.watertight ? launch_wavefront_quads<true>(p, w, sm_count, phases, stream)
+                          : launch_wavefront_quads<false>(p, w, sm_count, phases, stream);
+    if (!p.local_stack || dynamic) RDN_WF(MODE_WIDE4, false, 0);
+    // register tiers apply to the local-stack kernels
+    if (w.register_tier == 1) RDN_WF(MODE_WIDE4, true, 1);
+    if (w.register_tier == 2) RDN_WF(MODE_WIDE4, true, 2);
+    RDN_WF(MODE_WIDE4, true, 0);
+  };
+  if (phases != 3u || by_quads == 0u || by_quads == 3u) return run(phases);
+  const cudaError_t e = run(1u);
+  return e == cudaSuccess ? run(2u) : e;
 #undef RDN_WF
 }
 
