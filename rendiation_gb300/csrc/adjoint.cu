@@ -612,7 +612,9 @@ cudaError_t launch_attr_paths_mode(const TraceParams& p, const PathAdjointParams
 // 175,157 578 / 558, 301 / 297; 1,031,276 of three 2280 / 1945; 2,677,724 5355
 // / 4400). 64 registers without a bound on the blocks; with 5, 6, 7 and 8
 // blocks of 128 the last took 5170, 4790, 5208 and 5105.
-constexpr uint32_t kQuadPaths = 150000;
+// Fields of less than 1024^2 and small soups: up to quad_limit.
+constexpr uint32_t kQuadPathsLeast = 20000, kQuadPaths = 150000;
+constexpr float kQuadPathRays = 120.0f;
 
 template <int PASS, int MODE, bool LOCAL, bool WT, bool SPLIT>
 cudaError_t launch_ray_lanes(const TraceParams& p, const AdjointParams& a, uint32_t block, cudaStream_t stream) {
@@ -631,7 +633,8 @@ cudaError_t launch_ray_pass_wt(const TraceParams& p, const AdjointParams& a, int
   if (mode == MODE_THREADED) return launch_ray_lanes<PASS, MODE_THREADED, false, WT, false>(p, a, block, stream);
   const TraceParams q = wide4_params(p);
   if (!p.packed) return launch_ray_lanes<PASS, MODE_WIDE4, false, WT, false>(q, a, block, stream);
-  const QuadShareLaunch L = quad_share(a.count, q.local_stack != 0);
+  const QuadShareLaunch L = quad_share(q, a.count);
+  if (L.grid == 0u) return launch_ray_lanes<PASS, MODE_WIDE4, true, WT, false>(q, a, block, stream);
   static std::atomic<uint64_t> done{0};
   const auto fn = ray_pass_quad_kernel<PASS, WT>;
   const cudaError_t e = raise_smem_limit(done, {(const void*)fn});
@@ -665,7 +668,7 @@ cudaError_t launch_attr_paths(const TraceParams& p, const PathAdjointParams& a, 
   const TraceParams q = wide4_params(p);
   // instanced structures: quads at every size (64 instances of 20,000 triangles, 700,000 paths of two segments: 11300 us
   // one per lane, whose lanes part at the first of a ray's BLASes, 3430 with quads; 512 of 100: 3290, 1340)
-  if (p.packed && (a.count <= kQuadPaths || !q.local_stack || q.instanced))
+  if (p.packed && (a.count <= quad_limit(p, kQuadPathRays, kQuadPathsLeast, kQuadPaths) || !q.local_stack || q.instanced))
     return launch_attr_paths_mode<MODE_WIDE4, true, false>(p, a, adjoint, block, sm_count, stream);
   return q.local_stack ? launch_attr_paths_mode<MODE_WIDE4, false, true>(q, a, adjoint, block, sm_count, stream)
                        : launch_attr_paths_mode<MODE_WIDE4, false, false>(q, a, adjoint, block, sm_count, stream);

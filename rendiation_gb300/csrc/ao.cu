@@ -61,8 +61,11 @@ __global__ void __launch_bounds__(128) ao_kernel(TraceParams P, AoEnv A) {
 // (us for four samples on the 1024^2 field: 128^2 pixels, one per thread 582,
 // 8 a warp 303; 256^2 662, 8 487, 16 520; means of four cameras: 400x300 841,
 // 760; 400^2 930, 890; 512^2 1030, 1180; 800x500 1370, 1710). Above it pixels that are alike share their
-// nodes better one per lane.
-constexpr uint32_t kQuadPixels = 200000;
+// nodes better one per lane. Smaller trees: up to quad_limit (160,000 pixels of
+// the fields of 16^2, 64^2, 128^2, of two-child lanes: quads 2.08, 1.34, 0.91,
+// lanes 0.90, 0.78, 0.67; soups of 100, 1000: 1.28, 1.02 and 0.90, 0.76).
+constexpr uint32_t kQuadLeast = 40000, kQuadPixels = 200000;
+constexpr float kQuadRays = 180.0f;
 constexpr uint32_t ao_quad_batch(uint32_t pixels) { return pixels < 100000u ? 8u : 16u; }
 
 template <bool WT>
@@ -143,7 +146,7 @@ cudaError_t launch_ao_advance(uint32_t* counter, cudaStream_t st) {
 cudaError_t launch_ao(const TraceParams& p, const AoEnv& a, int mode, cudaStream_t st) {
   if (a.width == 0 || a.height == 0) return cudaSuccess;
   const uint32_t pixels = ao_dispatch_count(a.width, a.height);
-  if (mode != MODE_THREADED && p.packed && pixels <= kQuadPixels)
+  if (mode != MODE_THREADED && p.packed && pixels <= quad_limit(p, kQuadRays, kQuadLeast, kQuadPixels))
     return p.watertight ? launch_quads<true>(p, a, pixels, st) : launch_quads<false>(p, a, pixels, st);
   if (mode != MODE_THREADED) {
     const TraceParams q = wide4_params(p);

@@ -273,7 +273,11 @@ __global__ void __launch_bounds__(128, pt_min_blocks(TIER)) pt_refill_kernel(Tra
 // 662; means of four cameras: 400x300 952, 938; 400^2 1020, 1014; 512^2 1155,
 // 1293; 800x500 1360, 1580. 72 registers (7 blocks): 64 and 80 took 1192 and 1169 us against 1153
 // at 682x384.
+// Smaller trees: up to quad_limit (65,536 pixels of the fields of 16^2, 64^2,
+// 128^2, 256^2, of two-child lanes: quads 1.47, 1.16, 0.99, 0.85, lanes 0.93,
+// 0.88, 0.85, 0.83).
 constexpr uint32_t kQuadPixels = 200000;
+constexpr float kQuadRays = 90.0f;
 template <bool WT>
 __global__ void __launch_bounds__(128, 7) pt_refill_quad_kernel(TraceParams P, PtEnv E, uint32_t total, uint32_t batch) {
   extern __shared__ __align__(16) unsigned char quad_smem[];
@@ -544,7 +548,7 @@ cudaError_t launch_variant_wt(const TraceParams& p, const PtEnv& e, const PtWave
     return cudaGetLastError();
   }
   if constexpr (MODE != MODE_THREADED)
-    if (p.packed && total <= kQuadPixels) return launch_refill_quads<WT>(p, e, sm_count, st);
+    if (p.packed && total <= quad_limit(p, kQuadRays, 0u, kQuadPixels)) return launch_refill_quads<WT>(p, e, sm_count, st);
   // register tiers apply to the local-stack walks of MODE_WIDE4
   if constexpr (LOCAL && MODE == MODE_WIDE4) {
     if (e.register_tier == 1) return launch_refill<MODE, LOCAL, WT, 1>(p, e, sm_count, block, smem, st);

@@ -331,8 +331,11 @@ struct QuadHits {
 };
 constexpr uint32_t kShareBlock = 128;
 // From kShareSplit rays on, groups that differ are walked 32 a warp; from
-// kShareLanes on, groups that are alike one ray per lane (trace.cu's sizes).
-constexpr uint32_t kShareSplit = 48000, kShareLanes = 400000;
+// quad_limit on, groups that are alike one ray per lane (the hit query of
+// 262,144 camera rays on a field of 64^2 98 us by quads, 51 by lanes), and all
+// of them where the trees are small.
+constexpr uint32_t kShareSplit = 48000, kShareMost = 400000;
+constexpr float kShareRays = 255.0f;
 __host__ __device__ constexpr uint32_t quad_share_bytes(uint32_t stack_depth) {
   return (uint32_t)sizeof(QuadHits) + 4u * quad_warp_bytes(stack_depth);
 }
@@ -391,17 +394,19 @@ __device__ __forceinline__ bool quad_share_query(const TraceParams& p, const Qua
 
 }  // namespace dev
 
-// The share of a batch of `count` rays, and whether the groups that are alike
-// are left to a kernel with a ray per lane.
+// The share of a batch of `count` rays (no blocks: none of it), and whether the
+// groups that are alike, or all, are left to a kernel with a ray per lane.
 struct QuadShareLaunch {
   dev::QuadShare share;
   uint32_t grid;
   bool lanes;
 };
-inline QuadShareLaunch quad_share(uint32_t count, bool lanes_ok) {
+inline QuadShareLaunch quad_share(const TraceParams& p, uint32_t count) {
   const uint32_t differing = (uint32_t)(((uint64_t)count + 127) / 128), alike = (uint32_t)(((uint64_t)count + 31) / 32);
   if (count < dev::kShareSplit) return {{0u, false}, alike, false};
-  if (count < dev::kShareLanes || !lanes_ok) return {{differing, true}, differing + alike, false};
+  if (!p.local_stack || count < quad_limit(p, dev::kShareRays, dev::kShareSplit, dev::kShareMost))
+    return {{differing, true}, differing + alike, false};
+  if (small_trees(p)) return {{0u, false}, 0u, true};
   return {{differing, true}, differing, true};
 }
 

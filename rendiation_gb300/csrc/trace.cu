@@ -141,14 +141,17 @@ namespace {
 //                       16 79, 32 119; 1,000 random rays: 84 -> 47
 //   below kQuadBatch32  quads; rays that differ 16 a warp (48,000 random rays:
 //                       8 a warp 100, 16 88, 32 120), alike ones still 8
-//   below kLaneSplit    the same with 32 (131,072 random: 193 / 159 / 150;
+//   below quad_limit    the same with 32 (131,072 random: 193 / 159 / 150;
 //                       camera rays: 160,000 8 a warp 127 / 70, lanes 173 / 87;
 //                       327,680 215 / 101, lanes 237 / 98)
 //   from there on       alike rays one per lane (400,000: quads 259 / 102,
 //                       lanes 273 / 99; 786,432: 431 / 187, 323 / 112), the
 //                       rest quads (777,777 through a 150k soup: lanes 917,
 //                       quads 835; watertight 1200, 943)
-constexpr uint32_t kQuadSplit = 40000, kQuadBatch32 = 100000, kLaneSplit = 400000;
+// quad_limit is 400,000 for these; 262,144 camera rays on fields of 16^2, 64^2
+// and 128^2: quads 73, 90, 107 us, lanes 28, 43, 60, two-child lanes 32, 56, 88.
+constexpr uint32_t kQuadSplit = 40000, kQuadBatch32 = 100000, kQuadMost = 400000;
+constexpr float kQuadRays = 300.0f;
 
 template <int MODE, bool COUNT, bool LOCAL, bool WT, bool SPLIT>
 cudaError_t launch_lanes_wt(const TraceParams& p, uint32_t block, cudaStream_t stream) {
@@ -195,8 +198,10 @@ cudaError_t launch_trace(const TraceParams& p, int mode, bool counted, uint32_t 
   if (!p.packed) return local ? launch_lanes<MODE_WIDE4, false, true>(q, block, stream)
                              : launch_lanes<MODE_WIDE4, false, false>(q, block, stream);
   if (p.count < kQuadSplit) return launch_quads(q, 8, 0, stream);
-  if (p.count < kLaneSplit || !local) return launch_quads(q, p.count < kQuadBatch32 ? 16 : 32, 2, stream);
-  const cudaError_t e = launch_quads(q, 32, 1, stream);
+  const uint32_t batch = p.count < kQuadBatch32 ? 16 : 32;
+  if (!local || p.count < quad_limit(p, kQuadRays, kQuadSplit, kQuadMost)) return launch_quads(q, batch, 2, stream);
+  if (small_trees(p)) return launch_lanes<MODE_WIDE4, false, true>(q, block, stream);
+  const cudaError_t e = launch_quads(q, batch, 1, stream);
   return e == cudaSuccess ? launch_lanes<MODE_WIDE4, false, true, true>(q, block, stream) : e;
 }
 

@@ -78,6 +78,28 @@ inline TraceParams wide4_params(const TraceParams& p) {
   return q;
 }
 
+// Rays (pixels, paths) of a batch up to which four lanes per ray are its faster
+// walk: `per_square` times the square of the nodes that a line meets, between
+// `least` and `most`. Four lanes per ray finish a batch sooner that is bound by
+// its longest walks, and cost more where the chip is full; the longest walk
+// grows faster with the tree than the mean. Where the two met (camera queries):
+//   field of 16^2, 64^2, 128^2, 256^2, 512^2, 1024^2   10.7, 19.6, 24.2, 28.8, 33.4, 37.9 nodes
+//                                      40k, 65k, 95k, 150k, 240k, 400k rays
+//   soup of 12, 100, 1000, 10000       2.9, 7.8, 21, 57 nodes; 10k, 65k, 160k, above 320k rays
+// Neither the depth nor the triangles tell a field from a soup. The factors of
+// the kernels lie between these lines and those where two-child walks, one ray
+// per lane, were as fast.
+inline uint32_t quad_limit(const TraceParams& p, float per_square, uint32_t least, uint32_t most) {
+  const float n = per_square * p.line_nodes * p.line_nodes;
+  return n >= (float)most ? most : (n > (float)least ? (uint32_t)n : least);
+}
+// Trees so small that a batch above quad_limit goes by lanes whole: the second
+// kernel of a split batch costs more than its four lanes per ray gain (us,
+// 1920x1080 camera rays, two-child lanes / split / lanes: soups of 12 triangles
+// 32 / 69 / 32, of 300 58 / 86 / 47; 777,777 random rays 38 / 67 / 36, 175 /
+// 151 / 119). Rays that enter many instances gain more.
+inline bool small_trees(const TraceParams& p) { return p.line_nodes < (p.instanced ? 5.0f : 13.0f); }
+
 // stack entries the mode needs per thread
 uint32_t stack_entries(int mode, uint32_t max_binary_depth, uint32_t max_wide4_depth);
 

@@ -194,11 +194,19 @@ __global__ void __launch_bounds__(128, min_blocks(TIER)) primary_kernel(TracePar
 }
 
 // The same with four lanes per ray (quad.cuh): a warp claims `batch` pixels of
-// a tile. Both kernels of this kind run for frames of up to kQuadPixels, whose
-// slowest warps decide (us a frame, one ray per lane -> quads): 64^2 pixels 236
-// -> 110, 256^2 393 -> 216, 400^2 464 -> 340, 512^2 482 -> 442, but 640x512 499
-// -> 525, 1280x720 899 -> 1246.
-constexpr uint32_t kQuadPixels = 300000;
+// a tile. For frames of up to kQuadPixels, whose slowest warps decide (us a
+// frame on the 1024^2 field, one ray per lane -> quads: 64^2 pixels 236 -> 110,
+// 256^2 393 -> 216, 400^2 464 -> 340, 512^2 482 -> 442, but 640x512 499 -> 525,
+// 1280x720 899 -> 1246), and up to quad_limit where the trees are smaller:
+// 160,000 primaries of the fields of 16^2, 64^2, 128^2, 256^2 take, of the time
+// of two-child lanes, 2.04, 1.64, 1.24 and 0.86 by quads, 0.95, 0.84, 0.74 and
+// 0.66 by lanes; their secondary rays 1.50, 1.17, 1.02, 0.96 and 0.93, 0.89,
+// 0.83, 0.91. Those of soups, most of whose pixels hit nothing, are fewer and
+// take 0.4 to 0.8 by quads, so the secondary rays go by their own number.
+constexpr uint32_t kQuadPixelsLeast = 30000, kQuadPixels = 300000;
+constexpr float kQuadPrimaries = 155.0f;
+constexpr uint32_t kQuadSecondaryLeast = 100000;
+constexpr float kQuadSecondary = 410.0f;
 template <bool WT>
 __global__ void __launch_bounds__(128, 8) primary_quad_kernel(TraceParams p, WavefrontParams w, uint32_t batch) {
   extern __shared__ __align__(16) unsigned char quad_smem[];
@@ -251,6 +259,7 @@ __global__ void __launch_bounds__(128, min_blocks(TIER)) secondary_kernel(TraceP
   const uint32_t n_front = (uint32_t)bins, n = n_front + (uint32_t)(bins >> 32);
   const uint32_t cap = w.width * w.height;
   const uint32_t total = 2u * n;
+  if (w.least_rays && total < w.least_rays) return;
   const uint32_t lane = threadIdx.x & 31u;
   if (blockIdx.x == 0 && threadIdx.x == 0 && w.ray_counts) {
     w.ray_counts[0] = w.width * w.height;
@@ -287,7 +296,7 @@ __global__ void __launch_bounds__(128, min_blocks(TIER)) secondary_kernel(TraceP
 
 // The same with four lanes per ray (quad.cuh), a warp as many entries at a
 // time as the queues give every resident warp.
-template <bool WT>
+template <bool WT, bool LIMIT>
 __global__ void __launch_bounds__(128, 8) secondary_quad_kernel(TraceParams p, WavefrontParams w) {
   extern __shared__ __align__(16) unsigned char quad_smem[];
   const QuadWarp W = quad_warp(quad_smem, p.stack_depth4);
@@ -295,6 +304,7 @@ __global__ void __launch_bounds__(128, 8) secondary_quad_kernel(TraceParams p, W
   const uint32_t n_front = (uint32_t)bins, n = n_front + (uint32_t)(bins >> 32);
   const uint32_t cap = w.width * w.height;
   const uint32_t total = 2u * n;
+  if (LIMIT && total > w.most_rays) return;  // without a limit the first claim does not wait for the count
   // 131,072 rays took 104 us with 8 a warp, 127 with 16 and 152 with 32; 524,288 268, 242 and 230
   const uint32_t batch = total < 200000u ? 8u : (total < 400000u ? 16u : 32u);
   const uint32_t lane = threadIdx.x & 31u;
@@ -462,8 +472,10 @@ cudaError_t launch_wavefront_mode(const TraceParams& p, const WavefrontParams& w
     if (e != cudaSuccess) return e;
   }
   if (!(phases & 2u)) return cudaSuccess;
-  e = cudaMemsetAsync(w.work_counter, 0, 64, stream);
-  if (e != cudaSuccess) return e;
+  if (w.least_rays == 0u) {  // else the quads' launch before this one has zeroed it, and has not used it if this one runs
+    e = cudaMemsetAsync(w.work_counter, 0, 64, stream);
+    if (e != cudaSuccess) return e;
+  }
   // persistent secondary grid: enough resident blocks to fill every SM
   const bool dynamic = MODE != MODE_THREADED && w.refill != 0u && !LOCAL;
   int per_sm = 0;
@@ -488,8 +500,9 @@ cudaError_t launch_wavefront_quads(const TraceParams& p, const WavefrontParams& 
   constexpr uint32_t block = 64;
   const size_t smem = (size_t)quad_warp_bytes(p.stack_depth4) * (block / 32);
   static std::atomic<uint64_t> attr_done{0};
-  cudaError_t e =
-      raise_smem_limit(attr_done, {(const void*)primary_quad_kernel<WT>, (const void*)secondary_quad_kernel<WT>});
+  const auto secondary = w.most_rays ? secondary_quad_kernel<WT, true> : secondary_quad_kernel<WT, false>;
+  cudaError_t e = raise_smem_limit(attr_done, {(const void*)primary_quad_kernel<WT>, (const void*)secondary_quad_kernel<WT, true>,
+                                               (const void*)secondary_quad_kernel<WT, false>});
   if (e != cudaSuccess) return e;
   const uint64_t pixels = (uint64_t)((w.width + 3) / 4) * ((w.height + 7) / 8) * 32;
   // persistent grids: as many resident blocks as fill every SM, or fewer when the rays are
@@ -512,9 +525,9 @@ cudaError_t launch_wavefront_quads(const TraceParams& p, const WavefrontParams& 
   }
   if (!(phases & 2u)) return cudaSuccess;
   e = cudaMemsetAsync(w.work_counter, 0, 64, stream);
-  if (e == cudaSuccess) e = grid((const void*)secondary_quad_kernel<WT>, 2 * pixels, 8u, blocks);
+  if (e == cudaSuccess) e = grid((const void*)secondary, 2 * pixels, 8u, blocks);
   if (e != cudaSuccess) return e;
-  secondary_quad_kernel<WT><<<blocks, block, smem, stream>>>(p, w);
+  secondary<<<blocks, block, smem, stream>>>(p, w);
   return cudaGetLastError();
 }
 }  // namespace
@@ -526,8 +539,10 @@ cudaError_t launch_wavefront(const TraceParams& params, const WavefrontParams& w
   const size_t n = (size_t)w.width * w.height;
   if (n == 0) return cudaSuccess;
 #define RDN_WF(M, L, T)                                                                      \
-  return p.watertight ? launch_wavefront_mode<M, L, T, true>(p, w, block, sm_count, phases, stream) \
-                      : launch_wavefront_mode<M, L, T, false>(p, w, block, sm_count, phases, stream)
+  return p.watertight ? launch_wavefront_mode<M, L, T, true>(p, v, block, sm_count, phases, stream) \
+                      : launch_wavefront_mode<M, L, T, false>(p, v, block, sm_count, phases, stream)
+  WavefrontParams v = w;
+  v.least_rays = v.most_rays = 0u;
   if (mode == MODE_THREADED) {
     const TraceParams& p = params;
     RDN_WF(MODE_THREADED, false, 0);
@@ -535,25 +550,36 @@ cudaError_t launch_wavefront(const TraceParams& params, const WavefrontParams& w
   const TraceParams p = wide4_params(params);
   // dynamic fetch (w.refill) has its own secondary kernel, with stacks in shared memory
   const bool dynamic = w.refill != 0u && !(w.local_stack && p.local_stack);
-  // The phases (1 primaries, 2 secondary rays) that go by quads: both of a small frame, the secondary rays of an
-  // instanced structure always. One per lane the lanes part at the first of a ray's BLASes (us, secondary rays of
-  // 640x480 and 1920x1080 pixels, lanes / quads: 512 instances of 300 triangles 900, 1130 / 178, 303; 64 of 5,000
-  // 1040, 1620 / 271, 638; 216 of 6 x 100 2260, 2640 / 416, 925; the primaries are alike: 300, 500 / 525, 1450).
-  uint32_t by_quads = 0u;
-  if (p.packed && !dynamic) by_quads = n <= kQuadPixels ? 3u : (p.instanced ? 2u : 0u);
-  const auto run = [&](uint32_t phases) -> cudaError_t {
-    if (phases & by_quads)
-      return p.watertight ? launch_wavefront_quads<true>(p, w, sm_count, phases, stream)
-                          : launch_wavefront_quads<false>(p, w, sm_count, phases, stream);
+  // Primaries by quads in small frames.
+  const bool quads_ok = p.packed && !dynamic;
+  const bool quads1 = quads_ok && n <= quad_limit(p, kQuadPrimaries, kQuadPixelsLeast, kQuadPixels);
+  // Secondary rays by quads up to a number of rays that only the device knows: where the pixels leave it open both
+  // kernels are launched, and one of them returns at once. Those of an instanced structure always, since one per lane
+  // the lanes part at the first of a ray's BLASes (us, secondary rays of 640x480 and 1920x1080 pixels, lanes / quads: 512
+  // instances of 300 triangles 900, 1130 / 178, 303; 64 of 5,000 1040, 1620 / 271, 638; 216 of 6 x 100 2260, 2640 /
+  // 416, 925; the primaries are alike: 300, 500 / 525, 1450).
+  const uint32_t limit2 = quad_limit(p, kQuadSecondary, kQuadSecondaryLeast, 2u * kQuadPixels);
+  const bool quads2 = quads_ok && (p.instanced || n <= kQuadPixels);
+  const bool open2 = quads2 && !p.instanced && 2 * n > limit2;
+  const auto quads = [&](uint32_t phases) {
+    return p.watertight ? launch_wavefront_quads<true>(p, v, sm_count, phases, stream)
+                        : launch_wavefront_quads<false>(p, v, sm_count, phases, stream);
+  };
+  const auto lanes = [&](uint32_t phases) -> cudaError_t {
     if (!p.local_stack || dynamic) RDN_WF(MODE_WIDE4, false, 0);
     // register tiers apply to the local-stack kernels
     if (w.register_tier == 1) RDN_WF(MODE_WIDE4, true, 1);
     if (w.register_tier == 2) RDN_WF(MODE_WIDE4, true, 2);
     RDN_WF(MODE_WIDE4, true, 0);
   };
-  if (phases != 3u || by_quads == 0u || by_quads == 3u) return run(phases);
-  const cudaError_t e = run(1u);
-  return e == cudaSuccess ? run(2u) : e;
+  cudaError_t e = cudaSuccess;
+  if (phases & 1u) e = quads1 ? quads(1u) : lanes(1u);
+  if (e != cudaSuccess || !(phases & 2u)) return e;
+  if (open2) v.most_rays = limit2;
+  if (quads2) e = quads(2u);
+  if (e != cudaSuccess || (quads2 && !open2)) return e;
+  if (open2) v.least_rays = limit2 + 1u;
+  return lanes(2u);
 #undef RDN_WF
 }
 

@@ -47,6 +47,10 @@ struct WavefrontParams {
   uint32_t local_stack;
   // register budget of the local-stack kernels: 0 default (64), 1 = 72, 2 = 56
   uint32_t register_tier;
+  // set by launch_wavefront where both kinds of secondary kernel are launched:
+  // the lanes' runs from least_rays secondary rays on, the quads' up to
+  // most_rays (0: always; the count is known on the device only)
+  uint32_t least_rays, most_rays;
   // the launch covers rows [row0, row0 + height) of a frame of frame_height rows
   uint32_t row0, frame_height;
 };
