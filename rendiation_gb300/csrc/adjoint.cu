@@ -5,7 +5,7 @@
 // traverse.cuh), value = (1-u-v)*a[i0] + u*a[i1] + v*a[i2] with the hit
 // triangle's vertex attributes, loss = (value - target)^2; a miss contributes
 // nothing. The per-ray value and loss are written; the loss sum is accumulated
-// per warp and added once per warp.
+// and added once per warp or block.
 //
 // Adjoint (ATTR_ADJOINT): the hit is recomputed by tracing the ray again
 // instead of being stored by the forward pass. With r = 2 (value - target) * g
@@ -504,12 +504,25 @@ __device__ __forceinline__ float ray_pass(const TraceParams& p, const AdjointPar
   return 0.0f;
 }
 
-// The warp's losses to the sum: in double, one addition per warp.
+// The losses of the warp, or with BLOCK of the whole block (of up to 128
+// threads, every one of which calls), to the sum: in double, one addition each,
+// none for misses alone. Additions to one address take about a nanosecond each:
+// 2.07 M camera rays onto 12 triangles took 115 us with one a warp, 41 with one
+// a block that hits. Long walks hide them, and a block's barrier costs more
+// (2.07 M rays onto a field of 64^2: 298 us a warp, 305 a block).
+template <bool BLOCK>
 __device__ __forceinline__ void add_loss(const AdjointParams& a, float loss) {
   if (!a.loss_sum) return;
   double s = loss;
   for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-  if ((threadIdx.x & 31) == 0) atomicAdd(a.loss_sum, s);
+  if (BLOCK) {
+    __shared__ double warp_sums[4];
+    if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (uint32_t w = 1; w < blockDim.x >> 5; w++) s += warp_sums[w];
+  }
+  if ((threadIdx.x & (BLOCK ? 127 : 31)) == 0 && s != 0.0) atomicAdd(a.loss_sum, s);
 }
 
 // A ray per lane, in MODE's order. SPLIT: only the warps whose rays are alike.
@@ -536,7 +549,7 @@ __global__ void __launch_bounds__(128) ray_pass_kernel(TraceParams p, AdjointPar
     loss = ray_pass<PASS>(p, a, i, R);
   }
   __syncwarp();
-  if (PASS == ATTR_FORWARD) add_loss(a, loss);
+  if (PASS == ATTR_FORWARD) add_loss<!SPLIT>(a, loss);
 }
 
 // Four lanes per ray (quad.cuh): the ordered walks. 262,144 rays on the 256^2
@@ -552,7 +565,7 @@ __global__ void __launch_bounds__(kShareBlock, kQuadBlocks) ray_pass_quad_kernel
   if (!quad_share_query<WT>(p, S, a.rays, a.count, a.tlas_uniform, dyn_smem, i, valid, R)) return;
   const float loss = valid ? ray_pass<PASS>(p, a, i, R) : 0.0f;
   __syncwarp();
-  if (PASS == ATTR_FORWARD) add_loss(a, loss);
+  if (PASS == ATTR_FORWARD) add_loss<false>(a, loss);
 }
 
 __global__ void __launch_bounds__(256) hit_diff_recorded_adjoint_kernel(TraceParams p, AdjointParams a) {
