@@ -143,6 +143,97 @@ __global__ void __launch_bounds__(128) path_kernel(TraceParams p, PathParams q, 
   if (blockIdx.x == 0 && threadIdx.x == 0 && q.segment_counts) q.segment_counts[bounce] = n;
 }
 
+// Bounce 0 of large calls: a group of 32 primaries that are alike walks faster a
+// ray per lane. A look at 128 groups, path_vote_kernel, says whether most are;
+// if so path_alike_kernel goes through all, takes those that are and lists the
+// others for the quads, else the quads take all. (Both kernels over all groups,
+// each with its own vote, cost the calls without alike rays 5 % of bounce 0.)
+// 2.07 M camera rays onto the 1024^2 field, no bounce: two-child lanes 787 us, all
+// by quads 944, here 615; onto that of 64^2, up to two bounces: 1152, 1356, 1061.
+// As many random rays: 592 and 717 by quads, 602 and 725 here.
+enum { SPLIT_MOST_ALIKE = 0, SPLIT_LISTED = 1, SPLIT_CLAIMED = 2 };  // words of PathParams::split
+
+__device__ __forceinline__ void path_ray(const PathRay& e, RayCtx& R) {
+  R.o = make_float3(e.r0.x, e.r0.y, e.r0.z);
+  R.tmin = e.r0.w;
+  R.d = make_float3(e.r1.x, e.r1.y, e.r1.z);
+  R.tmax = e.r1.w;
+  R.cull_mask = 0xFFu;
+  R.ray_flags = 0u;
+}
+
+constexpr uint32_t kVoteThreads = 1024, kVotes = 4;
+__global__ void __launch_bounds__(kVoteThreads) path_vote_kernel(PathParams q, bool from_user,
+                                                                 const float4* __restrict__ in_rays,
+                                                                 const uint4* __restrict__ in_state) {
+  __shared__ uint32_t alike;
+  if (threadIdx.x == 0) alike = 0u;
+  __syncthreads();
+  constexpr uint32_t samples = kVoteThreads / 32u * kVotes;
+  const uint32_t groups = (uint32_t)(((uint64_t)q.count + 31u) / 32u);
+  PathRay e[kVotes];
+#pragma unroll
+  for (uint32_t k = 0; k < kVotes; k++) {
+    const uint32_t s = (threadIdx.x >> 5) * kVotes + k;
+    const uint32_t j = (uint32_t)((uint64_t)s * groups / samples) * 32u + (threadIdx.x & 31u);
+    e[k] = load_path(q, from_user, in_rays, in_state, j < q.count ? j : q.count - 1u);
+  }
+  uint32_t mine = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < kVotes; k++) {
+    RayCtx R;
+    path_ray(e[k], R);
+    mine += coherent_warp(R, e[k].tlas, true);
+  }
+  if ((threadIdx.x & 31u) == 0) atomicAdd(&alike, mine);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    q.split[SPLIT_MOST_ALIKE] = 2u * alike >= samples;
+    q.split[SPLIT_LISTED] = q.split[SPLIT_CLAIMED] = 0u;
+  }
+}
+
+template <bool WT>
+__global__ void __launch_bounds__(128) path_alike_kernel(TraceParams p, PathParams q, bool from_user,
+                                                         const float4* __restrict__ in_rays,
+                                                         const uint4* __restrict__ in_state,
+                                                         float4* __restrict__ out_rays, uint4* __restrict__ out_state) {
+  uint2 stack[kLocalStackEntries];
+  if (!q.split[SPLIT_MOST_ALIKE]) return;
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t groups = (uint32_t)(((uint64_t)q.count + 31u) / 32u);
+  for (;;) {
+    uint32_t g = 0;
+    if (lane == 0) g = atomicAdd(q.split + SPLIT_CLAIMED, 1u);
+    g = __shfl_sync(0xffffffffu, g, 0);
+    if (g >= groups) break;
+    const uint32_t j = g * 32u + lane;
+    const bool valid = j < q.count;
+    PathRay e{};
+    if (valid) e = load_path(q, from_user, in_rays, in_state, j);
+    RayCtx R;
+    path_ray(e, R);
+    if (!coherent_warp(R, e.tlas, valid)) {
+      if (lane == 0) q.split_list[atomicAdd(q.split + SPLIT_LISTED, 1u)] = g;
+      continue;
+    }
+    bool keep = false;
+    float4 nr0 = make_float4(0.f, 0.f, 0.f, 0.f), nr1 = nr0;
+    uint4 ns = make_uint4(0u, 0u, 0u, 0u);
+    if (valid) {
+      bool bad;
+      traverse_ray<MODE_WIDE4, false, BuiltinAnyHit, WT, 2, WT>(p, R, e.tlas, stack, 1u, bad);
+      keep = shade_path(p, q, 0u, e.id, e.tlas, e.throughput, R.o, R.d, R.best, nr0, nr1, ns);
+    }
+    const uint32_t slot = warp_append(q.queue_count, keep);
+    if (keep) {
+      out_rays[2 * (size_t)slot] = nr0;
+      out_rays[2 * (size_t)slot + 1] = nr1;
+      out_state[slot] = ns;
+    }
+  }
+}
+
 // One bounce with four lanes per ray (quad.cuh): the ordered walks. A warp
 // claims 32 queue entries, or fewer of a queue that would not give every
 // resident warp 32. The entry is read again for the shading, so that the walk
@@ -150,7 +241,8 @@ __global__ void __launch_bounds__(128) path_kernel(TraceParams p, PathParams q, 
 // direction, the case the quads are for: 64 soups (2.4 M triangles, 3.7 M
 // primaries, up to 4 bounces) 10151 us one ray per lane on two-child nodes,
 // 5515 with quads; blocks of 32, 64 or 128 threads within 0.4 %.
-template <bool WT>
+// SPLIT: bounce 0 after path_alike_kernel, the groups that it has listed.
+template <bool WT, bool SPLIT>
 __global__ void __launch_bounds__(128, 8) path_quad_kernel(TraceParams p, PathParams q, uint32_t bounce, bool from_user,
                                                            const float4* __restrict__ in_rays,
                                                            const uint4* __restrict__ in_state,
@@ -159,13 +251,15 @@ __global__ void __launch_bounds__(128, 8) path_quad_kernel(TraceParams p, PathPa
   extern __shared__ __align__(16) unsigned char quad_smem[];
   const uint32_t n = bounce == 0 ? q.count : *(volatile uint32_t*)(q.queue_count + bounce - 1);
   const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t batch = quad_batch(n);
+  const bool listed = SPLIT && q.split[SPLIT_MOST_ALIKE];
+  const uint32_t batch = listed ? 32u : quad_batch(n), end = listed ? 32u * q.split[SPLIT_LISTED] : n;
   uint32_t* work = q.work_counter + bounce;
   for (;;) {
     uint32_t base = 0;
     if (lane == 0) base = atomicAdd(work, batch);
     base = __shfl_sync(0xffffffffu, base, 0);
-    if (base >= n) break;
+    if (base >= end) break;
+    if (listed) base = 32u * q.split_list[base >> 5];
     const uint32_t j = base + lane;
     const bool valid = lane < batch && j < n;
     RayCtx R;
@@ -352,33 +446,48 @@ void paths_bind_scratch(PathParams& q, void* scratch) {
   off += up(n * 16);
   q.state_b = s + off;
   off += up(n * 16);
+  // the words before the queue counts; the list in an array that is free when bounce 0 runs
+  q.split = reinterpret_cast<uint32_t*>(s);
+  q.split_list = static_cast<uint32_t*>(q.rays_a);
   if (q.sort_key) {
     q.keys = reinterpret_cast<uint32_t*>(s + off);
     off += up(n * 4);
     q.idx = reinterpret_cast<uint32_t*>(s + off);
     off += up(n * 4);
     q.sort_scratch = s + off;
+    q.split_list = q.keys;
   }
 }
 
 namespace {
-// kernel variant: 0 a ray per lane, 1 dynamic fetch, 2 four lanes per ray
-enum PathVariant { PATH_LANES = 0, PATH_DYNAMIC = 1, PATH_QUADS = 2 };
+// kernel variant: a ray per lane (stacks in shared or local memory), dynamic
+// fetch, four lanes per ray, and the same with alike primaries a ray per lane
+enum PathVariant { PATH_LANES = 0, PATH_DYNAMIC = 1, PATH_QUADS = 2, PATH_LOCAL_LANES = 3, PATH_SPLIT = 4 };
+// Primaries from which a call is large (see quad_limit). Small trees go by lanes
+// in every bounce then (two bounces on the field of 16^2, us, quads / lanes /
+// two-child lanes: 160,000 camera primaries 133 / 99 / 108, random ones 98 / 117 /
+// 123; 2.07 M 965 / 533 / 614, 535 / 467 / 544; 65,536 85 / 85 / 89, 71 / 87 / 94).
+constexpr uint32_t kSplitLeast = 100000, kSplitMost = 400000;
+constexpr float kSplitRays = 260.0f;
 int path_variant(int mode, const TraceParams& p, const PathParams& q) {
   if (mode == MODE_THREADED) return PATH_LANES;
   if (q.refill != 0) return PATH_DYNAMIC;
-  return p.packed ? PATH_QUADS : PATH_LANES;
+  if (!p.packed) return PATH_LANES;
+  if (!wide4_params(p).local_stack || q.count < quad_limit(p, kSplitRays, kSplitLeast, kSplitMost)) return PATH_QUADS;
+  return small_trees(p) ? PATH_LOCAL_LANES : PATH_SPLIT;
 }
 // shared memory of a block: the variant's stacks
 size_t path_smem(int mode, int variant, const TraceParams& p, uint32_t block) {
-  if (variant == PATH_QUADS) return (size_t)quad_warp_bytes(p.stack_depth4) * (block / 32);
+  if (variant == PATH_QUADS || variant == PATH_SPLIT) return (size_t)quad_warp_bytes(p.stack_depth4) * (block / 32);
+  if (variant == PATH_LOCAL_LANES) return 0;
   return mode == MODE_THREADED ? 0 : (size_t)p.stack_depth4 * block * sizeof(uint2);
 }
 using PathKernel = void (*)(TraceParams, PathParams, uint32_t, bool, const float4*, const uint4*, float4*, uint4*);
 template <bool WT>
 PathKernel path_fn_wt(int mode, int variant) {
   if (mode == MODE_THREADED) return path_kernel<MODE_THREADED, false, WT>;
-  if (variant == PATH_QUADS) return path_quad_kernel<WT>;
+  if (variant == PATH_QUADS || variant == PATH_SPLIT) return path_quad_kernel<WT, false>;
+  if (variant == PATH_LOCAL_LANES) return path_kernel<MODE_WIDE4, true, WT>;
   return variant == PATH_DYNAMIC ? path_dynamic_kernel<MODE_WIDE4, WT> : path_kernel<MODE_WIDE4, false, WT>;
 }
 PathKernel path_fn(int mode, int variant, bool wt) {
@@ -391,9 +500,12 @@ cudaError_t prepare_paths(const TraceParams& p, const PathParams& q, int mode, u
   if (block == 0) block = 64;
   const int variant = path_variant(mode, p, q);
   const size_t smem = path_smem(mode, variant, p, block);
-  static std::atomic<uint64_t> attr_done[2][3][3] = {};
+  static std::atomic<uint64_t> attr_done[2][5][3] = {}, split_done{0};
   const void* fn = (const void*)path_fn(mode, variant, p.watertight != 0);
   cudaError_t e = raise_smem_limit(attr_done[p.watertight ? 1 : 0][variant][mode], {fn});
+  if (e != cudaSuccess) return e;
+  if (variant == PATH_SPLIT)
+    e = raise_smem_limit(split_done, {(const void*)path_quad_kernel<false, true>, (const void*)path_quad_kernel<true, true>});
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, (int)block, smem);
@@ -401,7 +513,7 @@ cudaError_t prepare_paths(const TraceParams& p, const PathParams& q, int mode, u
   if (per_sm < 1) per_sm = 1;
   // persistent grid, never larger than the primary queue needs
   uint32_t g = (uint32_t)(sm_count * per_sm);
-  const uint32_t per = variant == PATH_QUADS ? quad_batch(q.count) * (block / 32) : block;  // rays a block takes at a time
+  const uint32_t per = variant == PATH_QUADS || variant == PATH_SPLIT ? quad_batch(q.count) * (block / 32) : block;  // rays a block takes at a time
   const uint32_t need = (q.count + per - 1) / per;
   *grid = g > need ? need : g;
   return cudaSuccess;
@@ -454,7 +566,19 @@ cudaError_t record_paths(const TraceParams& p, const PathParams& q, int mode, ui
       out_r = (b & 1) ? ra : rb;
       out_s = (b & 1) ? sa : sb;
     }
-    fn<<<grid, block, smem, stream>>>(walk, q, b, from_user, in_r, in_s, out_r, out_s);
+    if (variant == PATH_SPLIT && b == 0) {
+      path_vote_kernel<<<1, kVoteThreads, 0, stream>>>(q, from_user, in_r, in_s);
+      e = cudaGetLastError();
+      if (e != cudaSuccess) return e;
+      const auto alike = p.watertight ? path_alike_kernel<true> : path_alike_kernel<false>;
+      alike<<<grid, block, 0, stream>>>(walk, q, from_user, in_r, in_s, out_r, out_s);
+      e = cudaGetLastError();
+      if (e != cudaSuccess) return e;
+      const PathKernel differing = p.watertight ? path_quad_kernel<true, true> : path_quad_kernel<false, true>;
+      differing<<<grid, block, smem, stream>>>(walk, q, b, from_user, in_r, in_s, out_r, out_s);
+    } else {
+      fn<<<grid, block, smem, stream>>>(walk, q, b, from_user, in_r, in_s, out_r, out_s);
+    }
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }

@@ -18,6 +18,8 @@ struct PathParams {
   // scratch (paths_bind_scratch)
   uint32_t* queue_count;       // max_bounces + 1 counters: entries appended by bounce b
   uint32_t* work_counter;      // max_bounces + 1 counters
+  uint32_t* split;             // bounce 0 of large calls: whether most primaries are alike, groups listed and claimed
+  uint32_t* split_list;        // ... and the groups of 32 left to the quads
   void* rays_a;
   void* rays_b;
   void* state_a;

@@ -173,3 +173,51 @@ def test_rendered_frames(cuda, kind, size):
                 out.append(R.result().copy())
             assert np.count_nonzero((out[0] != out[1]).any(-1)) <= width * height // 20_000
     assert P.check_errors() == (0, 0)
+
+
+@pytest.mark.parametrize("kind,size", SCENES)
+@pytest.mark.parametrize("watertight,sort_key,graph", [(0, 0, True), (rt.INTERSECT_WATERTIGHT, 0, False), (0, 1, False)])
+def test_paths(cuda, kind, size, watertight, sort_key, graph):
+    import torch
+
+    P = system(kind, size)
+    at = limit(P, 260.0, 100_000, 400_000)
+    for n in (at - 2, at + 33):
+        d = torch.from_numpy(rays_of(kind, n, n).view(np.float32).reshape(-1, 8).copy()).cuda()
+        out = []
+        for traversal in (rt.TRAVERSAL_REFERENCE, rt.TRAVERSAL_ORDERED, rt.TRAVERSAL_ORDERED_WIDE):
+            p = rt.Paths(P, d, max_bounces=3, seed=7, traversal=traversal | watertight, sort_key=sort_key)
+            if graph:
+                p.capture()
+                p.launch_graph()
+                p.launch_graph()
+            else:
+                p.run()
+            torch.cuda.synchronize()
+            out.append((p.results().copy(), p.segments()))
+        for got, segments in out[1:]:
+            assert np.count_nonzero(got != out[0][0]) <= n // 20_000
+            assert all(abs(a - b) <= n // 20_000 for a, b in zip(segments, out[0][1]))
+        assert out[0][1][0] == n and out[0][1][1] > 0
+    assert P.check_errors() == (0, 0)
+
+
+def test_paths_of_many_scenes(cuda):
+    """Groups that are alike end where the scene changes; an index that is not bound ends its path."""
+    import torch
+
+    from test_quads_gpu import soup_system
+
+    P = soup_system([scenes.triangle_soup(k, seed=k, offset=0.05) for k in (300, 2000, 6000)])
+    n = limit(P, 260.0, 100_000, 400_000) + 5
+    d = torch.from_numpy(rays_of("soup", n, 3).view(np.float32).reshape(-1, 8).copy()).cuda()
+    rng = np.random.default_rng(3)
+    for tidx in (np.repeat(rng.integers(0, 4, n // 48 + 1), 48)[:n], rng.integers(0, 3, n), np.sort(rng.integers(0, 4, n))):
+        t = torch.from_numpy(tidx.astype(np.int32)).cuda()
+        out = []
+        for traversal in (rt.TRAVERSAL_REFERENCE, rt.TRAVERSAL_ORDERED):
+            p = rt.Paths(P, d, t, max_bounces=2, seed=5, traversal=traversal)
+            p.run()
+            torch.cuda.synchronize()
+            out.append(p.results().copy())
+        assert np.count_nonzero(out[0] != out[1]) <= n // 20_000
