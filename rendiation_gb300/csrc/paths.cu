@@ -146,12 +146,14 @@ __global__ void __launch_bounds__(128) path_kernel(TraceParams p, PathParams q, 
 // Bounce 0 of large calls: a group of 32 primaries that are alike walks faster a
 // ray per lane. A look at 128 groups, path_vote_kernel, says whether most are;
 // if so path_alike_kernel goes through all, takes those that are and lists the
-// others for the quads, else the quads take all. (Both kernels over all groups,
-// each with its own vote, cost the calls without alike rays 5 % of bounce 0.)
+// others for the quads, and leaves the quads' usual launch nothing; else that
+// takes all. (Both kernels over all groups, each with its own vote, cost the
+// calls without alike rays 5 % of bounce 0; the quads' loop with a look at the
+// list 0.6 %.)
 // 2.07 M camera rays onto the 1024^2 field, no bounce: two-child lanes 787 us, all
 // by quads 944, here 615; onto that of 64^2, up to two bounces: 1152, 1356, 1061.
 // As many random rays: 592 and 717 by quads, 602 and 725 here.
-enum { SPLIT_MOST_ALIKE = 0, SPLIT_LISTED = 1, SPLIT_CLAIMED = 2 };  // words of PathParams::split
+enum { SPLIT_MOST_ALIKE = 0, SPLIT_LISTED = 1, SPLIT_CLAIMED = 2, SPLIT_TAKEN = 3 };  // words of PathParams::split
 
 __device__ __forceinline__ void path_ray(const PathRay& e, RayCtx& R) {
   R.o = make_float3(e.r0.x, e.r0.y, e.r0.z);
@@ -188,8 +190,10 @@ __global__ void __launch_bounds__(kVoteThreads) path_vote_kernel(PathParams q, b
   if ((threadIdx.x & 31u) == 0) atomicAdd(&alike, mine);
   __syncthreads();
   if (threadIdx.x == 0) {
-    q.split[SPLIT_MOST_ALIKE] = 2u * alike >= samples;
-    q.split[SPLIT_LISTED] = q.split[SPLIT_CLAIMED] = 0u;
+    const bool most = 2u * alike >= samples;
+    q.split[SPLIT_MOST_ALIKE] = most;
+    q.split[SPLIT_LISTED] = q.split[SPLIT_CLAIMED] = q.split[SPLIT_TAKEN] = 0u;
+    if (most) q.work_counter[0] = q.count;  // all claimed: bounce 0 is path_alike_kernel's and the list's
   }
 }
 
@@ -241,8 +245,8 @@ __global__ void __launch_bounds__(128) path_alike_kernel(TraceParams p, PathPara
 // direction, the case the quads are for: 64 soups (2.4 M triangles, 3.7 M
 // primaries, up to 4 bounces) 10151 us one ray per lane on two-child nodes,
 // 5515 with quads; blocks of 32, 64 or 128 threads within 0.4 %.
-// SPLIT: bounce 0 after path_alike_kernel, the groups that it has listed.
-template <bool WT, bool SPLIT>
+// LISTED: bounce 0 of the groups that path_alike_kernel has listed.
+template <bool WT, bool LISTED>
 __global__ void __launch_bounds__(128, 8) path_quad_kernel(TraceParams p, PathParams q, uint32_t bounce, bool from_user,
                                                            const float4* __restrict__ in_rays,
                                                            const uint4* __restrict__ in_state,
@@ -251,15 +255,15 @@ __global__ void __launch_bounds__(128, 8) path_quad_kernel(TraceParams p, PathPa
   extern __shared__ __align__(16) unsigned char quad_smem[];
   const uint32_t n = bounce == 0 ? q.count : *(volatile uint32_t*)(q.queue_count + bounce - 1);
   const uint32_t lane = threadIdx.x & 31u;
-  const bool listed = SPLIT && q.split[SPLIT_MOST_ALIKE];
-  const uint32_t batch = listed ? 32u : quad_batch(n), end = listed ? 32u * q.split[SPLIT_LISTED] : n;
-  uint32_t* work = q.work_counter + bounce;
+  if (LISTED && !q.split[SPLIT_MOST_ALIKE]) return;
+  const uint32_t batch = LISTED ? 32u : quad_batch(n), end = LISTED ? 32u * q.split[SPLIT_LISTED] : n;
+  uint32_t* work = LISTED ? q.split + SPLIT_TAKEN : q.work_counter + bounce;
   for (;;) {
     uint32_t base = 0;
     if (lane == 0) base = atomicAdd(work, batch);
     base = __shfl_sync(0xffffffffu, base, 0);
     if (base >= end) break;
-    if (listed) base = 32u * q.split_list[base >> 5];
+    if (LISTED) base = 32u * q.split_list[base >> 5];
     const uint32_t j = base + lane;
     const bool valid = lane < batch && j < n;
     RayCtx R;
@@ -574,11 +578,12 @@ cudaError_t record_paths(const TraceParams& p, const PathParams& q, int mode, ui
       alike<<<grid, block, 0, stream>>>(walk, q, from_user, in_r, in_s, out_r, out_s);
       e = cudaGetLastError();
       if (e != cudaSuccess) return e;
-      const PathKernel differing = p.watertight ? path_quad_kernel<true, true> : path_quad_kernel<false, true>;
-      differing<<<grid, block, smem, stream>>>(walk, q, b, from_user, in_r, in_s, out_r, out_s);
-    } else {
-      fn<<<grid, block, smem, stream>>>(walk, q, b, from_user, in_r, in_s, out_r, out_s);
+      const PathKernel listed = p.watertight ? path_quad_kernel<true, true> : path_quad_kernel<false, true>;
+      listed<<<grid, block, smem, stream>>>(walk, q, b, from_user, in_r, in_s, out_r, out_s);
+      e = cudaGetLastError();
+      if (e != cudaSuccess) return e;
     }
+    fn<<<grid, block, smem, stream>>>(walk, q, b, from_user, in_r, in_s, out_r, out_s);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
