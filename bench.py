@@ -278,14 +278,11 @@ def bench_wavefront(args, ws, rank):
         from rendiation_gb300.autotune import Autotuner, grid
 
         tuner = Autotuner(args.tune_cache)
-        # traversal stack in shared memory (local 0) or in local memory (1)
-        orders = [rt.TRAVERSAL_ORDERED, rt.TRAVERSAL_ORDERED_WIDE]
-        # register tier (regs) applies to the local-stack kernels
-        cands = (grid(traversal=orders, block=[32, 64, 128], local=[0])
-                 + grid(traversal=orders, block=[32, 64, 128], local=[1], regs=[0, 1, 2]))
+        # both ordered traversals walk the same nodes, with stacks in local memory but for dynamic fetch
+        orders = [rt.TRAVERSAL_ORDERED_WIDE]
+        cands = grid(traversal=orders, block=[32, 64, 128], local=[1], regs=[0, 1, 2])
         # secondary schedule: batches of 32 rays per warp (refill 0) or dynamic fetch
-        cands2 = (grid(traversal=orders, block=[32, 64, 128], refill=[0], local=[0])
-                  + grid(traversal=orders, block=[32, 64, 128], refill=[0], local=[1], regs=[0, 1, 2])
+        cands2 = (grid(traversal=orders, block=[32, 64, 128], refill=[0], local=[1], regs=[0, 1, 2])
                   + grid(traversal=orders, block=[64], refill=[8, 16], local=[0]))
 
         def run_phase(ph):
@@ -1096,9 +1093,9 @@ def bench_batched(args, ws=1, rank=0):
     if args.tune and args.traversal == "ordered":
         from rendiation_gb300.autotune import Autotuner, grid
 
-        orders = [rt.TRAVERSAL_ORDERED, rt.TRAVERSAL_ORDERED_WIDE]
-        cands = (grid(traversal=orders, block=[64, 128], sort_key=[rt.SORT_NONE], refill=[0], local=[0, 1])
-                 + grid(traversal=orders, block=[64], sort_key=[rt.SORT_SCENE_OCTANT], refill=[0], local=[0, 1])
+        orders = [rt.TRAVERSAL_ORDERED_WIDE]  # as for the frame: one layout, one place for the stacks
+        cands = (grid(traversal=orders, block=[64, 128], sort_key=[rt.SORT_NONE], refill=[0], local=[1])
+                 + grid(traversal=orders, block=[64], sort_key=[rt.SORT_SCENE_OCTANT], refill=[0], local=[1])
                  + grid(traversal=orders, block=[64], sort_key=[rt.SORT_NONE], refill=[8, 16], local=[0]))
 
         def run(c):

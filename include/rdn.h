@@ -153,21 +153,22 @@ typedef struct rdn_hit_ext {
 
 /* Traversal order.
  * RDN_TRAVERSAL_ORDERED (default): nearest-child-first stack traversal over
- *   64 B two-child nodes holding the reference's exact node boxes, with
- *   speculative leaf postponement (a lane that reaches a leaf keeps descending
- *   until its whole warp holds leaves, so triangle tests run together). Closest
- *   hits equal the reference's except among hits at exactly equal distance;
- *   first-hit (shadow) queries agree on hit/miss.
+ *   nodes holding the reference's exact node boxes, with speculative leaf
+ *   postponement (a lane that reaches a leaf keeps descending until its whole
+ *   warp holds leaves, so triangle tests run together). Closest hits equal the
+ *   reference's except among hits at exactly equal distance, of which any may be
+ *   returned (also by the number of rays of the call); first-hit (shadow)
+ *   queries agree on hit/miss.
  * RDN_TRAVERSAL_REFERENCE: the reference's stackless threaded hit/miss walk
  *   (traverse_cpu.rs:291-319) over its own 48 B node layout; bit-identical to
  *   the reference CPU traversal, including ties and which hit ends a search.
- * RDN_TRAVERSAL_ORDERED_WIDE: as ORDERED over 128 B four-child nodes collapsed
- *   from the same tree.
- * The two ordered values give the same results, and rdn_trace, the frames, the
- * paths, the task graph's trace tasks and the differentiable calls walk both on
- * the four-child nodes, one ray per lane or four lanes per ray by their number
- * of rays and by how alike a warp's rays are (rdn_trace_counted and
- * include/rdn_trace.cuh walk the nodes that are asked for). The launch knobs of
+ * RDN_TRAVERSAL_ORDERED_WIDE: as ORDERED.
+ * rdn_trace, the frames, the paths, the task graph's trace tasks and the
+ * differentiable calls walk both ordered values on 128 B four-child nodes
+ * collapsed from the reference's tree, one ray per lane or four lanes per ray by
+ * their number of rays, by how much a ray of the structure walks and by how
+ * alike a warp's rays are. rdn_trace_counted and include/rdn_trace.cuh walk 64 B
+ * two-child nodes for ORDERED, four-child ones for WIDE. The launch knobs of
  * the descriptors (block_size, local_stack, register_tier, speculation) change
  * no result and act where a ray has a lane of its own; stacks that fit 64
  * entries are in local memory there unless dynamic fetch is asked for. */
@@ -222,7 +223,8 @@ typedef struct rdn_trace_desc {
 /* ---- device status ----------------------------------------------------- */
 
 /* Bits of the device error word the kernels set instead of faulting. */
-#define RDN_ERROR_STACK_OVERFLOW 0x1u   /* a traversal stack push past its depth (unreachable by construction) */
+#define RDN_ERROR_STACK_OVERFLOW 0x1u   /* a traversal stack push past its depth (callers' kernels, rdn_trace.cuh; the
+                                           library's own stacks are sized from the tree) */
 #define RDN_ERROR_BAD_TLAS_INDEX 0x2u   /* a ray named a TLAS index that is not bound (the ray misses) */
 #define RDN_ERROR_ITERATION_LIMIT 0x4u  /* a dynamic-fetch warp reached its iteration limit and stopped */
 

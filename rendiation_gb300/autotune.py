@@ -6,12 +6,13 @@ shader/ray-tracing/src/backend/wavefront_compute/mod.rs:134). Here the knobs
 that decide GB300 throughput are chosen per workload by timing every candidate
 on the workload itself:
 
-* node layout of the ordered traversal (2-wide or 4-wide nodes),
-* block size (warps per block: occupancy against shared-memory stack size),
+* block size and register budget of the walks with a ray per lane,
+* leaf-postponement threshold of those walks,
+* dynamic fetch of the secondary rays or batches of 32,
 * ray-sort key of the batched executor (none, scene+octant, scene+octant+cell).
 
-The traversal stack depth is not a knob: a stack walk without restarts needs
-the tree depth, so it is derived from the built tree.
+The node layout, the stack's place and its depth are not knobs: the ordered
+walks use four-child nodes, and their stacks' size follows from the built tree.
 
 Each candidate is warmed up and then timed with CUDA events on the current
 stream; the median decides. Choices are cached in a JSON file (keyed by a

@@ -17,10 +17,10 @@
 // Measured (rdn_trace, us, one ray per lane -> quads): 777,777 random rays
 // through a 150k soup 917 -> 835 (watertight 1200 -> 943), 1,000,000 through
 // the 1024^2 field 407 -> 355, 1,000 rays through a 10k soup 84 -> 47, 65,536
-// camera rays onto it 85 -> 49. Only large batches of rays that are alike walk faster one per
-// lane, where a warp's lanes share the nodes they read (2.07 M camera rays:
-// 597 against 985). 64 registers a thread; before the steps were unrolled the
-// random rays took 885 us with 64, 910 with 72 and 938 with 56.
+// camera rays onto it 85 -> 49. Large batches of rays that are alike walk faster
+// one per lane, where a warp's lanes share the nodes they read (2.07 M camera
+// rays: 597 against 985), and on small trees batches from some 40,000 rays on
+// (quad_limit). 64 registers a thread; 72 and 56 cost the random rays 3 and 6 %.
 //
 // Results: every child box and every triangle is tested with the operations of
 // the per-lane walk, and a leaf's candidates are committed in the leaf's order
@@ -89,8 +89,8 @@ __device__ __forceinline__ QuadWarp quad_warp(unsigned char* smem, uint32_t stac
 // seam is the end of an image's row, or of a batch of the caller's: with every
 // ray held against the first, the rows' ends of a 1000x524 image, one group in
 // 31, went to the quads and made 305 us of camera rays 430. Which walk a ray
-// takes does not change its result; both kernels of a split query form the
-// same vote.
+// takes decides only exact-distance ties and which hit ends a first-hit search;
+// both kernels of a split query form the same vote.
 constexpr float kAlikeCos2 = 0.75f;
 constexpr int kSeams = 2;
 __device__ __forceinline__ bool coherent_warp(const RayCtx& R, uint32_t tidx, bool valid) {

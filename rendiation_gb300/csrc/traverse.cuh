@@ -420,9 +420,10 @@ __device__ __forceinline__ Wide4Load load_wide4_if(const float4* w, bool want) {
 // slab() on packed pairs of planes: the same subtractions and products (a - b
 // as a + (-b)), two to an instruction. The per-lane four-child walk is bound by
 // instruction issue (55-66 % of the slots, 6 to 17 of 32 lanes active), and a
-// box test falls from about 22 to 16 instructions: 2.07 M camera rays on the
-// 1024^2 field 880 -> 727 us (with the child-major node below; 597 with the
-// steps of descend()), the 1080p frame 2107 -> 1950 us (1659).
+// box test falls from about 22 to 16 instructions. With it and the child-major
+// node, 2.07 M camera rays on the 1024^2 field took 727 us instead of 880, the
+// 1080p frame 1950 instead of 2107 (before the steps of descend(): 597 and 1659
+// with those).
 template <bool WT>
 __device__ __forceinline__ bool slab2(float2 neg_o_xy, float2 neg_o_z, float2 inv_xy, float2 inv_z, float tmin,
                                       float tmax, const Wide4Load& c, float& t_near_max) {

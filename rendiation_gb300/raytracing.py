@@ -206,8 +206,9 @@ class AccelerationStructureSystem:
               local_stack=0, anyhit_mask=None):
         """rays: CUDA f32 tensor (N, 8); hits: CUDA f32 tensor (N, 4) (prim id stored as u32 bits);
         hits_ext: optional CUDA int32 tensor (N, 4); tlas_idx: optional CUDA int32 tensor (N,).
-        count overrides N (e.g. 0 for an empty batch). local_stack: traversal stacks in
-        local memory instead of shared memory (ordered walks). anyhit_mask: CUDA int32
+        count overrides N (e.g. 0 for an empty batch). local_stack: no effect on rdn_trace's
+        ordered walks (stacks of up to 64 entries are in local memory where a ray has a lane
+        of its own, those of four lanes per ray in shared memory). anyhit_mask: CUDA int32
         bit array over built triangles (ANYHIT_PRIMITIVE_MASK)."""
         import torch
 
